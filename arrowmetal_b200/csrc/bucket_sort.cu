@@ -1,0 +1,1570 @@
+// Single-key sort by buckets: each row moves once or twice through HBM to its bucket of a few thousand
+// rows, and every bucket is then ordered inside one CTA's shared memory.
+//
+//   1. buckets_kernel: up to 65,536 keys, evenly spread over the column, give the key
+//      distribution. The sampled key range is cut into 512 equal coarse cells, a coarse cell into up to
+//      2^11 equal fine cells by its share of the sample, a fine cell into equal sub-buckets by its
+//      estimated rows (light neighbours share a bucket): a monotone map key -> bucket of two table reads
+//      and one multiply, whose buckets hold about TARGET rows whatever the distribution.
+//   2. bucket_histogram_kernel reads the column once: exact rows of every bucket, and of every level-1
+//      bin of every chunk (a contiguous range of rows). bucket_starts_kernel turns them into starts, and
+//      decides: when a bucket is larger than BIG rows (heavily repeated keys), nothing has moved yet and
+//      the digit passes sort the column instead.
+//   3. level1_kernel, one CTA a chunk, scatters the chunk's rows to their level-1 bins (the bucket
+//      itself up to BINS1 buckets, else 128 buckets a bin), level2_kernel each bin's rows to their
+//      buckets. A row's place among its tile's rows of a bin comes from one shared-memory atomic, in no
+//      particular order: the row id that moves with it orders equal keys at the end. Rows are staged in
+//      shared memory by bin, so a bin's rows leave as one run. The null and NaN rows go straight to
+//      their final places, in row order (ballots, and the chunks' counts).
+//   4. bucket_sort_kernel orders each bucket by (key, row id): a counting step over 2,048 bins that
+//      divide the bucket's key range, then comparisons within the bin (a row or two), and writes ids,
+//      rebuilt keys and payload to their final rows.
+//
+// The order is the stable sort's: (key, row id) is what a stable sort orders by. What it replaces moved
+// rows stably (nine ballots a row and a look-back over the tiles before it, 8.4 and 5.8 warp
+// instructions a row in two passes bound by instruction issue); no step here needs the rows before a
+// tile, so there is no look-back and no ordering between tiles.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <type_traits>
+
+#include "am_internal.h"
+#include "bucket_sort.cuh"
+#include "key_encode.cuh"
+#include "radix_sort.cuh"
+#include "records.cuh"
+
+namespace am {
+namespace bs {
+
+using namespace rs;
+
+constexpr int COARSE_BITS = 9, COARSE = 1 << COARSE_BITS;
+constexpr int FINE_BITS = 11;                     // a coarse cell has at most 2^11 fine cells
+constexpr int FINE_GOAL = 512;                    // sum of 2^bits <= 2 x goal + COARSE
+constexpr int FINE = 2 * FINE_GOAL + COARSE;
+constexpr uint32_t MAX_BUCKETS = 40960;
+constexpr int BINS1 = 1024;                       // level-1 bins
+constexpr int S2 = 8, BINS2 = 1 << S2;            // buckets a level-1 bin of a two-level sort
+static_assert(MAX_BUCKETS / BINS2 <= 256, "level-1 bins of a two-level sort");
+constexpr int CAP = 2048;                         // rows the shared-memory sort of a bucket takes
+constexpr int BIG = 4096;                         // rows its slower form takes
+constexpr uint32_t TARGET = 1300;                 // rows a bucket is meant to hold
+constexpr uint32_t SAMPLES = 65536;               // keys looked at (every key of a shorter column)
+constexpr int CLUSTER = 8;                        // CTAs of the one-cluster kernels
+constexpr int BINS = 2048, BINS_LOG = 11;         // bins of the shared-memory sort
+constexpr uint32_t MAX_BIN = 32;                  // rows a bin may hold for the comparisons
+constexpr uint32_t META_SPLIT = 0x80000000u;
+constexpr int CUR_PAD = 8;                        // cursors 32 bytes apart: same-sector atomics queue
+constexpr int THREADS = 512, ITEMS = 7, TILE = THREADS * ITEMS, WARPS = THREADS / 32;
+constexpr int HTHREADS = 1024, HITEMS = 8;
+constexpr int MAX_CHUNKS = 296;                   // two level-1 CTAs on each of 148 SMs
+constexpr int LTHREADS = 256, LITEMS = CAP / LTHREADS, LBLOCKS = 4;
+
+struct Args {
+  State* st;
+  uint32_t *coarse, *fine, *bfirst, *bmeta, *bcount, *bpos, *cursor1, *cursor2, *chunk_bins, *chunk_cats;
+  uint32_t nsamples, nchunks, chunk_rows, bucket_cap, bins1_cap;
+  uint64_t n;
+  void* keys[2];
+  uint32_t* ids[2];
+  uint4* rec[2];                                  // with a payload: row id and payload fields (RecLayout), instead of ids
+  void *out, *key_out;
+  int32_t wide, key_pt, key_desc, nulls_first;
+  uint32_t* err;
+  SortSummary* sum;
+  RecLayout pay;
+};
+
+// ---- the map key -> (bucket, fine cell, position in the fine cell)
+//
+// x = key - lo, shifted so that the sampled range fills the word: the top 9 bits are the coarse cell, the
+// bits below lead the position within it.
+template <typename KeyT>
+struct Map {
+  KeyT lo, span;
+  uint32_t up, last, linear;
+};
+template <typename KeyT>
+__device__ __forceinline__ Map<KeyT> load_map(const State* st) {
+  return {KeyT(st->lo), KeyT(st->span), st->up, st->buckets - 1, st->linear};
+}
+// Fine cell `f` and the 32 bits below it, of x <= span.
+template <typename KeyT>
+__device__ __forceinline__ void cell_of(const Map<KeyT>& m, const uint32_t* coarse, KeyT x, uint32_t& f, uint32_t& frac) {
+  const KeyT y = KeyT(x << m.up);
+  constexpr int TOP = int(sizeof(KeyT)) * 8 - COARSE_BITS;
+  const uint32_t e = coarse[uint32_t(y >> TOP)], fb = e >> 16;
+  const KeyT z = KeyT(y << COARSE_BITS);
+  uint32_t hi;
+  if constexpr (sizeof(KeyT) == 8) {
+    hi = uint32_t(z >> 32);
+    frac = __funnelshift_l(uint32_t(z), hi, fb);
+  } else {
+    hi = z;
+    frac = z << fb;
+  }
+  f = (e & 0xFFFFu) + ((hi >> 1) >> (31u - fb));
+}
+template <typename KeyT>
+__device__ __forceinline__ uint32_t bucket_of(const Map<KeyT>& m, const uint32_t* coarse, const uint32_t* fine, KeyT key) {
+  const KeyT x = KeyT(key - m.lo);                 // a key below lo wraps past the span
+  if (x > m.span) return key < m.lo ? 0u : m.last;
+  if (m.linear) return 1u + __umulhi(uint32_t(KeyT(x << m.up) >> (8 * sizeof(KeyT) - 32)), m.linear);
+  uint32_t f, frac;
+  cell_of(m, coarse, x, f, frac);
+  const uint32_t e = fine[f];
+  return (e & 0xFFFFu) + __umulhi(frac, e >> 16);
+}
+
+__device__ __forceinline__ void load_tables(const Args& a, uint32_t* coarse, uint32_t* fine) {
+  if (a.st->linear) return;
+  for (int i = threadIdx.x; i < COARSE; i += blockDim.x) coarse[i] = a.coarse[i];
+  for (int i = threadIdx.x; i < FINE; i += blockDim.x) fine[i] = a.fine[i];
+}
+
+// A warp's NI x 32 rows from row w0 (item i of a lane: row w0 + 32 i + lane), rows before `end`, as
+// loaded: raw key bits, and lane i's word of the validity bitmap is item i's 32 rows.
+template <typename KeyT, int NI>
+struct RawTile {
+  KeyT key[NI];
+  uint32_t word;
+};
+template <int NI>
+__device__ __forceinline__ bool whole_words(const ColView& col, uint64_t w0, uint64_t end) {
+  return w0 + NI * 32 <= end && (col.valid_off & 31) == 0 && (reinterpret_cast<uintptr_t>(col.valid) & 3u) == 0;
+}
+template <typename KeyT, int NI>
+__device__ __forceinline__ void load_tile(const ColView& col, uint64_t w0, uint64_t end, RawTile<KeyT, NI>& r) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const bool plain = sizeof(KeyT) == 8 || col.pt == PT_I32 || col.pt == PT_U32 || col.pt == PT_F32;
+  if (w0 + NI * 32 <= end && plain) {
+    const KeyT* v = static_cast<const KeyT*>(col.values) + w0 + lane;
+#pragma unroll
+    for (int i = 0; i < NI; i++) r.key[i] = v[i * 32];
+  } else {
+    uint32_t row[NI], ok = 0;
+#pragma unroll
+    for (int i = 0; i < NI; i++) {
+      const uint64_t g = w0 + uint64_t(i) * 32 + lane;
+      row[i] = uint32_t(g);
+      if (g < end) ok |= 1u << i;
+    }
+    load_raw_rows<KeyT, NI>(col, row, ok, r.key);
+  }
+  r.word = 0;
+  if (col.valid && lane < uint32_t(NI) && whole_words<NI>(col, w0, end))
+    r.word = reinterpret_cast<const uint32_t*>(col.valid)[((uint64_t(col.valid_off) + w0) >> 5) + lane];
+}
+// Raw bits into keys; bit i of `values`, `nulls`, `nans` says what item i is. Keys of rows that are not
+// values mean nothing.
+template <typename KeyT, int NI>
+__device__ __forceinline__ void encode_tile(const ColView& col, uint64_t w0, uint64_t end, RawTile<KeyT, NI>& t,
+                                            uint32_t& values, uint32_t& nulls, uint32_t& nans) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t ok = (1u << NI) - 1u;
+  if (w0 + NI * 32 > end) {
+    ok = 0;
+#pragma unroll
+    for (int i = 0; i < NI; i++)
+      if (w0 + uint64_t(i) * 32 + lane < end) ok |= 1u << i;
+  }
+  values = ok;
+  if (col.valid) {
+    if (whole_words<NI>(col, w0, end)) {
+      values = 0;
+#pragma unroll
+      for (int i = 0; i < NI; i++) values |= ((__shfl_sync(0xffffffffu, t.word, i) >> lane) & 1u) << i;
+    } else {
+      values = striped_validity<NI>(col, w0, end, ok);
+    }
+  }
+  nulls = ok & ~values;
+  nans = 0;
+  constexpr KeyT SIGN = KeyT(KeyT(1) << (8 * sizeof(KeyT) - 1));
+  const KeyT flip = col.desc ? KeyT(~KeyT(0)) : KeyT(0);
+  if (sizeof(KeyT) == 8 ? col.pt == PT_F64 : (col.pt == PT_F32 || col.pt == PT_F16)) {
+    constexpr KeyT INF = sizeof(KeyT) == 8 ? KeyT(0x7FF0000000000000ull) : KeyT(0x7F800000u);
+    const bool total = col.float_order == FO_TOTAL;
+#pragma unroll
+    for (int i = 0; i < NI; i++) {
+      KeyT r = t.key[i];
+      if constexpr (sizeof(KeyT) == 4)
+        if (col.pt == PT_F16) r = f16_to_f32_bits(uint32_t(r));
+      const KeyT mag = KeyT(r & ~SIGN);
+      if (!total) {
+        if (mag > INF) {
+          if (col.nan_cat) nans |= 1u << i;
+          r = KeyT(INF | 1u);
+        }
+        if (mag == 0) r = 0;
+      }
+      t.key[i] = KeyT(r ^ (((r & SIGN) ? KeyT(~KeyT(0)) : SIGN) ^ flip));
+    }
+    nans &= values;
+    values &= ~nans;
+  } else {
+    const KeyT x = KeyT((sizeof(KeyT) == 8 ? (col.pt == PT_I64 ? SIGN : KeyT(0)) : (col.pt == PT_U32 ? KeyT(0) : SIGN)) ^ flip);
+#pragma unroll
+    for (int i = 0; i < NI; i++) t.key[i] ^= x;
+  }
+}
+
+// Exclusive scan of one value a thread over the block; `total` to every thread. Two barriers.
+template <int NT>
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* s_warp, uint32_t& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  __syncthreads();
+  if (lane == 31) s_warp[warp] = x;
+  __syncthreads();
+  const uint32_t c = lane < NT / 32 ? s_warp[lane] : 0u;
+  total = __reduce_add_sync(0xffffffffu, c);
+  return x - v + __reduce_add_sync(0xffffffffu, lane < warp ? c : 0u);
+}
+
+// ---- bulk copies between shared and global memory (addresses and sizes multiples of 16 bytes)
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
+// Shared memory written by this thread becomes visible to bulk copies issued after the next barrier.
+__device__ __forceinline__ void fence_bulk() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void bulk_store(void* dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_addr(src)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// Until this thread's bulk stores have read their shared memory; until they are complete.
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+__device__ __forceinline__ void mbar_init(uint64_t* bar) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_addr(dst)),
+               "l"(src), "r"(bytes), "r"(smem_addr(bar))
+               : "memory");
+}
+// Waits for the phase of `parity`: at most about a second, then false.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
+  for (uint32_t polls = 0; polls < (1u << 20); polls++) {
+    uint32_t done;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(done) : "r"(smem_addr(bar)), "r"(parity) : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+
+// ---- 1. the sample and the bucket map
+
+// One cluster of CTAs; each holds its share of the sample in registers, and sums counts over the
+// cluster's shared memories. (One CTA alone, its samples read twice from L2, took 60 us for 65,536.)
+struct PlanShared {
+  uint32_t coarse_cnt[COARSE];
+  uint32_t half_cnt[2 * FINE];           // the halves of the fine cells
+  uint32_t coarse[COARSE];
+  uint32_t warp[32];
+  uint32_t group[1024];
+  unsigned long long smax[CLUSTER], smin[CLUSTER], scnt[CLUSTER];
+  unsigned long long wmax[32], wmin[32];
+};
+
+template <typename KeyT>
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(1024)
+buckets_kernel(const __grid_constant__ ColView col, const __grid_constant__ Args a) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ PlanShared sm;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const uint32_t rank = cl.block_rank();
+  State* st = a.st;
+  cl.sync();                             // every CTA runs before its shared memory is written
+  // The sample: one row of each nsamples-th part of the column, at a mixed offset (no period of the data
+  // lines up), or every row. nsamples is SAMPLES or the rows.
+  constexpr int U = SAMPLES / (1024 * CLUSTER);
+  KeyT key[U];
+  uint32_t live = 0;
+  const bool full = a.nsamples == a.n;
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const uint32_t j = (rank * U + u) * 1024 + t;
+    key[u] = 0;
+    if (j < a.nsamples) {
+      uint64_t row = j;
+      if (!full) {
+        const uint64_t lo = uint64_t(j) * a.n / SAMPLES, hi = uint64_t(j + 1) * a.n / SAMPLES;
+        uint32_t h = j * 2654435761u;
+        h ^= h >> 15;
+        h *= 2246822519u;
+        h ^= h >> 13;
+        row = lo + __umulhi(h, uint32_t(hi - lo));
+      }
+      const bool valid = !col.valid || bit_at(col.valid, col.valid_off + int64_t(row));
+      int cat;
+      key[u] = key_from_raw<KeyT>(col, load_raw<KeyT>(col, row), valid, cat);
+      if (cat == 0) live |= 1u << u;
+    }
+  }
+  for (int i = t; i < COARSE; i += 1024) sm.coarse_cnt[i] = 0;
+  for (int i = t; i < 2 * FINE; i += 1024) sm.half_cnt[i] = 0;
+  // The sampled range, over the cluster.
+  {
+    uint64_t mx = 0, mn = 0;
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if ((live >> u) & 1u) {
+        mx = max(mx, uint64_t(key[u]));
+        mn = max(mn, ~uint64_t(key[u]));
+      }
+    mx = warp_max_u64(mx);
+    mn = warp_max_u64(mn);
+    const uint32_t c = __reduce_add_sync(0xffffffffu, __popc(live));
+    if (lane == 0) {
+      sm.wmax[warp] = mx;
+      sm.wmin[warp] = mn;
+      sm.warp[warp] = c;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const uint64_t bx = warp_max_u64(sm.wmax[lane]), bn = warp_max_u64(sm.wmin[lane]);
+      const uint32_t bc = __reduce_add_sync(0xffffffffu, sm.warp[lane]);
+      if (lane < CLUSTER) {
+        PlanShared* o = cl.map_shared_rank(&sm, lane);
+        o->smax[rank] = bx;
+        o->smin[rank] = bn;
+        o->scnt[rank] = bc;
+      }
+    }
+  }
+  cl.sync();
+  uint64_t vmax = 0, vmin_inv = 0;
+  uint32_t sv = 0;
+#pragma unroll
+  for (int r = 0; r < CLUSTER; r++) {
+    vmax = max(vmax, uint64_t(sm.smax[r]));
+    vmin_inv = max(vmin_inv, uint64_t(sm.smin[r]));
+    sv += uint32_t(sm.scnt[r]);
+  }
+  const unsigned long long lo = sv ? ~vmin_inv : 0ull, span = sv ? vmax - lo : 0ull;
+  const int bits = max(COARSE_BITS, span ? 64 - __clzll((long long)span) : 0);
+  const uint32_t shc = uint32_t(bits - COARSE_BITS);        // key bits below a coarse cell
+  const Map<KeyT> map{KeyT(lo), KeyT(span), uint32_t(sizeof(KeyT)) * 8u - uint32_t(bits), 0u, 0u};
+#pragma unroll
+  for (int u = 0; u < U; u++)
+    if ((live >> u) & 1u) atomicAdd(&sm.coarse_cnt[uint32_t(KeyT(key[u] - map.lo) >> shc)], 1u);
+  cl.sync();
+  uint32_t in_cell = 0;                  // the sample's keys in coarse cell t
+  if (t < COARSE) {
+#pragma unroll
+    for (int r = 0; r < CLUSTER; r++) in_cell += cl.map_shared_rank(&sm, r)->coarse_cnt[t];
+  }
+  // Evenly spread keys (every coarse cell's count within 4.5 deviations of its width's share) need no
+  // tables: equal cuts of the range, filled to TARGET rows (a deviation the test cannot see still
+  // fits CAP).
+  {
+    uint32_t off = 0;
+    if (t < COARSE) {
+      const unsigned long long c0 = (unsigned long long)t << shc, w = 1ull << shc;
+      const float keys_in = c0 > span ? 0.0f : span - c0 >= w ? float(w) : float(span - c0) + 1.0f;
+      const float e = float(sv) * keys_in / (float(span) + 1.0f);
+      off = fabsf(float(in_cell) - e) > 4.5f * sqrtf(e) + 3.0f ? 1u : 0u;
+    }
+    const bool even = !__syncthreads_or(int(off)) && sv >= 16u * COARSE && shc > 0;
+    if (even) {
+      const float est = float(a.n) * float(sv) / float(a.nsamples);
+      const float range = bits == 64 ? 18446744073709551616.0f : float(1ull << bits);
+      const uint32_t cuts = uint32_t(ceilf(est / float(TARGET) * (range / (float(span) + 1.0f))));
+      const uint32_t top = uint32_t(KeyT(KeyT(span) << map.up) >> (8 * sizeof(KeyT) - 32));
+      const uint32_t nb = __umulhi(top, cuts) + 3u;
+      if (nb <= a.bucket_cap) {
+        for (uint32_t b = rank * 1024 + t; b < nb; b += 1024 * CLUSTER) {
+          const bool outer = b == 0 || b == nb - 1;
+          a.bmeta[b] = META_SPLIT | (outer ? 0u : cuts);
+          a.bfirst[b] = (outer ? 0xFFFFu : map.up) << 16;
+        }
+        if (t == 0 && rank == 0) {
+          st->lo = lo;
+          st->span = span;
+          st->up = map.up;
+          st->linear = cuts;
+          st->buckets = nb;
+          st->s2 = nb <= a.bins1_cap ? 0u : uint32_t(S2);
+          st->bins1 = nb <= a.bins1_cap ? nb : (nb + BINS2 - 1) >> S2;
+          st->mode = MODE_BUCKETS;
+        }
+        cl.sync();                       // no CTA leaves while another reads its counts
+        return;
+      }
+    }
+  }
+  // Fine cells of each coarse cell: 2^fb, from its share of the sample (about FINE_GOAL cells over the
+  // column, fewer when the sample is small: at least 24 sampled rows a cell on average).
+  const uint32_t goal = min(uint32_t(FINE_GOAL), max(1u, sv / 24u));
+  uint32_t fb = 0, width = 0;
+  if (t < COARSE) {
+    const uint32_t want = sv ? uint32_t(uint64_t(in_cell) * goal / sv) : 0u;
+    fb = want > 1u ? 32u - __clz(want - 1u) : 0u;
+    fb = min(fb, min(uint32_t(FINE_BITS), shc));
+    width = 1u << fb;
+  }
+  uint32_t nfine;
+  const uint32_t fbase = block_scan<1024>(width, sm.warp, nfine);
+  if (t < COARSE) {
+    sm.coarse[t] = fbase | (fb << 16);
+    if (rank == 0) a.coarse[t] = sm.coarse[t];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < U; u++)
+    if ((live >> u) & 1u) {
+      uint32_t f, frac;
+      cell_of(map, sm.coarse, KeyT(key[u] - map.lo), f, frac);
+      atomicAdd(&sm.half_cnt[2 * f + (frac >> 31)], 1u);
+    }
+  cl.sync();
+  if (rank == 0) {
+    for (int i = t; i < 2 * FINE; i += 1024) {
+      uint32_t c = sm.half_cnt[i];
+#pragma unroll
+      for (int r = 1; r < CLUSTER; r++) c += cl.map_shared_rank(&sm, r)->half_cnt[i];
+      sm.half_cnt[i] = c;
+    }
+  }
+  cl.sync();
+  if (rank != 0) return;
+  const uint32_t* coarse = sm.coarse;
+  // Rows of each fine cell, at the upper end of what the sample says; single-key cells (nothing left to
+  // split) that surely exceed a bucket end the attempt here.
+  constexpr int PER = (FINE + 1023) / 1024;
+  const float scale = float(a.n) / float(a.nsamples);
+  uint32_t rows[PER], dense[PER], room[PER], below[PER];     // below: what shifts a key's distance from lo to its place in the cell
+  uint32_t bad = 0;
+#pragma unroll
+  for (int q = 0; q < PER; q++) {
+    const uint32_t f = uint32_t(t) * PER + q;
+    rows[q] = 0;
+    dense[q] = 0;
+    room[q] = 1;
+    below[q] = 0;
+    if (f >= nfine) continue;
+    const uint32_t h0 = sm.half_cnt[2 * f], h1 = sm.half_cnt[2 * f + 1];
+    const float c = float(h0 + h1), h = float(max(h0, h1));
+    rows[q] = full ? h0 + h1 : uint32_t((c + sqrtf(c) + 1.0f) * scale);
+    // Split by the fuller half: keys are not even within a cell that spans a factor of two of a float's range.
+    dense[q] = 2u * (full ? max(h0, h1) : uint32_t((h + sqrtf(h) + 1.0f) * scale));
+    // The fine cell's coarse cell: the last one starting at or before it.
+    uint32_t l = 0, r = COARSE;
+    while (r - l > 1) {
+      const uint32_t mid = (l + r) >> 1;
+      if ((coarse[mid] & 0xFFFFu) <= f) l = mid;
+      else r = mid;
+    }
+    const uint32_t left = shc - (coarse[l] >> 16);           // key bits below the fine cell
+    room[q] = left >= 16 ? 65535u : 1u << left;
+    below[q] = uint32_t(sizeof(KeyT)) * 8u - left;
+    if (room[q] == 1u && (c - 4.0f * sqrtf(c)) * scale > float(BIG)) bad = 1;
+  }
+  bad = __syncthreads_or(bad);
+  // Buckets: a heavy cell (over half a target) is split into equal parts; light neighbours share one.
+  // With more buckets than fit, larger targets.
+  uint32_t target = TARGET, total = 0, base[PER], m[PER];
+  bool start[PER];
+  for (int attempt = 0; attempt < 4 && !bad; attempt++) {
+    const uint32_t half = target / 2;
+    uint32_t light = 0;
+#pragma unroll
+    for (int q = 0; q < PER; q++)
+      if (rows[q] <= half) light += rows[q];
+    uint32_t all;
+    uint32_t before = block_scan<1024>(light, sm.warp, all);
+    // The group of the cell before this thread's first one.
+    uint32_t group[PER];
+#pragma unroll
+    for (int q = 0; q < PER; q++) {
+      const bool heavy = rows[q] > half;
+      group[q] = heavy ? 0xFFFFFFFFu : before / half;
+      if (!heavy) before += rows[q];
+    }
+    sm.group[t] = group[PER - 1];
+    __syncthreads();
+    uint32_t prev = t ? sm.group[t - 1] : 0xFFFFFFFFu, add = 0;
+#pragma unroll
+    for (int q = 0; q < PER; q++) {
+      const uint32_t f = uint32_t(t) * PER + q;
+      m[q] = 1;
+      start[q] = group[q] == 0xFFFFFFFFu || group[q] != prev;
+      if (group[q] == 0xFFFFFFFFu) m[q] = min((dense[q] + target - 1) / target, room[q]);
+      prev = group[q];
+      base[q] = add;
+      if (f < nfine && start[q]) add += m[q];
+    }
+    const uint32_t off = block_scan<1024>(add, sm.warp, total);
+#pragma unroll
+    for (int q = 0; q < PER; q++) base[q] += off;
+    if (total + 2 <= a.bucket_cap) break;
+    target += target / 4;
+  }
+  if (bad || total + 2 > a.bucket_cap || sv == 0) {
+    if (t == 0) st->mode = MODE_FALLBACK;
+    return;
+  }
+  // The tables. Bucket 0 and the last take the keys outside the sampled range.
+#pragma unroll
+  for (int q = 0; q < PER; q++) {
+    const uint32_t f = uint32_t(t) * PER + q;
+    if (f >= nfine) continue;
+    const uint32_t b = 1u + base[q] - (start[q] ? 0u : 1u);
+    a.fine[f] = b | (m[q] << 16);
+    if (rows[q] > target / 2) {
+      for (uint32_t k = 0; k < m[q]; k++) {
+        a.bfirst[b + k] = below[q] << 16;
+        a.bmeta[b + k] = META_SPLIT | m[q];
+      }
+    } else {
+      if (start[q]) a.bfirst[b] = f;
+      atomicMax(&a.bmeta[b], f);               // the last cell of the bucket (bmeta starts at zero)
+    }
+  }
+  if (t == 0) {
+    const uint32_t nb = total + 2;
+    a.bmeta[0] = META_SPLIT;
+    a.bmeta[nb - 1] = META_SPLIT;
+    a.bfirst[0] = 0xFFFF0000u;
+    a.bfirst[nb - 1] = 0xFFFF0000u;
+    st->lo = lo;
+    st->span = span;
+    st->up = map.up;
+    st->buckets = nb;
+    st->s2 = nb <= a.bins1_cap ? 0u : uint32_t(S2);
+    st->bins1 = nb <= a.bins1_cap ? nb : (nb + BINS2 - 1) >> S2;
+    st->mode = MODE_BUCKETS;
+  }
+}
+
+// ---- 2. exact counts
+//
+// One read of the column (63 us for 45M keys and 16,384 bins on a B200: the HBM copy rate). Each CTA
+// takes consecutive chunks; a chunk's level-1 counts are the growth of its bins' sums over the chunk.
+template <typename KeyT>
+__global__ void __launch_bounds__(HTHREADS) bucket_histogram_kernel(const __grid_constant__ ColView col,
+                                                                   const __grid_constant__ Args a) {
+  extern __shared__ __align__(16) unsigned char hsm[];
+  State* st = a.st;
+  if (st->mode != MODE_BUCKETS) return;
+  uint32_t* bins = reinterpret_cast<uint32_t*>(hsm);
+  __shared__ uint32_t coarse[COARSE], fine[FINE], prev[BINS1];
+  __shared__ uint32_t s_null, s_nan;
+  __shared__ unsigned long long s_or;
+  const uint32_t nb = st->buckets, s2 = st->s2, nbins = st->bins1;
+  load_tables(a, coarse, fine);
+  for (uint32_t i = threadIdx.x; i < nb; i += HTHREADS) bins[i] = 0;
+  for (int i = threadIdx.x; i < BINS1; i += HTHREADS) prev[i] = 0;
+  if (threadIdx.x == 0) {
+    s_null = 0;
+    s_nan = 0;
+    s_or = 0;
+  }
+  __syncthreads();
+  const Map<KeyT> map = load_map<KeyT>(st);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  KeyT diff = 0;                        // bits that differ from lo's in some key
+  uint32_t values = 0, all_null = 0, all_nan = 0;
+  const uint32_t c0 = uint32_t(uint64_t(blockIdx.x) * a.nchunks / gridDim.x);
+  const uint32_t c1 = uint32_t(uint64_t(blockIdx.x + 1) * a.nchunks / gridDim.x);
+  for (uint32_t c = c0; c < c1; c++) {
+    const uint64_t first = uint64_t(c) * a.chunk_rows, end = min(a.n, first + a.chunk_rows);
+    uint32_t n_null = 0, n_nan = 0;
+    for (uint64_t w0 = first + uint64_t(warp) * (HITEMS * 32); w0 < end; w0 += HTHREADS * HITEMS) {
+      RawTile<KeyT, HITEMS> r;
+      uint32_t is_value, is_null, is_nan;
+      load_tile(col, w0, end, r);
+      encode_tile(col, w0, end, r, is_value, is_null, is_nan);
+      values += __popc(is_value);
+      n_null += __popc(is_null);
+      n_nan += __popc(is_nan);
+#pragma unroll
+      for (int i = 0; i < HITEMS; i++) {
+        if (!((is_value >> i) & 1u)) continue;
+        diff |= r.key[i] ^ map.lo;
+        atomicAdd(bins + bucket_of(map, coarse, fine, r.key[i]), 1u);
+      }
+    }
+    n_null = __reduce_add_sync(0xffffffffu, n_null);
+    n_nan = __reduce_add_sync(0xffffffffu, n_nan);
+    if (lane == 0) {
+      if (n_null) atomicAdd(&s_null, n_null);
+      if (n_nan) atomicAdd(&s_nan, n_nan);
+    }
+    __syncthreads();
+    if (s2 == 0) {
+      for (uint32_t d = threadIdx.x; d < nbins; d += HTHREADS) {
+        a.chunk_bins[size_t(c) * BINS1 + d] = bins[d] - prev[d];
+        prev[d] = bins[d];
+      }
+    } else {
+      for (uint32_t d = warp; d < nbins; d += HTHREADS / 32) {
+        uint32_t sum = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < BINS2; q += 32) {
+          const uint32_t b = (d << S2) + q + lane;
+          sum += b < nb ? bins[b] : 0u;
+        }
+        sum = __reduce_add_sync(0xffffffffu, sum);
+        if (lane == 0) {
+          a.chunk_bins[size_t(c) * BINS1 + d] = sum - prev[d];
+          prev[d] = sum;
+        }
+      }
+    }
+    if (threadIdx.x == 0) {
+      a.chunk_cats[2 * c] = s_null;
+      a.chunk_cats[2 * c + 1] = s_nan;
+      all_null += s_null;
+      all_nan += s_nan;
+      s_null = 0;
+      s_nan = 0;
+    }
+    __syncthreads();
+  }
+  diff = warp_or<KeyT>(diff);
+  values = __reduce_add_sync(0xffffffffu, values);
+  if (lane == 0) {
+    atomicOr(&s_or, (unsigned long long)diff);
+    if (values) atomicAdd(&st->n_value, values);
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < nb; i += HTHREADS)
+    if (bins[i]) atomicAdd(a.bcount + i, bins[i]);
+  if (threadIdx.x == 0) {
+    if (all_null) atomicAdd(&st->n_null, all_null);
+    if (all_nan) atomicAdd(&st->n_nan, all_nan);
+    atomicOr(&st->diff, s_or);
+  }
+}
+
+// One cluster: bucket starts, cursors, the chunks' null and NaN starts, and the decision.
+template <typename KeyT>
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(1024) bucket_starts_kernel(const __grid_constant__ Args a) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ uint32_t s_warp[32], s_sum[CLUSTER], s_max[CLUSTER];
+  State* st = a.st;
+  if (st->mode != MODE_BUCKETS) return;
+  cl.sync();                             // every CTA runs before its shared memory is written
+  constexpr uint32_t PER = 8;
+  static_assert(MAX_BUCKETS <= CLUSTER * 1024 * PER, "one round of the cluster takes every bucket");
+  const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, rank = cl.block_rank();
+  const uint32_t nb = st->buckets, s2 = st->s2;
+  // CTA r takes the r-th of equal shares (a multiple of PER), a thread PER buckets in a row.
+  const uint32_t share = (nb + CLUSTER * PER - 1) / (CLUSTER * PER) * PER;
+  const uint32_t b = rank * share + t * PER;
+  uint32_t c[PER], sum = 0, big = 0;
+#pragma unroll
+  for (uint32_t q = 0; q < PER; q++) {
+    c[q] = t * PER < share && b + q < nb ? a.bcount[b + q] : 0u;
+    sum += c[q];
+    big = max(big, c[q]);
+  }
+  uint32_t tot;
+  uint32_t at = block_scan<1024>(sum, s_warp, tot);
+  big = __reduce_max_sync(0xffffffffu, big);
+  __syncthreads();
+  if (lane == 0) s_warp[warp] = big;
+  __syncthreads();
+  big = __reduce_max_sync(0xffffffffu, s_warp[lane]);
+  if (t < uint32_t(CLUSTER)) {
+    cl.map_shared_rank(s_sum, t)[rank] = tot;
+    cl.map_shared_rank(s_max, t)[rank] = big;
+  }
+  cl.sync();
+  uint32_t carry = 0;
+  for (uint32_t r = 0; r < uint32_t(CLUSTER); r++) {
+    if (r < rank) at += s_sum[r];
+    carry += s_sum[r];
+    big = max(big, s_max[r]);
+  }
+#pragma unroll
+  for (uint32_t q = 0; q < PER; q++) {
+    if (t * PER < share && b + q < nb) {
+      a.bpos[b + q] = at;
+      a.cursor2[size_t(b + q) * CUR_PAD] = at;
+      if (((b + q) & ((1u << s2) - 1u)) == 0u) a.cursor1[size_t((b + q) >> s2) * CUR_PAD] = at;
+      at += c[q];
+    }
+  }
+  if (rank != 0) return;
+  uint32_t all;
+  const uint32_t nulls = t < a.nchunks ? a.chunk_cats[2 * t] : 0u;
+  const uint32_t nans = t < a.nchunks ? a.chunk_cats[2 * t + 1] : 0u;
+  const uint32_t null0 = block_scan<1024>(nulls, s_warp, all);
+  const uint32_t nan0 = block_scan<1024>(nans, s_warp, all);
+  if (t < a.nchunks) {
+    a.chunk_cats[2 * t] = null0;
+    a.chunk_cats[2 * t + 1] = nan0;
+  }
+  if (t == 0) {
+    a.bpos[nb] = carry;
+    st->max_bucket = big;
+    if (carry != st->n_value) atomicOr(a.err, ERR_BOUNDS);
+    if (big > uint32_t(BIG) || carry != st->n_value) {
+      st->mode = MODE_FALLBACK;
+    } else {
+      // The counters of the digit passes' sort: the key's digits that vary. A two-level sort's two
+      // passes stand in for them.
+      uint32_t active = 0;
+      for (uint32_t d = 0; d < sizeof(KeyT); d++) active += (st->diff >> (8 * d)) & 255u ? 1u : 0u;
+      a.sum->value_rows = st->n_value;
+      a.sum->null_rows = st->n_null;
+      a.sum->nan_rows = st->n_nan;
+      a.sum->passes_run = s2 ? 2u : max(1u, active);
+      a.sum->passes_total = uint32_t(sizeof(KeyT));
+    }
+  }
+}
+
+// ---- 3. rows to their buckets
+
+template <typename KeyT, int PAY>
+struct TileShared {
+  static constexpr int NB = PAY ? BINS1 / 2 : BINS1;
+  uint32_t coarse[COARSE], fine[FINE];
+  // Rows of the tile per bin, then the bins' starts in it; what added to a row's place in the tile gives
+  // its destination; the chunk's next destination in each bin.
+  uint32_t start[NB], delta[NB], at[NB];
+  uint32_t warp[32];
+  uint32_t cats[WARPS][2];
+  uint4 rec[PAY ? TILE : 1];
+  KeyT key[TILE];
+  // Per staged row: its bin, and without records (which hold the row id) its place in the tile below it.
+  std::conditional_t<PAY != 0, uint16_t, uint32_t> word[TILE];
+};
+
+__device__ __forceinline__ void store_id(const Args& a, uint64_t dst, uint32_t id) {
+  if (!a.out) return;
+  if (a.wide) static_cast<uint64_t*>(a.out)[dst] = id;
+  else static_cast<uint32_t*>(a.out)[dst] = id;
+}
+
+template <typename KeyT, int PAY>
+__global__ void __launch_bounds__(THREADS, 2) level1_kernel(const __grid_constant__ ColView col,
+                                                           const __grid_constant__ Args a) {
+  extern __shared__ __align__(16) unsigned char tsm[];
+  using SM = TileShared<KeyT, PAY>;
+  SM& sm = *reinterpret_cast<SM*>(tsm);
+  const State* st = a.st;
+  if (st->mode != MODE_BUCKETS) return;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const uint32_t lt = (1u << lane) - 1u;
+  const uint32_t s2 = st->s2, nbins = st->bins1;
+  const Map<KeyT> map = load_map<KeyT>(st);
+  load_tables(a, sm.coarse, sm.fine);
+  const uint32_t c = blockIdx.x;
+  const uint64_t first = uint64_t(c) * a.chunk_rows, end = min(a.n, first + a.chunk_rows);
+  // The chunk's share of every bin, reserved once (chunks reserve in any order).
+  for (int d = t; d < SM::NB; d += THREADS) {
+    uint32_t at = 0;
+    if (uint32_t(d) < nbins) {
+      const uint32_t mine = a.chunk_bins[size_t(c) * BINS1 + d];
+      if (mine) at = atomicAdd(a.cursor1 + size_t(d) * CUR_PAD, mine);
+    }
+    sm.at[d] = at;
+    sm.start[d] = 0;
+  }
+  const bool cats = col.valid || col.nan_cat;
+  uint32_t null_at = a.chunk_cats[2 * c], nan_at = a.chunk_cats[2 * c + 1];
+  const uint32_t nv = st->n_value, nn = st->n_null, nx = st->n_nan;
+  null_at += a.nulls_first ? 0u : nv + nx;
+  nan_at += a.nulls_first ? nn : nv;
+  KeyT* __restrict__ kout = static_cast<KeyT*>(a.keys[0]);
+  uint32_t* __restrict__ iout = a.ids[0];
+  uint4* __restrict__ rout = a.rec[0];
+  const uint32_t wofs = uint32_t(warp) * (ITEMS * 32) + uint32_t(lane);
+  const bool direct = PAY && a.pay.pair;           // the payload words are two columns as they are
+  const uint64_t* wsrc = direct ? static_cast<const uint64_t*>(a.pay.src[a.pay.wide]) : nullptr;
+  const uint32_t* hsrc = direct ? static_cast<const uint32_t*>(a.pay.src[a.pay.narrow]) : nullptr;
+  RawTile<KeyT, ITEMS> r;
+  uint64_t pw[PAY ? ITEMS : 1];
+  uint32_t ph[PAY ? ITEMS : 1];
+  auto load_rows = [&](uint64_t tile) {
+    load_tile(col, tile + (wofs - lane), end, r);
+    if constexpr (PAY) {
+      if (direct) {
+        const uint64_t* w = wsrc + tile + wofs;
+        const uint32_t* h = hsrc + tile + wofs;
+        const uint64_t left = end - tile;
+#pragma unroll
+        for (int i = 0; i < ITEMS; i++)
+          if (wofs + i * 32 < left) {
+            pw[i] = w[i * 32];
+            ph[i] = h[i * 32];
+          }
+      }
+    }
+  };
+  if (first < end) load_rows(first);
+  __syncthreads();
+  for (uint64_t tile = first; tile < end; tile += TILE) {
+    uint32_t values, nulls, nans;
+    encode_tile(col, tile + (wofs - lane), end, r, values, nulls, nans);
+    uint32_t slot[ITEMS];               // bin << 16 | place among the tile's rows of the bin
+#pragma unroll
+    for (int i = 0; i < ITEMS; i++) {
+      if (!((values >> i) & 1u)) continue;
+      const uint32_t d = bucket_of(map, sm.coarse, sm.fine, r.key[i]) >> s2;
+      slot[i] = (d << 16) | atomicAdd(&sm.start[d], 1u);
+    }
+    if (cats) {
+      const uint32_t wn = __reduce_add_sync(0xffffffffu, __popc(nulls)), wx = __reduce_add_sync(0xffffffffu, __popc(nans));
+      if (lane == 0) {
+        sm.cats[warp][0] = wn;
+        sm.cats[warp][1] = wx;
+      }
+    }
+    __syncthreads();
+    // The last tile's records have left shared memory before this one's are staged.
+    if constexpr (PAY) bulk_wait_read();
+    // Bin counts into starts: one or two bins a thread.
+    constexpr int PER = SM::NB / THREADS;
+    static_assert(PER == 1 || PER == 2, "bins a thread");
+    const uint32_t c0 = sm.start[PER * t], c1 = PER == 2 ? sm.start[PER * t + PER - 1] : 0u;
+    uint32_t tile_n;
+    const uint32_t s0 = block_scan<THREADS>(c0 + c1, sm.warp, tile_n);
+    const uint32_t at0 = sm.at[PER * t];
+    sm.start[PER * t] = s0;
+    sm.delta[PER * t] = at0 - s0;
+    sm.at[PER * t] = at0 + c0;
+    if constexpr (PER == 2) {
+      const uint32_t at1 = sm.at[2 * t + 1];
+      sm.start[2 * t + 1] = s0 + c0;
+      sm.delta[2 * t + 1] = at1 - (s0 + c0);
+      sm.at[2 * t + 1] = at1 + c1;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ITEMS; i++) {
+      if (!((values >> i) & 1u)) continue;
+      const uint32_t pos = sm.start[slot[i] >> 16] + (slot[i] & 0xFFFFu);
+      sm.key[pos] = r.key[i];
+      if constexpr (PAY) {
+        sm.word[pos] = uint16_t(slot[i] >> 16);
+        const uint32_t row = uint32_t(tile) + wofs + uint32_t(i) * 32;
+        sm.rec[pos] = direct ? make_uint4(row, uint32_t(pw[i]), uint32_t(pw[i] >> 32), ph[i]) : build_record(a.pay, row);
+      } else {
+        sm.word[pos] = (slot[i] & 0xFFFF0000u) | (wofs + i * 32);
+      }
+    }
+    // Null and NaN rows wait behind the values, in row order: they go straight to their final places.
+    uint32_t tn = 0, tx = 0;
+    if (cats) {
+      uint32_t wn = 0, wx = 0;
+#pragma unroll
+      for (int v = 0; v < WARPS; v++) {
+        const uint2 q = *reinterpret_cast<const uint2*>(sm.cats[v]);
+        if (v < warp) {
+          wn += q.x;
+          wx += q.y;
+        }
+        tn += q.x;
+        tx += q.y;
+      }
+      // (A tile's rows are at most TILE: behind the values there is room for the others.)
+      if (tn) {
+        uint32_t p = tile_n + wn;
+#pragma unroll
+        for (int i = 0; i < ITEMS; i++) {
+          const bool is = (nulls >> i) & 1u;
+          const uint32_t m = __ballot_sync(0xffffffffu, is);
+          if (is) sm.word[p + __popc(m & lt)] = wofs + i * 32;
+          p += __popc(m);
+        }
+      }
+      if (tx) {
+        uint32_t p = tile_n + tn + wx;
+#pragma unroll
+        for (int i = 0; i < ITEMS; i++) {
+          const bool is = (nans >> i) & 1u;
+          const uint32_t m = __ballot_sync(0xffffffffu, is);
+          if (is) sm.word[p + __popc(m & lt)] = wofs + i * 32;
+          p += __popc(m);
+        }
+      }
+    }
+    // The next tile's rows arrive while this one leaves.
+    if (tile + TILE < end) load_rows(tile + TILE);
+    if constexpr (PAY) fence_bulk();
+    __syncthreads();
+    if constexpr (PAY) {
+      // Thread d sends bin d's records as one copy; it runs while the next tile is read and ranked.
+      static_assert(PER == 1, "one bin a thread");
+      if (c0) {
+        if (at0 + c0 <= nv) bulk_store(rout + at0, sm.rec + s0, c0 * 16u);
+        else atomicOr(a.err, ERR_BOUNDS);
+      }
+      bulk_commit();
+    }
+    const int nit = int(tile_n + THREADS - 1 - t) / THREADS;
+#pragma unroll
+    for (int i = 0; i < ITEMS; i++) {
+      if (i >= nit) break;
+      const uint32_t j = uint32_t(i) * THREADS + t;
+      const uint32_t word = sm.word[j];
+      const uint32_t dst = sm.delta[PAY ? word : word >> 16] + j;
+      if (dst >= nv) {
+        atomicOr(a.err, ERR_BOUNDS);
+        continue;
+      }
+      kout[dst] = sm.key[j];
+      if constexpr (!PAY) iout[dst] = uint32_t(tile) + (word & 0xFFFFu);
+    }
+    for (uint32_t j = tile_n + t; j < tile_n + tn + tx; j += THREADS) {
+      const uint32_t q = j - tile_n, row = uint32_t(tile) + sm.word[j];
+      const uint32_t dst = q < tn ? null_at + q : nan_at + (q - tn);
+      if (dst >= a.n) {
+        atomicOr(a.err, ERR_BOUNDS);
+        continue;
+      }
+      store_id(a, dst, row);
+      if constexpr (PAY) unpack_record(a.pay, build_record(a.pay, row), dst);
+      if (a.key_out) store_width(a.key_out, dst, pt_bytes(a.key_pt), 0ull);
+    }
+    null_at += tn;
+    nan_at += tx;
+    for (int d = t; d < SM::NB; d += THREADS) sm.start[d] = 0;
+    __syncthreads();
+  }
+  if constexpr (PAY) bulk_wait_all();
+}
+
+template <typename KeyT, int PAY>
+struct Tile2Shared {
+  uint32_t coarse[COARSE], fine[FINE];
+  uint32_t tiles[MAX_BUCKETS / BINS2 + 1];      // tiles before each level-1 bin
+  uint32_t start[BINS2], delta[BINS2];
+  uint32_t warp[32];
+  std::conditional_t<PAY != 0, uint4, uint32_t> rec[TILE];      // records, or row ids
+  KeyT key[TILE];
+  uint8_t bin[TILE];
+};
+
+// Level 2: tiles of one level-1 bin's rows to its 128 buckets. A tile reserves its rows of a bucket with
+// one atomic.
+template <typename KeyT, int PAY>
+__global__ void __launch_bounds__(THREADS, 2) level2_kernel(const __grid_constant__ Args a) {
+  extern __shared__ __align__(16) unsigned char tsm[];
+  using SM = Tile2Shared<KeyT, PAY>;
+  SM& sm = *reinterpret_cast<SM*>(tsm);
+  const State* st = a.st;
+  if (st->mode != MODE_BUCKETS || st->s2 == 0) return;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const uint32_t nbins = st->bins1, nb = st->buckets, nv = st->n_value;
+  const Map<KeyT> map = load_map<KeyT>(st);
+  load_tables(a, sm.coarse, sm.fine);
+  auto bin_start = [&](uint32_t d) { return a.bpos[min(d << S2, nb)]; };
+  uint32_t ntiles;
+  {
+    const uint32_t rows = uint32_t(t) < nbins ? bin_start(t + 1) - bin_start(t) : 0u;
+    const uint32_t before = block_scan<THREADS>((rows + TILE - 1) / TILE, sm.warp, ntiles);
+    if (t <= int(MAX_BUCKETS / BINS2)) sm.tiles[t] = before;
+  }
+  const KeyT* __restrict__ kin = static_cast<const KeyT*>(a.keys[0]);
+  KeyT* __restrict__ kout = static_cast<KeyT*>(a.keys[1]);
+  const uint32_t t0 = uint32_t(uint64_t(blockIdx.x) * ntiles / gridDim.x);
+  const uint32_t t1 = uint32_t(uint64_t(blockIdx.x + 1) * ntiles / gridDim.x);
+  if (t < BINS2) sm.start[t] = 0;
+  __syncthreads();
+  uint32_t d = 0;
+  if (t0 < t1) {                         // the bin of the first tile: the last one starting at or before it
+    uint32_t l = 0, r = nbins;
+    while (r - l > 1) {
+      const uint32_t mid = (l + r) >> 1;
+      if (sm.tiles[mid] <= t0) l = mid;
+      else r = mid;
+    }
+    d = l;
+  }
+  using RecT = std::conditional_t<PAY != 0, uint4, uint32_t>;
+  const RecT* __restrict__ rin = reinterpret_cast<const RecT*>(PAY ? static_cast<const void*>(a.rec[0]) : a.ids[0]);
+  RecT* __restrict__ rout = reinterpret_cast<RecT*>(PAY ? static_cast<void*>(a.rec[1]) : a.ids[1]);
+  KeyT key[ITEMS];
+  // Tile q's first row and rows; its keys.
+  uint32_t first = 0, tile_n = 0;
+  int nit = 0;                          // this thread's rows of it: row i x THREADS + t, i < nit
+  auto load = [&](uint32_t q) {
+    while (d + 1 < nbins && sm.tiles[d + 1] <= q) d++;
+    const uint32_t end = bin_start(d + 1);
+    first = bin_start(d) + (q - sm.tiles[d]) * TILE;
+    tile_n = min(uint32_t(TILE), end - first);
+    nit = int((tile_n + THREADS - 1 - t) / THREADS);
+    const KeyT* p = kin + first + t;
+#pragma unroll
+    for (int i = 0; i < ITEMS; i++) {
+      if (i >= nit) break;
+      key[i] = p[i * THREADS];
+    }
+  };
+  if (t0 < t1) load(t0);
+  for (uint32_t q = t0; q < t1; q++) {
+    const uint32_t b0 = d << S2, row0 = first;
+    const int ni = nit;
+    uint32_t slot[ITEMS];
+#pragma unroll
+    for (int i = 0; i < ITEMS; i++) {
+      if (i >= ni) break;
+      const uint32_t b = (bucket_of(map, sm.coarse, sm.fine, key[i]) - b0) & uint32_t(BINS2 - 1);
+      slot[i] = (b << 16) | atomicAdd(&sm.start[b], 1u);
+    }
+    RecT rec[ITEMS];
+    const RecT* rp = rin + row0 + t;
+#pragma unroll
+    for (int i = 0; i < ITEMS; i++) {
+      if (i >= ni) break;
+      rec[i] = rp[i * THREADS];
+    }
+    __syncthreads();
+    uint32_t run = 0, run_at = 0, run_dst = 0;    // this thread's bucket: rows, where in the tile, where to
+    if (warp < BINS2 / 32) {
+      // The buckets' starts in the tile: each of these warps its own 32 buckets after the ones before.
+      if constexpr (PAY) bulk_wait_read();        // the last tile's records have left
+      const uint32_t c = sm.start[t];
+      uint32_t x = c, before = 0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      for (int v = 0; v < warp; v++) before += sm.start[v * 32 + lane];
+      before = __reduce_add_sync(0xffffffffu, before);
+      run = c;
+      run_at = before + x - c;
+      run_dst = c ? atomicAdd(a.cursor2 + size_t(b0 + t) * CUR_PAD, c) : 0u;
+      sm.delta[t] = run_dst - run_at;
+      asm volatile("bar.sync 1, %0;" ::"n"(BINS2) : "memory");
+      sm.start[t] = run_at;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ITEMS; i++) {
+      if (i >= ni) break;
+      const uint32_t b = slot[i] >> 16, pos = sm.start[b] + (slot[i] & 0xFFFFu);
+      sm.key[pos] = key[i];
+      sm.rec[pos] = rec[i];
+      sm.bin[pos] = uint8_t(b);
+    }
+    if (q + 1 < t1) load(q + 1);
+    if constexpr (PAY) fence_bulk();
+    __syncthreads();
+    if constexpr (PAY) {
+      if (run) {
+        if (run_dst + run <= nv) bulk_store(rout + run_dst, sm.rec + run_at, run * 16u);
+        else atomicOr(a.err, ERR_BOUNDS);
+      }
+      bulk_commit();
+    }
+    if (t < BINS2) sm.start[t] = 0;
+#pragma unroll
+    for (int i = 0; i < ITEMS; i++) {
+      const uint32_t j = uint32_t(i) * THREADS + t;
+      if (i >= ni) break;
+      const uint32_t dst = sm.delta[sm.bin[j]] + j;
+      if (dst >= nv) {
+        atomicOr(a.err, ERR_BOUNDS);
+        continue;
+      }
+      kout[dst] = sm.key[j];
+      if constexpr (!PAY) rout[dst] = sm.rec[j];
+    }
+    __syncthreads();
+  }
+  if constexpr (PAY) bulk_wait_all();
+}
+
+// ---- 4. each bucket in shared memory
+
+// A CTA's shared memory: the fast form's arrays, or the slower one's keys and places of up to BIG rows.
+template <typename KeyT, int PAY>
+struct LocalShared {
+  uint64_t full;                        // the bucket's records have arrived
+  uint32_t warp[32];
+  uint32_t crowded;
+  union {
+    struct {
+      union {
+        struct {
+          uint32_t start[BINS + 4];     // rows per bin, then where each bin starts
+          uint32_t word[CAP];           // by bin: the row's position below its bin, then its place in the bucket
+        };
+        KeyT key[CAP];                  // in order
+      };
+      uint32_t id[PAY ? 1 : CAP];       // the rows' ids, as they come; then in order
+      uint16_t place[PAY ? CAP : 2];    // in order: the row's place in the bucket
+      alignas(16) uint4 rec[PAY ? CAP : 1];     // the rows' records, as they come
+    };
+    struct {
+      KeyT key[BIG];
+      uint16_t place[BIG];
+    } slow;
+  };
+};
+
+// A bucket of more than CAP rows, or with many equal or very close keys: bitonic sort of (key, row id),
+// the ids of equal keys read where the rows are.
+template <typename KeyT, typename IdOf>
+__device__ __forceinline__ void bitonic_rows(KeyT* key, uint16_t* place, uint32_t size, const KeyT* in, IdOf&& id_of) {
+  uint32_t p = 2;
+  while (p < size) p <<= 1;
+  for (uint32_t i = threadIdx.x; i < p; i += LTHREADS) {
+    key[i] = i < size ? in[i] : KeyT(~KeyT(0));
+    place[i] = uint16_t(i);             // places from `size` on come after every row
+  }
+  __syncthreads();
+  for (uint32_t k = 2; k <= p; k <<= 1) {
+    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+      for (uint32_t q = threadIdx.x; q < p / 2; q += LTHREADS) {
+        const uint32_t i = 2 * q - (q & (j - 1)), l = i + j;
+        const KeyT ki = key[i], kl = key[l];
+        bool less = kl < ki;
+        if (kl == ki) {
+          const uint32_t pi = place[i], pl = place[l];
+          less = pl >= size ? false : pi >= size ? true : id_of(pl) < id_of(pi);
+        }
+        if (less == ((i & k) == 0)) {
+          key[i] = kl;
+          key[l] = ki;
+          const uint16_t pi = place[i];
+          place[i] = place[l];
+          place[l] = pi;
+        }
+      }
+      __syncthreads();
+    }
+  }
+}
+
+// A row leaves: its id, its key as the column's value, its payload.
+template <typename KeyT>
+struct KeyOut {
+  bool xored;                           // an integer key of the key's own width leaves by one XOR
+  KeyT bits;
+  __device__ __forceinline__ explicit KeyOut(const Args& a)
+      : xored(a.key_pt == PT_I64 || a.key_pt == PT_U64 || a.key_pt == PT_I32 || a.key_pt == PT_U32),
+        bits(KeyT(((a.key_pt == PT_I64 || a.key_pt == PT_I32) ? KeyT(KeyT(1) << (8 * sizeof(KeyT) - 1)) : KeyT(0)) ^
+                  (a.key_desc ? KeyT(~KeyT(0)) : KeyT(0)))) {}
+};
+
+template <typename KeyT, int PAY>
+__global__ void __launch_bounds__(LTHREADS, LBLOCKS) bucket_sort_kernel(const __grid_constant__ Args a) {
+  extern __shared__ __align__(16) unsigned char lsm[];
+  using SM = LocalShared<KeyT, PAY>;
+  SM& sm = *reinterpret_cast<SM*>(lsm);
+  const State* st = a.st;
+  if (st->mode != MODE_BUCKETS) return;
+  const uint32_t t = threadIdx.x;
+  const uint32_t nb = st->buckets, src = st->s2 ? 1u : 0u;
+  const uint64_t vbase = a.nulls_first ? uint64_t(st->n_null) + st->n_nan : 0ull;
+  const Map<KeyT> map = load_map<KeyT>(st);
+  const KeyOut<KeyT> ko(a);
+  const int kw = pt_bytes(a.key_pt);
+  constexpr uint32_t SUB = 32 - BINS_LOG;          // position bits below the bin
+  static_assert(CAP <= (1 << BINS_LOG), "a place fits beside the position bits below the bin");
+
+  // The bucket at hand: its rows, its part of the map, and this thread's keys of it (item i is the
+  // bucket's row i x LTHREADS + t; items below nit).
+  uint32_t first = 0, size = 0, meta = 0, f0 = 0;
+  int nit = 0;
+  KeyT key[LITEMS];
+  auto next_bucket = [&](uint32_t b) {             // the next one with rows, from b on
+    for (; b < nb; b += gridDim.x) {
+      first = a.bpos[b];
+      size = a.bpos[b + 1] - first;
+      if (size == 0) continue;
+      meta = a.bmeta[b];
+      f0 = a.bfirst[b];
+      break;
+    }
+    return b;
+  };
+  auto load_rows = [&] {
+    nit = size <= uint32_t(CAP) ? int((size + LTHREADS - 1 - t) / LTHREADS) : 0;
+    const KeyT* kin = static_cast<const KeyT*>(a.keys[src]) + first + t;
+#pragma unroll
+    for (int i = 0; i < LITEMS; i++) {
+      if (i >= nit) break;
+      key[i] = kin[i * LTHREADS];
+    }
+  };
+  auto load_records = [&] {                        // by thread 0, into the free buffer
+    if constexpr (PAY)
+      if (size <= uint32_t(CAP)) bulk_load(sm.rec, a.rec[src] + first, size * 16u, &sm.full);
+  };
+  if (t == 0) {
+    sm.crowded = 0;
+    mbar_init(&sm.full);
+  }
+  for (int x = t; x < BINS; x += LTHREADS) sm.start[x] = 0;
+  __syncthreads();
+  uint32_t b = next_bucket(blockIdx.x), parity = 0;
+  if (b < nb) {
+    load_rows();
+    if (t == 0) load_records();
+  }
+  while (b < nb) {
+    const uint32_t rows = size, row0 = first;
+    const int ni = nit;
+    const KeyT* __restrict__ kin = static_cast<const KeyT*>(a.keys[src]) + row0;
+    const uint32_t* __restrict__ iin = a.ids[src] + row0;
+    const uint4* __restrict__ rin = a.rec[src] + row0;
+    auto id_of = [&](uint32_t p) { return PAY ? rin[p].x : iin[p]; };
+    const uint64_t dst0 = vbase + row0;
+    if (dst0 + rows > a.n || rows > uint32_t(BIG)) {       // the scan rules both out
+      if (t == 0) atomicOr(a.err, ERR_BOUNDS);
+      if (PAY && rows <= uint32_t(CAP)) (void)mbar_wait(&sm.full, parity);
+      break;
+    }
+    // Rows that agree on their positions agree on their keys: no key bits lie below a position's 32.
+    const bool exact = (meta & META_SPLIT) && meta != META_SPLIT && uint32_t(sizeof(KeyT)) * 8u - (f0 >> 16) <= 32u;
+    bool fast = rows <= uint32_t(CAP);
+    uint32_t at[LITEMS];                           // the row's place among its bin's; by bin; in order
+    if (fast) {
+      uint32_t pos[LITEMS];
+      uint32_t id[PAY ? 1 : LITEMS];
+      if constexpr (!PAY) {
+#pragma unroll
+        for (int i = 0; i < LITEMS; i++) {
+          if (i >= ni) break;
+          id[i] = iin[t + i * LTHREADS];
+        }
+      }
+      // A row's position in the bucket's key range, as 32 bits: in a split cell the part of
+      // (position in the cell) x (buckets of the cell) below the bucket number; in a bucket of several
+      // cells, (cell, position in it). Its top bits are the bin.
+      if (meta & META_SPLIT) {
+        const uint32_t sh = f0 >> 16, mul = meta & ~META_SPLIT;     // mul 0: keys outside the sampled range
+        const uint32_t sh0 = sh == 0xFFFFu ? 0u : sh >> 1, sh1 = sh == 0xFFFFu ? 0u : sh - (sh >> 1);
+#pragma unroll
+        for (int i = 0; i < LITEMS; i++) {
+          if (i >= ni) break;
+          const KeyT z = KeyT(KeyT(KeyT(key[i] - map.lo) << sh0) << sh1);      // sh may be the key's width
+          pos[i] = uint32_t(z >> (8 * sizeof(KeyT) - 32)) * mul;
+          at[i] = atomicAdd(&sm.start[pos[i] >> SUB], 1u);
+        }
+      } else {
+        const uint32_t cells = meta - f0 + 1u, k = cells > 1u ? 32u - __clz(cells - 1u) : 0u;
+#pragma unroll
+        for (int i = 0; i < LITEMS; i++) {
+          if (i >= ni) break;
+          uint32_t f, frac;
+          cell_of(map, a.coarse, KeyT(key[i] - map.lo), f, frac);
+          pos[i] = uint32_t(((uint64_t(f - f0) << 32) | frac) >> k);
+          at[i] = atomicAdd(&sm.start[pos[i] >> SUB], 1u);
+        }
+      }
+      __syncthreads();
+      {
+        constexpr int PER = BINS / LTHREADS;
+        static_assert(PER % 4 == 0, "whole vectors of bins a thread");
+        uint4 c[PER / 4];
+        uint32_t sum = 0, mx = 0, all;
+#pragma unroll
+        for (int q = 0; q < PER / 4; q++) {
+          c[q] = *reinterpret_cast<const uint4*>(&sm.start[t * PER + 4 * q]);
+          sum += c[q].x + c[q].y + c[q].z + c[q].w;
+          mx = max(mx, max(max(c[q].x, c[q].y), max(c[q].z, c[q].w)));
+        }
+        if (mx > MAX_BIN) sm.crowded = 1;
+        uint32_t s = block_scan<LTHREADS>(sum, sm.warp, all);
+#pragma unroll
+        for (int q = 0; q < PER / 4; q++) {
+          *reinterpret_cast<uint4*>(&sm.start[t * PER + 4 * q]) =
+              make_uint4(s, s + c[q].x, s + c[q].x + c[q].y, s + c[q].x + c[q].y + c[q].z);
+          s += c[q].x + c[q].y + c[q].z + c[q].w;
+        }
+        if (t == LTHREADS - 1) sm.start[BINS] = rows;
+      }
+      __syncthreads();
+      fast = sm.crowded == 0;
+      if (fast) {
+#pragma unroll
+        for (int i = 0; i < LITEMS; i++) {
+          if (i >= ni) break;
+          const uint32_t s0 = sm.start[pos[i] >> SUB], r = t + i * LTHREADS;
+          sm.word[s0 + at[i]] = (pos[i] << BINS_LOG) | r;
+          if constexpr (!PAY) sm.id[r] = id[i];
+          at[i] = s0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < LITEMS; i++) {
+          if (i >= ni) break;
+          const uint32_t s0 = at[i], s1 = sm.start[(pos[i] >> SUB) + 1];
+          if (s1 - s0 > 1) {
+            // Rows of the bin that come before: by the position bits below the bin; rows that agree on
+            // them too by the whole key, equal keys by row id.
+            const uint32_t me = (pos[i] << BINS_LOG) | (t + i * LTHREADS);
+            uint32_t rank = s0, same = 0;
+#pragma unroll 1
+            for (uint32_t q = s0; q < s1; q++) {
+              const uint32_t o = sm.word[q];
+              rank += o < me ? 1u : 0u;
+              same += (o ^ me) < uint32_t(1 << BINS_LOG) ? 1u : 0u;
+            }
+            if (same > 1) {
+              rank = s0;
+              const uint32_t mine = PAY ? id_of(me & (BINS - 1)) : sm.id[me & (BINS - 1)];
+#pragma unroll 1
+              for (uint32_t q = s0; q < s1; q++) {
+                const uint32_t o = sm.word[q], p = o & (BINS - 1);
+                if ((o ^ me) >= uint32_t(1 << BINS_LOG)) {
+                  rank += o < me ? 1u : 0u;
+                } else {
+                  const KeyT k = exact ? key[i] : kin[p];
+                  rank += k < key[i] || (k == key[i] && (PAY ? id_of(p) : sm.id[p]) < mine) ? 1u : 0u;
+                }
+              }
+            }
+            at[i] = rank;
+          }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < LITEMS; i++) {
+          if (i >= ni) break;
+          sm.key[at[i]] = key[i];
+          if constexpr (PAY) sm.place[at[i]] = uint16_t(t + i * LTHREADS);
+          else sm.id[at[i]] = id[i];
+        }
+      }
+    }
+    // The next bucket's keys arrive while this one leaves.
+    const uint32_t bn = next_bucket(b + gridDim.x);
+    if (bn < nb) load_rows();
+    __syncthreads();
+    if (fast) {
+      if constexpr (!PAY) {
+        if (a.out) {
+          if (a.wide) {
+            uint64_t* o = static_cast<uint64_t*>(a.out) + dst0 + t;
+#pragma unroll
+            for (int i = 0; i < LITEMS; i++) {
+              if (i >= ni) break;
+              o[i * LTHREADS] = sm.id[t + i * LTHREADS];
+            }
+          } else {
+            uint32_t* o = static_cast<uint32_t*>(a.out) + dst0 + t;
+#pragma unroll
+            for (int i = 0; i < LITEMS; i++) {
+              if (i >= ni) break;
+              o[i * LTHREADS] = sm.id[t + i * LTHREADS];
+            }
+          }
+        }
+      }
+      if (a.key_out) {
+        if (ko.xored) {
+          KeyT* o = static_cast<KeyT*>(a.key_out) + dst0 + t;
+#pragma unroll
+          for (int i = 0; i < LITEMS; i++) {
+            if (i >= ni) break;
+            o[i * LTHREADS] = sm.key[t + i * LTHREADS] ^ ko.bits;
+          }
+        } else {
+          for (uint32_t r = t; r < rows; r += LTHREADS)
+            store_width(a.key_out, dst0 + r, kw, unkey_bits<KeyT>(sm.key[r], a.key_pt, a.key_desc));
+        }
+      }
+      if constexpr (PAY) {
+        if (!mbar_wait(&sm.full, parity)) {
+          atomicOr(a.err, ERR_LOOKBACK_TIMEOUT);
+          return;
+        }
+        if (a.pay.pair && !a.out) {
+          uint64_t* w = static_cast<uint64_t*>(a.pay.dst[a.pay.wide]) + dst0 + t;
+          uint32_t* h = static_cast<uint32_t*>(a.pay.dst[a.pay.narrow]) + dst0 + t;
+#pragma unroll
+          for (int i = 0; i < LITEMS; i++) {
+            if (i >= ni) break;
+            const uint4 v = sm.rec[sm.place[t + i * LTHREADS]];
+            w[i * LTHREADS] = uint64_t(v.y) | (uint64_t(v.z) << 32);
+            h[i * LTHREADS] = v.w;
+          }
+        } else {
+          for (uint32_t r = t; r < rows; r += LTHREADS) {
+            const uint4 v = sm.rec[sm.place[r]];
+            store_id(a, dst0 + r, v.x);
+            unpack_record(a.pay, v, dst0 + r);
+          }
+        }
+      }
+    } else {
+      // Records of a crowded bucket are on their way into the memory used here.
+      if constexpr (PAY) {
+        if (rows <= uint32_t(CAP) && !mbar_wait(&sm.full, parity)) {
+          atomicOr(a.err, ERR_LOOKBACK_TIMEOUT);
+          return;
+        }
+        __syncthreads();
+      }
+      bitonic_rows(sm.slow.key, sm.slow.place, rows, kin, id_of);
+      for (uint32_t r = t; r < rows; r += LTHREADS) {
+        const uint32_t p = sm.slow.place[r];
+        store_id(a, dst0 + r, id_of(p));
+        if (a.key_out) store_width(a.key_out, dst0 + r, kw, unkey_bits<KeyT>(sm.slow.key[r], a.key_pt, a.key_desc));
+        if constexpr (PAY) unpack_record(a.pay, rin[p], dst0 + r);
+      }
+      if constexpr (PAY) fence_bulk();
+    }
+    if (PAY && rows <= uint32_t(CAP)) parity ^= 1u;
+    b = bn;
+    __syncthreads();
+    for (int x = t; x < BINS; x += LTHREADS) sm.start[x] = 0;
+    if (t == 0) {
+      sm.crowded = 0;
+      if (b < nb) load_records();
+    }
+    __syncthreads();
+  }
+}
+
+// ---- host side
+
+static uint32_t bucket_cap(uint64_t n) {
+  const uint64_t want = 4 * (n / TARGET) + 256;
+  return uint32_t(std::min<uint64_t>(MAX_BUCKETS, (want + 1023) & ~uint64_t(1023)));
+}
+namespace {
+struct Layout {
+  size_t state, bcount, bmeta, zeroed, coarse, fine, bfirst, bpos, cursor1, cursor2, chunk_bins, chunk_cats, total;
+  explicit Layout(uint64_t n) {
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+      const size_t r = at;
+      at = (at + bytes + 255) & ~size_t(255);
+      return r;
+    };
+    const size_t nb = bucket_cap(n);
+    state = take(sizeof(State));
+    bcount = take(nb * 4);
+    bmeta = take(nb * 4);
+    zeroed = at;
+    coarse = take(COARSE * 4);
+    fine = take(FINE * 4);
+    bfirst = take(nb * 4);
+    bpos = take((nb + 1) * 4);
+    cursor1 = take(size_t(BINS1) * CUR_PAD * 4);
+    cursor2 = take(nb * CUR_PAD * 4);
+    chunk_bins = take(size_t(MAX_CHUNKS) * BINS1 * 4);
+    chunk_cats = take(size_t(MAX_CHUNKS) * 8);
+    total = at;
+  }
+};
+
+template <typename F>
+void smem_limit(F fn, size_t bytes) {
+  AM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+}
+
+template <typename KeyT, int PAY>
+void launch_moves(const ColView& cv, const Args& a, cudaStream_t s) {
+  static std::once_flag once;
+  std::call_once(once, [] {
+    smem_limit(level1_kernel<KeyT, PAY>, sizeof(TileShared<KeyT, PAY>));
+    smem_limit(level2_kernel<KeyT, PAY>, sizeof(Tile2Shared<KeyT, PAY>));
+    smem_limit(bucket_sort_kernel<KeyT, PAY>, sizeof(LocalShared<KeyT, PAY>));
+  });
+  const int sms = device().sm_count;
+  {
+    KernelTimer kt("bucket_level1", s);
+    level1_kernel<KeyT, PAY><<<a.nchunks, THREADS, sizeof(TileShared<KeyT, PAY>), s>>>(cv, a);
+    AM_CUDA(cudaGetLastError());
+  }
+  if (a.bucket_cap > a.bins1_cap) {
+    KernelTimer kt("bucket_level2", s);
+    level2_kernel<KeyT, PAY><<<sms * 2, THREADS, sizeof(Tile2Shared<KeyT, PAY>), s>>>(a);
+    AM_CUDA(cudaGetLastError());
+  }
+  {
+    KernelTimer kt("bucket_sort", s);
+    const int grid = int(std::min<uint32_t>(a.bucket_cap, uint32_t(sms * LBLOCKS)));
+    bucket_sort_kernel<KeyT, PAY><<<grid, LTHREADS, sizeof(LocalShared<KeyT, PAY>), s>>>(a);
+    AM_CUDA(cudaGetLastError());
+  }
+}
+
+template <typename KeyT>
+void launch_all(const Sort& b, const Args& a, int pay, cudaStream_t s) {
+  {
+    KernelTimer kt("bucket_plan", s);
+    buckets_kernel<KeyT><<<CLUSTER, 1024, 0, s>>>(b.col, a);
+    AM_CUDA(cudaGetLastError());
+  }
+  static std::once_flag once;
+  std::call_once(once, [] { smem_limit(bucket_histogram_kernel<KeyT>, size_t(MAX_BUCKETS) * 4); });
+  {
+    KernelTimer kt("bucket_histogram", s);
+    const int grid = int(std::min<uint32_t>(a.nchunks, uint32_t(device().sm_count)));
+    bucket_histogram_kernel<KeyT><<<grid, HTHREADS, size_t(a.bucket_cap) * 4, s>>>(b.col, a);
+    AM_CUDA(cudaGetLastError());
+  }
+  {
+    KernelTimer kt("bucket_scan", s);
+    bucket_starts_kernel<KeyT><<<CLUSTER, 1024, 0, s>>>(a);
+    AM_CUDA(cudaGetLastError());
+  }
+  if (pay) launch_moves<KeyT, 1>(b.col, a, s);
+  else launch_moves<KeyT, 0>(b.col, a, s);
+}
+}  // namespace
+
+size_t scratch_bytes(uint64_t n) { return Layout(n).total; }
+size_t zeroed_bytes(uint64_t n) { return Layout(n).zeroed; }
+
+State* enqueue(const Sort& b, cudaStream_t s) {
+  const Layout L(b.n);
+  auto at = [&](size_t off) { return reinterpret_cast<uint32_t*>(b.scratch + off); };
+  Args a{};
+  a.st = reinterpret_cast<State*>(b.scratch + L.state);
+  a.coarse = at(L.coarse);
+  a.fine = at(L.fine);
+  a.bfirst = at(L.bfirst);
+  a.bmeta = at(L.bmeta);
+  a.bcount = at(L.bcount);
+  a.bpos = at(L.bpos);
+  a.cursor1 = at(L.cursor1);
+  a.cursor2 = at(L.cursor2);
+  a.chunk_bins = at(L.chunk_bins);
+  a.chunk_cats = at(L.chunk_cats);
+  a.nsamples = uint32_t(std::min<uint64_t>(b.n, SAMPLES));
+  a.bucket_cap = bucket_cap(b.n);
+  const uint64_t per = (b.n + MAX_CHUNKS - 1) / MAX_CHUNKS;
+  a.chunk_rows = uint32_t((per + TILE - 1) / TILE * TILE);
+  a.nchunks = uint32_t((b.n + a.chunk_rows - 1) / a.chunk_rows);
+  a.n = b.n;
+  for (int i = 0; i < 2; i++) {
+    a.keys[i] = b.keys[i];
+    a.ids[i] = reinterpret_cast<uint32_t*>(b.ids[i]);
+    a.rec[i] = reinterpret_cast<uint4*>(b.ids[i]);
+  }
+  a.out = b.out;
+  a.wide = b.wide ? 1 : 0;
+  a.key_out = b.key_out;
+  a.key_pt = b.key_pt;
+  a.key_desc = b.key_desc ? 1 : 0;
+  a.nulls_first = b.nulls_first ? 1 : 0;
+  a.err = b.err;
+  a.sum = b.summary;
+  if (b.payload) a.pay = b.rec;
+  const int pay = b.payload ? 1 : 0;
+  a.bins1_cap = b.payload ? BINS1 / 2 : BINS1;
+  if (b.key_bytes == 8) launch_all<uint64_t>(b, a, pay, s);
+  else launch_all<uint32_t>(b, a, pay, s);
+  return a.st;
+}
+
+}  // namespace bs
+}  // namespace am

@@ -1,0 +1,56 @@
+// The bucket sort of one key (bucket_sort.cu): what the radix sort's host side (radix_sort.cu) hands it.
+#pragma once
+
+#include <stdint.h>
+
+#include "radix_sort.cuh"
+
+namespace am {
+namespace bs {
+
+constexpr uint32_t MODE_BUCKETS = 1, MODE_FALLBACK = 2;
+
+// What the sampling, the histogram and the scan decide, read by the kernels after them. All zero when a
+// sort starts.
+struct State {
+  unsigned long long lo, span;           // smallest sampled key, and the largest's distance from it
+  unsigned long long diff;               // bits in which some value key differs from lo
+  uint32_t mode;
+  uint32_t up;                           // (key - lo) << up: the sampled range fills the word
+  uint32_t linear;                       // not 0: the range is cut into this many equal buckets
+  uint32_t buckets, s2, bins1;           // buckets; level 1 sorts by bucket >> s2 into bins1 bins
+  uint32_t n_value, n_null, n_nan;
+  uint32_t max_bucket, pad;
+};
+
+// One bucket sort. `rec` (may be NULL): the payload columns that ride with the rows.
+struct Sort {
+  rs::ColView col;
+  int key_bytes;
+  uint64_t n;
+  char* scratch;                         // `scratch_bytes(n)` bytes, the first `zeroed_bytes(n)` zero
+  void* keys[2];                         // n keys each
+  char* ids[2];                          // n x 4 bytes, or n x 16 with a payload
+  bool payload;
+  rs::RecLayout rec;
+  void* out;                             // the order (NULL: not wanted)
+  bool wide;
+  void* key_out;                         // the sorted key column (NULL: not wanted)
+  int key_pt;
+  bool key_desc, nulls_first;
+  uint32_t* err;
+  rs::SortSummary* summary;
+};
+
+// Rows a bucket sort takes: from one shared-memory sort's worth up to what MAX_BUCKETS buckets hold.
+constexpr uint64_t MIN_ROWS = 4097;
+constexpr uint64_t MAX_ROWS = uint64_t(60) << 20;
+
+size_t scratch_bytes(uint64_t n);
+size_t zeroed_bytes(uint64_t n);
+// Enqueues the sort; afterwards State::mode says whether it ran (MODE_BUCKETS) or its rows are as they
+// were (MODE_FALLBACK: the digit passes must run). Returns the State on the device.
+State* enqueue(const Sort& b, cudaStream_t s);
+
+}  // namespace bs
+}  // namespace am

@@ -28,9 +28,10 @@
 #include <type_traits>
 
 #include "am_internal.h"
-#include "radix_sort.cuh"
+#include "bucket_sort.cuh"
 #include "key_encode.cuh"
-
+#include "radix_sort.cuh"
+#include "records.cuh"
 
 namespace am {
 namespace rs {
@@ -320,7 +321,7 @@ __device__ void plan_body(const PlanArgs& a, KeyStats* __restrict__ st, KeyPlan*
     const uint32_t total = (k == 0) ? st[0].n_value : n;
     if (t == 0) s_max = 0;
     __syncthreads();
-    uint32_t c = st[k].hist[d][t];
+    uint32_t c = t < 256 ? st[k].hist[d][t] : 0u;
     uint32_t m = __reduce_max_sync(0xffffffffu, c);
     if ((t & 31) == 0) atomicMax(&s_max, m);
     __syncthreads();
@@ -405,10 +406,10 @@ __device__ void plan_body(const PlanArgs& a, KeyStats* __restrict__ st, KeyPlan*
       __syncthreads();
       continue;
     }
-    s_vals[t] = st[k].hist[d][t];
+    if (t < 256) s_vals[t] = st[k].hist[d][t];
     __syncthreads();
     block_exclusive_scan_256(s_vals, s_out, &s_total, s_warp);
-    p.bin_base[t] = s_out[t];
+    if (t < 256) p.bin_base[t] = s_out[t];
     if (t == 0) {
       const uint32_t m = st[0].n_value, nn = st[0].n_null, nnan = st[0].n_nan;
       if (k == 0 && a.nulls_first[0]) {
@@ -716,78 +717,11 @@ struct PassShared {
   IdT ids[sizeof(IdT) == 2 ? 1 : TILE];   // row ids (passes that carry them)
 };
 
-// Inverse of the integer and totalOrder key maps (SortSource.swift:131-190 read backwards): the value
-// bits of a key, at the key's width.
-template <typename KeyT>
-__device__ __forceinline__ uint64_t unkey_bits(KeyT k, int pt, int desc) {
-  if (desc) k = KeyT(~k);
-  if constexpr (sizeof(KeyT) == 8) {
-    const uint64_t S = 0x8000000000000000ull;
-    if (pt == PT_I64) return k ^ S;
-    if (pt == PT_F64) return (k & S) ? (k ^ S) : ~k;
-    return k;
-  } else {
-    const uint32_t S = 0x80000000u;
-    if (pt == PT_U32) return k;
-    if (pt == PT_F32) return (k & S) ? (k ^ S) : uint32_t(~k);
-    return uint32_t(k ^ S);          // int32 and the narrow types widened to it (truncated on store)
-  }
-}
-
-__device__ __forceinline__ void store_width(void* base, uint64_t i, int width, uint64_t v) {
-  switch (width) {
-    case 8: static_cast<uint64_t*>(base)[i] = v; break;
-    case 4: static_cast<uint32_t*>(base)[i] = uint32_t(v); break;
-    case 2: static_cast<uint16_t*>(base)[i] = uint16_t(v); break;
-    default: static_cast<uint8_t*>(base)[i] = uint8_t(v); break;
-  }
-}
-// ---- payload records (RecLayout)
-
-__device__ __forceinline__ uint64_t load_width(const void* base, uint64_t i, int width) {
-  switch (width) {
-    case 8: return static_cast<const uint64_t*>(base)[i];
-    case 4: return static_cast<const uint32_t*>(base)[i];
-    case 2: return static_cast<const uint16_t*>(base)[i];
-    default: return static_cast<const uint8_t*>(base)[i];
-  }
-}
-
-// Row `row`'s record: its id and its payload fields read from the columns.
-__device__ __forceinline__ uint4 build_record(const RecLayout& L, uint32_t row) {
-  if (L.pair) {
-    const uint64_t w = static_cast<const uint64_t*>(L.src[L.wide])[row];
-    return make_uint4(row, uint32_t(w), uint32_t(w >> 32), static_cast<const uint32_t*>(L.src[L.narrow])[row]);
-  }
-  uint64_t lo = 0;           // payload bytes 0-7
-  uint32_t hi = 0;           // payload bytes 8-11
-  for (int c = 0; c < L.ncols; c++) {
-    const uint64_t v = load_width(L.src[c], row, L.width[c]);
-    const int o = L.off[c];
-    if (o < 8) lo |= v << (8 * o);
-    else hi |= uint32_t(v) << (8 * (o - 8));
-  }
-  return make_uint4(row, uint32_t(lo), uint32_t(lo >> 32), hi);
-}
-
-// A record's payload fields, written to row `dst` of the sorted payload columns.
-__device__ __forceinline__ void unpack_record(const RecLayout& L, const uint4& r, uint64_t dst) {
-  const uint64_t lo = uint64_t(r.y) | (uint64_t(r.z) << 32);
-  if (L.pair) {
-    static_cast<uint64_t*>(L.dst[L.wide])[dst] = lo;
-    static_cast<uint32_t*>(L.dst[L.narrow])[dst] = r.w;
-    return;
-  }
-  for (int c = 0; c < L.ncols; c++) {
-    const int o = L.off[c];
-    const uint64_t v = o < 8 ? (lo >> (8 * o)) : uint64_t(r.w >> (8 * (o - 8)));
-    store_width(L.dst[c], dst, L.width[c], v);
-  }
-}
-
-template <typename KeyT, typename StatusT, int THREADS, int ITEMS, bool SEG, bool REC = false>
-__global__ void __launch_bounds__(THREADS, 2)
-onesweep_pass_kernel(const __grid_constant__ PassArgs pa, const __grid_constant__ ColView col_arg) {
+// One pass over the tiles, by every block of the launch. `pass_desc`, `tickets` and `epoch` are the
+// pass's own (a launch may run several passes one after the other).
+template <typename KeyT, typename StatusT, int THREADS, int ITEMS, bool SEG, bool REC>
+__device__ __forceinline__ void onesweep_pass(const PassArgs& pa, const ColView& col_arg, const PassDesc* pass_desc,
+                                              uint32_t* tickets, uint32_t epoch) {
   static_assert(THREADS >= NBINS && THREADS % 32 == 0, "one thread per digit bin");
   static_assert(THREADS * ITEMS <= 65536, "tile-local ranks are 16-bit");
   static_assert(!(SEG && REC), "record passes sort one array");
@@ -807,8 +741,9 @@ onesweep_pass_kernel(const __grid_constant__ PassArgs pa, const __grid_constant_
   uint32_t flags = 0, shift = 0, ntiles = 0;
   uint64_t count = 0;
   int si = -1, di = -1;
-  const KeyT* __restrict__ keys_in = nullptr;
-  const uint32_t* __restrict__ ids_in = nullptr;
+  // Not __restrict__: several passes of one launch read what earlier ones wrote.
+  const KeyT* keys_in = nullptr;
+  const uint32_t* ids_in = nullptr;
   KeyT* __restrict__ keys_out = nullptr;
   uint32_t* __restrict__ ids_out = nullptr;
   auto bind = [&](uint64_t row_off) {
@@ -828,19 +763,18 @@ onesweep_pass_kernel(const __grid_constant__ PassArgs pa, const __grid_constant_
   void* final_out = pa.final_out;
   const ColView* colp = &col_arg;
   if constexpr (!SEG) {
-    copy_words(&sm.desc, pa.desc, int(sizeof(PassDesc) / 4));
+    copy_words(&sm.desc, pass_desc, int(sizeof(PassDesc) / 4));
     __syncthreads();
     if (!sm.desc.active) return;
     bind(0);
     kplan = *pa.kplan;
   }
-  const uint32_t epoch = pa.epoch;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t lt_mask = (1u << lane) - 1u;
 
   for (;;) {
     if (threadIdx.x == 0) {
-      const uint32_t t = atomicAdd(pa.tile_counter, 1u);
+      const uint32_t t = atomicAdd(tickets, 1u);
       sm.ticket = t;
       if constexpr (SEG) {
         // The segment of tile t: the last s with tile_start[s] <= t.
@@ -862,7 +796,7 @@ onesweep_pass_kernel(const __grid_constant__ PassArgs pa, const __grid_constant_
     if constexpr (SEG) {
       if (T >= pa.total_tiles) break;
       const uint32_t seg = sm.seg;
-      copy_words(&sm.desc, pa.desc + size_t(seg) * pa.nslots + pa.slot, int(sizeof(PassDesc) / 4));
+      copy_words(&sm.desc, pass_desc + size_t(seg) * pa.nslots + pa.slot, int(sizeof(PassDesc) / 4));
       copy_words(&sm.sdesc, pa.segs + seg, int(sizeof(SegDesc) / 4));
       __syncthreads();
       bind(sm.sdesc.row_off);
@@ -1116,7 +1050,7 @@ onesweep_pass_kernel(const __grid_constant__ PassArgs pa, const __grid_constant_
       // payload columns in the first pass; a row reaching its final place has its record unpacked.
       // Two rows a thread per round, their record loads in flight together (each is a random read
       // within the tile's span, an L2 round trip).
-      const uint4* __restrict__ rin = reinterpret_cast<const uint4*>(ids_in);
+      const uint4* rin = reinterpret_cast<const uint4*>(ids_in);
       uint4* __restrict__ rout = reinterpret_cast<uint4*>(ids_out);
       constexpr int U = 2;
       const bool encode = (flags & PF_ENCODE) != 0;
@@ -1223,6 +1157,83 @@ onesweep_pass_kernel(const __grid_constant__ PassArgs pa, const __grid_constant_
       }
     }
     __syncthreads();
+  }
+}
+
+template <typename KeyT, typename StatusT, int THREADS, int ITEMS, bool SEG, bool REC = false>
+__global__ void __launch_bounds__(THREADS, 2)
+onesweep_pass_kernel(const __grid_constant__ PassArgs pa, const __grid_constant__ ColView col) {
+  onesweep_pass<KeyT, StatusT, THREADS, ITEMS, SEG, REC>(pa, col, pa.desc, pa.tile_counter, pa.epoch);
+}
+
+// ------------------------------------------------------------------------------------------------
+// The digit passes in one launch: the histogram, the plan and every active pass of one key, with a
+// barrier over the grid between them. It follows every bucket sort (bucket_sort.cu) and returns at once
+// unless that found a bucket too large, which only the device knows: one inactive launch costs 2 us
+// where the passes' own 18 would cost 36.
+
+// A barrier over the grid (a cooperative launch: every block is resident). Bounded: false after a
+// second, with the error word set, and the block then leaves.
+__device__ __forceinline__ bool grid_barrier(uint32_t* arrived, uint32_t& round, uint32_t* err) {
+  __shared__ uint32_t s_ok;
+  __syncthreads();
+  round++;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(arrived, 1u);
+    const uint32_t want = round * gridDim.x;
+    const uint64_t t0 = globaltimer_ns();
+    uint32_t ok = 1, polls = 0;
+    while (ld_relaxed_u32(arrived) < want) {
+      __nanosleep(64);
+      if ((++polls & 63u) == 0u && globaltimer_ns() - t0 > LOOKBACK_TIMEOUT_NS) {
+        atomicOr(err, ERR_LOOKBACK_TIMEOUT);
+        ok = 0;
+        break;
+      }
+    }
+    __threadfence();
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0u;
+}
+
+struct AllPassesArgs {
+  PassArgs pass;
+  PlanArgs plan;
+  KeyStats* stats;
+  KeyPlan* kplan;
+  PassDesc* desc;
+  SortSummary* sum;
+  uint32_t* tickets;
+  uint32_t* arrived;
+  const uint32_t* mode;      // bs::MODE_FALLBACK: run
+  uint64_t status16;         // the look-back words, in 16-byte units
+};
+
+template <typename KeyT, int THREADS, int ITEMS, bool REC>
+__global__ void __launch_bounds__(THREADS, 2)
+all_passes_kernel(const __grid_constant__ AllPassesArgs a, const __grid_constant__ ColView col) {
+  if (*a.mode != bs::MODE_FALLBACK) return;
+  uint32_t round = 0;
+  constexpr int HI = 4;
+  constexpr uint64_t CHUNK = uint64_t(THREADS) * HI;
+  histogram_rows<KeyT, THREADS, HI, false>(col, a.stats, uint64_t(blockIdx.x) * CHUNK, a.plan.n, uint64_t(gridDim.x) * CHUNK);
+  if (!grid_barrier(a.arrived, round, a.pass.err)) return;
+  if (blockIdx.x == 0) {
+    plan_body(a.plan, a.stats, a.kplan, a.desc, a.sum);
+    // The sample and the count read the rows before the passes.
+    if (threadIdx.x == 0) a.sum->passes_run += 2;
+  }
+  for (int sl = 0; sl < a.plan.nslots; sl++) {
+    if (!grid_barrier(a.arrived, round, a.pass.err)) return;
+    if (!*reinterpret_cast<const volatile uint32_t*>(&a.desc[sl].active)) continue;
+    uint4* words = static_cast<uint4*>(a.pass.status);
+    for (uint64_t i = uint64_t(blockIdx.x) * THREADS + threadIdx.x; i < a.status16; i += uint64_t(gridDim.x) * THREADS)
+      words[i] = make_uint4(0, 0, 0, 0);
+    if (!grid_barrier(a.arrived, round, a.pass.err)) return;
+    onesweep_pass<KeyT, uint32_t, THREADS, ITEMS, false, REC>(a.pass, col, a.desc + sl, a.tickets + sl, 0u);
   }
 }
 
@@ -1761,6 +1772,7 @@ struct PassConfig;
 template <> struct PassConfig<uint32_t> { static constexpr int THREADS = 512, ITEMS = 10; };
 template <> struct PassConfig<uint64_t> { static constexpr int THREADS = 512, ITEMS = 10; };
 constexpr int HIST_THREADS = 256, HIST_ITEMS = 8;
+constexpr int MAX_ONE_KEY = 8;        // digit passes of one key
 
 template <typename KeyT, int ITEMS = PassConfig<KeyT>::ITEMS, int THREADS = PassConfig<KeyT>::THREADS, bool REC = false>
 static size_t pass_smem() {
@@ -1955,6 +1967,154 @@ bool payload_record_layout(const std::vector<am_array*>& cols, rs::RecLayout* L)
   return true;
 }
 
+// The sorted key column's buffers (a key_dst of a sort by `key` over n rows).
+static void alloc_key_column(am_array* key_dst, const SortKey& key, uint64_t n, cudaStream_t s) {
+  const size_t words = size_t((n + 127) / 128) * 4;
+  key_dst->values = DevBuffer::alloc(n * pt_bytes(key.col->pt) + 16, s);
+  key_dst->last_stream = s;
+  if (key.col->null_count != 0) {
+    key_dst->validity = DevBuffer::alloc(words * 4, s);
+    key_dst->null_count_dev = DevBuffer::alloc(sizeof(unsigned long long), s);
+    // The sorted column has the input's null rows: a known count needs no device round trip.
+    key_dst->null_count = key.col->null_count > 0 ? key.col->null_count : -1;
+  } else {
+    key_dst->null_count = 0;
+  }
+}
+
+// What follows every sort: the sorted key column's validity (one block of nulls at one end), and the
+// counters, which arrive asynchronously (am_last_sort_stats waits for them).
+static void finish_sort(const SortKey& key, uint64_t n, am_array* key_dst, const rs::SortSummary* sum, bool payload,
+                        am_sort_stats* stats, cudaStream_t s) {
+  using namespace rs;
+  const int fin_grid = int(std::min<uint64_t>((n + 8191) / 8192, uint64_t(device().sm_count) * 4));
+  if (key_dst && key_dst->validity) {
+    KernelTimer kt("sort_finish", s);
+    key_validity_kernel<<<std::max(fin_grid, 1), 256, 0, s>>>(sum, key.nulls_first ? 1 : 0,
+                                                            static_cast<uint32_t*>(key_dst->validity->ptr), n,
+                                                            static_cast<unsigned long long*>(key_dst->null_count_dev->ptr));
+    AM_CUDA(cudaGetLastError());
+  }
+  if (key_dst) key_dst->ready = std::make_shared<ReadyEvent>(s);
+  if (stats) {
+    stats->rows = int64_t(n);
+    stats->payload_in_records = payload ? 1 : 0;
+    AM_CUDA(cudaMemcpyAsync(last_summary_host(), sum, sizeof(SortSummary), cudaMemcpyDeviceToHost, s));
+    tls().stats_stream = s;
+  }
+}
+
+template <typename KeyT, bool REC>
+static void launch_all_passes(const rs::AllPassesArgs& a, const rs::ColView& cv, uint64_t n, cudaStream_t s) {
+  using namespace rs;
+  using C = PassConfig<KeyT>;
+  auto fn = all_passes_kernel<KeyT, C::THREADS, C::ITEMS, REC>;
+  const size_t smem = pass_smem<KeyT, C::ITEMS, C::THREADS, REC>();
+  static int blocks = 0;
+  static std::once_flag once;
+  std::call_once(once, [&] {
+    AM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    int b = 0;
+    AM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, C::THREADS, smem));
+    blocks = b;
+  });
+  if (blocks < 1) throw Error("radix sort: the digit passes do not fit the device");
+  const uint64_t tiles = (n + uint64_t(C::THREADS) * C::ITEMS - 1) / (uint64_t(C::THREADS) * C::ITEMS);
+  const int grid = int(std::min<uint64_t>(tiles, uint64_t(device().sm_count) * blocks));
+  KernelTimer kt("radix_all_passes", s);
+  void* args[] = {const_cast<AllPassesArgs*>(&a), const_cast<ColView*>(&cv)};
+  AM_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(fn), dim3(uint32_t(grid)), dim3(C::THREADS), args, smem, s));
+}
+
+// One key sorted by buckets (bucket_sort.cu), or, when the device finds a bucket too large, by the digit
+// passes in one launch.
+static void sort_by_buckets(const SortKey& key, const rs::PlanArgs& pa, uint64_t n, int kb, void* out, int index_width,
+                            am_array* key_dst, const rs::RecLayout* payload, bool carry_ids, cudaStream_t s,
+                            am_sort_stats* stats) {
+  using namespace rs;
+  auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
+  // Zeroed: the digit passes' state and the bucket sort's own; then its tables, then the rows' buffers.
+  const size_t off_kplan = sizeof(KeyStats);
+  const size_t off_desc = up(off_kplan + sizeof(KeyPlan));
+  const size_t off_tick = up(off_desc + sizeof(PassDesc) * MAX_ONE_KEY);
+  const size_t off_sum = off_tick + sizeof(uint32_t) * (MAX_ONE_KEY + 4);
+  const size_t off_bs = up(off_sum + sizeof(SortSummary));
+  const size_t off_keys = up(off_bs + bs::scratch_bytes(n));
+  const size_t kbuf = up(n * size_t(kb));
+  const size_t ibuf = up(payload ? n * sizeof(uint4) : n * sizeof(uint32_t));
+  ScratchBlock scratch(s, off_keys + 2 * kbuf + 2 * ibuf);
+  char* base = scratch.data();
+  AM_CUDA(cudaMemsetAsync(base, 0, off_bs + bs::zeroed_bytes(n), s));
+  if (key_dst) alloc_key_column(key_dst, key, n, s);
+  const uint64_t tile = min_super();
+  const uint64_t tiles = (n + tile - 1) / tile;
+  StreamScratch& sc = stream_scratch(s, size_t(tiles) * NBINS);
+  SortSummary* sum = reinterpret_cast<SortSummary*>(base + off_sum);
+
+  bs::Sort b{};
+  b.col = make_view(key);
+  b.key_bytes = kb;
+  b.n = n;
+  b.scratch = base + off_bs;
+  b.payload = payload != nullptr;
+  if (payload) b.rec = *payload;
+  b.out = out;
+  b.wide = index_width == 8;
+  for (int i = 0; i < 2; i++) {
+    b.keys[i] = base + off_keys + size_t(i) * kbuf;
+    b.ids[i] = base + off_keys + 2 * kbuf + size_t(i) * ibuf;
+  }
+  if (key_dst) b.key_out = key_dst->values->ptr;
+  b.key_pt = key.col->pt;
+  b.key_desc = key.descending;
+  b.nulls_first = key.nulls_first;
+  b.err = sc.err;
+  b.summary = sum;
+  const bs::State* st = bs::enqueue(b, s);
+
+  AllPassesArgs a{};
+  PassArgs& p = a.pass;
+  for (int i = 0; i < 2; i++) {
+    p.keys[i] = b.keys[i];
+    p.ids[i] = reinterpret_cast<uint32_t*>(b.ids[i]);
+  }
+  a.kplan = reinterpret_cast<KeyPlan*>(base + off_kplan);
+  p.kplan = a.kplan;
+  p.final_out = out;
+  p.status = sc.status;
+  p.err = sc.err;
+  p.carry_ids = carry_ids ? 1 : 0;
+  if (key_dst) {
+    p.key_out_mode = KEY_OUT_UNKEY;
+    p.key_out_pt = key.col->pt;
+    p.key_desc = key.descending ? 1 : 0;
+    p.key_float_order = key.float_order;
+    p.key_out = key_dst->values->ptr;
+  }
+  if (payload) {
+    p.rec_mode = 1;
+    p.rec = *payload;
+  }
+  a.plan = pa;
+  a.stats = reinterpret_cast<KeyStats*>(base);
+  a.desc = reinterpret_cast<PassDesc*>(base + off_desc);
+  a.sum = sum;
+  a.tickets = reinterpret_cast<uint32_t*>(base + off_tick);
+  a.arrived = a.tickets + MAX_ONE_KEY;
+  a.mode = &st->mode;
+  a.status16 = (tiles * NBINS * sizeof(uint32_t) + 15) / 16;
+  // The passes use the stream's look-back words with no epoch: later 64-bit users start over.
+  sc.epoch = (1u << 30) - 1;
+  if (kb == 8) {
+    if (payload) launch_all_passes<uint64_t, true>(a, b.col, n, s);
+    else launch_all_passes<uint64_t, false>(a, b.col, n, s);
+  } else {
+    if (payload) launch_all_passes<uint32_t, true>(a, b.col, n, s);
+    else launch_all_passes<uint32_t, false>(a, b.col, n, s);
+  }
+  finish_sort(key, n, key_dst, sum, payload != nullptr, stats, s);
+}
+
 void radix_argsort(const std::vector<SortKey>& keys, int64_t n, void* out, int index_width, cudaStream_t s,
                    am_sort_stats* stats) {
   radix_sort(keys, n, out, index_width, nullptr, s, stats);
@@ -2025,6 +2185,12 @@ void radix_sort(const std::vector<SortKey>& keys_in, int64_t n64, void* out, int
   int max_kb = 4;
   for (auto& k : keys) max_kb = std::max(max_kb, pt_key_bytes(k.col->pt));
 
+  // One key of a size that buckets serve: the bucket sort, with the digit passes behind it.
+  if (K == 1 && n >= bs::MIN_ROWS && n <= bs::MAX_ROWS && !debug_skip_first_tile()) {
+    sort_by_buckets(keys[0], pa, n, max_kb, out, index_width, key_dst, payload, carry_ids, s, stats);
+    return;
+  }
+
   // Per-call scratch: stats, plans, pass descriptors, tickets, summary (one memset), then the
   // ping-pong key and id buffers.
   // A single 8-byte key over at least 2^21 rows may take the two-level sort (the device decides).
@@ -2060,19 +2226,7 @@ void radix_sort(const std::vector<SortKey>& keys_in, int64_t n64, void* out, int
   void* kbufB = base + header + kbuf;
   uint32_t* ibufA = carry_ids ? reinterpret_cast<uint32_t*>(base + header + 2 * kbuf) : nullptr;
   uint32_t* ibufB = carry_ids ? reinterpret_cast<uint32_t*>(base + header + 2 * kbuf + ibuf) : nullptr;
-  if (key_dst) {
-    const size_t words = size_t((n + 127) / 128) * 4;
-    key_dst->values = DevBuffer::alloc(n * pt_bytes(keys[0].col->pt) + 16, s);
-    key_dst->last_stream = s;
-    if (keys[0].col->null_count != 0) {
-      key_dst->validity = DevBuffer::alloc(words * 4, s);
-      key_dst->null_count_dev = DevBuffer::alloc(sizeof(unsigned long long), s);
-      // The sorted column has the input's null rows: a known count needs no device round trip.
-      key_dst->null_count = keys[0].col->null_count > 0 ? keys[0].col->null_count : -1;
-    } else {
-      key_dst->null_count = 0;
-    }
-  }
+  if (key_dst) alloc_key_column(key_dst, keys[0], n, s);
   if (debug_skip_first_tile()) {
     // Test hook: every pass's ticket starts at 1, so tile 0 is never processed and the look-back of
     // tile 1 runs into its time limit.
@@ -2208,23 +2362,7 @@ void radix_sort(const std::vector<SortKey>& keys_in, int64_t n64, void* out, int
       else launch_pass<uint32_t, uint64_t>(a, cv, n, s);
     }
   }
-  // The sorted key column's validity: one block of nulls at one end.
-  const int fin_grid = int(std::min<uint64_t>((n + 8191) / 8192, uint64_t(device().sm_count) * 4));
-  if (key_dst && key_dst->validity) {
-    KernelTimer kt("sort_finish", s);
-    key_validity_kernel<<<std::max(fin_grid, 1), 256, 0, s>>>(sum, keys[0].nulls_first ? 1 : 0,
-                                                            static_cast<uint32_t*>(key_dst->validity->ptr), n,
-                                                            static_cast<unsigned long long*>(key_dst->null_count_dev->ptr));
-    AM_CUDA(cudaGetLastError());
-  }
-  if (key_dst) key_dst->ready = std::make_shared<ReadyEvent>(s);
-  if (stats) {
-    // Counters arrive asynchronously; am_last_sort_stats waits for them.
-    stats->rows = int64_t(n);
-    stats->payload_in_records = payload ? 1 : 0;
-    AM_CUDA(cudaMemcpyAsync(last_summary_host(), sum, sizeof(SortSummary), cudaMemcpyDeviceToHost, s));
-    tls().stats_stream = s;
-  }
+  finish_sort(keys[0], n, key_dst, sum, payload != nullptr, stats, s);
 }
 
 

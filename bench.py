@@ -751,7 +751,9 @@ def algorithmic_bytes(n, m, passes, local_sort=False, records=False):
       each value row's key and record (24 B) and each null row's key value and payload (8 + 12 B);
     - a middle pass reads and writes 24 B a value row;
     - the local sorts (or the last pass) read 24 B a value row and write its key value and payload
-      (8 + 12 B)."""
+      (8 + 12 B).
+
+    The bucket sort (bucket_* kernels) moves the same bytes as a histogram, two passes and local sorts."""
     src = 8 * n + n / 8
     if records:
         first = src + 12 * n + 24 * m + 20 * (n - m)
@@ -762,7 +764,8 @@ def algorithmic_bytes(n, m, passes, local_sort=False, records=False):
             pass_bytes = first + (passes - 1) * 48 * m
         else:
             pass_bytes = first + (passes - 2) * 48 * m + last
-        out = {"radix_histogram": src, "radix_onesweep_pass": pass_bytes, "sort_finish": n / 8}
+        out = {"radix_histogram": src, "radix_onesweep_pass": pass_bytes, "sort_finish": n / 8,
+               "bucket_histogram": src, "bucket_level1": first, "bucket_level2": 48 * m, "bucket_sort": last}
         if local_sort:
             out["radix_local_sort"] = last
         return out
@@ -772,7 +775,9 @@ def algorithmic_bytes(n, m, passes, local_sort=False, records=False):
         first = src + 12 * m + 12 * (n - m)
         pass_bytes = first + (passes - 2) * 24 * m + 24 * m
     out = {"radix_histogram": src, "radix_onesweep_pass": pass_bytes,
-           "take_gather": 4 * n + 2 * (8 + 4) * n, "sort_finish": n / 8}
+           "take_gather": 4 * n + 2 * (8 + 4) * n, "sort_finish": n / 8,
+           "bucket_histogram": src, "bucket_level1": src + 12 * m + 12 * (n - m), "bucket_level2": 24 * m,
+           "bucket_sort": 24 * m}
     if local_sort:
         out["radix_local_sort"] = 24 * m
     return out

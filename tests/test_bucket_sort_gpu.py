@@ -1,0 +1,99 @@
+"""The bucket sort of one key (bucket_sort.cu) where it can go wrong: the smallest column it takes, rows
+around a tile and around the sample size, one and two levels of bins, both key widths, keys spread
+evenly (equal cuts) and unevenly (cells), buckets of one repeated key (the slow form, and the digit
+passes when none can hold it), and null and NaN rows; each against the oracle's stable order, with and
+without payload columns beside the key."""
+import numpy as np
+import pyarrow as pa
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+TILE = 512 * 7
+CASES = [(4097, "even"), (TILE * 2 - 1, "normal"), (TILE * 2 + 1, "normal32"), (65535, "even32"), (65536, "normal"),
+         (65537, "repeats"), (200_003, "clusters"), (700_001, "even"), (1_500_000, "normal32"), (1_500_001, "repeats"),
+         (3_000_017, "normal"), (3_000_017, "one_value"), (5_000_011, "even"), (2_000_003, "narrow"), (2_000_003, "exponential")]
+
+
+def keys(kind, n, rng):
+    if kind == "even":
+        return rng.integers(0, 2**40, n, dtype=np.int64)
+    if kind == "even32":
+        return rng.integers(-2**31, 2**31, n).astype(np.int32)
+    if kind in ("normal", "normal32"):
+        v = rng.standard_normal(n).astype(np.float32 if kind == "normal32" else np.float64)
+        v[rng.random(n) < 0.01] = np.nan
+        v[rng.random(n) < 0.0005] = -0.0
+        v[rng.random(n) < 0.0005] = 0.0
+        return v
+    if kind == "repeats":                       # 3,000 rows a value: more than the fast form takes
+        return rng.integers(0, max(2, n // 3000), n).astype(np.int64) * 7919
+    if kind == "clusters":                      # a few values repeated about a thousand times among others
+        v = rng.integers(0, 2**50, n, dtype=np.int64)
+        hit = rng.random(n) < 0.2
+        v[hit] = rng.integers(0, 40, int(hit.sum())) * 2**43 + 5
+        return v
+    if kind == "one_value":                     # no bucket holds it: the digit passes
+        v = rng.integers(0, 2**40, n, dtype=np.int64)
+        v[rng.random(n) < 0.3] = 123_456_789_012
+        return v
+    if kind == "narrow":
+        return rng.integers(-100, 100, n).astype(np.int16)
+    return (rng.exponential(1e5, n)).astype(np.int64)
+
+
+@pytest.mark.parametrize("n,kind", CASES)
+def test_against_the_oracle(am, oracle, n, kind):
+    rng = np.random.default_rng(n + len(kind))
+    v = keys(kind, n, rng)
+    for nulls, desc, place, order in ((0.0, False, "at_end", "ieee"), (0.1, True, "at_start", "nan_largest"),
+                                      (0.3, False, "at_start", "ieee"), (0.02, True, "at_end", "total")):
+        arr = pa.array(v, mask=rng.random(n) < nulls if nulls else None, from_pandas=False)
+        want = oracle.argsort(arr, desc, place, order, threads=4)
+        m = am.MetalArray.from_arrow(arr)
+        assert np.array_equal(m.argsort(desc, place, order).to_arrow().to_numpy(), want)
+        assert np.array_equal(m.argsort64(desc, place, order).to_arrow().to_numpy(), want)
+        p1, p2 = rng.standard_normal(n), rng.integers(-2**31, 2**31, n).astype(np.int32)
+        src = am.PlanSource("t", {"k": m, "a": pa.array(p1), "b": pa.array(p2)})
+        by = [["k", desc, {"nulls": "first" if place == "at_start" else "last", "float_order": order}]]
+        out = am.run_plan({"op": "sort", "by": by, "input": {"op": "scan", "source": "t"}}, [src])
+        assert np.array_equal(out["a"].to_arrow().to_numpy(), p1[want])
+        assert np.array_equal(out["b"].to_arrow().to_numpy(), p2[want])
+        got, sorted_copy, exp = out["k"].to_arrow(), m.sort(desc, place, order).to_arrow(), arr.take(pa.array(want))
+        valid = np.asarray(exp.is_valid())
+        width = arr.type.bit_width // 8
+        bits = [np.frombuffer(a.buffers()[1], np.uint8, n * width).reshape(n, width)[valid] for a in (got, sorted_copy, exp)]
+        assert np.array_equal(np.asarray(got.is_valid()), valid) and np.array_equal(np.asarray(sorted_copy.is_valid()), valid)
+        assert np.array_equal(bits[0], bits[2]) and np.array_equal(bits[1], bits[2])
+
+
+@pytest.mark.parametrize("offset", [1, 32, 37])
+def test_sliced_columns(am, oracle, offset):
+    # A validity bitmap that starts inside a word, and values off their alignment.
+    rng = np.random.default_rng(offset)
+    base = pa.array(rng.integers(0, 2**40, 100_000), mask=rng.random(100_000) < 0.2)
+    part = base.slice(offset, 90_001)
+    m = am.MetalArray.from_arrow(base).slice(offset, 90_001)
+    assert np.array_equal(m.argsort().to_arrow().to_numpy(), oracle.argsort(part))
+
+
+def test_concurrent_threads(am, oracle):
+    # Each thread sorts on its own stream, with its own scratch.
+    import threading
+    rng = np.random.default_rng(3)
+    arrays = [pa.array(rng.standard_normal(300_000 + 1000 * i)) for i in range(4)]
+    want = [oracle.argsort(a) for a in arrays]
+    bad = []
+
+    def work(i):
+        m = am.MetalArray.from_arrow(arrays[i])
+        for _ in range(20):
+            if not np.array_equal(m.argsort().to_arrow().to_numpy(), want[i]):
+                bad.append(i)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
