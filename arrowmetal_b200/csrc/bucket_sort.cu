@@ -53,6 +53,7 @@ constexpr int BIG = 4096;                         // rows its slower form takes
 constexpr uint32_t TARGET = 1300;                 // rows a bucket is meant to hold
 constexpr uint32_t SAMPLES = 65536;               // keys looked at (every key of a shorter column)
 constexpr int CLUSTER = 8;                        // CTAs of the one-cluster kernels
+constexpr uint32_t ONE_CAP = 1024;                // buckets of a column of at most SAMPLES rows
 constexpr int BINS = 2048, BINS_LOG = 11;         // bins of the shared-memory sort
 constexpr uint32_t MAX_BIN = 32;                  // rows a bin may hold for the comparisons
 constexpr uint32_t META_SPLIT = 0x80000000u;
@@ -71,7 +72,8 @@ struct Args {
   uint32_t* ids[2];
   uint4* rec[2];                                  // with a payload: row id and payload fields (RecLayout), instead of ids
   void *out, *key_out;
-  int32_t wide, key_pt, key_desc, nulls_first;
+  int32_t wide, key_pt, key_desc, nulls_first, has_payload;
+  int32_t one_launch;                             // the plan's launch counts and moves the rows too
   uint32_t* err;
   SortSummary* sum;
   RecLayout pay;
@@ -229,6 +231,12 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* s_warp, uin
   return x - v + __reduce_add_sync(0xffffffffu, lane < warp ? c : 0u);
 }
 
+__device__ __forceinline__ void store_id(const Args& a, uint64_t dst, uint32_t id) {
+  if (!a.out) return;
+  if (a.wide) static_cast<uint64_t*>(a.out)[dst] = id;
+  else static_cast<uint32_t*>(a.out)[dst] = id;
+}
+
 // ---- bulk copies between shared and global memory (addresses and sizes multiples of 16 bytes)
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
@@ -274,171 +282,35 @@ struct PlanShared {
   uint32_t group[1024];
   unsigned long long smax[CLUSTER], smin[CLUSTER], scnt[CLUSTER];
   unsigned long long wmax[32], wmin[32];
+  uint32_t mode, buckets, linear;        // the plan, from the first CTA
+  // One launch for the counts and the moves too (columns of at most SAMPLES rows): the fine cells, the
+  // CTA's rows of each bucket, where they go, its null and NaN rows by item and warp, and their sums.
+  uint32_t fine[FINE];
+  uint32_t bins[ONE_CAP], start[ONE_CAP];
+  uint32_t cats[2][SAMPLES / (1024 * CLUSTER) * 32];
+  uint32_t ncats[2];
+  unsigned long long diff;
 };
 
-template <typename KeyT>
-__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(1024)
-buckets_kernel(const __grid_constant__ ColView col, const __grid_constant__ Args a) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cl = cg::this_cluster();
-  __shared__ PlanShared sm;
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const uint32_t rank = cl.block_rank();
+__device__ __forceinline__ void tell_plan(const Args& a, unsigned long long lo, unsigned long long span, uint32_t up,
+                                          uint32_t buckets, uint32_t linear) {
   State* st = a.st;
-  cl.sync();                             // every CTA runs before its shared memory is written
-  // The sample: one row of each nsamples-th part of the column, at a mixed offset (no period of the data
-  // lines up), or every row. nsamples is SAMPLES or the rows.
-  constexpr int U = SAMPLES / (1024 * CLUSTER);
-  KeyT key[U];
-  uint32_t live = 0;
-  const bool full = a.nsamples == a.n;
-#pragma unroll
-  for (int u = 0; u < U; u++) {
-    const uint32_t j = (rank * U + u) * 1024 + t;
-    key[u] = 0;
-    if (j < a.nsamples) {
-      uint64_t row = j;
-      if (!full) {
-        const uint64_t lo = uint64_t(j) * a.n / SAMPLES, hi = uint64_t(j + 1) * a.n / SAMPLES;
-        uint32_t h = j * 2654435761u;
-        h ^= h >> 15;
-        h *= 2246822519u;
-        h ^= h >> 13;
-        row = lo + __umulhi(h, uint32_t(hi - lo));
-      }
-      const bool valid = !col.valid || bit_at(col.valid, col.valid_off + int64_t(row));
-      int cat;
-      key[u] = key_from_raw<KeyT>(col, load_raw<KeyT>(col, row), valid, cat);
-      if (cat == 0) live |= 1u << u;
-    }
-  }
-  for (int i = t; i < COARSE; i += 1024) sm.coarse_cnt[i] = 0;
-  for (int i = t; i < 2 * FINE; i += 1024) sm.half_cnt[i] = 0;
-  // The sampled range, over the cluster.
-  {
-    uint64_t mx = 0, mn = 0;
-#pragma unroll
-    for (int u = 0; u < U; u++)
-      if ((live >> u) & 1u) {
-        mx = max(mx, uint64_t(key[u]));
-        mn = max(mn, ~uint64_t(key[u]));
-      }
-    mx = warp_max_u64(mx);
-    mn = warp_max_u64(mn);
-    const uint32_t c = __reduce_add_sync(0xffffffffu, __popc(live));
-    if (lane == 0) {
-      sm.wmax[warp] = mx;
-      sm.wmin[warp] = mn;
-      sm.warp[warp] = c;
-    }
-    __syncthreads();
-    if (warp == 0) {
-      const uint64_t bx = warp_max_u64(sm.wmax[lane]), bn = warp_max_u64(sm.wmin[lane]);
-      const uint32_t bc = __reduce_add_sync(0xffffffffu, sm.warp[lane]);
-      if (lane < CLUSTER) {
-        PlanShared* o = cl.map_shared_rank(&sm, lane);
-        o->smax[rank] = bx;
-        o->smin[rank] = bn;
-        o->scnt[rank] = bc;
-      }
-    }
-  }
-  cl.sync();
-  uint64_t vmax = 0, vmin_inv = 0;
-  uint32_t sv = 0;
-#pragma unroll
-  for (int r = 0; r < CLUSTER; r++) {
-    vmax = max(vmax, uint64_t(sm.smax[r]));
-    vmin_inv = max(vmin_inv, uint64_t(sm.smin[r]));
-    sv += uint32_t(sm.scnt[r]);
-  }
-  const unsigned long long lo = sv ? ~vmin_inv : 0ull, span = sv ? vmax - lo : 0ull;
-  const int bits = max(COARSE_BITS, span ? 64 - __clzll((long long)span) : 0);
-  const uint32_t shc = uint32_t(bits - COARSE_BITS);        // key bits below a coarse cell
-  const Map<KeyT> map{KeyT(lo), KeyT(span), uint32_t(sizeof(KeyT)) * 8u - uint32_t(bits), 0u, 0u};
-#pragma unroll
-  for (int u = 0; u < U; u++)
-    if ((live >> u) & 1u) atomicAdd(&sm.coarse_cnt[uint32_t(KeyT(key[u] - map.lo) >> shc)], 1u);
-  cl.sync();
-  uint32_t in_cell = 0;                  // the sample's keys in coarse cell t
-  if (t < COARSE) {
-#pragma unroll
-    for (int r = 0; r < CLUSTER; r++) in_cell += cl.map_shared_rank(&sm, r)->coarse_cnt[t];
-  }
-  // Evenly spread keys (every coarse cell's count within 4.5 deviations of its width's share) need no
-  // tables: equal cuts of the range, filled to TARGET rows (a deviation the test cannot see still
-  // fits CAP).
-  {
-    uint32_t off = 0;
-    if (t < COARSE) {
-      const unsigned long long c0 = (unsigned long long)t << shc, w = 1ull << shc;
-      const float keys_in = c0 > span ? 0.0f : span - c0 >= w ? float(w) : float(span - c0) + 1.0f;
-      const float e = float(sv) * keys_in / (float(span) + 1.0f);
-      off = fabsf(float(in_cell) - e) > 4.5f * sqrtf(e) + 3.0f ? 1u : 0u;
-    }
-    const bool even = !__syncthreads_or(int(off)) && sv >= 16u * COARSE && shc > 0;
-    if (even) {
-      const float est = float(a.n) * float(sv) / float(a.nsamples);
-      const float range = bits == 64 ? 18446744073709551616.0f : float(1ull << bits);
-      const uint32_t cuts = uint32_t(ceilf(est / float(TARGET) * (range / (float(span) + 1.0f))));
-      const uint32_t top = uint32_t(KeyT(KeyT(span) << map.up) >> (8 * sizeof(KeyT) - 32));
-      const uint32_t nb = __umulhi(top, cuts) + 3u;
-      if (nb <= a.bucket_cap) {
-        for (uint32_t b = rank * 1024 + t; b < nb; b += 1024 * CLUSTER) {
-          const bool outer = b == 0 || b == nb - 1;
-          a.bmeta[b] = META_SPLIT | (outer ? 0u : cuts);
-          a.bfirst[b] = (outer ? 0xFFFFu : map.up) << 16;
-        }
-        if (t == 0 && rank == 0) {
-          st->lo = lo;
-          st->span = span;
-          st->up = map.up;
-          st->linear = cuts;
-          st->buckets = nb;
-          st->s2 = nb <= a.bins1_cap ? 0u : uint32_t(S2);
-          st->bins1 = nb <= a.bins1_cap ? nb : (nb + BINS2 - 1) >> S2;
-          st->mode = MODE_BUCKETS;
-        }
-        cl.sync();                       // no CTA leaves while another reads its counts
-        return;
-      }
-    }
-  }
-  // Fine cells of each coarse cell: 2^fb, from its share of the sample (about FINE_GOAL cells over the
-  // column, fewer when the sample is small: at least 24 sampled rows a cell on average).
-  const uint32_t goal = min(uint32_t(FINE_GOAL), max(1u, sv / 24u));
-  uint32_t fb = 0, width = 0;
-  if (t < COARSE) {
-    const uint32_t want = sv ? uint32_t(uint64_t(in_cell) * goal / sv) : 0u;
-    fb = want > 1u ? 32u - __clz(want - 1u) : 0u;
-    fb = min(fb, min(uint32_t(FINE_BITS), shc));
-    width = 1u << fb;
-  }
-  uint32_t nfine;
-  const uint32_t fbase = block_scan<1024>(width, sm.warp, nfine);
-  if (t < COARSE) {
-    sm.coarse[t] = fbase | (fb << 16);
-    if (rank == 0) a.coarse[t] = sm.coarse[t];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int u = 0; u < U; u++)
-    if ((live >> u) & 1u) {
-      uint32_t f, frac;
-      cell_of(map, sm.coarse, KeyT(key[u] - map.lo), f, frac);
-      atomicAdd(&sm.half_cnt[2 * f + (frac >> 31)], 1u);
-    }
-  cl.sync();
-  if (rank == 0) {
-    for (int i = t; i < 2 * FINE; i += 1024) {
-      uint32_t c = sm.half_cnt[i];
-#pragma unroll
-      for (int r = 1; r < CLUSTER; r++) c += cl.map_shared_rank(&sm, r)->half_cnt[i];
-      sm.half_cnt[i] = c;
-    }
-  }
-  cl.sync();
-  if (rank != 0) return;
+  st->lo = lo;
+  st->span = span;
+  st->up = up;
+  st->linear = linear;
+  st->buckets = buckets;
+  st->s2 = buckets <= a.bins1_cap ? 0u : uint32_t(S2);
+  st->bins1 = buckets <= a.bins1_cap ? buckets : (buckets + BINS2 - 1) >> S2;
+  st->mode = MODE_BUCKETS;
+}
+
+// The first CTA, with the cluster's counts of the half cells: buckets from the fine cells' rows.
+template <typename KeyT>
+__device__ void plan_cells(const Args& a, PlanShared& sm, const Map<KeyT>& map, unsigned long long lo, unsigned long long span,
+                           uint32_t shc, uint32_t sv, uint32_t nfine, bool full) {
+  const int t = threadIdx.x;
+  State* st = a.st;
   const uint32_t* coarse = sm.coarse;
   // Rows of each fine cell, at the upper end of what the sample says; single-key cells (nothing left to
   // split) that surely exceed a bucket end the attempt here.
@@ -512,7 +384,10 @@ buckets_kernel(const __grid_constant__ ColView col, const __grid_constant__ Args
     target += target / 4;
   }
   if (bad || total + 2 > a.bucket_cap || sv == 0) {
-    if (t == 0) st->mode = MODE_FALLBACK;
+    if (t == 0) {
+      st->mode = MODE_FALLBACK;
+      sm.mode = MODE_FALLBACK;
+    }
     return;
   }
   // The tables. Bucket 0 and the last take the keys outside the sampled range.
@@ -522,6 +397,7 @@ buckets_kernel(const __grid_constant__ ColView col, const __grid_constant__ Args
     if (f >= nfine) continue;
     const uint32_t b = 1u + base[q] - (start[q] ? 0u : 1u);
     a.fine[f] = b | (m[q] << 16);
+    sm.fine[f] = b | (m[q] << 16);
     if (rows[q] > target / 2) {
       for (uint32_t k = 0; k < m[q]; k++) {
         a.bfirst[b + k] = below[q] << 16;
@@ -538,14 +414,299 @@ buckets_kernel(const __grid_constant__ ColView col, const __grid_constant__ Args
     a.bmeta[nb - 1] = META_SPLIT;
     a.bfirst[0] = 0xFFFF0000u;
     a.bfirst[nb - 1] = 0xFFFF0000u;
-    st->lo = lo;
-    st->span = span;
-    st->up = map.up;
-    st->buckets = nb;
-    st->s2 = nb <= a.bins1_cap ? 0u : uint32_t(S2);
-    st->bins1 = nb <= a.bins1_cap ? nb : (nb + BINS2 - 1) >> S2;
-    st->mode = MODE_BUCKETS;
+    sm.buckets = nb;
+    sm.mode = MODE_BUCKETS;
+    tell_plan(a, lo, span, map.up, nb, 0u);
   }
+}
+
+template <typename KeyT>
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(1024)
+buckets_kernel(const __grid_constant__ ColView col, const __grid_constant__ Args a) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ PlanShared sm;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const uint32_t rank = cl.block_rank();
+  State* st = a.st;
+  cl.sync();                             // every CTA runs before its shared memory is written
+  // The sample: one row of each nsamples-th part of the column, at a mixed offset (no period of the data
+  // lines up), or every row. nsamples is SAMPLES or the rows.
+  constexpr int U = SAMPLES / (1024 * CLUSTER);
+  KeyT key[U];
+  uint32_t live = 0, nulls = 0, nans = 0;
+  const bool full = a.nsamples == a.n;
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const uint32_t j = (rank * U + u) * 1024 + t;
+    key[u] = 0;
+    if (j < a.nsamples) {
+      uint64_t row = j;
+      if (!full) {
+        const uint64_t lo = uint64_t(j) * a.n / SAMPLES, hi = uint64_t(j + 1) * a.n / SAMPLES;
+        uint32_t h = j * 2654435761u;
+        h ^= h >> 15;
+        h *= 2246822519u;
+        h ^= h >> 13;
+        row = lo + __umulhi(h, uint32_t(hi - lo));
+      }
+      const bool valid = !col.valid || bit_at(col.valid, col.valid_off + int64_t(row));
+      int cat;
+      key[u] = key_from_raw<KeyT>(col, load_raw<KeyT>(col, row), valid, cat);
+      if (cat == 0) live |= 1u << u;
+      else if (cat == 1) nans |= 1u << u;
+      else nulls |= 1u << u;
+    }
+  }
+  for (int i = t; i < COARSE; i += 1024) sm.coarse_cnt[i] = 0;
+  for (int i = t; i < 2 * FINE; i += 1024) sm.half_cnt[i] = 0;
+  // The sampled range, over the cluster.
+  {
+    uint64_t mx = 0, mn = 0;
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if ((live >> u) & 1u) {
+        mx = max(mx, uint64_t(key[u]));
+        mn = max(mn, ~uint64_t(key[u]));
+      }
+    mx = warp_max_u64(mx);
+    mn = warp_max_u64(mn);
+    const uint32_t c = __reduce_add_sync(0xffffffffu, __popc(live));
+    if (lane == 0) {
+      sm.wmax[warp] = mx;
+      sm.wmin[warp] = mn;
+      sm.warp[warp] = c;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const uint64_t bx = warp_max_u64(sm.wmax[lane]), bn = warp_max_u64(sm.wmin[lane]);
+      const uint32_t bc = __reduce_add_sync(0xffffffffu, sm.warp[lane]);
+      if (lane < CLUSTER) {
+        PlanShared* o = cl.map_shared_rank(&sm, lane);
+        o->smax[rank] = bx;
+        o->smin[rank] = bn;
+        o->scnt[rank] = bc;
+      }
+    }
+  }
+  cl.sync();
+  uint64_t vmax = 0, vmin_inv = 0;
+  uint32_t sv = 0;
+#pragma unroll
+  for (int r = 0; r < CLUSTER; r++) {
+    vmax = max(vmax, uint64_t(sm.smax[r]));
+    vmin_inv = max(vmin_inv, uint64_t(sm.smin[r]));
+    sv += uint32_t(sm.scnt[r]);
+  }
+  const unsigned long long lo = sv ? ~vmin_inv : 0ull, span = sv ? vmax - lo : 0ull;
+  const int bits = max(COARSE_BITS, span ? 64 - __clzll((long long)span) : 0);
+  const uint32_t shc = uint32_t(bits - COARSE_BITS);        // key bits below a coarse cell
+  const Map<KeyT> map{KeyT(lo), KeyT(span), uint32_t(sizeof(KeyT)) * 8u - uint32_t(bits), 0u, 0u};
+#pragma unroll
+  for (int u = 0; u < U; u++)
+    if ((live >> u) & 1u) atomicAdd(&sm.coarse_cnt[uint32_t(KeyT(key[u] - map.lo) >> shc)], 1u);
+  cl.sync();
+  uint32_t in_cell = 0;                  // the sample's keys in coarse cell t
+  if (t < COARSE) {
+#pragma unroll
+    for (int r = 0; r < CLUSTER; r++) in_cell += cl.map_shared_rank(&sm, r)->coarse_cnt[t];
+  }
+  bool planned = false;
+  if (t == 0) sm.linear = 0;
+  // Evenly spread keys (every coarse cell's count within 4.5 deviations of its width's share) need no
+  // tables: equal cuts of the range, filled to TARGET rows (a deviation the test cannot see still
+  // fits CAP).
+  {
+    uint32_t off = 0;
+    if (t < COARSE) {
+      const unsigned long long c0 = (unsigned long long)t << shc, w = 1ull << shc;
+      const float keys_in = c0 > span ? 0.0f : span - c0 >= w ? float(w) : float(span - c0) + 1.0f;
+      const float e = float(sv) * keys_in / (float(span) + 1.0f);
+      off = fabsf(float(in_cell) - e) > 4.5f * sqrtf(e) + 3.0f ? 1u : 0u;
+    }
+    const bool even = !__syncthreads_or(int(off)) && sv >= 16u * COARSE && shc > 0;
+    if (even) {
+      const float est = float(a.n) * float(sv) / float(a.nsamples);
+      const float range = bits == 64 ? 18446744073709551616.0f : float(1ull << bits);
+      const uint32_t cuts = uint32_t(ceilf(est / float(TARGET) * (range / (float(span) + 1.0f))));
+      const uint32_t top = uint32_t(KeyT(KeyT(span) << map.up) >> (8 * sizeof(KeyT) - 32));
+      const uint32_t nb = __umulhi(top, cuts) + 3u;
+      if (nb <= a.bucket_cap) {
+        for (uint32_t b = rank * 1024 + t; b < nb; b += 1024 * CLUSTER) {
+          const bool outer = b == 0 || b == nb - 1;
+          a.bmeta[b] = META_SPLIT | (outer ? 0u : cuts);
+          a.bfirst[b] = (outer ? 0xFFFFu : map.up) << 16;
+        }
+        if (t == 0 && rank == 0) {
+          sm.linear = cuts;
+          sm.buckets = nb;
+          sm.mode = MODE_BUCKETS;
+          tell_plan(a, lo, span, map.up, nb, cuts);
+        }
+        planned = true;
+      }
+    }
+  }
+  if (!planned) {
+    // Fine cells of each coarse cell: 2^fb, from its share of the sample (about FINE_GOAL cells over the
+    // column, fewer when the sample is small: at least 24 sampled rows a cell on average).
+    const uint32_t goal = min(uint32_t(FINE_GOAL), max(1u, sv / 24u));
+    uint32_t fb = 0, width = 0;
+    if (t < COARSE) {
+      const uint32_t want = sv ? uint32_t(uint64_t(in_cell) * goal / sv) : 0u;
+      fb = want > 1u ? 32u - __clz(want - 1u) : 0u;
+      fb = min(fb, min(uint32_t(FINE_BITS), shc));
+      width = 1u << fb;
+    }
+    uint32_t nfine;
+    const uint32_t fbase = block_scan<1024>(width, sm.warp, nfine);
+    if (t < COARSE) {
+      sm.coarse[t] = fbase | (fb << 16);
+      if (rank == 0) a.coarse[t] = sm.coarse[t];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if ((live >> u) & 1u) {
+        uint32_t f, frac;
+        cell_of(map, sm.coarse, KeyT(key[u] - map.lo), f, frac);
+        atomicAdd(&sm.half_cnt[2 * f + (frac >> 31)], 1u);
+      }
+    cl.sync();
+    if (rank == 0) {
+      for (int i = t; i < 2 * FINE; i += 1024) {
+        uint32_t c = sm.half_cnt[i];
+#pragma unroll
+        for (int r = 1; r < CLUSTER; r++) c += cl.map_shared_rank(&sm, r)->half_cnt[i];
+        sm.half_cnt[i] = c;
+      }
+    }
+    if (rank == 0) {
+      __syncthreads();
+      plan_cells<KeyT>(a, sm, map, lo, span, shc, sv, nfine, full);
+    }
+  }
+  cl.sync();                             // no CTA leaves, or goes on, before the plan stands
+  if (!a.one_launch) return;
+
+  // ---- a column of at most SAMPLES rows, every one of them in the cluster's registers: its counts and
+  // moves too, without the launches of steps 2 and 3.
+  const PlanShared* p0 = cl.map_shared_rank(&sm, 0);
+  const uint32_t nb = p0->buckets, linear = p0->linear;
+  bool go = p0->mode == MODE_BUCKETS;
+  if (go && !linear)
+    for (int i = t; i < FINE; i += 1024) sm.fine[i] = rank == 0 ? sm.fine[i] : p0->fine[i];
+  if (t < int(ONE_CAP)) sm.bins[t] = 0;
+  if (t == 0) sm.diff = 0;
+  __syncthreads();
+  const Map<KeyT> all{KeyT(lo), KeyT(span), map.up, nb - 1, linear};
+  uint32_t slot[U];                      // bucket << 16 | place among the CTA's rows of it
+  KeyT diff = 0;
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const bool is = (live >> u) & 1u;
+    if (go && is) {
+      const uint32_t b = bucket_of(all, sm.coarse, sm.fine, key[u]);
+      slot[u] = (b << 16) | atomicAdd(&sm.bins[b], 1u);
+      diff |= key[u] ^ KeyT(lo);
+    }
+    const uint32_t wn = __popc(__ballot_sync(0xffffffffu, (nulls >> u) & 1u));
+    const uint32_t wx = __popc(__ballot_sync(0xffffffffu, (nans >> u) & 1u));
+    if (lane == 0) {
+      sm.cats[0][u * 32 + warp] = wn;
+      sm.cats[1][u * 32 + warp] = wx;
+    }
+  }
+  diff = warp_or<KeyT>(diff);
+  if (lane == 0 && diff) atomicOr(&sm.diff, (unsigned long long)diff);
+  __syncthreads();
+  // Null and NaN rows before each (item, warp) of the CTA: rows in order, items first.
+  uint32_t n_null, n_nan;
+  const uint32_t mine_null = t < U * 32 ? sm.cats[0][t] : 0u, mine_nan = t < U * 32 ? sm.cats[1][t] : 0u;
+  const uint32_t before_null = block_scan<1024>(mine_null, sm.warp, n_null);
+  const uint32_t before_nan = block_scan<1024>(mine_nan, sm.warp, n_nan);
+  if (t < U * 32) {
+    sm.cats[0][t] = before_null;
+    sm.cats[1][t] = before_nan;
+  }
+  if (t == 0) {
+    sm.ncats[0] = n_null;
+    sm.ncats[1] = n_nan;
+  }
+  cl.sync();
+  uint32_t rows = 0, ahead = 0, null_at = 0, nan_at = 0, nn = 0, nx = 0;
+  unsigned long long dall = 0;
+  for (int r = 0; r < CLUSTER; r++) {
+    const PlanShared* o = cl.map_shared_rank(&sm, r);
+    const uint32_t c = t < int(ONE_CAP) ? o->bins[t] : 0u;
+    if (uint32_t(r) < rank) ahead += c;
+    rows += c;
+    const uint32_t cn = o->ncats[0], cx = o->ncats[1];
+    if (uint32_t(r) < rank) {
+      null_at += cn;
+      nan_at += cx;
+    }
+    nn += cn;
+    nx += cx;
+    dall |= o->diff;
+  }
+  uint32_t values;
+  const uint32_t at = block_scan<1024>(rows, sm.warp, values);
+  sm.start[t] = at + ahead;
+  const uint32_t over = __syncthreads_or(int(rows > uint32_t(BIG)));
+  go = go && !over;
+  if (rank == 0) {
+    if (go && uint32_t(t) < nb) a.bpos[t] = at;
+    if (t == 0) {
+      st->n_value = values;
+      st->n_null = nn;
+      st->n_nan = nx;
+      if (go) {
+        a.bpos[nb] = values;
+        uint32_t active = 0;
+        for (uint32_t d = 0; d < sizeof(KeyT); d++) active += (dall >> (8 * d)) & 255u ? 1u : 0u;
+        a.sum->value_rows = values;
+        a.sum->null_rows = nn;
+        a.sum->nan_rows = nx;
+        a.sum->passes_run = max(1u, active);
+        a.sum->passes_total = uint32_t(sizeof(KeyT));
+      } else {
+        st->mode = MODE_FALLBACK;
+      }
+    }
+  }
+  if (go) {
+    null_at += a.nulls_first ? 0u : values + nx;
+    nan_at += a.nulls_first ? nn : values;
+    const uint32_t lt = (1u << lane) - 1u;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const uint32_t row = (rank * U + u) * 1024 + t;
+      const bool isn = (nulls >> u) & 1u, isx = (nans >> u) & 1u;
+      const uint32_t bn = __ballot_sync(0xffffffffu, isn), bx = __ballot_sync(0xffffffffu, isx);
+      if ((live >> u) & 1u) {
+        const uint32_t dst = sm.start[slot[u] >> 16] + (slot[u] & 0xFFFFu);
+        if (dst < values) {
+          static_cast<KeyT*>(a.keys[0])[dst] = key[u];
+          if (a.has_payload) a.rec[0][dst] = build_record(a.pay, row);
+          else a.ids[0][dst] = row;
+        } else {
+          atomicOr(a.err, ERR_BOUNDS);
+        }
+      } else if (isn || isx) {
+        const uint32_t dst = isn ? null_at + sm.cats[0][u * 32 + warp] + __popc(bn & lt)
+                                 : nan_at + sm.cats[1][u * 32 + warp] + __popc(bx & lt);
+        if (dst < a.n) {
+          store_id(a, dst, row);
+          if (a.has_payload) unpack_record(a.pay, build_record(a.pay, row), dst);
+          if (a.key_out) store_width(a.key_out, dst, pt_bytes(a.key_pt), 0ull);
+        } else {
+          atomicOr(a.err, ERR_BOUNDS);
+        }
+      }
+    }
+  }
+  cl.sync();                             // no CTA leaves while another reads its counts
 }
 
 // ---- 2. exact counts
@@ -745,12 +906,6 @@ struct TileShared {
   // Per staged row: its bin, and without records (which hold the row id) its place in the tile below it.
   std::conditional_t<PAY != 0, uint16_t, uint32_t> word[TILE];
 };
-
-__device__ __forceinline__ void store_id(const Args& a, uint64_t dst, uint32_t id) {
-  if (!a.out) return;
-  if (a.wide) static_cast<uint64_t*>(a.out)[dst] = id;
-  else static_cast<uint32_t*>(a.out)[dst] = id;
-}
 
 template <typename KeyT, int PAY>
 __global__ void __launch_bounds__(THREADS, 2) level1_kernel(const __grid_constant__ ColView col,
@@ -1373,9 +1528,6 @@ __global__ void __launch_bounds__(LTHREADS, LBLOCKS) bucket_sort_kernel(const __
             if (i >= ni) break;
             o[i * LTHREADS] = sm.key[t + i * LTHREADS] ^ ko.bits;
           }
-        } else {
-          for (uint32_t r = t; r < rows; r += LTHREADS)
-            store_width(a.key_out, dst0 + r, kw, unkey_bits<KeyT>(sm.key[r], a.key_pt, a.key_desc));
         }
       }
       if constexpr (PAY) {
@@ -1383,6 +1535,14 @@ __global__ void __launch_bounds__(LTHREADS, LBLOCKS) bucket_sort_kernel(const __
           atomicOr(a.err, ERR_LOOKBACK_TIMEOUT);
           return;
         }
+      }
+      if (a.key_out && !ko.xored) {
+        for (uint32_t r = t; r < rows; r += LTHREADS) {
+          const KeyT k = sm.key[r];
+          store_width(a.key_out, dst0 + r, kw, unkey_bits<KeyT>(k, a.key_pt, a.key_desc));
+        }
+      }
+      if constexpr (PAY) {
         if (a.pay.pair && !a.out) {
           uint64_t* w = static_cast<uint64_t*>(a.pay.dst[a.pay.wide]) + dst0 + t;
           uint32_t* h = static_cast<uint32_t*>(a.pay.dst[a.pay.narrow]) + dst0 + t;
@@ -1413,8 +1573,9 @@ __global__ void __launch_bounds__(LTHREADS, LBLOCKS) bucket_sort_kernel(const __
       bitonic_rows(sm.slow.key, sm.slow.place, rows, kin, id_of);
       for (uint32_t r = t; r < rows; r += LTHREADS) {
         const uint32_t p = sm.slow.place[r];
+        const KeyT k = sm.slow.key[r];
         store_id(a, dst0 + r, id_of(p));
-        if (a.key_out) store_width(a.key_out, dst0 + r, kw, unkey_bits<KeyT>(sm.slow.key[r], a.key_pt, a.key_desc));
+        if (a.key_out) store_width(a.key_out, dst0 + r, kw, unkey_bits<KeyT>(k, a.key_pt, a.key_desc));
         if constexpr (PAY) unpack_record(a.pay, rin[p], dst0 + r);
       }
       if constexpr (PAY) fence_bulk();
@@ -1478,15 +1639,17 @@ void launch_moves(const ColView& cv, const Args& a, cudaStream_t s) {
     smem_limit(bucket_sort_kernel<KeyT, PAY>, sizeof(LocalShared<KeyT, PAY>));
   });
   const int sms = device().sm_count;
-  {
-    KernelTimer kt("bucket_level1", s);
-    level1_kernel<KeyT, PAY><<<a.nchunks, THREADS, sizeof(TileShared<KeyT, PAY>), s>>>(cv, a);
-    AM_CUDA(cudaGetLastError());
-  }
-  if (a.bucket_cap > a.bins1_cap) {
-    KernelTimer kt("bucket_level2", s);
-    level2_kernel<KeyT, PAY><<<sms * 2, THREADS, sizeof(Tile2Shared<KeyT, PAY>), s>>>(a);
-    AM_CUDA(cudaGetLastError());
+  if (!a.one_launch) {
+    {
+      KernelTimer kt("bucket_level1", s);
+      level1_kernel<KeyT, PAY><<<a.nchunks, THREADS, sizeof(TileShared<KeyT, PAY>), s>>>(cv, a);
+      AM_CUDA(cudaGetLastError());
+    }
+    if (a.bucket_cap > a.bins1_cap) {
+      KernelTimer kt("bucket_level2", s);
+      level2_kernel<KeyT, PAY><<<sms * 2, THREADS, sizeof(Tile2Shared<KeyT, PAY>), s>>>(a);
+      AM_CUDA(cudaGetLastError());
+    }
   }
   {
     KernelTimer kt("bucket_sort", s);
@@ -1503,18 +1666,20 @@ void launch_all(const Sort& b, const Args& a, int pay, cudaStream_t s) {
     buckets_kernel<KeyT><<<CLUSTER, 1024, 0, s>>>(b.col, a);
     AM_CUDA(cudaGetLastError());
   }
-  static std::once_flag once;
-  std::call_once(once, [] { smem_limit(bucket_histogram_kernel<KeyT>, size_t(MAX_BUCKETS) * 4); });
-  {
-    KernelTimer kt("bucket_histogram", s);
-    const int grid = int(std::min<uint32_t>(a.nchunks, uint32_t(device().sm_count)));
-    bucket_histogram_kernel<KeyT><<<grid, HTHREADS, size_t(a.bucket_cap) * 4, s>>>(b.col, a);
-    AM_CUDA(cudaGetLastError());
-  }
-  {
-    KernelTimer kt("bucket_scan", s);
-    bucket_starts_kernel<KeyT><<<CLUSTER, 1024, 0, s>>>(a);
-    AM_CUDA(cudaGetLastError());
+  if (!a.one_launch) {
+    static std::once_flag once;
+    std::call_once(once, [] { smem_limit(bucket_histogram_kernel<KeyT>, size_t(MAX_BUCKETS) * 4); });
+    {
+      KernelTimer kt("bucket_histogram", s);
+      const int grid = int(std::min<uint32_t>(a.nchunks, uint32_t(device().sm_count)));
+      bucket_histogram_kernel<KeyT><<<grid, HTHREADS, size_t(a.bucket_cap) * 4, s>>>(b.col, a);
+      AM_CUDA(cudaGetLastError());
+    }
+    {
+      KernelTimer kt("bucket_scan", s);
+      bucket_starts_kernel<KeyT><<<CLUSTER, 1024, 0, s>>>(a);
+      AM_CUDA(cudaGetLastError());
+    }
   }
   if (pay) launch_moves<KeyT, 1>(b.col, a, s);
   else launch_moves<KeyT, 0>(b.col, a, s);
@@ -1561,6 +1726,12 @@ State* enqueue(const Sort& b, cudaStream_t s) {
   if (b.payload) a.pay = b.rec;
   const int pay = b.payload ? 1 : 0;
   a.bins1_cap = b.payload ? BINS1 / 2 : BINS1;
+  a.has_payload = b.payload ? 1 : 0;
+  a.one_launch = b.n <= SAMPLES ? 1 : 0;
+  if (a.one_launch) {
+    a.bucket_cap = std::min(a.bucket_cap, ONE_CAP);
+    a.bins1_cap = ONE_CAP;
+  }
   if (b.key_bytes == 8) launch_all<uint64_t>(b, a, pay, s);
   else launch_all<uint32_t>(b, a, pay, s);
   return a.st;

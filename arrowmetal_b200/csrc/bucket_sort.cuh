@@ -42,8 +42,7 @@ struct Sort {
   rs::SortSummary* summary;
 };
 
-// Rows a bucket sort takes: from one shared-memory sort's worth up to what MAX_BUCKETS buckets hold.
-constexpr uint64_t MIN_ROWS = 4097;
+// Rows a bucket sort takes: up to what MAX_BUCKETS buckets hold.
 constexpr uint64_t MAX_ROWS = uint64_t(60) << 20;
 
 size_t scratch_bytes(uint64_t n);

@@ -2186,7 +2186,7 @@ void radix_sort(const std::vector<SortKey>& keys_in, int64_t n64, void* out, int
   for (auto& k : keys) max_kb = std::max(max_kb, pt_key_bytes(k.col->pt));
 
   // One key of a size that buckets serve: the bucket sort, with the digit passes behind it.
-  if (K == 1 && n >= bs::MIN_ROWS && n <= bs::MAX_ROWS && !debug_skip_first_tile()) {
+  if (K == 1 && n <= bs::MAX_ROWS && !debug_skip_first_tile()) {
     sort_by_buckets(keys[0], pa, n, max_kb, out, index_width, key_dst, payload, carry_ids, s, stats);
     return;
   }

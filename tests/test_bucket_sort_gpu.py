@@ -1,5 +1,5 @@
-"""The bucket sort of one key (bucket_sort.cu) where it can go wrong: the smallest column it takes, rows
-around a tile and around the sample size, one and two levels of bins, both key widths, keys spread
+"""The bucket sort of one key (bucket_sort.cu) where it can go wrong: the smallest columns, rows around a
+tile and around the sample size (up to which one launch plans, counts and moves), one and two levels of bins, both key widths, keys spread
 evenly (equal cuts) and unevenly (cells), buckets of one repeated key (the slow form, and the digit
 passes when none can hold it), and null and NaN rows; each against the oracle's stable order, with and
 without payload columns beside the key."""
@@ -10,7 +10,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 TILE = 512 * 7
-CASES = [(4097, "even"), (TILE * 2 - 1, "normal"), (TILE * 2 + 1, "normal32"), (65535, "even32"), (65536, "normal"),
+CASES = [(1, "even"), (33, "normal"), (2003, "even"), (2048, "repeats"), (4097, "even"), (TILE * 2 - 1, "normal"), (TILE * 2 + 1, "normal32"), (65535, "even32"), (65536, "normal"),
          (65537, "repeats"), (200_003, "clusters"), (700_001, "even"), (1_500_000, "normal32"), (1_500_001, "repeats"),
          (3_000_017, "normal"), (3_000_017, "one_value"), (5_000_011, "even"), (2_000_003, "narrow"), (2_000_003, "exponential")]
 
