@@ -929,7 +929,7 @@ int am_sort_ex2(am_array* a, int descending, int null_placement, int float_order
     k[0] = SortKey{a, descending != 0, null_placement == 1, float_order};
     // A key map that is a bijection: the sorted column is rebuilt from the sorted keys, no gather
     // (the reference's sortedByInvertingKeys, Sources/ArrowMetal/Kernels/Sort.swift:509-619).
-    if (a->length > 0 && float_order_ok(float_order) >= 0 && key_invertible(k[0])) {
+    if (a->length > 0 && float_order_ok(float_order) >= 0 && key_rebuildable(k[0])) {
       check_index_rows(a->length, "sort");
       cudaStream_t s = stream();
       use_on(a, s);

@@ -289,8 +289,11 @@ am_array* radix_top_k(const SortKey& key, int64_t k, cudaStream_t s);
 am_array* low_cardinality_ranks(const SortKey& k, cudaStream_t s);
 // True when the key column can be rebuilt from its sorted keys (the key map is a bijection).
 bool key_invertible(const SortKey& k);
+// True when a sort can write the sorted key column beside the order: an invertible key, or a float key
+// whose order ties values (the bucket sort reads those few, and the null rows, from the column).
+bool key_rebuildable(const SortKey& k);
 // The sort engine. `out` (may be NULL) receives the index array; `key_dst` (may be NULL; one
-// key_invertible key only) receives the sorted key column, rebuilt from the sorted keys by the last
+// key_rebuildable key only) receives the sorted key column, rebuilt from the sorted keys by the last
 // pass, so a sorted copy of the key needs no gather. `payload` (may be NULL; one key only): payload
 // columns carried through the sort in row records and written, sorted, to their destinations.
 void radix_sort(const std::vector<SortKey>& keys, int64_t n, void* out, int index_width, am_array* key_dst,

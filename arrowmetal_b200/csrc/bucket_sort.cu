@@ -72,6 +72,8 @@ struct Args {
   uint32_t* ids[2];
   uint4* rec[2];                                  // with a payload: row id and payload fields (RecLayout), instead of ids
   void *out, *key_out;
+  const void* key_src;                            // not NULL: keys that stand for several values are read here
+  unsigned long long twin0, twin1;                // those keys: a zero's, a NaN's
   int32_t wide, key_pt, key_desc, nulls_first, has_payload;
   int32_t one_launch;                             // the plan's launch counts and moves the rows too
   uint32_t* err;
@@ -235,6 +237,11 @@ __device__ __forceinline__ void store_id(const Args& a, uint64_t dst, uint32_t i
   if (!a.out) return;
   if (a.wide) static_cast<uint64_t*>(a.out)[dst] = id;
   else static_cast<uint32_t*>(a.out)[dst] = id;
+}
+
+// The key column's bits at a row, where a row's key does not give them (0 where null rows are written as 0).
+__device__ __forceinline__ uint64_t source_bits(const Args& a, uint32_t row) {
+  return a.key_src ? load_width(a.key_src, row, pt_bytes(a.key_pt)) : 0ull;
 }
 
 // ---- bulk copies between shared and global memory (addresses and sizes multiples of 16 bytes)
@@ -699,7 +706,7 @@ buckets_kernel(const __grid_constant__ ColView col, const __grid_constant__ Args
         if (dst < a.n) {
           store_id(a, dst, row);
           if (a.has_payload) unpack_record(a.pay, build_record(a.pay, row), dst);
-          if (a.key_out) store_width(a.key_out, dst, pt_bytes(a.key_pt), 0ull);
+          if (a.key_out) store_width(a.key_out, dst, pt_bytes(a.key_pt), source_bits(a, row));
         } else {
           atomicOr(a.err, ERR_BOUNDS);
         }
@@ -1087,7 +1094,7 @@ __global__ void __launch_bounds__(THREADS, 2) level1_kernel(const __grid_constan
       }
       store_id(a, dst, row);
       if constexpr (PAY) unpack_record(a.pay, build_record(a.pay, row), dst);
-      if (a.key_out) store_width(a.key_out, dst, pt_bytes(a.key_pt), 0ull);
+      if (a.key_out) store_width(a.key_out, dst, pt_bytes(a.key_pt), source_bits(a, row));
     }
     null_at += tn;
     nan_at += tx;
@@ -1539,7 +1546,14 @@ __global__ void __launch_bounds__(LTHREADS, LBLOCKS) bucket_sort_kernel(const __
       if (a.key_out && !ko.xored) {
         for (uint32_t r = t; r < rows; r += LTHREADS) {
           const KeyT k = sm.key[r];
-          store_width(a.key_out, dst0 + r, kw, unkey_bits<KeyT>(k, a.key_pt, a.key_desc));
+          uint64_t v = unkey_bits<KeyT>(k, a.key_pt, a.key_desc);
+          if (a.key_src && (k == KeyT(a.twin0) || k == KeyT(a.twin1))) {
+            uint32_t id;
+            if constexpr (PAY) id = sm.rec[sm.place[r]].x;
+            else id = sm.id[r];
+            v = source_bits(a, id);
+          }
+          store_width(a.key_out, dst0 + r, kw, v);
         }
       }
       if constexpr (PAY) {
@@ -1575,7 +1589,9 @@ __global__ void __launch_bounds__(LTHREADS, LBLOCKS) bucket_sort_kernel(const __
         const uint32_t p = sm.slow.place[r];
         const KeyT k = sm.slow.key[r];
         store_id(a, dst0 + r, id_of(p));
-        if (a.key_out) store_width(a.key_out, dst0 + r, kw, unkey_bits<KeyT>(k, a.key_pt, a.key_desc));
+        if (a.key_out)
+          store_width(a.key_out, dst0 + r, kw, a.key_src && (k == KeyT(a.twin0) || k == KeyT(a.twin1))
+                                                   ? source_bits(a, id_of(p)) : unkey_bits<KeyT>(k, a.key_pt, a.key_desc));
         if constexpr (PAY) unpack_record(a.pay, rin[p], dst0 + r);
       }
       if constexpr (PAY) fence_bulk();
@@ -1719,6 +1735,14 @@ State* enqueue(const Sort& b, cudaStream_t s) {
   a.wide = b.wide ? 1 : 0;
   a.key_out = b.key_out;
   a.key_pt = b.key_pt;
+  if (b.key_source) {
+    // Keys of both zeros, and of every NaN: a column's own bits are read back for them.
+    const bool wide = b.key_bytes == 8;
+    const unsigned long long flip = b.key_desc ? ~0ull : 0ull, sign = wide ? 1ull << 63 : 1ull << 31;
+    a.key_src = b.col.values;
+    a.twin0 = sign ^ flip;
+    a.twin1 = (sign | (wide ? 0x7FF0000000000001ull : 0x7F800001ull)) ^ flip;
+  }
   a.key_desc = b.key_desc ? 1 : 0;
   a.nulls_first = b.nulls_first ? 1 : 0;
   a.err = b.err;

@@ -37,6 +37,7 @@ struct Sort {
   bool wide;
   void* key_out;                         // the sorted key column (NULL: not wanted)
   int key_pt;
+  bool key_source;                       // a float order that ties values: null rows, zeros and NaNs keep their own bits
   bool key_desc, nulls_first;
   uint32_t* err;
   rs::SortSummary* summary;

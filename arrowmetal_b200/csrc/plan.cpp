@@ -211,7 +211,7 @@ Frame sort_frame(Frame f, const std::vector<KeySpec>& keys) {
   if (keys.size() == 1 && !f.perm && f.rows > 0) {
     SortKey key{f.cols[size_t(which[0])], keys[0].desc, keys[0].nulls_first, keys[0].float_order};
     if (key.float_order < 0 || key.float_order > 2) throw invalid("unknown float_order " + std::to_string(key.float_order));
-    if (key_invertible(key)) {
+    if (key_rebuildable(key)) {
       check_index_rows(f.rows, "sort");
       cudaStream_t s = stream();
       use_on(key.col, s);

@@ -1096,6 +1096,8 @@ __device__ __forceinline__ void onesweep_pass(const PassArgs& pa, const ColView&
           if (pa.key_out_mode == KEY_OUT_UNKEY)
             store_width(pa.key_out, dst, pt_bytes(pa.key_out_pt),
                         d < RADIX ? unkey_bits<KeyT>(sm.keys[j], pa.key_out_pt, pa.key_desc) : 0ull);
+          else if (pa.key_out_mode == KEY_OUT_SOURCE)
+            store_width(pa.key_out, dst, pt_bytes(pa.key_out_pt), load_width(col.values, r[u].x, pt_bytes(pa.key_out_pt)));
         }
       }
     } else if (merged) {
@@ -1127,7 +1129,7 @@ __device__ __forceinline__ void onesweep_pass(const PassArgs& pa, const ColView&
     }
     // The sorted key column: value rows from their keys in the last pass, null rows (first pass of the
     // most significant key) as zero. Record passes write it in their own loop, beside the payload.
-    if (!REC && pa.key_out_mode == KEY_OUT_UNKEY && (last || (flags & PF_ROUTE))) {
+    if (!REC && pa.key_out_mode != KEY_OUT_NONE && (last || (flags & PF_ROUTE))) {
       const int kw = pt_bytes(pa.key_out_pt);
       for (uint32_t j = threadIdx.x; j < tile_n; j += THREADS) {
         const uint32_t d = dig_at(j);
@@ -1135,7 +1137,9 @@ __device__ __forceinline__ void onesweep_pass(const PassArgs& pa, const ColView&
         uint32_t dst = sm.gdelta[d] + j;
         if (d < RADIX) dst += sm.desc.value_base;
         if (dst >= out_rows) { atomicOr(pa.err, ERR_BOUNDS); continue; }
-        const uint64_t v = d < RADIX ? unkey_bits<KeyT>(sm.keys[j], pa.key_out_pt, pa.key_desc) : 0ull;
+        uint64_t v;
+        if (pa.key_out_mode == KEY_OUT_SOURCE) v = load_width(col.values, sm.ids[REC ? 0 : j], kw);
+        else v = d < RADIX ? unkey_bits<KeyT>(sm.keys[j], pa.key_out_pt, pa.key_desc) : 0ull;
         store_width(pa.key_out, dst, kw, v);
       }
     }
@@ -1933,6 +1937,12 @@ bool key_invertible(const SortKey& k) {
   }
 }
 
+bool key_rebuildable(const SortKey& k) {
+  if (key_invertible(k)) return true;
+  return !k.col->dictionary && (k.col->pt == PT_F32 || k.col->pt == PT_F64) && uint64_t(k.col->length) <= bs::MAX_ROWS &&
+         !debug_skip_first_tile();
+}
+
 bool payload_record_layout(const std::vector<am_array*>& cols, rs::RecLayout* L) {
   using namespace rs;
   if (cols.empty() || cols.size() > size_t(REC_MAX_COLS)) return false;
@@ -2066,6 +2076,7 @@ static void sort_by_buckets(const SortKey& key, const rs::PlanArgs& pa, uint64_t
   }
   if (key_dst) b.key_out = key_dst->values->ptr;
   b.key_pt = key.col->pt;
+  b.key_source = key_dst && !key_invertible(key);
   b.key_desc = key.descending;
   b.nulls_first = key.nulls_first;
   b.err = sc.err;
@@ -2083,9 +2094,9 @@ static void sort_by_buckets(const SortKey& key, const rs::PlanArgs& pa, uint64_t
   p.final_out = out;
   p.status = sc.status;
   p.err = sc.err;
-  p.carry_ids = carry_ids ? 1 : 0;
+  p.carry_ids = carry_ids || b.key_source ? 1 : 0;
   if (key_dst) {
-    p.key_out_mode = KEY_OUT_UNKEY;
+    p.key_out_mode = b.key_source ? KEY_OUT_SOURCE : KEY_OUT_UNKEY;
     p.key_out_pt = key.col->pt;
     p.key_desc = key.descending ? 1 : 0;
     p.key_float_order = key.float_order;
@@ -2147,8 +2158,8 @@ void radix_sort(const std::vector<SortKey>& keys_in, int64_t n64, void* out, int
     if (pt_var(k.col->pt)) throw Error("radix_sort: string keys must be expanded to their chunk keys first");
   if (n64 <= 0) return;
   const uint64_t n = uint64_t(n64);
-  if (key_dst && (K != 1 || !key_invertible(keys[0])))
-    throw invalid("the sorted key column is rebuilt only for one integer or totalOrder float key");
+  if (key_dst && (K != 1 || !key_rebuildable(keys[0])))
+    throw invalid("the sorted key column is rebuilt only for one integer or float key");
   if (payload && K != 1) throw invalid("payload columns ride through a sort by one key only");
   // Row ids move through the passes when an index is wanted or a lower key's column is gathered;
   // with payload columns, 16-byte row records (id and payload) move instead.

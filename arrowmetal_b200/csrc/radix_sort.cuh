@@ -113,7 +113,8 @@ struct RecLayout {
 };
 
 // key_out modes: the sorted key column itself, produced by inverting the key map in the last pass.
-constexpr int KEY_OUT_NONE = 0, KEY_OUT_UNKEY = 1;
+// KEY_OUT_SOURCE: read from the key column by row id (float orders that tie values).
+constexpr int KEY_OUT_NONE = 0, KEY_OUT_UNKEY = 1, KEY_OUT_SOURCE = 2;
 
 struct PassArgs {
   const PassDesc* desc;
