@@ -72,6 +72,8 @@ struct Args {
   uint32_t* ids[2];
   uint4* rec[2];                                  // with a payload: row id and payload fields (RecLayout), instead of ids
   void *out, *key_out;
+  const void* src_keys;                           // not NULL: the rows are these keys, with these ids, and no column
+  const uint32_t* src_ids;
   const void* key_src;                            // not NULL: keys that stand for several values are read here
   unsigned long long twin0, twin1;                // those keys: a zero's, a NaN's
   int32_t wide, key_pt, key_desc, nulls_first, has_payload;
@@ -457,9 +459,13 @@ buckets_kernel(const __grid_constant__ ColView col, const __grid_constant__ Args
         h ^= h >> 13;
         row = lo + __umulhi(h, uint32_t(hi - lo));
       }
-      const bool valid = !col.valid || bit_at(col.valid, col.valid_off + int64_t(row));
-      int cat;
-      key[u] = key_from_raw<KeyT>(col, load_raw<KeyT>(col, row), valid, cat);
+      int cat = 0;
+      if (a.src_ids) {
+        key[u] = static_cast<const KeyT*>(a.src_keys)[row];
+      } else {
+        const bool valid = !col.valid || bit_at(col.valid, col.valid_off + int64_t(row));
+        key[u] = key_from_raw<KeyT>(col, load_raw<KeyT>(col, row), valid, cat);
+      }
       if (cat == 0) live |= 1u << u;
       else if (cat == 1) nans |= 1u << u;
       else nulls |= 1u << u;
@@ -696,7 +702,7 @@ buckets_kernel(const __grid_constant__ ColView col, const __grid_constant__ Args
         if (dst < values) {
           static_cast<KeyT*>(a.keys[0])[dst] = key[u];
           if (a.has_payload) a.rec[0][dst] = build_record(a.pay, row);
-          else a.ids[0][dst] = row;
+          else a.ids[0][dst] = a.src_ids ? a.src_ids[row] : row;
         } else {
           atomicOr(a.err, ERR_BOUNDS);
         }
@@ -1608,6 +1614,164 @@ __global__ void __launch_bounds__(LTHREADS, LBLOCKS) bucket_sort_kernel(const __
   }
 }
 
+// ---- 5. the first k rows
+//
+// A sampled threshold that the k-th smallest key is almost surely at or below, one read of the column
+// that keeps the rows at or below it, and the bucket sort of those few (key, row) pairs, whose first k
+// row ids are the answer. The pairs are kept in no order: (key, row id) orders them.
+
+// One cluster: the threshold. Selection by 8-bit digits of the sampled keys' distance from the smallest,
+// until the digit's keys are few beyond the wanted ones.
+struct FirstShared {
+  uint32_t cnt[2][256];
+  uint32_t warp[32];
+  uint32_t pick[3];                      // the digit, the keys before it, its keys
+  unsigned long long smax[CLUSTER], smin[CLUSTER], scnt[CLUSTER];
+  unsigned long long wmax[32], wmin[32];
+};
+
+template <typename KeyT>
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(1024)
+first_threshold_kernel(const __grid_constant__ ColView col, uint64_t n, uint64_t k, FirstState* __restrict__ fs) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ FirstShared sm;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const uint32_t rank = cl.block_rank();
+  cl.sync();                             // every CTA runs before its shared memory is written
+  constexpr int U = SAMPLES / (1024 * CLUSTER);
+  KeyT key[U];
+  uint32_t live = 0;
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const uint32_t j = (rank * U + u) * 1024 + t;
+    const uint64_t lo = uint64_t(j) * n / SAMPLES, hi = uint64_t(j + 1) * n / SAMPLES;
+    uint32_t h = j * 2654435761u;
+    h ^= h >> 15;
+    h *= 2246822519u;
+    h ^= h >> 13;
+    const uint64_t row = lo + __umulhi(h, uint32_t(hi - lo));
+    const bool valid = !col.valid || bit_at(col.valid, col.valid_off + int64_t(row));
+    int cat;
+    key[u] = key_from_raw<KeyT>(col, load_raw<KeyT>(col, row), valid, cat);
+    if (cat == 0) live |= 1u << u;
+  }
+  uint64_t mx = 0, mn = 0;
+#pragma unroll
+  for (int u = 0; u < U; u++)
+    if ((live >> u) & 1u) {
+      mx = max(mx, uint64_t(key[u]));
+      mn = max(mn, ~uint64_t(key[u]));
+    }
+  mx = warp_max_u64(mx);
+  mn = warp_max_u64(mn);
+  const uint32_t c = __reduce_add_sync(0xffffffffu, __popc(live));
+  if (lane == 0) {
+    sm.wmax[warp] = mx;
+    sm.wmin[warp] = mn;
+    sm.warp[warp] = c;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    const uint64_t bx = warp_max_u64(sm.wmax[lane]), bn = warp_max_u64(sm.wmin[lane]);
+    const uint32_t bc = __reduce_add_sync(0xffffffffu, sm.warp[lane]);
+    if (lane < CLUSTER) {
+      FirstShared* o = cl.map_shared_rank(&sm, lane);
+      o->smax[rank] = bx;
+      o->smin[rank] = bn;
+      o->scnt[rank] = bc;
+    }
+  }
+  cl.sync();
+  uint64_t vmax = 0, vmin_inv = 0;
+  uint32_t sv = 0;
+#pragma unroll
+  for (int r = 0; r < CLUSTER; r++) {
+    vmax = max(vmax, uint64_t(sm.smax[r]));
+    vmin_inv = max(vmin_inv, uint64_t(sm.smin[r]));
+    sv += uint32_t(sm.scnt[r]);
+  }
+  // The sampled rank that holds k rows with a margin of four deviations.
+  const float mu = float(k) * float(SAMPLES) / float(n);
+  const uint32_t want = uint32_t(mu + 4.0f * sqrtf(mu) + 8.0f);
+  if (sv < want) {                       // (the same in every CTA)
+    if (rank == 0 && t == 0) fs->limit = ~0ull;
+    cl.sync();
+    return;
+  }
+  const uint64_t lo = ~vmin_inv, span = vmax - lo;
+  const int bits = span ? 64 - __clzll((long long)span) : 1;
+  uint64_t prefix = 0;                   // the digits chosen so far, of (key - lo) in `bits` bits
+  int shift = bits;
+  uint32_t left = want;
+  for (int round = 0; shift > 0; round++) {
+    const int step = shift < 8 ? shift : 8, next = shift - step, buf = round & 1;
+    if (t < 256) sm.cnt[buf][t] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const uint64_t x = uint64_t(key[u]) - lo;
+      if (((live >> u) & 1u) && (shift >= 64 || (x >> shift) == prefix)) atomicAdd(&sm.cnt[buf][(x >> next) & ((1u << step) - 1u)], 1u);
+    }
+    cl.sync();
+    uint32_t mine = 0;
+    if (t < 256)
+      for (int r = 0; r < CLUSTER; r++) mine += cl.map_shared_rank(&sm, r)->cnt[buf][t];
+    uint32_t all;
+    const uint32_t before = block_scan<1024>(mine, sm.warp, all);
+    if (t < 256 && before < left && left <= before + mine) {
+      sm.pick[0] = t;
+      sm.pick[1] = before;
+      sm.pick[2] = mine;
+    }
+    __syncthreads();
+    prefix = (shift >= 64 ? 0ull : prefix << step) | sm.pick[0];
+    left -= sm.pick[1];
+    shift = next;
+    if (sm.pick[2] - left <= want / 4 + 8) break;
+    __syncthreads();
+  }
+  if (rank == 0 && t == 0) {
+    const uint64_t x = shift ? (prefix << shift) | ((1ull << shift) - 1ull) : prefix;
+    fs->limit = lo + (x < span ? x : span);
+  }
+  cl.sync();                             // no CTA leaves while another reads its counts
+}
+
+// Rows whose key is at most the limit, appended as (key, row) pairs; pairs past `cap` are only counted.
+template <typename KeyT>
+__global__ void __launch_bounds__(256) first_collect_kernel(const __grid_constant__ ColView col, uint64_t n, FirstState* __restrict__ fs,
+                                                            uint32_t cap, KeyT* __restrict__ keys, uint32_t* __restrict__ rows) {
+  constexpr int NI = 8;
+  const KeyT limit = KeyT(fs->limit);
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+  const uint64_t step = uint64_t(gridDim.x) * (256 * NI);
+  for (uint64_t w0 = uint64_t(blockIdx.x) * (256 * NI) + warp * (NI * 32); w0 < n; w0 += step) {
+    RawTile<KeyT, NI> r;
+    uint32_t values, nulls, nans;
+    load_tile(col, w0, n, r);
+    encode_tile(col, w0, n, r, values, nulls, nans);
+    uint32_t hit = 0;
+#pragma unroll
+    for (int i = 0; i < NI; i++)
+      if (((values >> i) & 1u) && r.key[i] <= limit) hit |= 1u << i;
+    if (!__any_sync(0xffffffffu, hit != 0u)) continue;
+#pragma unroll
+    for (int i = 0; i < NI; i++) {
+      const bool is = (hit >> i) & 1u;
+      const uint32_t m = __ballot_sync(0xffffffffu, is);
+      if (m == 0u) continue;
+      uint32_t at = 0;
+      if (lane == 0) at = atomicAdd(&fs->count, uint32_t(__popc(m)));
+      at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & lt);
+      if (is && at < cap) {
+        keys[at] = r.key[i];
+        rows[at] = uint32_t(w0) + uint32_t(i) * 32 + lane;
+      }
+    }
+  }
+}
+
 // ---- host side
 
 static uint32_t bucket_cap(uint64_t n) {
@@ -1702,6 +1866,26 @@ void launch_all(const Sort& b, const Args& a, int pay, cudaStream_t s) {
 }
 }  // namespace
 
+void enqueue_first(const ColView& col, int key_bytes, uint64_t n, uint64_t k, FirstState* fs, void* keys, uint32_t* rows,
+                   cudaStream_t s) {
+  AM_CUDA(cudaMemsetAsync(fs, 0, sizeof(FirstState), s));
+  const uint64_t tiles = (n + 256 * 8 - 1) / (256 * 8);
+  const int grid = int(std::min<uint64_t>(tiles, uint64_t(device().sm_count) * 8));
+  auto go = [&](auto tag) {
+    using KeyT = decltype(tag);
+    {
+      KernelTimer kt("topk_threshold", s);
+      first_threshold_kernel<KeyT><<<CLUSTER, 1024, 0, s>>>(col, n, k, fs);
+      AM_CUDA(cudaGetLastError());
+    }
+    KernelTimer kt("topk_collect", s);
+    first_collect_kernel<KeyT><<<grid, 256, 0, s>>>(col, n, fs, SAMPLES, static_cast<KeyT*>(keys), rows);
+    AM_CUDA(cudaGetLastError());
+  };
+  if (key_bytes == 8) go(uint64_t(0));
+  else go(uint32_t(0));
+}
+
 size_t scratch_bytes(uint64_t n) { return Layout(n).total; }
 size_t zeroed_bytes(uint64_t n) { return Layout(n).zeroed; }
 
@@ -1731,6 +1915,8 @@ State* enqueue(const Sort& b, cudaStream_t s) {
     a.ids[i] = reinterpret_cast<uint32_t*>(b.ids[i]);
     a.rec[i] = reinterpret_cast<uint4*>(b.ids[i]);
   }
+  a.src_keys = b.src_keys;
+  a.src_ids = b.src_ids;
   a.out = b.out;
   a.wide = b.wide ? 1 : 0;
   a.key_out = b.key_out;

@@ -23,11 +23,19 @@ struct State {
   uint32_t max_bucket, pad;
 };
 
+// The first rows' selection: keys up to `limit` are kept, `count` of them.
+struct FirstState {
+  unsigned long long limit;
+  uint32_t count, pad;
+};
+
 // One bucket sort. `rec` (may be NULL): the payload columns that ride with the rows.
 struct Sort {
   rs::ColView col;
   int key_bytes;
   uint64_t n;
+  const void* src_keys;                  // not NULL: at most MAX_PAIRS rows given as keys and row ids, no column
+  const uint32_t* src_ids;
   char* scratch;                         // `scratch_bytes(n)` bytes, the first `zeroed_bytes(n)` zero
   void* keys[2];                         // n keys each
   char* ids[2];                          // n x 4 bytes, or n x 16 with a payload
@@ -46,11 +54,18 @@ struct Sort {
 // Rows a bucket sort takes: up to what MAX_BUCKETS buckets hold.
 constexpr uint64_t MAX_ROWS = uint64_t(60) << 20;
 
+constexpr uint64_t MAX_PAIRS = 65536;
+
 size_t scratch_bytes(uint64_t n);
 size_t zeroed_bytes(uint64_t n);
 // Enqueues the sort; afterwards State::mode says whether it ran (MODE_BUCKETS) or its rows are as they
 // were (MODE_FALLBACK: the digit passes must run). Returns the State on the device.
 State* enqueue(const Sort& b, cudaStream_t s);
+// Enqueues the choice of a key limit that at least the k smallest value keys are almost surely within, and
+// one read of the column that appends the rows within it, as (key, row id) pairs in no order, to arrays
+// of MAX_PAIRS; fs->count says how many there are. n is at least MAX_PAIRS.
+void enqueue_first(const rs::ColView& col, int key_bytes, uint64_t n, uint64_t k, FirstState* fs, void* keys, uint32_t* rows,
+                   cudaStream_t s);
 
 }  // namespace bs
 }  // namespace am

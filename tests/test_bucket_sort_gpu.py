@@ -123,3 +123,19 @@ def test_rebuilt_float_keys_keep_their_bits(am, n, kind, order):
             assert got.null_count == want.null_count
             assert got.buffers()[1].to_pybytes()[:n * v.dtype.itemsize] == want.buffers()[1].to_pybytes()[:n * v.dtype.itemsize]
             assert np.array_equal(np.asarray(got.is_valid()), np.asarray(want.is_valid()))
+
+
+@pytest.mark.parametrize("n,k,kind", [(2**19, 1, "even"), (600_011, 1000, "normal"), (2_000_003, 20_000, "even32"),
+                                      (3_000_017, 500, "one_value"), (600_011, 30_000, "normal32"), (700_001, 5000, "narrow")])
+def test_first_rows_are_the_sorts_first(am, n, k, kind):
+    # The sampled limit and its fallbacks: few and many rows wanted, equal keys at the limit, nulls first.
+    rng = np.random.default_rng(n + k)
+    v = keys(kind, n, rng)
+    if kind == "one_value":
+        v[v == 123_456_789_012] = 0
+    for nulls in (0.0, 0.3):
+        m = am.MetalArray.from_arrow(pa.array(v, mask=rng.random(n) < nulls if nulls else None, from_pandas=False))
+        for largest, place, order in ((True, "at_end", "ieee"), (False, "at_start", "nan_largest"), (False, "at_end", "total")):
+            want = m.argsort(largest, place, order).to_arrow().to_numpy()[:k]
+            got = m.top_k(k, largest, place, order).to_arrow().to_numpy()
+            assert np.array_equal(got, want), (nulls, largest, place, order)
