@@ -365,6 +365,11 @@ am_array* dictionary_key_column(const SortKey& k, cudaStream_t s);
 void argsort_any(const std::vector<SortKey>& keys, int64_t n, void* out, int width, cudaStream_t s,
                  am_sort_stats* stats);
 
+// The argsort of one string column by buckets of its leading characters, equal ones ordered by the strings
+// themselves; false when that cannot be (many rows share them): `out` then holds
+// nothing and the derived keys must be sorted. Waits for the answer to that.
+bool string_argsort(const SortKey& key, int64_t n, void* out, int width, cudaStream_t s, am_sort_stats* stats);
+
 // Copies a host Arrow array (a dictionary array with its dictionary) into HBM on stream `s`; the caller
 // keeps and releases the struct.
 am_array* import_copy(const ArrowSchema* schema, const ArrowArray* array, cudaStream_t s);
@@ -375,6 +380,9 @@ am_array* import_copy(const ArrowSchema* schema, const ArrowArray* array, cudaSt
 // derives chunks [first, first + count) and, when asked, the length (chunk 0 carries the nulls).
 int string_chunk_count(const am_array* a, cudaStream_t s);
 std::vector<am_array*> string_key_columns(const am_array* a, int first, int count, bool with_length, cudaStream_t s);
+// The one-key form of a string column for the bucket sort (strings.cu): a uint64 key column with the
+// column's nulls; word 8 of `chars` (device memory) receives the characters a key holds.
+am_array* string_order_key(const am_array* a, bool desc, BufPtr& chars, cudaStream_t s);
 void take_strings(am_array* src, am_array* idx, am_array* out, bool check_range, cudaStream_t s);
 
 // Gathers `count` columns through one index array. outs[i] must be new arrays of indices' length.

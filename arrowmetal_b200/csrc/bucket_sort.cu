@@ -80,6 +80,7 @@ struct Args {
   int32_t one_launch;                             // the plan's launch counts and moves the rows too
   uint32_t* err;
   SortSummary* sum;
+  StringTies ties;
   RecLayout pay;
 };
 
@@ -1255,6 +1256,34 @@ __global__ void __launch_bounds__(THREADS, 2) level2_kernel(const __grid_constan
 
 // ---- 4. each bucket in shared memory
 
+// Row a before row b, their keys being equal: by row id, or first by the strings behind the keys.
+template <int TIES>
+__device__ __forceinline__ bool tied_before(const StringTies& s, uint32_t a, uint32_t b) {
+  if constexpr (TIES != 0) {
+    uint64_t oa, ob, la, lb;
+    if (s.wide) {
+      const int64_t* o = static_cast<const int64_t*>(s.offsets);
+      oa = uint64_t(o[a]);
+      ob = uint64_t(o[b]);
+      la = uint64_t(o[a + 1ull]) - oa;
+      lb = uint64_t(o[b + 1ull]) - ob;
+    } else {
+      const int32_t* o = static_cast<const int32_t*>(s.offsets);
+      oa = uint64_t(uint32_t(o[a]));
+      ob = uint64_t(uint32_t(o[b]));
+      la = uint64_t(uint32_t(o[a + 1ull])) - oa;
+      lb = uint64_t(uint32_t(o[b + 1ull])) - ob;
+    }
+    const uint64_t n = la < lb ? la : lb;
+    for (uint64_t i = *s.chars; i < n; i++) {
+      const uint8_t x = s.bytes[oa + i], y = s.bytes[ob + i];
+      if (x != y) return (x < y) != (s.desc != 0);
+    }
+    if (la != lb) return (la < lb) != (s.desc != 0);
+  }
+  return a < b;
+}
+
 // A CTA's shared memory: the fast form's arrays, or the slower one's keys and places of up to BIG rows.
 template <typename KeyT, int PAY>
 struct LocalShared {
@@ -1283,8 +1312,9 @@ struct LocalShared {
 
 // A bucket of more than CAP rows, or with many equal or very close keys: bitonic sort of (key, row id),
 // the ids of equal keys read where the rows are.
-template <typename KeyT, typename IdOf>
-__device__ __forceinline__ void bitonic_rows(KeyT* key, uint16_t* place, uint32_t size, const KeyT* in, IdOf&& id_of) {
+template <int TIES, typename KeyT, typename IdOf>
+__device__ __forceinline__ void bitonic_rows(KeyT* key, uint16_t* place, uint32_t size, const KeyT* in, IdOf&& id_of,
+                                             const StringTies& ties) {
   uint32_t p = 2;
   while (p < size) p <<= 1;
   for (uint32_t i = threadIdx.x; i < p; i += LTHREADS) {
@@ -1300,7 +1330,7 @@ __device__ __forceinline__ void bitonic_rows(KeyT* key, uint16_t* place, uint32_
         bool less = kl < ki;
         if (kl == ki) {
           const uint32_t pi = place[i], pl = place[l];
-          less = pl >= size ? false : pi >= size ? true : id_of(pl) < id_of(pi);
+          less = pl >= size ? false : pi >= size ? true : tied_before<TIES>(ties, id_of(pl), id_of(pi));
         }
         if (less == ((i & k) == 0)) {
           key[i] = kl;
@@ -1326,7 +1356,7 @@ struct KeyOut {
                   (a.key_desc ? KeyT(~KeyT(0)) : KeyT(0)))) {}
 };
 
-template <typename KeyT, int PAY>
+template <typename KeyT, int PAY, int TIES>
 __global__ void __launch_bounds__(LTHREADS, LBLOCKS) bucket_sort_kernel(const __grid_constant__ Args a) {
   extern __shared__ __align__(16) unsigned char lsm[];
   using SM = LocalShared<KeyT, PAY>;
@@ -1492,7 +1522,7 @@ __global__ void __launch_bounds__(LTHREADS, LBLOCKS) bucket_sort_kernel(const __
                   rank += o < me ? 1u : 0u;
                 } else {
                   const KeyT k = exact ? key[i] : kin[p];
-                  rank += k < key[i] || (k == key[i] && (PAY ? id_of(p) : sm.id[p]) < mine) ? 1u : 0u;
+                  rank += k < key[i] || (k == key[i] && tied_before<TIES>(a.ties, PAY ? id_of(p) : sm.id[p], mine)) ? 1u : 0u;
                 }
               }
             }
@@ -1590,7 +1620,7 @@ __global__ void __launch_bounds__(LTHREADS, LBLOCKS) bucket_sort_kernel(const __
         }
         __syncthreads();
       }
-      bitonic_rows(sm.slow.key, sm.slow.place, rows, kin, id_of);
+      bitonic_rows<TIES>(sm.slow.key, sm.slow.place, rows, kin, id_of, a.ties);
       for (uint32_t r = t; r < rows; r += LTHREADS) {
         const uint32_t p = sm.slow.place[r];
         const KeyT k = sm.slow.key[r];
@@ -1810,13 +1840,13 @@ void smem_limit(F fn, size_t bytes) {
   AM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
 }
 
-template <typename KeyT, int PAY>
+template <typename KeyT, int PAY, int TIES>
 void launch_moves(const ColView& cv, const Args& a, cudaStream_t s) {
   static std::once_flag once;
   std::call_once(once, [] {
     smem_limit(level1_kernel<KeyT, PAY>, sizeof(TileShared<KeyT, PAY>));
     smem_limit(level2_kernel<KeyT, PAY>, sizeof(Tile2Shared<KeyT, PAY>));
-    smem_limit(bucket_sort_kernel<KeyT, PAY>, sizeof(LocalShared<KeyT, PAY>));
+    smem_limit(bucket_sort_kernel<KeyT, PAY, TIES>, sizeof(LocalShared<KeyT, PAY>));
   });
   const int sms = device().sm_count;
   if (!a.one_launch) {
@@ -1834,7 +1864,7 @@ void launch_moves(const ColView& cv, const Args& a, cudaStream_t s) {
   {
     KernelTimer kt("bucket_sort", s);
     const int grid = int(std::min<uint32_t>(a.bucket_cap, uint32_t(sms * LBLOCKS)));
-    bucket_sort_kernel<KeyT, PAY><<<grid, LTHREADS, sizeof(LocalShared<KeyT, PAY>), s>>>(a);
+    bucket_sort_kernel<KeyT, PAY, TIES><<<grid, LTHREADS, sizeof(LocalShared<KeyT, PAY>), s>>>(a);
     AM_CUDA(cudaGetLastError());
   }
 }
@@ -1861,8 +1891,14 @@ void launch_all(const Sort& b, const Args& a, int pay, cudaStream_t s) {
       AM_CUDA(cudaGetLastError());
     }
   }
-  if (pay) launch_moves<KeyT, 1>(b.col, a, s);
-  else launch_moves<KeyT, 0>(b.col, a, s);
+  if constexpr (sizeof(KeyT) == 8) {
+    if (a.ties.offsets) {
+      launch_moves<KeyT, 0, 1>(b.col, a, s);
+      return;
+    }
+  }
+  if (pay) launch_moves<KeyT, 1, 0>(b.col, a, s);
+  else launch_moves<KeyT, 0, 0>(b.col, a, s);
 }
 }  // namespace
 
@@ -1915,6 +1951,7 @@ State* enqueue(const Sort& b, cudaStream_t s) {
     a.ids[i] = reinterpret_cast<uint32_t*>(b.ids[i]);
     a.rec[i] = reinterpret_cast<uint4*>(b.ids[i]);
   }
+  a.ties = b.ties;
   a.src_keys = b.src_keys;
   a.src_ids = b.src_ids;
   a.out = b.out;

@@ -23,6 +23,16 @@ struct State {
   uint32_t max_bucket, pad;
 };
 
+// Strings behind 8-byte keys of their leading characters (strings.cu): rows of equal keys order by the rest
+// of their strings, then by row id.
+struct StringTies {
+  const void* offsets;                   // row 0's offset; NULL: no strings
+  const uint8_t* bytes;
+  const uint32_t* chars;                 // device memory: the characters a key holds
+  int32_t wide;                          // 64-bit offsets
+  int32_t desc;
+};
+
 // The first rows' selection: keys up to `limit` are kept, `count` of them.
 struct FirstState {
   unsigned long long limit;
@@ -39,6 +49,7 @@ struct Sort {
   char* scratch;                         // `scratch_bytes(n)` bytes, the first `zeroed_bytes(n)` zero
   void* keys[2];                         // n keys each
   char* ids[2];                          // n x 4 bytes, or n x 16 with a payload
+  StringTies ties;
   bool payload;
   rs::RecLayout rec;
   void* out;                             // the order (NULL: not wanted)

@@ -754,6 +754,8 @@ std::vector<am_array*> materialize(const std::vector<Piece>& p, size_t lo, size_
 void argsort_any(const std::vector<SortKey>& keys, int64_t n, void* out, int width, cudaStream_t s,
                  am_sort_stats* stats) {
   if (n <= 0) return;
+  // (The derived keys' path reads the longest string back before it sorts; this one only its outcome.)
+  if (keys.size() == 1 && pt_var(keys[0].col->pt) && string_argsort(keys[0], n, out, width, s, stats)) return;
   std::vector<am_array*> owned;
   std::vector<Piece> pieces;
   auto release_all = [&](std::vector<am_array*>& v) {

@@ -2126,6 +2126,55 @@ static void sort_by_buckets(const SortKey& key, const rs::PlanArgs& pa, uint64_t
   finish_sort(key, n, key_dst, sum, payload != nullptr, stats, s);
 }
 
+bool string_argsort(const SortKey& key, int64_t n64, void* out, int index_width, cudaStream_t s, am_sort_stats* stats) {
+  using namespace rs;
+  const uint64_t n = uint64_t(n64);
+  if (n == 0 || n > bs::MAX_ROWS || debug_skip_first_tile()) return false;
+  const am_array* a = key.col;
+  BufPtr chars;
+  struct Release {
+    am_array* c;
+    ~Release() { am::release(c); }
+  } column{string_order_key(a, key.descending, chars, s)};
+  auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
+  const size_t off_bs = up(sizeof(SortSummary));
+  const size_t off_keys = up(off_bs + bs::scratch_bytes(n));
+  const size_t kbuf = up(n * 8), ibuf = up(n * 4);
+  ScratchBlock scratch(s, off_keys + 2 * kbuf + 2 * ibuf);
+  char* base = scratch.data();
+  AM_CUDA(cudaMemsetAsync(base, 0, off_bs + bs::zeroed_bytes(n), s));
+  SortSummary* sum = reinterpret_cast<SortSummary*>(base);
+  const SortKey first{column.c, key.descending, key.nulls_first, 0};
+  bs::Sort b{};
+  b.col = make_view(first);
+  b.key_bytes = 8;
+  b.n = n;
+  b.ties.offsets = static_cast<const char*>(a->values->ptr) + size_t(a->value_offset) * size_t(pt_bytes(a->pt));
+  b.ties.bytes = a->bytes ? static_cast<const uint8_t*>(a->bytes->ptr) : nullptr;
+  b.ties.chars = static_cast<const uint32_t*>(chars->ptr) + 8;
+  b.ties.wide = a->pt == PT_LSTR ? 1 : 0;
+  b.ties.desc = key.descending ? 1 : 0;
+  b.scratch = base + off_bs;
+  for (int i = 0; i < 2; i++) {
+    b.keys[i] = base + off_keys + size_t(i) * kbuf;
+    b.ids[i] = base + off_keys + 2 * kbuf + size_t(i) * ibuf;
+  }
+  b.out = out;
+  b.wide = index_width == 8;
+  b.key_pt = PT_U64;
+  b.nulls_first = key.nulls_first;
+  b.err = stream_scratch(s, 0).err;
+  b.summary = sum;
+  const bs::State* st = bs::enqueue(b, s);
+  static thread_local uint32_t* host = nullptr;
+  if (!host) host = static_cast<uint32_t*>(pinned_alloc(16));
+  AM_CUDA(cudaMemcpyAsync(host, &st->mode, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  AM_CUDA(cudaStreamSynchronize(s));
+  if (*host != bs::MODE_BUCKETS) return false;
+  finish_sort(first, n, nullptr, sum, false, stats, s);
+  return true;
+}
+
 void radix_argsort(const std::vector<SortKey>& keys, int64_t n, void* out, int index_width, cudaStream_t s,
                    am_sort_stats* stats) {
   radix_sort(keys, n, out, index_width, nullptr, s, stats);

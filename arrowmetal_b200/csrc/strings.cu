@@ -10,6 +10,12 @@
 // length comes first. Null rows are routed by the first chunk, which carries the column's validity; a
 // descending sort reverses every derived key.
 //
+// One string column sorts by buckets (bucket_sort.cu) of a single 8-byte key first: its leading characters
+// as digits over the column's own alphabet (the bytes that occur, in order, after a digit 0 for the end),
+// as many as 64 bits hold: 13 of lowercase letters, 7 of any bytes. A string that ends within them leaves
+// the digits below its end to its row number, so a short string however often repeated spreads over
+// its own range of keys in row order. Rows of equal keys order by the rest of their strings.
+//
 // Take gathers the rows' lengths, scans them into the output offsets and copies each row's bytes.
 #include <algorithm>
 
@@ -69,6 +75,97 @@ __global__ void __launch_bounds__(256) chunk_kernel(const OffT* __restrict__ off
       chunks[j][r] = v;
     }
     if (length) length[r] = LenT(l);
+  }
+}
+
+// ---- the one-key form
+
+// Which bytes the rows' strings use (null rows' slots too: a larger alphabet, the same order).
+template <typename OffT>
+__global__ void __launch_bounds__(256) byte_use_kernel(const OffT* __restrict__ off, const uint8_t* __restrict__ bytes, uint64_t n,
+                                                       uint32_t* __restrict__ used) {
+  __shared__ uint32_t seen[8];
+  if (threadIdx.x < 8) seen[threadIdx.x] = 0;
+  __syncthreads();
+  const uint64_t first = uint64_t(off[0]), end = uint64_t(off[n]);
+  uint32_t mine[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  auto add = [&](uint32_t b) {
+#pragma unroll
+    for (int w = 0; w < 8; w++) mine[w] |= (b >> 5) == uint32_t(w) ? 1u << (b & 31u) : 0u;
+  };
+  // Whole 16-byte pieces, then the bytes before and after them.
+  const uint64_t lo = (first + 15) & ~uint64_t(15), hi = end & ~uint64_t(15);
+  const uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x, step = uint64_t(gridDim.x) * blockDim.x;
+  if (lo < hi && (reinterpret_cast<uintptr_t>(bytes) & 15u) == 0) {
+    for (uint64_t i = lo / 16 + t; i < hi / 16; i += step) {
+      const uint4 v = reinterpret_cast<const uint4*>(bytes)[i];
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+#pragma unroll
+        for (int b = 0; b < 4; b++) add((w[q] >> (8 * b)) & 255u);
+    }
+    for (uint64_t i = first + t; i < lo; i += step) add(bytes[i]);
+    for (uint64_t i = hi + t; i < end; i += step) add(bytes[i]);
+  } else {
+    for (uint64_t i = first + t; i < end; i += step) add(bytes[i]);
+  }
+#pragma unroll
+  for (int w = 0; w < 8; w++) {
+    const uint32_t m = __reduce_or_sync(0xffffffffu, mine[w]);
+    if ((threadIdx.x & 31) == 0 && m) atomicOr(&seen[w], m);
+  }
+  __syncthreads();
+  if (threadIdx.x < 8 && seen[threadIdx.x]) atomicOr(used + threadIdx.x, seen[threadIdx.x]);
+}
+
+constexpr int KEY_CHARS = 24;            // at most so many characters, however small the alphabet
+
+// Keys of the rows, and (in used[8]) the characters a key holds.
+template <typename OffT>
+__global__ void __launch_bounds__(256) string_key_kernel(const OffT* __restrict__ off, const uint8_t* __restrict__ bytes, uint64_t n,
+                                                         int desc, uint32_t* __restrict__ used, uint64_t* __restrict__ keys) {
+  __shared__ uint16_t digit[256];
+  __shared__ uint64_t power[KEY_CHARS + 1];
+  __shared__ int s_chars;
+  const int t = threadIdx.x;
+  {
+    uint32_t before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+      const uint32_t m = used[w];
+      if (w < (t >> 5)) before += __popc(m);
+      all += __popc(m);
+    }
+    digit[t] = uint16_t(before + __popc(used[t >> 5] & ((2u << (t & 31)) - 1u)));    // 1 up; 0 is the end
+    if (t == 0) {
+      const uint64_t base = uint64_t(all) + 1;
+      int c = 0;
+      uint64_t p = 1;
+      power[0] = 1;
+      while (c < KEY_CHARS && p <= ~0ull / base) {
+        p *= base;
+        power[++c] = p;
+      }
+      s_chars = c;
+      if (blockIdx.x == 0) used[8] = uint32_t(c);
+    }
+  }
+  __syncthreads();
+  const int chars = s_chars;
+  const int idbits = n > 1 ? 64 - __clzll((long long)(n - 1)) : 1;
+  for (uint64_t r = uint64_t(blockIdx.x) * blockDim.x + t; r < n; r += uint64_t(gridDim.x) * blockDim.x) {
+    uint64_t s, l;
+    row_span(off, int64_t(r), s, l);
+    const int m = l < uint64_t(chars) ? int(l) : chars;
+    uint64_t k = 0;
+    for (int i = 0; i < m; i++) k = k * power[1] + digit[bytes[s + i]];
+    if (m < chars) {
+      // The end's digit 0, and the row's share of the digits below it (rows in order, both directions).
+      const uint64_t id = desc ? n - 1 - r : r;
+      k = k * power[chars - m] + __umul64hi(power[chars - m - 1], id << (64 - idbits));
+    }
+    keys[r] = k;
   }
 }
 
@@ -393,6 +490,38 @@ int string_chunk_count(const am_array* a, cudaStream_t s) {
   const uint64_t m = std::max<uint64_t>(1, (maxlen + 7) / 8);
   if (m > (uint64_t(1) << 24)) throw unsupported("string keys longer than 128 MiB");
   return int(m);
+}
+
+am_array* string_order_key(const am_array* a, bool desc, BufPtr& chars, cudaStream_t s) {
+  const uint64_t n = uint64_t(a->length);
+  am_array* c = new_array(PT_U64, "L", int64_t(n));
+  try {
+    c->values = DevBuffer::alloc(size_t(n) * 8 + 16, s);
+    c->last_stream = s;
+    chars = DevBuffer::alloc(64, s);
+    uint32_t* used = static_cast<uint32_t*>(chars->ptr);
+    AM_CUDA(cudaMemsetAsync(used, 0, 64, s));
+    const uint8_t* bytes = a->bytes ? static_cast<const uint8_t*>(a->bytes->ptr) : nullptr;
+    KernelTimer kt("string_key", s);
+    auto go = [&](auto tag) {
+      using OffT = decltype(tag);
+      const OffT* off = offsets_at_row0<OffT>(a);
+      if (bytes) byte_use_kernel<OffT><<<device().sm_count * 4, 256, 0, s>>>(off, bytes, n, used);
+      AM_CUDA(cudaGetLastError());
+      string_key_kernel<OffT><<<grid_for(n, 256), 256, 0, s>>>(off, bytes, n, desc ? 1 : 0, used, static_cast<uint64_t*>(c->values->ptr));
+      AM_CUDA(cudaGetLastError());
+    };
+    if (a->pt == PT_LSTR) go(int64_t(0));
+    else go(int32_t(0));
+    c->validity = a->validity;
+    c->validity_offset = a->validity_offset;
+    c->null_count = a->null_count;
+    c->null_count_dev = a->null_count_dev;
+  } catch (...) {
+    release(c);
+    throw;
+  }
+  return c;
 }
 
 std::vector<am_array*> string_key_columns(const am_array* a, int first, int count, bool with_length, cudaStream_t s) {

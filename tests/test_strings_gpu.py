@@ -201,3 +201,31 @@ def test_null_slots_that_span_bytes_keep_row_order(am):
             want = pc.array_sort_indices(arr, order="descending" if desc else "ascending",
                                          null_placement=placement).to_numpy()
             assert np.array_equal(got, want), (desc, placement)
+
+
+@pytest.mark.parametrize("n,kind", [(1, "letters"), (3000, "letters"), (70_001, "prefix"), (300_007, "letters"), (300_007, "few"),
+                                    (300_007, "low_bytes"), (200_003, "repeats"), (150_001, "empty"), (100_003, "all_bytes")])
+def test_string_order_by_buckets(am, n, kind):
+    # Keys of leading characters: alphabets of 1 to 256 bytes, many empty and short strings, strings equal
+    # in all a key holds, strings repeated too often for any bucket; slices, both offset widths, nulls.
+    rng = np.random.default_rng(n + len(kind))
+    top = {"letters": 25, "prefix": 30, "few": 2, "low_bytes": 14, "repeats": 9, "empty": 1, "all_bytes": 12}[kind]
+    lens = rng.integers(0, top, n)
+    if kind == "prefix":
+        lens = lens + 20
+    offsets = np.concatenate([[0], np.cumsum(lens)])
+    lo, hi = {"low_bytes": (0, 3), "all_bytes": (0, 256)}.get(kind, (97, 123))
+    data = rng.integers(lo, hi, offsets[-1]).astype(np.uint8).tobytes()
+    vals = [data[offsets[i]:offsets[i + 1]] for i in range(n)]
+    if kind == "prefix":
+        vals = [b"a common beginning of " + v[-3:] if i % 40 == 0 else v for i, v in enumerate(vals)]
+    if kind == "repeats":
+        vals = [b"%05d" % int(rng.integers(0, max(1, n // 900))) + b"x" * (i % 3) for i in range(n)]
+    for typ in (pa.binary(), pa.large_binary()):
+        mask = rng.random(n) < 0.05
+        for arr in (pa.array(vals, typ), pa.array([None if m else v for v, m in zip(vals, mask)], typ)):
+            part = arr.slice(min(3, n - 1))
+            m = am.MetalArray.from_arrow(arr).slice(min(3, n - 1), len(part))
+            for desc, place in ((False, "at_end"), (True, "at_start")):
+                want = pc.sort_indices(pa.table({"s": part}), [("s", "descending" if desc else "ascending")], null_placement=place)
+                assert np.array_equal(m.argsort(desc, place).to_arrow().to_numpy(), want.to_numpy()), (typ, desc)
