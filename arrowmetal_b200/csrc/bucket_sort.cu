@@ -27,6 +27,8 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <cstring>
+#include <memory>
 #include <type_traits>
 
 #include "am_internal.h"
@@ -67,6 +69,7 @@ struct Args {
   State* st;
   uint32_t *coarse, *fine, *bfirst, *bmeta, *bcount, *bpos, *cursor1, *cursor2, *chunk_bins, *chunk_cats;
   uint32_t nsamples, nchunks, chunk_rows, bucket_cap, bins1_cap;
+  uint32_t hist_grid, level2_grid, sort_grid;     // CTAs that take part in those steps
   uint64_t n;
   void* keys[2];
   uint32_t* ids[2];
@@ -431,8 +434,7 @@ __device__ void plan_cells(const Args& a, PlanShared& sm, const Map<KeyT>& map, 
 }
 
 template <typename KeyT>
-__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(1024)
-buckets_kernel(const __grid_constant__ ColView col, const __grid_constant__ Args a) {
+__device__ __forceinline__ void buckets_body(const ColView& col, const Args& a) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   __shared__ PlanShared sm;
@@ -728,11 +730,10 @@ buckets_kernel(const __grid_constant__ ColView col, const __grid_constant__ Args
 // One read of the column (63 us for 45M keys and 16,384 bins on a B200: the HBM copy rate). Each CTA
 // takes consecutive chunks; a chunk's level-1 counts are the growth of its bins' sums over the chunk.
 template <typename KeyT>
-__global__ void __launch_bounds__(HTHREADS) bucket_histogram_kernel(const __grid_constant__ ColView col,
-                                                                   const __grid_constant__ Args a) {
+__device__ __forceinline__ void histogram_body(const ColView& col, const Args& a) {
   extern __shared__ __align__(16) unsigned char hsm[];
   State* st = a.st;
-  if (st->mode != MODE_BUCKETS) return;
+  if (blockIdx.x >= a.hist_grid || st->mode != MODE_BUCKETS) return;
   uint32_t* bins = reinterpret_cast<uint32_t*>(hsm);
   __shared__ uint32_t coarse[COARSE], fine[FINE], prev[BINS1];
   __shared__ uint32_t s_null, s_nan;
@@ -751,8 +752,8 @@ __global__ void __launch_bounds__(HTHREADS) bucket_histogram_kernel(const __grid
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   KeyT diff = 0;                        // bits that differ from lo's in some key
   uint32_t values = 0, all_null = 0, all_nan = 0;
-  const uint32_t c0 = uint32_t(uint64_t(blockIdx.x) * a.nchunks / gridDim.x);
-  const uint32_t c1 = uint32_t(uint64_t(blockIdx.x + 1) * a.nchunks / gridDim.x);
+  const uint32_t c0 = uint32_t(uint64_t(blockIdx.x) * a.nchunks / a.hist_grid);
+  const uint32_t c1 = uint32_t(uint64_t(blockIdx.x + 1) * a.nchunks / a.hist_grid);
   for (uint32_t c = c0; c < c1; c++) {
     const uint64_t first = uint64_t(c) * a.chunk_rows, end = min(a.n, first + a.chunk_rows);
     uint32_t n_null = 0, n_nan = 0;
@@ -826,12 +827,12 @@ __global__ void __launch_bounds__(HTHREADS) bucket_histogram_kernel(const __grid
 
 // One cluster: bucket starts, cursors, the chunks' null and NaN starts, and the decision.
 template <typename KeyT>
-__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(1024) bucket_starts_kernel(const __grid_constant__ Args a) {
+__device__ __forceinline__ void starts_body(const Args& a) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   __shared__ uint32_t s_warp[32], s_sum[CLUSTER], s_max[CLUSTER];
   State* st = a.st;
-  if (st->mode != MODE_BUCKETS) return;
+  if (a.one_launch || st->mode != MODE_BUCKETS) return;
   cl.sync();                             // every CTA runs before its shared memory is written
   constexpr uint32_t PER = 8;
   static_assert(MAX_BUCKETS <= CLUSTER * 1024 * PER, "one round of the cluster takes every bucket");
@@ -922,13 +923,12 @@ struct TileShared {
 };
 
 template <typename KeyT, int PAY>
-__global__ void __launch_bounds__(THREADS, 2) level1_kernel(const __grid_constant__ ColView col,
-                                                           const __grid_constant__ Args a) {
+__device__ __forceinline__ void level1_body(const ColView& col, const Args& a) {
   extern __shared__ __align__(16) unsigned char tsm[];
   using SM = TileShared<KeyT, PAY>;
   SM& sm = *reinterpret_cast<SM*>(tsm);
   const State* st = a.st;
-  if (st->mode != MODE_BUCKETS) return;
+  if (blockIdx.x >= a.nchunks || st->mode != MODE_BUCKETS) return;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const uint32_t lt = (1u << lane) - 1u;
   const uint32_t s2 = st->s2, nbins = st->bins1;
@@ -1125,12 +1125,12 @@ struct Tile2Shared {
 // Level 2: tiles of one level-1 bin's rows to its 128 buckets. A tile reserves its rows of a bucket with
 // one atomic.
 template <typename KeyT, int PAY>
-__global__ void __launch_bounds__(THREADS, 2) level2_kernel(const __grid_constant__ Args a) {
+__device__ __forceinline__ void level2_body(const Args& a) {
   extern __shared__ __align__(16) unsigned char tsm[];
   using SM = Tile2Shared<KeyT, PAY>;
   SM& sm = *reinterpret_cast<SM*>(tsm);
   const State* st = a.st;
-  if (st->mode != MODE_BUCKETS || st->s2 == 0) return;
+  if (blockIdx.x >= a.level2_grid || st->mode != MODE_BUCKETS || st->s2 == 0) return;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const uint32_t nbins = st->bins1, nb = st->buckets, nv = st->n_value;
   const Map<KeyT> map = load_map<KeyT>(st);
@@ -1144,8 +1144,8 @@ __global__ void __launch_bounds__(THREADS, 2) level2_kernel(const __grid_constan
   }
   const KeyT* __restrict__ kin = static_cast<const KeyT*>(a.keys[0]);
   KeyT* __restrict__ kout = static_cast<KeyT*>(a.keys[1]);
-  const uint32_t t0 = uint32_t(uint64_t(blockIdx.x) * ntiles / gridDim.x);
-  const uint32_t t1 = uint32_t(uint64_t(blockIdx.x + 1) * ntiles / gridDim.x);
+  const uint32_t t0 = uint32_t(uint64_t(blockIdx.x) * ntiles / a.level2_grid);
+  const uint32_t t1 = uint32_t(uint64_t(blockIdx.x + 1) * ntiles / a.level2_grid);
   if (t < BINS2) sm.start[t] = 0;
   __syncthreads();
   uint32_t d = 0;
@@ -1256,10 +1256,12 @@ __global__ void __launch_bounds__(THREADS, 2) level2_kernel(const __grid_constan
 
 // ---- 4. each bucket in shared memory
 
-// Row a before row b, their keys being equal: by row id, or first by the strings behind the keys.
+constexpr int TIES_ID = 0, TIES_STRING = 1;
+
+// Row a before row b, their keys being equal: by row id, or first by the strings behind them.
 template <int TIES>
 __device__ __forceinline__ bool tied_before(const StringTies& s, uint32_t a, uint32_t b) {
-  if constexpr (TIES != 0) {
+  if constexpr (TIES == TIES_STRING) {
     uint64_t oa, ob, la, lb;
     if (s.wide) {
       const int64_t* o = static_cast<const int64_t*>(s.offsets);
@@ -1357,12 +1359,12 @@ struct KeyOut {
 };
 
 template <typename KeyT, int PAY, int TIES>
-__global__ void __launch_bounds__(LTHREADS, LBLOCKS) bucket_sort_kernel(const __grid_constant__ Args a) {
+__device__ __forceinline__ void sort_body(const Args& a) {
   extern __shared__ __align__(16) unsigned char lsm[];
   using SM = LocalShared<KeyT, PAY>;
   SM& sm = *reinterpret_cast<SM*>(lsm);
   const State* st = a.st;
-  if (st->mode != MODE_BUCKETS) return;
+  if (blockIdx.x >= a.sort_grid || st->mode != MODE_BUCKETS) return;
   const uint32_t t = threadIdx.x;
   const uint32_t nb = st->buckets, src = st->s2 ? 1u : 0u;
   const uint64_t vbase = a.nulls_first ? uint64_t(st->n_null) + st->n_nan : 0ull;
@@ -1378,7 +1380,7 @@ __global__ void __launch_bounds__(LTHREADS, LBLOCKS) bucket_sort_kernel(const __
   int nit = 0;
   KeyT key[LITEMS];
   auto next_bucket = [&](uint32_t b) {             // the next one with rows, from b on
-    for (; b < nb; b += gridDim.x) {
+    for (; b < nb; b += a.sort_grid) {
       first = a.bpos[b];
       size = a.bpos[b + 1] - first;
       if (size == 0) continue;
@@ -1540,7 +1542,7 @@ __global__ void __launch_bounds__(LTHREADS, LBLOCKS) bucket_sort_kernel(const __
       }
     }
     // The next bucket's keys arrive while this one leaves.
-    const uint32_t bn = next_bucket(b + gridDim.x);
+    const uint32_t bn = next_bucket(b + a.sort_grid);
     if (bn < nb) load_rows();
     __syncthreads();
     if (fast) {
@@ -1642,6 +1644,74 @@ __global__ void __launch_bounds__(LTHREADS, LBLOCKS) bucket_sort_kernel(const __
     }
     __syncthreads();
   }
+}
+
+// ---- the launches: of one sort, and of a batch's sorts (one a row of the grid)
+
+template <typename KeyT>
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(1024)
+buckets_kernel(const __grid_constant__ ColView col, const __grid_constant__ Args a) {
+  buckets_body<KeyT>(col, a);
+}
+template <typename KeyT>
+__global__ void __launch_bounds__(HTHREADS)
+bucket_histogram_kernel(const __grid_constant__ ColView col, const __grid_constant__ Args a) {
+  histogram_body<KeyT>(col, a);
+}
+template <typename KeyT>
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(1024) bucket_starts_kernel(const __grid_constant__ Args a) {
+  starts_body<KeyT>(a);
+}
+template <typename KeyT, int PAY>
+__global__ void __launch_bounds__(THREADS, 2) level1_kernel(const __grid_constant__ ColView col, const __grid_constant__ Args a) {
+  level1_body<KeyT, PAY>(col, a);
+}
+template <typename KeyT, int PAY>
+__global__ void __launch_bounds__(THREADS, 2) level2_kernel(const __grid_constant__ Args a) {
+  level2_body<KeyT, PAY>(a);
+}
+template <typename KeyT, int PAY, int TIES>
+__global__ void __launch_bounds__(LTHREADS, LBLOCKS) bucket_sort_kernel(const __grid_constant__ Args a) {
+  sort_body<KeyT, PAY, TIES>(a);
+}
+
+struct alignas(16) BatchItem {
+  ColView col;
+  Args a;
+};
+__device__ __forceinline__ const BatchItem& batch_item(const BatchItem* __restrict__ items) {
+  __shared__ BatchItem it;
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(items + blockIdx.y);
+  for (uint32_t i = threadIdx.x; i < sizeof(BatchItem) / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(&it)[i] = src[i];
+  __syncthreads();
+  return it;
+}
+template <typename KeyT>
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(1024) batch_buckets_kernel(const BatchItem* __restrict__ items) {
+  const BatchItem& it = batch_item(items);
+  buckets_body<KeyT>(it.col, it.a);
+}
+template <typename KeyT>
+__global__ void __launch_bounds__(HTHREADS) batch_histogram_kernel(const BatchItem* __restrict__ items) {
+  const BatchItem& it = batch_item(items);
+  histogram_body<KeyT>(it.col, it.a);
+}
+template <typename KeyT>
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(1024) batch_starts_kernel(const BatchItem* __restrict__ items) {
+  starts_body<KeyT>(batch_item(items).a);
+}
+template <typename KeyT>
+__global__ void __launch_bounds__(THREADS, 2) batch_level1_kernel(const BatchItem* __restrict__ items) {
+  const BatchItem& it = batch_item(items);
+  level1_body<KeyT, 0>(it.col, it.a);
+}
+template <typename KeyT>
+__global__ void __launch_bounds__(THREADS, 2) batch_level2_kernel(const BatchItem* __restrict__ items) {
+  level2_body<KeyT, 0>(batch_item(items).a);
+}
+template <typename KeyT>
+__global__ void __launch_bounds__(LTHREADS, LBLOCKS) batch_sort_kernel(const BatchItem* __restrict__ items) {
+  sort_body<KeyT, 0, TIES_ID>(batch_item(items).a);
 }
 
 // ---- 5. the first k rows
@@ -1809,6 +1879,12 @@ static uint32_t bucket_cap(uint64_t n) {
   return uint32_t(std::min<uint64_t>(MAX_BUCKETS, (want + 1023) & ~uint64_t(1023)));
 }
 namespace {
+uint32_t rows_per_chunk(uint64_t n) {
+  const uint64_t per = (n + MAX_CHUNKS - 1) / MAX_CHUNKS;
+  return uint32_t((per + TILE - 1) / TILE * TILE);
+}
+uint32_t chunks_of(uint64_t n) { return n <= SAMPLES ? 0u : uint32_t((n + rows_per_chunk(n) - 1) / rows_per_chunk(n)); }
+
 struct Layout {
   size_t state, bcount, bmeta, zeroed, coarse, fine, bfirst, bpos, cursor1, cursor2, chunk_bins, chunk_cats, total;
   explicit Layout(uint64_t n) {
@@ -1829,8 +1905,8 @@ struct Layout {
     bpos = take((nb + 1) * 4);
     cursor1 = take(size_t(BINS1) * CUR_PAD * 4);
     cursor2 = take(nb * CUR_PAD * 4);
-    chunk_bins = take(size_t(MAX_CHUNKS) * BINS1 * 4);
-    chunk_cats = take(size_t(MAX_CHUNKS) * 8);
+    chunk_bins = take(size_t(chunks_of(n)) * BINS1 * 4);
+    chunk_cats = take(size_t(chunks_of(n)) * 8);
     total = at;
   }
 };
@@ -1848,7 +1924,6 @@ void launch_moves(const ColView& cv, const Args& a, cudaStream_t s) {
     smem_limit(level2_kernel<KeyT, PAY>, sizeof(Tile2Shared<KeyT, PAY>));
     smem_limit(bucket_sort_kernel<KeyT, PAY, TIES>, sizeof(LocalShared<KeyT, PAY>));
   });
-  const int sms = device().sm_count;
   if (!a.one_launch) {
     {
       KernelTimer kt("bucket_level1", s);
@@ -1857,14 +1932,13 @@ void launch_moves(const ColView& cv, const Args& a, cudaStream_t s) {
     }
     if (a.bucket_cap > a.bins1_cap) {
       KernelTimer kt("bucket_level2", s);
-      level2_kernel<KeyT, PAY><<<sms * 2, THREADS, sizeof(Tile2Shared<KeyT, PAY>), s>>>(a);
+      level2_kernel<KeyT, PAY><<<a.level2_grid, THREADS, sizeof(Tile2Shared<KeyT, PAY>), s>>>(a);
       AM_CUDA(cudaGetLastError());
     }
   }
   {
     KernelTimer kt("bucket_sort", s);
-    const int grid = int(std::min<uint32_t>(a.bucket_cap, uint32_t(sms * LBLOCKS)));
-    bucket_sort_kernel<KeyT, PAY, TIES><<<grid, LTHREADS, sizeof(LocalShared<KeyT, PAY>), s>>>(a);
+    bucket_sort_kernel<KeyT, PAY, TIES><<<a.sort_grid, LTHREADS, sizeof(LocalShared<KeyT, PAY>), s>>>(a);
     AM_CUDA(cudaGetLastError());
   }
 }
@@ -1881,8 +1955,7 @@ void launch_all(const Sort& b, const Args& a, int pay, cudaStream_t s) {
     std::call_once(once, [] { smem_limit(bucket_histogram_kernel<KeyT>, size_t(MAX_BUCKETS) * 4); });
     {
       KernelTimer kt("bucket_histogram", s);
-      const int grid = int(std::min<uint32_t>(a.nchunks, uint32_t(device().sm_count)));
-      bucket_histogram_kernel<KeyT><<<grid, HTHREADS, size_t(a.bucket_cap) * 4, s>>>(b.col, a);
+      bucket_histogram_kernel<KeyT><<<a.hist_grid, HTHREADS, size_t(a.bucket_cap) * 4, s>>>(b.col, a);
       AM_CUDA(cudaGetLastError());
     }
     {
@@ -1893,12 +1966,12 @@ void launch_all(const Sort& b, const Args& a, int pay, cudaStream_t s) {
   }
   if constexpr (sizeof(KeyT) == 8) {
     if (a.ties.offsets) {
-      launch_moves<KeyT, 0, 1>(b.col, a, s);
+      launch_moves<KeyT, 0, TIES_STRING>(b.col, a, s);
       return;
     }
   }
-  if (pay) launch_moves<KeyT, 1, 0>(b.col, a, s);
-  else launch_moves<KeyT, 0, 0>(b.col, a, s);
+  if (pay) launch_moves<KeyT, 1, TIES_ID>(b.col, a, s);
+  else launch_moves<KeyT, 0, TIES_ID>(b.col, a, s);
 }
 }  // namespace
 
@@ -1925,11 +1998,13 @@ void enqueue_first(const ColView& col, int key_bytes, uint64_t n, uint64_t k, Fi
 size_t scratch_bytes(uint64_t n) { return Layout(n).total; }
 size_t zeroed_bytes(uint64_t n) { return Layout(n).zeroed; }
 
-State* enqueue(const Sort& b, cudaStream_t s) {
+static Args make_args(const Sort& b) {
   const Layout L(b.n);
-  auto at = [&](size_t off) { return reinterpret_cast<uint32_t*>(b.scratch + off); };
+  auto at = [&](size_t off) {
+    return reinterpret_cast<uint32_t*>(off < L.zeroed && b.zeroed ? b.zeroed + off : b.scratch + off);
+  };
   Args a{};
-  a.st = reinterpret_cast<State*>(b.scratch + L.state);
+  a.st = reinterpret_cast<State*>(at(L.state));
   a.coarse = at(L.coarse);
   a.fine = at(L.fine);
   a.bfirst = at(L.bfirst);
@@ -1942,9 +2017,8 @@ State* enqueue(const Sort& b, cudaStream_t s) {
   a.chunk_cats = at(L.chunk_cats);
   a.nsamples = uint32_t(std::min<uint64_t>(b.n, SAMPLES));
   a.bucket_cap = bucket_cap(b.n);
-  const uint64_t per = (b.n + MAX_CHUNKS - 1) / MAX_CHUNKS;
-  a.chunk_rows = uint32_t((per + TILE - 1) / TILE * TILE);
-  a.nchunks = uint32_t((b.n + a.chunk_rows - 1) / a.chunk_rows);
+  a.chunk_rows = rows_per_chunk(b.n);
+  a.nchunks = chunks_of(b.n);
   a.n = b.n;
   for (int i = 0; i < 2; i++) {
     a.keys[i] = b.keys[i];
@@ -1971,7 +2045,6 @@ State* enqueue(const Sort& b, cudaStream_t s) {
   a.err = b.err;
   a.sum = b.summary;
   if (b.payload) a.pay = b.rec;
-  const int pay = b.payload ? 1 : 0;
   a.bins1_cap = b.payload ? BINS1 / 2 : BINS1;
   a.has_payload = b.payload ? 1 : 0;
   a.one_launch = b.n <= SAMPLES ? 1 : 0;
@@ -1979,9 +2052,92 @@ State* enqueue(const Sort& b, cudaStream_t s) {
     a.bucket_cap = std::min(a.bucket_cap, ONE_CAP);
     a.bins1_cap = ONE_CAP;
   }
+  const uint32_t sms = uint32_t(device().sm_count);
+  a.hist_grid = std::min(a.nchunks, sms);
+  a.level2_grid = uint32_t(std::min<uint64_t>((b.n + TILE - 1) / TILE, sms * 2));
+  a.sort_grid = uint32_t(std::min<uint64_t>(b.n / (TARGET / 2) + 3, sms * LBLOCKS));
+  return a;
+}
+
+State* enqueue(const Sort& b, cudaStream_t s) {
+  const Args a = make_args(b);
+  const int pay = b.payload ? 1 : 0;
   if (b.key_bytes == 8) launch_all<uint64_t>(b, a, pay, s);
   else launch_all<uint32_t>(b, a, pay, s);
   return a.st;
+}
+
+size_t batch_item_bytes() { return sizeof(BatchItem); }
+
+void fill_batch_item(const Sort& b, void* item) {
+  BatchItem it{};
+  it.col = b.col;
+  it.a = make_args(b);
+  std::memcpy(item, &it, sizeof(it));
+}
+
+namespace {
+template <typename KeyT>
+void launch_batch(const BatchItem* items, const BatchItem* host, uint32_t count, bool timed, cudaStream_t s) {
+  prepare_batch(int(sizeof(KeyT)));
+  uint32_t hist = 0, chunks = 0, level2 = 0, sort = 0, cap = 0;
+  for (uint32_t i = 0; i < count; i++) {
+    const Args& a = host[i].a;
+    sort = std::max(sort, a.sort_grid);
+    if (a.one_launch) continue;
+    hist = std::max(hist, a.hist_grid);
+    chunks = std::max(chunks, a.nchunks);
+    cap = std::max(cap, a.bucket_cap);
+    if (a.bucket_cap > a.bins1_cap) level2 = std::max(level2, a.level2_grid);
+  }
+  // A grid has at most 65,535 rows.
+  for (uint32_t at = 0; at < count; at += 65535) {
+    const uint32_t rows = std::min<uint32_t>(count - at, 65535);
+    const BatchItem* it = items + at;
+    auto step = [&](const char* name, auto&& launch) {
+      std::unique_ptr<KernelTimer> kt(timed ? new KernelTimer(name, s) : nullptr);
+      launch();
+      AM_CUDA(cudaGetLastError());
+    };
+    step("batch_plan", [&] { batch_buckets_kernel<KeyT><<<dim3(CLUSTER, rows), 1024, 0, s>>>(it); });
+    if (hist) {
+      step("batch_histogram", [&] { batch_histogram_kernel<KeyT><<<dim3(hist, rows), HTHREADS, size_t(cap) * 4, s>>>(it); });
+      step("batch_scan", [&] { batch_starts_kernel<KeyT><<<dim3(CLUSTER, rows), 1024, 0, s>>>(it); });
+      step("batch_level1", [&] {
+        batch_level1_kernel<KeyT><<<dim3(chunks, rows), THREADS, sizeof(TileShared<KeyT, 0>), s>>>(it);
+      });
+    }
+    if (level2)
+      step("batch_level2", [&] {
+        batch_level2_kernel<KeyT><<<dim3(level2, rows), THREADS, sizeof(Tile2Shared<KeyT, 0>), s>>>(it);
+      });
+    step("batch_sort", [&] {
+      batch_sort_kernel<KeyT><<<dim3(sort, rows), LTHREADS, sizeof(LocalShared<KeyT, 0>), s>>>(it);
+    });
+  }
+}
+template <typename KeyT>
+void prepare() {
+  static std::once_flag once;
+  std::call_once(once, [] {
+    smem_limit(batch_histogram_kernel<KeyT>, size_t(MAX_BUCKETS) * 4);
+    smem_limit(batch_level1_kernel<KeyT>, sizeof(TileShared<KeyT, 0>));
+    smem_limit(batch_level2_kernel<KeyT>, sizeof(Tile2Shared<KeyT, 0>));
+    smem_limit(batch_sort_kernel<KeyT>, sizeof(LocalShared<KeyT, 0>));
+  });
+}
+}  // namespace
+
+void prepare_batch(int key_bytes) {
+  if (key_bytes == 8) prepare<uint64_t>();
+  else prepare<uint32_t>();
+}
+
+void enqueue_batch(const void* items, const void* host_items, uint32_t count, int key_bytes, bool timed, cudaStream_t s) {
+  const BatchItem* it = static_cast<const BatchItem*>(items);
+  const BatchItem* h = static_cast<const BatchItem*>(host_items);
+  if (key_bytes == 8) launch_batch<uint64_t>(it, h, count, timed, s);
+  else launch_batch<uint32_t>(it, h, count, timed, s);
 }
 
 }  // namespace bs

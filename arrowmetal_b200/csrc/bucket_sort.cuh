@@ -47,6 +47,7 @@ struct Sort {
   const void* src_keys;                  // not NULL: at most MAX_PAIRS rows given as keys and row ids, no column
   const uint32_t* src_ids;
   char* scratch;                         // `scratch_bytes(n)` bytes, the first `zeroed_bytes(n)` zero
+  char* zeroed;                          // not NULL: those zero bytes are here instead
   void* keys[2];                         // n keys each
   char* ids[2];                          // n x 4 bytes, or n x 16 with a payload
   StringTies ties;
@@ -72,6 +73,12 @@ size_t zeroed_bytes(uint64_t n);
 // Enqueues the sort; afterwards State::mode says whether it ran (MODE_BUCKETS) or its rows are as they
 // were (MODE_FALLBACK: the digit passes must run). Returns the State on the device.
 State* enqueue(const Sort& b, cudaStream_t s);
+// A batch of sorts of one key width in one launch a step: an item a sort, filled on the host, read by the
+// kernels from device memory (no payload, no strings). `prepare_batch` before a stream is captured.
+size_t batch_item_bytes();
+void fill_batch_item(const Sort& b, void* item);
+void prepare_batch(int key_bytes);
+void enqueue_batch(const void* items, const void* host_items, uint32_t count, int key_bytes, bool timed, cudaStream_t s);
 // Enqueues the choice of a key limit that at least the k smallest value keys are almost surely within, and
 // one read of the column that appends the rows within it, as (key, row id) pairs in no order, to arrays
 // of MAX_PAIRS; fs->count says how many there are. n is at least MAX_PAIRS.

@@ -21,6 +21,7 @@
 // inside its first pass.
 #include <algorithm>
 #include <atomic>
+#include <cstddef>
 #include <cstdlib>
 #include <list>
 #include <memory>
@@ -1216,28 +1217,62 @@ struct AllPassesArgs {
   uint64_t status16;         // the look-back words, in 16-byte units
 };
 
+// False when a barrier ran out.
 template <typename KeyT, int THREADS, int ITEMS, bool REC>
-__global__ void __launch_bounds__(THREADS, 2)
-all_passes_kernel(const __grid_constant__ AllPassesArgs a, const __grid_constant__ ColView col) {
-  if (*a.mode != bs::MODE_FALLBACK) return;
+__device__ __forceinline__ bool run_all_passes(const AllPassesArgs& a, const ColView& col) {
   uint32_t round = 0;
   constexpr int HI = 4;
   constexpr uint64_t CHUNK = uint64_t(THREADS) * HI;
   histogram_rows<KeyT, THREADS, HI, false>(col, a.stats, uint64_t(blockIdx.x) * CHUNK, a.plan.n, uint64_t(gridDim.x) * CHUNK);
-  if (!grid_barrier(a.arrived, round, a.pass.err)) return;
+  if (!grid_barrier(a.arrived, round, a.pass.err)) return false;
   if (blockIdx.x == 0) {
     plan_body(a.plan, a.stats, a.kplan, a.desc, a.sum);
     // The sample and the count read the rows before the passes.
     if (threadIdx.x == 0) a.sum->passes_run += 2;
   }
   for (int sl = 0; sl < a.plan.nslots; sl++) {
-    if (!grid_barrier(a.arrived, round, a.pass.err)) return;
+    if (!grid_barrier(a.arrived, round, a.pass.err)) return false;
     if (!*reinterpret_cast<const volatile uint32_t*>(&a.desc[sl].active)) continue;
     uint4* words = static_cast<uint4*>(a.pass.status);
     for (uint64_t i = uint64_t(blockIdx.x) * THREADS + threadIdx.x; i < a.status16; i += uint64_t(gridDim.x) * THREADS)
       words[i] = make_uint4(0, 0, 0, 0);
-    if (!grid_barrier(a.arrived, round, a.pass.err)) return;
+    if (!grid_barrier(a.arrived, round, a.pass.err)) return false;
     onesweep_pass<KeyT, uint32_t, THREADS, ITEMS, false, REC>(a.pass, col, a.desc + sl, a.tickets + sl, 0u);
+  }
+  return true;
+}
+
+template <typename KeyT, int THREADS, int ITEMS, bool REC>
+__global__ void __launch_bounds__(THREADS, 2)
+all_passes_kernel(const __grid_constant__ AllPassesArgs a, const __grid_constant__ ColView col) {
+  if (*a.mode != bs::MODE_FALLBACK) return;
+  (void)run_all_passes<KeyT, THREADS, ITEMS, REC>(a, col);
+}
+
+// The same for a batch's arrays, one after the other by the whole grid: those whose buckets were too large.
+struct alignas(16) AllPassesItem {
+  AllPassesArgs a;
+  ColView col;
+};
+template <typename KeyT, int THREADS, int ITEMS>
+__global__ void __launch_bounds__(THREADS, 2)
+batch_all_passes_kernel(const AllPassesItem* __restrict__ items, const uint32_t* const* __restrict__ modes, uint32_t count) {
+  __shared__ AllPassesItem it;
+  for (uint32_t base = 0; base < count; base += THREADS) {
+    // A block's threads look at as many arrays at once; most batches have none to do.
+    const bool mine = base + threadIdx.x < count && *modes[base + threadIdx.x] == bs::MODE_FALLBACK;
+    if (!__syncthreads_or(int(mine))) continue;
+    for (uint32_t i = base; i < count && i < base + THREADS; i++) {
+      if (*modes[i] != bs::MODE_FALLBACK) continue;
+      __syncthreads();
+      const uint32_t* src = reinterpret_cast<const uint32_t*>(items + i);
+      for (uint32_t w = threadIdx.x; w < sizeof(AllPassesItem) / 4; w += THREADS) reinterpret_cast<uint32_t*>(&it)[w] = src[w];
+      __syncthreads();
+      if (!run_all_passes<KeyT, THREADS, ITEMS, false>(it.a, it.col)) return;
+      // The next array uses the same look-back words.
+      uint32_t round = 0;
+      if (!grid_barrier(it.a.arrived + 1, round, it.a.pass.err)) return;
+    }
   }
 }
 
@@ -2695,6 +2730,227 @@ void sort_segment_class(const std::vector<SortKey>& keys, const std::vector<void
   dfree(base, s);
 }
 
+// The arrays of a size class by the bucket sort (bucket_sort.cu), every step one launch for all of them,
+// then the digit passes of the arrays whose buckets were too large. 48 arrays of 1e3 to 1e6 rows (int64 and
+// float32): the graph's kernels 737 us as digit passes, 481 so, the call 1,300 and 973; six steps each with
+// work for the whole chip take the place of up to ten passes that wait on one another's tiles.
+template <typename KeyT>
+struct BucketLayout {
+  static constexpr size_t up(size_t b) { return (b + 255) & ~size_t(255); }
+  static constexpr size_t kOffKplan = sizeof(KeyStats), kOffDesc = (kOffKplan + sizeof(KeyPlan) + 255) & ~size_t(255);
+  static constexpr size_t kOffTick = (kOffDesc + sizeof(PassDesc) * MAX_ONE_KEY + 255) & ~size_t(255);
+  static constexpr size_t kOffSum = kOffTick + sizeof(uint32_t) * (MAX_ONE_KEY + 4);
+  static constexpr size_t kOffBs = (kOffSum + sizeof(SortSummary) + 255) & ~size_t(255);
+  uint32_t G = 0;
+  std::vector<uint32_t> lens;
+  size_t off_passes = 0, off_modes = 0, tables = 0, off_zeroed = 0, zeroed = 0, total = 0;
+  uint64_t max_tiles = 0;
+  std::vector<size_t> z_at, s_at, k_at, i_at;           // each array's zeroed bytes, tables, keys, ids
+
+  BucketLayout(const std::vector<SortKey>& keys, const std::vector<size_t>& group) {
+    G = uint32_t(group.size());
+    off_passes = up(bs::batch_item_bytes() * G);
+    off_modes = up(off_passes + sizeof(AllPassesItem) * G);
+    tables = up(off_modes + sizeof(void*) * G);
+    off_zeroed = tables;
+    size_t at = off_zeroed;
+    for (size_t i : group) {
+      const uint64_t n = uint64_t(keys[i].col->length);
+      lens.push_back(uint32_t(n));
+      max_tiles = std::max(max_tiles, (n + min_super() - 1) / min_super());
+      z_at.push_back(at);
+      at = up(at + kOffBs + bs::zeroed_bytes(n));
+    }
+    zeroed = at - off_zeroed;
+    for (size_t i : group) {
+      const uint64_t n = uint64_t(keys[i].col->length);
+      s_at.push_back(at);
+      at = up(at + bs::scratch_bytes(n));
+      k_at.push_back(at);
+      at += 2 * up(n * sizeof(KeyT));
+      i_at.push_back(at);
+      at += 2 * up(n * 4);
+    }
+    total = at;
+  }
+
+  // The tables, for scratch at `base`.
+  std::vector<char> fill(const std::vector<SortKey>& keys, const std::vector<void*>& outs, const std::vector<size_t>& group,
+                         char* base, void* status, uint32_t* err) const {
+    std::vector<char> host(tables, 0);
+    for (uint32_t g = 0; g < G; g++) {
+      const SortKey& key = keys[group[g]];
+      const uint64_t n = lens[g];
+      char* z = base + z_at[g];
+      bs::Sort b{};
+      b.col = make_view(key);
+      b.key_bytes = int(sizeof(KeyT));
+      b.n = n;
+      b.zeroed = z + kOffBs;
+      b.scratch = base + s_at[g];
+      for (int i = 0; i < 2; i++) {
+        b.keys[i] = base + k_at[g] + size_t(i) * up(n * sizeof(KeyT));
+        b.ids[i] = base + i_at[g] + size_t(i) * up(n * 4);
+      }
+      b.out = outs[group[g]];
+      b.key_pt = key.col->pt;
+      b.key_desc = key.descending;
+      b.nulls_first = key.nulls_first;
+      b.err = err;
+      b.summary = reinterpret_cast<SortSummary*>(z + kOffSum);
+      bs::fill_batch_item(b, host.data() + bs::batch_item_bytes() * g);
+
+      AllPassesItem it{};
+      AllPassesArgs& a = it.a;
+      it.col = b.col;
+      for (int i = 0; i < 2; i++) {
+        a.pass.keys[i] = b.keys[i];
+        a.pass.ids[i] = reinterpret_cast<uint32_t*>(b.ids[i]);
+      }
+      a.kplan = reinterpret_cast<KeyPlan*>(z + kOffKplan);
+      a.pass.kplan = a.kplan;
+      a.pass.final_out = b.out;
+      a.pass.status = status;
+      a.pass.err = err;
+      a.pass.carry_ids = 1;
+      a.plan.n = n;
+      a.plan.nkeys = 1;
+      a.plan.nslots = int(sizeof(KeyT));
+      a.plan.key_bytes[0] = uint8_t(sizeof(KeyT));
+      a.plan.nulls_first[0] = key.nulls_first ? 1 : 0;
+      for (int d = 0; d < int(sizeof(KeyT)); d++) a.plan.slot_digit[d] = int8_t(d);
+      a.stats = reinterpret_cast<KeyStats*>(z);
+      a.desc = reinterpret_cast<PassDesc*>(z + kOffDesc);
+      a.sum = b.summary;
+      a.tickets = reinterpret_cast<uint32_t*>(z + kOffTick);
+      a.arrived = a.tickets + MAX_ONE_KEY;
+      a.mode = reinterpret_cast<const uint32_t*>(z + kOffBs + offsetof(bs::State, mode));
+      a.status16 = ((n + min_super() - 1) / min_super() * NBINS * sizeof(uint32_t) + 15) / 16;
+      std::memcpy(host.data() + off_passes + sizeof(AllPassesItem) * g, &it, sizeof(it));
+      std::memcpy(host.data() + off_modes + sizeof(void*) * g, &a.mode, sizeof(void*));
+    }
+    return host;
+  }
+};
+
+template <typename KeyT>
+int batch_all_passes_blocks() {
+  using C = PassConfig<KeyT>;
+  static int blocks = 0;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    auto fn = batch_all_passes_kernel<KeyT, C::THREADS, C::ITEMS>;
+    AM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(pass_smem<KeyT>())));
+    AM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, C::THREADS, pass_smem<KeyT>()));
+  });
+  if (blocks < 1) throw Error("radix sort: the digit passes do not fit the device");
+  return blocks;
+}
+
+template <typename KeyT>
+void enqueue_buckets(const BucketLayout<KeyT>& L, char* base, const void* pinned_tables, const char* host_tables, bool timed,
+                     cudaStream_t s) {
+  using C = PassConfig<KeyT>;
+  if (pinned_tables) AM_CUDA(cudaMemcpyAsync(base, pinned_tables, L.tables, cudaMemcpyHostToDevice, s));
+  AM_CUDA(cudaMemsetAsync(base + L.off_zeroed, 0, L.zeroed, s));
+  bs::enqueue_batch(base, host_tables, L.G, int(sizeof(KeyT)), timed, s);
+  const int grid = int(std::max<uint64_t>(1, std::min<uint64_t>(L.max_tiles, uint64_t(device().sm_count) * batch_all_passes_blocks<KeyT>())));
+  const AllPassesItem* items = reinterpret_cast<const AllPassesItem*>(base + L.off_passes);
+  const uint32_t* const* modes = reinterpret_cast<const uint32_t* const*>(base + L.off_modes);
+  uint32_t count = L.G;
+  void* args[] = {&items, &modes, &count};
+  std::unique_ptr<KernelTimer> kt(timed ? new KernelTimer("batch_all_passes", s) : nullptr);
+  AM_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(batch_all_passes_kernel<KeyT, C::THREADS, C::ITEMS>),
+                                      dim3(uint32_t(grid)), dim3(C::THREADS), args, pass_smem<KeyT>(), s));
+}
+
+template <typename KeyT>
+void sort_segment_buckets(const std::vector<SortKey>& keys, const std::vector<void*>& outs, const std::vector<size_t>& group_in,
+                          bool allow_graph, cudaStream_t s) {
+  std::vector<size_t> group, large;
+  for (size_t i : group_in) (uint64_t(keys[i].col->length) <= bs::MAX_ROWS ? group : large).push_back(i);
+  if (!large.empty()) sort_segment_class<KeyT, 512, 8>(keys, outs, large, allow_graph, s);
+  if (group.empty()) return;
+  BucketLayout<KeyT> L(keys, group);
+  const size_t status_bytes = size_t(L.max_tiles) * NBINS * sizeof(uint32_t);
+  StreamScratch& sc = stream_scratch(s, (status_bytes + 7) / 8);
+  sc.epoch = (1u << 30) - 1;               // its words are used without an epoch: later users start over
+  bs::prepare_batch(int(sizeof(KeyT)));
+  (void)batch_all_passes_blocks<KeyT>();
+  if (allow_graph && graphs_enabled() && L.total <= kGraphMaxScratch) {
+    GraphCache& c = graph_cache();
+    const int width = int(sizeof(KeyT)) * 100000 + 99999;        // no tile shape has this code
+    BatchGraph* g = nullptr;
+    for (auto it = c.graphs.begin(); it != c.graphs.end(); ++it)
+      if ((*it)->width == width && (*it)->stream == s && (*it)->lens == L.lens) {
+        c.graphs.splice(c.graphs.begin(), c.graphs, it);
+        g = c.graphs.front().get();
+        break;
+      }
+    if (!g) {
+      bool seen = false;
+      for (auto& sh : c.seen)
+        if (sh.first == width && sh.second == L.lens) seen = true;
+      if (!seen) {
+        c.seen.emplace_front(width, L.lens);
+        if (c.seen.size() > 16) c.seen.pop_back();
+      } else {
+        auto ng = std::make_unique<BatchGraph>();
+        ng->width = width;
+        ng->stream = s;
+        ng->lens = L.lens;
+        ng->tables = L.tables;
+        AM_CUDA(cudaMalloc(reinterpret_cast<void**>(&ng->base), L.total));
+        AM_CUDA(cudaMalloc(&ng->status, std::max<size_t>(status_bytes + 16, 16)));
+        const std::vector<char> host = L.fill(keys, outs, group, ng->base, ng->status, sc.err);
+        for (auto& sl : ng->slot) {
+          sl.host = pinned_alloc(L.tables);
+          AM_CUDA(cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming));
+          cudaGraph_t graph = nullptr;
+          AM_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+          try {
+            enqueue_buckets<KeyT>(L, ng->base, sl.host, host.data(), false, s);
+          } catch (...) {
+            cudaGraph_t discard = nullptr;
+            (void)cudaStreamEndCapture(s, &discard);
+            if (discard) (void)cudaGraphDestroy(discard);
+            throw;
+          }
+          AM_CUDA(cudaStreamEndCapture(s, &graph));
+          const cudaError_t e = cudaGraphInstantiate(&sl.exec, graph, 0);
+          (void)cudaGraphDestroy(graph);
+          AM_CUDA(e);
+        }
+        c.graphs.push_front(std::move(ng));
+        if (c.graphs.size() > kGraphCacheEntries) c.graphs.pop_back();
+        g = c.graphs.front().get();
+      }
+    }
+    if (g) {
+      BatchGraph::Slot& sl = g->slot[g->next];
+      g->next ^= 1;
+      if (sl.launched) AM_CUDA(cudaEventSynchronize(sl.done));
+      const std::vector<char> host = L.fill(keys, outs, group, g->base, g->status, sc.err);
+      std::memcpy(sl.host, host.data(), L.tables);
+      KernelTimer kt("batch_graph", s);
+      AM_CUDA(cudaGraphLaunch(sl.exec, s));
+      AM_CUDA(cudaEventRecord(sl.done, s));
+      sl.launched = true;
+      return;
+    }
+  }
+  char* base = static_cast<char*>(dmalloc(L.total, s));
+  try {
+    const std::vector<char> host = L.fill(keys, outs, group, base, sc.status, sc.err);
+    copy_h2d(base, host.data(), L.tables, s);
+    enqueue_buckets<KeyT>(L, base, nullptr, host.data(), true, s);
+  } catch (...) {
+    dfree(base, s);
+    throw;
+  }
+  dfree(base, s);
+}
+
 // One launch sorts every array of a size class that fits a CTA (at most CTA_SORT_ROWS rows).
 template <typename KeyT, int THREADS, int ITEMS, int DBITS>
 void sort_segment_cta(const std::vector<SortKey>& keys, const std::vector<void*>& outs,
@@ -2735,14 +2991,17 @@ void sort_segment_cta(const std::vector<SortKey>& keys, const std::vector<void*>
 //
 // A batch's arrays of one key width fall into three size classes: up to CTA_SORT_ROWS rows, up to
 // SMALL_ARRAY_ROWS, and larger. Each class has its candidate shapes: the digit passes with a tile of
-// `threads` x `items` rows, or (the smallest class) one CTA per array with `threads` threads, `items`
-// rows a thread and `digit_bits`-bit digits. The first batch whose class holds at least its class's
+// `threads` x `items` rows, (the smallest class) one CTA per array with `threads` threads, `items`
+// rows a thread and `digit_bits`-bit digits, or (the larger ones) the bucket sort. The first batch whose class holds at least its class's
 // tuning rows (2^18, 2^20 and 2^21 rows) runs the class with every candidate, timed by CUDA events (each run leaves the same,
 // final output), and the fastest serves the class from then on. ARROWMETAL_SEG_ITEMS=4 or 8 fixes the
 // passes' tile at 512 x 4 or 512 x 8 rows for every class instead.
 constexpr uint32_t CTA_SORT_ROWS = 4096;
 constexpr uint32_t SMALL_ARRAY_ROWS = 16384;
 constexpr int SEG_CLASSES = 3;
+// Small arrays beyond which an untuned batch gives each one CTA. A bucket sort's plan is a cluster of eight
+// CTAs an array, some eighteen of which run at a time: up to here one round or two beside the larger arrays'.
+constexpr size_t CTA_SORT_ARRAYS = 32;
 
 struct SegShape {
   int method;          // 0: digit passes, 1: one CTA per array
@@ -2751,11 +3010,13 @@ struct SegShape {
 constexpr SegShape kSegShapes[] = {
     {0, 512, 8, 8}, {0, 512, 4, 8}, {0, 384, 12, 8},
     {1, 256, 16, 8}, {1, 256, 16, 4}, {1, 512, 8, 8}, {1, 512, 8, 4},
+    {0, 512, 7, 8},      // the bucket sort's passes
 };
+constexpr int BUCKET_SHAPE = 7;
 constexpr int kNumSegShapes = int(sizeof(kSegShapes) / sizeof(kSegShapes[0]));
 const std::vector<int>& class_candidates(int cls) {
-  static const std::vector<int> c0 = {3, 4, 5, 6, 1}, c12 = {0, 1, 2};
-  static_assert(kNumSegShapes == 7, "every shape is a candidate of some class");
+  static const std::vector<int> c0 = {3, 4, 5, 6, 1}, c12 = {BUCKET_SHAPE, 0, 1, 2};
+  static_assert(kNumSegShapes == 8, "every shape is a candidate of some class");
   return cls == 0 ? c0 : c12;
 }
 uint64_t class_tune_rows(int cls) { return cls == 0 ? (uint64_t(1) << 18) : cls == 1 ? (uint64_t(1) << 20) : (uint64_t(2) << 20); }
@@ -2789,7 +3050,8 @@ void run_segment_shape(int shape, const std::vector<SortKey>& keys, const std::v
     case 3: sort_segment_cta<KeyT, 256, 16, 8>(keys, outs, group, s); break;
     case 4: sort_segment_cta<KeyT, 256, 16, 4>(keys, outs, group, s); break;
     case 5: sort_segment_cta<KeyT, 512, 8, 8>(keys, outs, group, s); break;
-    default: sort_segment_cta<KeyT, 512, 8, 4>(keys, outs, group, s); break;
+    case 6: sort_segment_cta<KeyT, 512, 8, 4>(keys, outs, group, s); break;
+    default: sort_segment_buckets<KeyT>(keys, outs, group, allow_graph, s); break;
   }
 }
 
@@ -2805,6 +3067,7 @@ void sort_segment_group(const std::vector<SortKey>& keys, const std::vector<void
     cls_rows[c] += n;
   }
   const int width = int(sizeof(KeyT));
+  std::vector<size_t> buckets;             // arrays of every class that sorts by buckets: one batch of launches
   for (int c = 0; c < SEG_CLASSES; c++) {
     if (cls[c].empty()) continue;
     if (const int f = forced_items()) {
@@ -2824,6 +3087,8 @@ void sort_segment_group(const std::vector<SortKey>& keys, const std::vector<void
       AM_CUDA(cudaEventCreate(&e0));
       AM_CUDA(cudaEventCreate(&e1));
       for (size_t k = 0; k < cand.size(); k++) {
+        // Once before: the first run of a shape loads its kernels and grows the scratch.
+        run_segment_shape<KeyT>(cand[k], keys, outs, cls[c], false, s);
         AM_CUDA(cudaEventRecord(e0, s));
         run_segment_shape<KeyT>(cand[k], keys, outs, cls[c], false, s);
         AM_CUDA(cudaEventRecord(e1, s));
@@ -2837,9 +3102,12 @@ void sort_segment_group(const std::vector<SortKey>& keys, const std::vector<void
       g_tuned_shape[width == 8][c] = cand[best];
       continue;
     }
-    if (shape < 0) shape = c == 0 ? 5 : 0;     // untuned: one CTA per array, or 512 x 8 tiles
-    run_segment_shape<KeyT>(shape, keys, outs, cls[c], true, s);
+    // Untuned: buckets, but one CTA per array for many small ones (a cluster each would queue for the SMs).
+    if (shape < 0) shape = c == 0 && cls[c].size() > CTA_SORT_ARRAYS ? 5 : BUCKET_SHAPE;
+    if (shape == BUCKET_SHAPE) buckets.insert(buckets.end(), cls[c].begin(), cls[c].end());
+    else run_segment_shape<KeyT>(shape, keys, outs, cls[c], true, s);
   }
+  if (!buckets.empty()) run_segment_shape<KeyT>(BUCKET_SHAPE, keys, outs, buckets, true, s);
 }
 
 }  // namespace

@@ -179,3 +179,17 @@ def test_autotuner_records_its_choice_per_size_class(am, oracle):
             assert c == 0 and s["threads"] * s["items"] >= 4096
     assert shapes[(8, 0)]["max_rows"] == 4096 and shapes[(8, 2)]["max_rows"] == -1
     check_batch(am, oracle, arrays, opts)
+
+
+@pytest.mark.parametrize("kinds", [("int64", "int64_small", "float64"), ("float32", "int8", "int32")])
+def test_batches_by_buckets(am, oracle, kinds):
+    # One launch a step for arrays of one launch each (up to 65,536 rows) and of all steps, with arrays of
+    # few values (no bucket holds them: their digit passes run behind), small ones beside them, and the
+    # same shapes again (a graph replays).
+    rng = np.random.default_rng(500 + len(kinds[0]))
+    lengths = [4097, 65_535, 65_536, 65_537, 7, 0, 1000, 300_007, 20_011, 130_000, 1, 700_001]
+    arrays = [random_array(rng, kinds[i % 3], n) for i, n in enumerate(lengths)]
+    arrays.append(random_array(rng, "int64_small" if kinds[0] == "int64" else "int8", 250_003))
+    for call in range(4):
+        opts = [(bool(rng.integers(2)), PLACEMENTS[rng.integers(2)], ORDERS[rng.integers(3)]) for _ in arrays]
+        check_batch(am, oracle, arrays, opts)
