@@ -349,6 +349,11 @@ am_array* radix_partition_nth(const SortKey& key, int64_t pivot, cudaStream_t s)
 enum RankFn : int {
   RANK_MIN = 0, RANK_MAX, RANK_FIRST, RANK_DENSE, RANK_QUANTILE, RANK_NORMAL64, RANK_NORMAL32, RANK_PERCENT, RANK_CUME
 };
+// Ranks (min, max or first) of a column's rows straight out of the bucket sort: false when it does not
+// take them. Otherwise either ranks[] holds them, or (the buckets being too large) perm[] holds the
+// column's order; *mode (device memory) says which: bs::MODE_FALLBACK for the order.
+bool rank_by_buckets(const SortKey& key, int64_t n, int fn, bool merge_nan, uint32_t* ranks, uint32_t* perm, uint32_t* mode,
+                     cudaStream_t s);
 am_array* rank_of(am_array* a, int fn, bool desc, bool nulls_first, bool merge_nan, cudaStream_t s,
                   int float_order = 0);
 // The distinct values, ascending or in order of first appearance; `counts_out` (may be NULL) receives

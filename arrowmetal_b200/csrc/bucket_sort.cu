@@ -84,6 +84,7 @@ struct Args {
   uint32_t* err;
   SortSummary* sum;
   StringTies ties;
+  RankOut ranks;
   RecLayout pay;
 };
 
@@ -243,6 +244,24 @@ __device__ __forceinline__ void store_id(const Args& a, uint64_t dst, uint32_t i
   if (!a.out) return;
   if (a.wide) static_cast<uint64_t*>(a.out)[dst] = id;
   else static_cast<uint32_t*>(a.out)[dst] = id;
+}
+
+// The rank of a null or NaN row at position `dst` of the order, beside nv values.
+__device__ __forceinline__ void store_category_rank(const Args& a, uint32_t row, uint32_t dst, bool is_null, uint32_t nv,
+                                                    uint32_t nn, uint32_t nx) {
+  if (!a.ranks.out) return;
+  uint32_t lo, hi;                       // the row's equals: positions [lo, hi)
+  if (a.ranks.merge) {
+    lo = a.nulls_first ? 0u : nv;
+    hi = lo + nn + nx;
+  } else if (is_null) {
+    lo = a.nulls_first ? 0u : nv + nx;
+    hi = lo + nn;
+  } else {
+    lo = a.nulls_first ? nn : nv;
+    hi = lo + nx;
+  }
+  a.ranks.out[row] = a.ranks.mode == RANK_FIRST_OF ? lo + 1 : a.ranks.mode == RANK_LAST_OF ? hi : dst + 1;
 }
 
 // The key column's bits at a row, where a row's key does not give them (0 where null rows are written as 0).
@@ -714,6 +733,7 @@ __device__ __forceinline__ void buckets_body(const ColView& col, const Args& a) 
                                  : nan_at + sm.cats[1][u * 32 + warp] + __popc(bx & lt);
         if (dst < a.n) {
           store_id(a, dst, row);
+          store_category_rank(a, row, dst, isn, values, nn, nx);
           if (a.has_payload) unpack_record(a.pay, build_record(a.pay, row), dst);
           if (a.key_out) store_width(a.key_out, dst, pt_bytes(a.key_pt), source_bits(a, row));
         } else {
@@ -1100,6 +1120,7 @@ __device__ __forceinline__ void level1_body(const ColView& col, const Args& a) {
         continue;
       }
       store_id(a, dst, row);
+      if constexpr (!PAY) store_category_rank(a, row, dst, q < tn, nv, nn, nx);
       if constexpr (PAY) unpack_record(a.pay, build_record(a.pay, row), dst);
       if (a.key_out) store_width(a.key_out, dst, pt_bytes(a.key_pt), source_bits(a, row));
     }
@@ -1547,6 +1568,23 @@ __device__ __forceinline__ void sort_body(const Args& a) {
     __syncthreads();
     if (fast) {
       if constexpr (!PAY) {
+        if (a.ranks.out) {
+          // Equal keys share a bin, so a run of them is at most MAX_BIN rows: the walk to its end is short.
+          for (uint32_t r = t; r < rows; r += LTHREADS) {
+            const KeyT k = sm.key[r];
+            uint32_t p = r + 1;
+            if (a.ranks.mode == RANK_FIRST_OF) {
+              p = r;
+              while (p > 0 && sm.key[p - 1] == k) p--;
+              p++;
+            } else if (a.ranks.mode == RANK_LAST_OF) {
+              while (p < rows && sm.key[p] == k) p++;
+            }
+            const uint32_t row = sm.id[r];
+            if (row < a.n) a.ranks.out[row] = uint32_t(dst0) + p;
+            else atomicOr(a.err, ERR_BOUNDS);
+          }
+        }
         if (a.out) {
           if (a.wide) {
             uint64_t* o = static_cast<uint64_t*>(a.out) + dst0 + t;
@@ -1627,6 +1665,25 @@ __device__ __forceinline__ void sort_body(const Args& a) {
         const uint32_t p = sm.slow.place[r];
         const KeyT k = sm.slow.key[r];
         store_id(a, dst0 + r, id_of(p));
+        if constexpr (!PAY) {
+          if (a.ranks.out) {
+            // The run's end by bisection: the first row not before (or the first after) the key.
+            uint32_t lo = 0, hi = rows;
+            if (a.ranks.mode == RANK_OWN) {
+              lo = r;
+            } else {
+              while (lo < hi) {
+                const uint32_t mid = (lo + hi) >> 1;
+                const KeyT o = sm.slow.key[mid];
+                if (a.ranks.mode == RANK_FIRST_OF ? o < k : o <= k) lo = mid + 1;
+                else hi = mid;
+              }
+            }
+            const uint32_t row = id_of(p);
+            if (row < a.n) a.ranks.out[row] = uint32_t(dst0) + lo + (a.ranks.mode == RANK_LAST_OF ? 0u : 1u);
+            else atomicOr(a.err, ERR_BOUNDS);
+          }
+        }
         if (a.key_out)
           store_width(a.key_out, dst0 + r, kw, a.key_src && (k == KeyT(a.twin0) || k == KeyT(a.twin1))
                                                    ? source_bits(a, id_of(p)) : unkey_bits<KeyT>(k, a.key_pt, a.key_desc));
@@ -2026,6 +2083,7 @@ static Args make_args(const Sort& b) {
     a.rec[i] = reinterpret_cast<uint4*>(b.ids[i]);
   }
   a.ties = b.ties;
+  a.ranks = b.ranks;
   a.src_keys = b.src_keys;
   a.src_ids = b.src_ids;
   a.out = b.out;

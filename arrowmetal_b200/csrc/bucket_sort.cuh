@@ -33,6 +33,16 @@ struct StringTies {
   int32_t desc;
 };
 
+// Ranks instead of an order: out[row] = 1 + the first position of the row's equal keys (RANK_FIRST_OF), the
+// last one's (RANK_LAST_OF), or its own position's (RANK_OWN); null and NaN rows are equal rows each, or
+// (merge) all of them together.
+constexpr int RANK_FIRST_OF = 1, RANK_LAST_OF = 2, RANK_OWN = 3;
+struct RankOut {
+  uint32_t* out;                         // NULL: no ranks
+  int32_t mode;
+  int32_t merge;
+};
+
 // The first rows' selection: keys up to `limit` are kept, `count` of them.
 struct FirstState {
   unsigned long long limit;
@@ -51,6 +61,7 @@ struct Sort {
   void* keys[2];                         // n keys each
   char* ids[2];                          // n x 4 bytes, or n x 16 with a payload
   StringTies ties;
+  RankOut ranks;
   bool payload;
   rs::RecLayout rec;
   void* out;                             // the order (NULL: not wanted)

@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "am_internal.h"
+#include "bucket_sort.cuh"
 #include "key_encode.cuh"
 #include "radix_sort.cuh"
 
@@ -29,6 +30,10 @@ namespace {
 
 constexpr int RUN_THREADS = 256, RUN_ITEMS = 16;
 constexpr uint64_t RUN_CHUNK = uint64_t(RUN_THREADS) * RUN_ITEMS;
+
+// The steps after a bucket sort that may have written the ranks itself: nothing to do then (`gate`, when
+// given, is its mode).
+__device__ __forceinline__ bool closed(const uint32_t* gate) { return gate && *gate != bs::MODE_FALLBACK; }
 
 // A string column as the run marks read it.
 struct StrView {
@@ -111,7 +116,8 @@ template <typename KeyT>
 __global__ void __launch_bounds__(RUN_THREADS) run_marks_kernel(const __grid_constant__ ColView c, int merge_nan,
                                                                 const uint32_t* __restrict__ perm, uint64_t m,
                                                                 uint8_t* __restrict__ marks,
-                                                                uint32_t* __restrict__ block_counts) {
+                                                                uint32_t* __restrict__ block_counts, const uint32_t* gate) {
+  if (closed(gate)) return;
   __shared__ uint32_t s_warp[RUN_THREADS / 32];
   const uint64_t base = uint64_t(blockIdx.x) * RUN_CHUNK + uint64_t(threadIdx.x) * RUN_ITEMS;
   uint8_t mk[RUN_ITEMS];
@@ -169,7 +175,8 @@ __global__ void __launch_bounds__(RUN_THREADS) run_marks_str_kernel(const __grid
 }
 
 // 2. One block: exclusive scan of the block counts in place; the total run count lands at [blocks].
-__global__ void __launch_bounds__(1024) run_scan_kernel(uint32_t* __restrict__ counts, uint32_t blocks) {
+__global__ void __launch_bounds__(1024) run_scan_kernel(uint32_t* __restrict__ counts, uint32_t blocks, const uint32_t* gate) {
+  if (closed(gate)) return;
   __shared__ uint32_t s[32];
   __shared__ uint32_t carry;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -206,7 +213,8 @@ __global__ void __launch_bounds__(RUN_THREADS) run_ids_kernel(const uint8_t* __r
                                                               const uint32_t* __restrict__ perm, uint64_t m,
                                                               uint32_t* __restrict__ run_of_pos,
                                                               uint32_t* __restrict__ starts,
-                                                              uint32_t* __restrict__ heads) {
+                                                              uint32_t* __restrict__ heads, const uint32_t* gate) {
+  if (closed(gate)) return;
   __shared__ uint32_t s_warp[RUN_THREADS / 32];
   const uint64_t base = uint64_t(blockIdx.x) * RUN_CHUNK + uint64_t(threadIdx.x) * RUN_ITEMS;
   uint8_t mk[RUN_ITEMS];
@@ -245,7 +253,8 @@ enum Finish { FIN_MIN = 0, FIN_MAX, FIN_QUANTILE, FIN_NORMAL64, FIN_NORMAL32, FI
 __global__ void __launch_bounds__(256) rank_finish_kernel(const uint32_t* run_of_pos,
                                                           const uint32_t* __restrict__ starts,
                                                           const uint32_t* __restrict__ total_runs, uint64_t n,
-                                                          int mode, void* out) {
+                                                          int mode, void* out, const uint32_t* gate) {
+  if (closed(gate)) return;
   const uint32_t runs = *total_runs;
   for (uint64_t r = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; r < n; r += uint64_t(gridDim.x) * blockDim.x) {
     const uint32_t g = run_of_pos[r];
@@ -282,7 +291,8 @@ __global__ void __launch_bounds__(SC_THREADS) bucket_pairs_kernel(const uint32_t
                                                                   const V* __restrict__ val, uint64_t n, int shift,
                                                                   int nb, uint32_t* __restrict__ cursor,
                                                                   uint32_t* __restrict__ rows_out, V* __restrict__ vals_out,
-                                                                  uint32_t* __restrict__ err) {
+                                                                  uint32_t* __restrict__ err, const uint32_t* gate) {
+  if (closed(gate)) return;
   __shared__ uint32_t wcnt[SC_WARPS][SC_MAX_BUCKETS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t lt = (1u << lane) - 1u;
@@ -350,7 +360,9 @@ __global__ void __launch_bounds__(SC_THREADS) bucket_pairs_kernel(const uint32_t
 
 template <typename V>
 __global__ void __launch_bounds__(256) drain_pairs_kernel(const uint32_t* __restrict__ rows, const V* __restrict__ vals,
-                                                          uint64_t n, V* __restrict__ out, uint32_t* __restrict__ err) {
+                                                          uint64_t n, V* __restrict__ out, uint32_t* __restrict__ err,
+                                                          const uint32_t* gate) {
+  if (closed(gate)) return;
   for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
     const uint32_t r = rows[i];
     if (r < n) out[r] = vals[i];
@@ -478,7 +490,8 @@ struct Runs {
   const uint32_t* total() const { return static_cast<const uint32_t*>(counts->ptr) + blocks; }
 };
 
-Runs mark_runs(am_array* a, const uint32_t* perm, uint64_t m, bool merge_nan, int float_order, cudaStream_t s) {
+Runs mark_runs(am_array* a, const uint32_t* perm, uint64_t m, bool merge_nan, int float_order, cudaStream_t s,
+               const uint32_t* gate = nullptr) {
   Runs r;
   r.blocks = uint32_t((m + RUN_CHUNK - 1) / RUN_CHUNK);
   r.marks = DevBuffer::alloc(size_t(m) + 16, s);
@@ -494,27 +507,27 @@ Runs mark_runs(am_array* a, const uint32_t* perm, uint64_t m, bool merge_nan, in
   } else {
     const ColView c = make_view(SortKey{a, false, false, float_order});
     if (pt_key_bytes(a->pt) == 8)
-      run_marks_kernel<uint64_t><<<r.blocks, RUN_THREADS, 0, s>>>(c, merge_nan ? 1 : 0, perm, m, marks, counts);
-    else run_marks_kernel<uint32_t><<<r.blocks, RUN_THREADS, 0, s>>>(c, merge_nan ? 1 : 0, perm, m, marks, counts);
+      run_marks_kernel<uint64_t><<<r.blocks, RUN_THREADS, 0, s>>>(c, merge_nan ? 1 : 0, perm, m, marks, counts, gate);
+    else run_marks_kernel<uint32_t><<<r.blocks, RUN_THREADS, 0, s>>>(c, merge_nan ? 1 : 0, perm, m, marks, counts, gate);
   }
   AM_CUDA(cudaGetLastError());
-  run_scan_kernel<<<1, 1024, 0, s>>>(counts, r.blocks);
+  run_scan_kernel<<<1, 1024, 0, s>>>(counts, r.blocks, gate);
   AM_CUDA(cudaGetLastError());
   return r;
 }
 
 void run_ids(const Runs& r, const uint32_t* perm, uint64_t m, uint32_t* run_of_row, uint32_t* starts, uint32_t* heads,
-             cudaStream_t s) {
+             cudaStream_t s, const uint32_t* gate = nullptr) {
   KernelTimer kt("run_ids", s);
   run_ids_kernel<<<r.blocks, RUN_THREADS, 0, s>>>(static_cast<const uint8_t*>(r.marks->ptr),
                                                   static_cast<const uint32_t*>(r.counts->ptr), perm, m, run_of_row,
-                                                  starts, heads);
+                                                  starts, heads, gate);
   AM_CUDA(cudaGetLastError());
 }
 
 // out[perm[i]] = vals[i] for i < n (vals NULL: i + 1), perm a permutation of [0, n).
 template <typename V>
-void scatter_to_rows(const uint32_t* perm, const V* vals, uint64_t n, V* out, cudaStream_t s) {
+void scatter_to_rows(const uint32_t* perm, const V* vals, uint64_t n, V* out, cudaStream_t s, const uint32_t* gate = nullptr) {
   int bits = 0;
   while ((uint64_t(1) << bits) < n) bits++;
   // At most 64 buckets: a block's 4,096 pairs make runs of ~64 per bucket, and a bucket's rows (at
@@ -532,10 +545,10 @@ void scatter_to_rows(const uint32_t* perm, const V* vals, uint64_t n, V* out, cu
   bucket_pairs_kernel<V><<<blocks, SC_THREADS, 0, s>>>(perm, vals, n, shift, nb,
                                                                     static_cast<uint32_t*>(cursor->ptr),
                                                                     static_cast<uint32_t*>(rows->ptr),
-                                                                    static_cast<V*>(pv->ptr), err);
+                                                                    static_cast<V*>(pv->ptr), err, gate);
   AM_CUDA(cudaGetLastError());
   drain_pairs_kernel<V><<<grid_for(n), 256, 0, s>>>(static_cast<const uint32_t*>(rows->ptr),
-                                                    static_cast<const V*>(pv->ptr), n, out, err);
+                                                    static_cast<const V*>(pv->ptr), n, out, err, gate);
   AM_CUDA(cudaGetLastError());
 }
 
@@ -571,32 +584,40 @@ am_array* rank_of(am_array* a, int fn, bool desc, bool nulls_first, bool merge_n
   if (n == 0) return out;
   try {
     use_on(a, s);
-    BufPtr perm = sorted_order(a, desc, nulls_first, float_order, s);
+    // The ranks come out of the sort itself, or (its buckets being too large, which the device finds out)
+    // the order does; the steps after it then run, as they do for the orders that take no such sort.
+    BufPtr perm = DevBuffer::alloc(size_t(n) * 4 + 16, s);
+    const SortKey key{a, desc, nulls_first, float_order};
+    uint32_t* mode = static_cast<uint32_t*>(perm->ptr) + n;
+    const uint32_t* gate = nullptr;
+    if (rank_by_buckets(key, n, fn, merge_nan, static_cast<uint32_t*>(out->values->ptr), static_cast<uint32_t*>(perm->ptr), mode, s))
+      gate = mode;
+    else argsort_any({key}, n, perm->ptr, 4, s, nullptr);
     const uint32_t* p = static_cast<const uint32_t*>(perm->ptr);
     if (fn == RANK_FIRST) {
-      scatter_to_rows<uint32_t>(p, nullptr, uint64_t(n), static_cast<uint32_t*>(out->values->ptr), s);
+      scatter_to_rows<uint32_t>(p, nullptr, uint64_t(n), static_cast<uint32_t*>(out->values->ptr), s, gate);
       return out;
     }
-    const Runs r = mark_runs(a, p, uint64_t(n), merge_nan, float_order, s);
+    const Runs r = mark_runs(a, p, uint64_t(n), merge_nan, float_order, s, gate);
     // Run numbers by position; the uint32 answers are computed in place, the float ones beside them.
     BufPtr run_of_pos = DevBuffer::alloc(size_t(n) * 4 + 16, s);
     uint32_t* rp = static_cast<uint32_t*>(run_of_pos->ptr);
     BufPtr starts = fn == RANK_DENSE ? nullptr : DevBuffer::alloc(size_t(n) * 4 + 16, s);
-    run_ids(r, p, uint64_t(n), rp, starts ? static_cast<uint32_t*>(starts->ptr) : nullptr, nullptr, s);
+    run_ids(r, p, uint64_t(n), rp, starts ? static_cast<uint32_t*>(starts->ptr) : nullptr, nullptr, s, gate);
     BufPtr val_pos = (f32 || f64) ? DevBuffer::alloc(size_t(n) * (f64 ? 8 : 4) + 16, s) : nullptr;
     if (fn != RANK_DENSE) {
       static const int finish[] = {FIN_MIN, FIN_MAX, -1, -1, FIN_QUANTILE, FIN_NORMAL64, FIN_NORMAL32, FIN_PERCENT, FIN_CUME};
       KernelTimer kt("rank_finish", s);
       rank_finish_kernel<<<grid_for(uint64_t(n)), 256, 0, s>>>(rp, static_cast<const uint32_t*>(starts->ptr),
                                                                r.total(), uint64_t(n), finish[fn],
-                                                               val_pos ? val_pos->ptr : static_cast<void*>(rp));
+                                                               val_pos ? val_pos->ptr : static_cast<void*>(rp), gate);
       AM_CUDA(cudaGetLastError());
     }
     if (f64) scatter_to_rows<double>(p, static_cast<const double*>(val_pos->ptr), uint64_t(n),
                                      static_cast<double*>(out->values->ptr), s);
     else if (f32) scatter_to_rows<float>(p, static_cast<const float*>(val_pos->ptr), uint64_t(n),
                                          static_cast<float*>(out->values->ptr), s);
-    else scatter_to_rows<uint32_t>(p, rp, uint64_t(n), static_cast<uint32_t*>(out->values->ptr), s);
+    else scatter_to_rows<uint32_t>(p, rp, uint64_t(n), static_cast<uint32_t*>(out->values->ptr), s, gate);
     // The scratch buffers are freed in stream order after the kernels that read them.
   } catch (...) {
     release(out);

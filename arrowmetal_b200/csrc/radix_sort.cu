@@ -1812,6 +1812,9 @@ template <> struct PassConfig<uint32_t> { static constexpr int THREADS = 512, IT
 template <> struct PassConfig<uint64_t> { static constexpr int THREADS = 512, ITEMS = 10; };
 constexpr int HIST_THREADS = 256, HIST_ITEMS = 8;
 constexpr int MAX_ONE_KEY = 8;        // digit passes of one key
+// Ranks leave the bucket sort as random 4-byte stores: while the whole rank column (64 MB here) stays in L2.
+// 8M int64 keys with nulls, min: 867 us by an order, run marks and a scatter, 342 so.
+constexpr uint64_t RANK_BUCKET_ROWS = uint64_t(1) << 24;
 
 template <typename KeyT, int ITEMS = PassConfig<KeyT>::ITEMS, int THREADS = PassConfig<KeyT>::THREADS, bool REC = false>
 static size_t pass_smem() {
@@ -2075,7 +2078,7 @@ static void launch_all_passes(const rs::AllPassesArgs& a, const rs::ColView& cv,
 // passes in one launch.
 static void sort_by_buckets(const SortKey& key, const rs::PlanArgs& pa, uint64_t n, int kb, void* out, int index_width,
                             am_array* key_dst, const rs::RecLayout* payload, bool carry_ids, cudaStream_t s,
-                            am_sort_stats* stats) {
+                            am_sort_stats* stats, const bs::RankOut* ranks = nullptr, uint32_t* mode_out = nullptr) {
   using namespace rs;
   auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
   // Zeroed: the digit passes' state and the bucket sort's own; then its tables, then the rows' buffers.
@@ -2103,7 +2106,8 @@ static void sort_by_buckets(const SortKey& key, const rs::PlanArgs& pa, uint64_t
   b.scratch = base + off_bs;
   b.payload = payload != nullptr;
   if (payload) b.rec = *payload;
-  b.out = out;
+  b.out = ranks ? nullptr : out;         // ranks are written instead of the order, unless the passes run
+  if (ranks) b.ranks = *ranks;
   b.wide = index_width == 8;
   for (int i = 0; i < 2; i++) {
     b.keys[i] = base + off_keys + size_t(i) * kbuf;
@@ -2158,7 +2162,32 @@ static void sort_by_buckets(const SortKey& key, const rs::PlanArgs& pa, uint64_t
     if (payload) launch_all_passes<uint32_t, true>(a, b.col, n, s);
     else launch_all_passes<uint32_t, false>(a, b.col, n, s);
   }
+  if (mode_out) AM_CUDA(cudaMemcpyAsync(mode_out, &st->mode, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
   finish_sort(key, n, key_dst, sum, payload != nullptr, stats, s);
+}
+
+bool rank_by_buckets(const SortKey& key, int64_t n64, int fn, bool merge_nan, uint32_t* ranks, uint32_t* perm, uint32_t* mode,
+                     cudaStream_t s) {
+  using namespace rs;
+  const uint64_t n = uint64_t(n64);
+  if (n == 0 || n > RANK_BUCKET_ROWS || pt_var(key.col->pt) || key.col->dictionary || debug_skip_first_tile()) return false;
+  if (fn != RANK_MIN && fn != RANK_MAX && fn != RANK_FIRST) return false;
+  // A key of few distinct values sorts by its dense rank in one pass; its order is ranked as before.
+  if (am_array* r = low_cardinality_ranks(key, s)) {
+    am::release(r);
+    return false;
+  }
+  PlanArgs pa{};
+  const int kb = pt_key_bytes(key.col->pt);
+  pa.n = n;
+  pa.nkeys = 1;
+  pa.nslots = kb;
+  pa.key_bytes[0] = uint8_t(kb);
+  pa.nulls_first[0] = key.nulls_first ? 1 : 0;
+  for (int d = 0; d < kb; d++) pa.slot_digit[d] = int8_t(d);
+  const bs::RankOut out{ranks, fn == RANK_MIN ? bs::RANK_FIRST_OF : fn == RANK_MAX ? bs::RANK_LAST_OF : bs::RANK_OWN, merge_nan ? 1 : 0};
+  sort_by_buckets(key, pa, n, kb, perm, 4, nullptr, nullptr, true, s, nullptr, &out, mode);
+  return true;
 }
 
 bool string_argsort(const SortKey& key, int64_t n64, void* out, int index_width, cudaStream_t s, am_sort_stats* stats) {

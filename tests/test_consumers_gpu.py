@@ -266,3 +266,28 @@ def test_unique_large_strings(am):
     assert m.unique("sorted").to_arrow().to_pylist() == sorted(seen)
     vc = m.value_counts("sorted").to_arrow()
     assert vc.field("counts").to_pylist() == [seen[k] for k in sorted(seen)]
+
+
+@pytest.mark.parametrize("n", [2003, 65_536, 65_537, 900_001])
+@pytest.mark.parametrize("kind", ["spread", "runs", "repeats", "one_value", "floats"])
+def test_ranks_out_of_the_buckets(am, oracle, n, kind):
+    # Ranks written by the bucket sort: distinct keys, short runs, runs beyond the fast form, a value no
+    # bucket holds (the order and the steps after it), NaN and null rows tied or not.
+    rng = np.random.default_rng(n + len(kind))
+    v = {"spread": lambda: rng.integers(0, 2**40, n), "runs": lambda: rng.integers(0, n // 3 + 1, n) * 1000003,
+         "repeats": lambda: rng.integers(0, max(2, n // 3000), n), "one_value": lambda: np.where(rng.random(n) < 0.4, 7, rng.integers(0, 2**40, n)),
+         "floats": lambda: rng.standard_normal(n).round(2)}[kind]()
+    if kind == "floats":
+        v[rng.random(n) < 0.05] = np.nan
+        v[rng.random(n) < 0.02] = -0.0
+    arr = pa.array(v, mask=rng.random(n) < 0.1, from_pandas=False)
+    m = am.MetalArray.from_arrow(arr)
+    for desc, placement in ((False, "at_end"), (True, "at_start")):
+        for tb in ("min", "max", "first"):
+            want = oracle.rank(arr, tb, desc, placement)
+            got = np_of(m.rank("descending" if desc else "ascending", placement, tb))
+            assert np.array_equal(got, want), (desc, placement, tb)
+    order = np_of(m.argsort())
+    rows = np.empty(n, np.uint32)
+    rows[order] = np.arange(1, n + 1)
+    assert np.array_equal(np_of(m.row_number()), rows)
