@@ -1063,27 +1063,28 @@ __device__ __forceinline__ void level1_body(const ColView& col, const Args& a) {
         tn += q.x;
         tx += q.y;
       }
-      // (A tile's rows are at most TILE: behind the values there is room for the others.)
-      if (tn) {
-        uint32_t p = tile_n + wn;
+      // (A tile's rows are at most TILE: behind the values there is room for the others.) With a payload
+      // their records wait there too, from the registers they were loaded to: read again from the columns
+      // at the store, each row's 16 bytes cost two more 32-byte sectors (50M rows, 10% nulls: the step
+      // 716 us, 682 so).
+      auto stage = [&](uint32_t rows, uint32_t p) {
 #pragma unroll
         for (int i = 0; i < ITEMS; i++) {
-          const bool is = (nulls >> i) & 1u;
+          const bool is = (rows >> i) & 1u;
           const uint32_t m = __ballot_sync(0xffffffffu, is);
-          if (is) sm.word[p + __popc(m & lt)] = wofs + i * 32;
+          if (is) {
+            const uint32_t at = p + __popc(m & lt);
+            sm.word[at] = wofs + i * 32;
+            if constexpr (PAY) {
+              const uint32_t row = uint32_t(tile) + wofs + uint32_t(i) * 32;
+              sm.rec[at] = direct ? make_uint4(row, uint32_t(pw[i]), uint32_t(pw[i] >> 32), ph[i]) : build_record(a.pay, row);
+            }
+          }
           p += __popc(m);
         }
-      }
-      if (tx) {
-        uint32_t p = tile_n + tn + wx;
-#pragma unroll
-        for (int i = 0; i < ITEMS; i++) {
-          const bool is = (nans >> i) & 1u;
-          const uint32_t m = __ballot_sync(0xffffffffu, is);
-          if (is) sm.word[p + __popc(m & lt)] = wofs + i * 32;
-          p += __popc(m);
-        }
-      }
+      };
+      if (tn) stage(nulls, tile_n + wn);
+      if (tx) stage(nans, tile_n + tn + wx);
     }
     // The next tile's rows arrive while this one leaves.
     if (tile + TILE < end) load_rows(tile + TILE);
@@ -1121,7 +1122,7 @@ __device__ __forceinline__ void level1_body(const ColView& col, const Args& a) {
       }
       store_id(a, dst, row);
       if constexpr (!PAY) store_category_rank(a, row, dst, q < tn, nv, nn, nx);
-      if constexpr (PAY) unpack_record(a.pay, build_record(a.pay, row), dst);
+      if constexpr (PAY) unpack_record(a.pay, sm.rec[j], dst);
       if (a.key_out) store_width(a.key_out, dst, pt_bytes(a.key_pt), source_bits(a, row));
     }
     null_at += tn;
