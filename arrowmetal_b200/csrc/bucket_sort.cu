@@ -57,6 +57,7 @@ constexpr uint32_t SAMPLES = 65536;               // keys looked at (every key o
 constexpr int CLUSTER = 8;                        // CTAs of the one-cluster kernels
 constexpr uint32_t ONE_CAP = 1024;                // buckets of a column of at most SAMPLES rows
 constexpr int BINS = 2048, BINS_LOG = 11;         // bins of the shared-memory sort
+constexpr uint32_t CATS = 2 + FREQUENT;           // a chunk's rows apart from the buckets: null, NaN, each frequent key
 constexpr uint32_t MAX_BIN = 32;                  // rows a bin may hold for the comparisons
 constexpr uint32_t META_SPLIT = 0x80000000u;
 constexpr int CUR_PAD = 8;                        // cursors 32 bytes apart: same-sector atomics queue
@@ -80,6 +81,7 @@ struct Args {
   const void* key_src;                            // not NULL: keys that stand for several values are read here
   unsigned long long twin0, twin1;                // those keys: a zero's, a NaN's
   int32_t wide, key_pt, key_desc, nulls_first, has_payload;
+  int32_t frequent;                               // set frequent keys apart
   int32_t one_launch;                             // the plan's launch counts and moves the rows too
   uint32_t* err;
   SortSummary* sum;
@@ -452,7 +454,112 @@ __device__ void plan_cells(const Args& a, PlanShared& sm, const Map<KeyT>& map, 
   }
 }
 
-template <typename KeyT>
+// Sets frequent keys apart: up to FREQUENT that hold at least 1/512 of the sample and more rows than half
+// of BIG. The sample's keys are counted by a hash into 2,048 counters (about 32 each); in a counter four
+// times that one key has the majority, so each of its bits is the majority's bit. A wrong guess is a key of
+// another counter, or a key of few rows: nothing depends on either. Returns which of this thread's keys
+// they are. (key2 of a 16M-row lexsort, a float with 80 K rows each of zero and both infinities: without,
+// no bucket holds those rows and eight digit passes run, 1,300 us.)
+constexpr int COUNTERS_LOG = 11, COUNTERS = 1 << COUNTERS_LOG;
+template <typename KeyT, int U>
+__device__ uint32_t take_frequent(const Args& a, PlanShared& sm, const KeyT (&key)[U], uint32_t live) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  static_assert(COUNTERS <= 2 * FINE && FREQUENT * 64 + FREQUENT + FREQUENT * 2 <= 1024, "they borrow the plan's arrays");
+  constexpr uint32_t NONE = 0xFFFFFFFFu;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  uint32_t* counter = sm.half_cnt;
+  uint32_t* votes = sm.group;                      // by key and bit, then the voters, then the keys' words
+  uint32_t* voters = votes + FREQUENT * 64;
+  uint32_t* words = voters + FREQUENT;
+  auto counter_of = [](KeyT k) { return uint32_t((uint64_t(k) * 0x9E3779B97F4A7C15ull) >> (64 - COUNTERS_LOG)); };
+  for (int i = t; i < COUNTERS; i += 1024) counter[i] = 0;
+  if (t < FREQUENT * 64 + FREQUENT) votes[t] = 0;
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < U; u++)
+    if ((live >> u) & 1u) atomicAdd(&counter[counter_of(key[u])], 1u);
+  cl.sync();
+  uint32_t best[COUNTERS / 1024];                  // count << COUNTERS_LOG | counter
+#pragma unroll
+  for (int q = 0; q < COUNTERS / 1024; q++) {
+    uint32_t c = 0;
+#pragma unroll
+    for (int r = 0; r < CLUSTER; r++) c += cl.map_shared_rank(&sm, r)->half_cnt[q * 1024 + t];
+    best[q] = (c << COUNTERS_LOG) | uint32_t(q * 1024 + t);
+  }
+  const uint32_t least = max(4 * SAMPLES / COUNTERS, uint32_t(float(BIG / 2) * float(a.nsamples) / float(a.n)));
+  uint32_t at[FREQUENT];
+#pragma unroll
+  for (int h = 0; h < FREQUENT; h++) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int q = 0; q < COUNTERS / 1024; q++) m = max(m, best[q]);
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (lane == 0) sm.warp[warp] = m;
+    __syncthreads();
+    m = __reduce_max_sync(0xffffffffu, sm.warp[lane]);
+    __syncthreads();
+    at[h] = (m >> COUNTERS_LOG) >= least ? m & uint32_t(COUNTERS - 1) : NONE;
+#pragma unroll
+    for (int q = 0; q < COUNTERS / 1024; q++)
+      if (best[q] == m) best[q] = 0;
+  }
+  // A quarter of the sample votes.
+  constexpr int BITS = int(sizeof(KeyT)) * 8;
+#pragma unroll
+  for (int u = 0; u < (U + 3) / 4; u++) {
+    const uint32_t mine = (live >> u) & 1u ? counter_of(key[u]) : NONE - 1;
+#pragma unroll
+    for (int h = 0; h < FREQUENT; h++) {
+      const uint32_t who = __ballot_sync(0xffffffffu, mine == at[h]);
+      if (!who) continue;
+      if (lane == 0) atomicAdd(&voters[h], uint32_t(__popc(who)));
+      for (int bit = 0; bit < BITS; bit++) {
+        const uint32_t ones = who & __ballot_sync(0xffffffffu, (key[u] >> bit) & 1);
+        if (lane == (bit & 31) && ones) atomicAdd(&votes[h * 64 + bit], uint32_t(__popc(ones)));
+      }
+    }
+  }
+  cl.sync();
+  if (t < FREQUENT * 64) {
+    uint32_t yes = 0, all = 0;
+#pragma unroll
+    for (int r = 0; r < CLUSTER; r++) {
+      const PlanShared* o = cl.map_shared_rank(&sm, r);
+      yes += o->group[t];
+      all += o->group[FREQUENT * 64 + (t >> 6)];
+    }
+    const uint32_t w = __ballot_sync(0xffffffffu, 2 * yes > all);
+    if (lane == 0) words[t >> 5] = w;
+  }
+  __syncthreads();
+  // Ascending; keys of different counters differ.
+  KeyT found[FREQUENT];
+  uint32_t n = 0, hit = 0;
+#pragma unroll
+  for (int h = 0; h < FREQUENT; h++) {
+    const KeyT k = KeyT(uint64_t(words[2 * h]) | (uint64_t(words[2 * h + 1]) << 32));
+    found[h] = k;
+    if (at[h] == NONE || counter_of(k) != at[h]) continue;
+    uint32_t before = 0;
+#pragma unroll
+    for (int g = 0; g < FREQUENT; g++) {
+      const KeyT o = KeyT(uint64_t(words[2 * g]) | (uint64_t(words[2 * g + 1]) << 32));
+      if (g != h && at[g] != NONE && counter_of(o) == at[g] && o < k) before++;
+    }
+    if (t == 0 && cl.block_rank() == 0) a.st->key[before] = k;
+    n++;
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (((live >> u) & 1u) && key[u] == k) hit |= 1u << u;
+  }
+  if (t == 0 && cl.block_rank() == 0) a.st->nkeys = n;
+  __syncthreads();                                 // the borrowed arrays are free
+  return hit;
+}
+
+template <typename KeyT, bool FREQ = false>
 __device__ __forceinline__ void buckets_body(const ColView& col, const Args& a) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
@@ -493,6 +600,7 @@ __device__ __forceinline__ void buckets_body(const ColView& col, const Args& a) 
       else nulls |= 1u << u;
     }
   }
+  if constexpr (FREQ) live &= ~take_frequent<KeyT, U>(a, sm, key, live);
   for (int i = t; i < COARSE; i += 1024) sm.coarse_cnt[i] = 0;
   for (int i = t; i < 2 * FINE; i += 1024) sm.half_cnt[i] = 0;
   // The sampled range, over the cluster.
@@ -749,17 +857,22 @@ __device__ __forceinline__ void buckets_body(const ColView& col, const Args& a) 
 //
 // One read of the column (63 us for 45M keys and 16,384 bins on a B200: the HBM copy rate). Each CTA
 // takes consecutive chunks; a chunk's level-1 counts are the growth of its bins' sums over the chunk.
-template <typename KeyT>
+template <typename KeyT, bool FREQ = false>
 __device__ __forceinline__ void histogram_body(const ColView& col, const Args& a) {
   extern __shared__ __align__(16) unsigned char hsm[];
   State* st = a.st;
   if (blockIdx.x >= a.hist_grid || st->mode != MODE_BUCKETS) return;
   uint32_t* bins = reinterpret_cast<uint32_t*>(hsm);
   __shared__ uint32_t coarse[COARSE], fine[FINE], prev[BINS1];
-  __shared__ uint32_t s_null, s_nan;
+  __shared__ uint32_t s_null, s_nan, s_rows[FREQUENT];
+  __shared__ KeyT s_key[FREQUENT];
   __shared__ unsigned long long s_or;
-  const uint32_t nb = st->buckets, s2 = st->s2, nbins = st->bins1;
+  const uint32_t nb = st->buckets, s2 = st->s2, nbins = st->bins1, nkeys = FREQ ? st->nkeys : 0u;
   load_tables(a, coarse, fine);
+  if (threadIdx.x < uint32_t(FREQUENT)) {
+    s_key[threadIdx.x] = KeyT(st->key[threadIdx.x]);
+    s_rows[threadIdx.x] = 0;
+  }
   for (uint32_t i = threadIdx.x; i < nb; i += HTHREADS) bins[i] = 0;
   for (int i = threadIdx.x; i < BINS1; i += HTHREADS) prev[i] = 0;
   if (threadIdx.x == 0) {
@@ -772,11 +885,12 @@ __device__ __forceinline__ void histogram_body(const ColView& col, const Args& a
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   KeyT diff = 0;                        // bits that differ from lo's in some key
   uint32_t values = 0, all_null = 0, all_nan = 0;
+  uint32_t below[FREQUENT] = {};        // value rows before each frequent key
   const uint32_t c0 = uint32_t(uint64_t(blockIdx.x) * a.nchunks / a.hist_grid);
   const uint32_t c1 = uint32_t(uint64_t(blockIdx.x + 1) * a.nchunks / a.hist_grid);
   for (uint32_t c = c0; c < c1; c++) {
     const uint64_t first = uint64_t(c) * a.chunk_rows, end = min(a.n, first + a.chunk_rows);
-    uint32_t n_null = 0, n_nan = 0;
+    uint32_t n_null = 0, n_nan = 0, n_key[FREQUENT] = {};
     for (uint64_t w0 = first + uint64_t(warp) * (HITEMS * 32); w0 < end; w0 += HTHREADS * HITEMS) {
       RawTile<KeyT, HITEMS> r;
       uint32_t is_value, is_null, is_nan;
@@ -785,6 +899,26 @@ __device__ __forceinline__ void histogram_body(const ColView& col, const Args& a
       values += __popc(is_value);
       n_null += __popc(is_null);
       n_nan += __popc(is_nan);
+      if (nkeys) {
+        uint32_t apart = 0;
+#pragma unroll
+        for (int h = 0; h < FREQUENT; h++) {
+          if (uint32_t(h) >= nkeys) break;
+          const KeyT k = s_key[h];
+          uint32_t same = 0, less = 0;
+#pragma unroll
+          for (int i = 0; i < HITEMS; i++) {
+            same |= uint32_t(r.key[i] == k) << i;
+            less |= uint32_t(r.key[i] < k) << i;
+          }
+          same &= is_value;
+          below[h] += __popc(less & is_value);
+          n_key[h] += __popc(same);
+          if (same) diff |= k ^ map.lo;
+          apart |= same;
+        }
+        is_value &= ~apart;
+      }
 #pragma unroll
       for (int i = 0; i < HITEMS; i++) {
         if (!((is_value >> i) & 1u)) continue;
@@ -797,6 +931,12 @@ __device__ __forceinline__ void histogram_body(const ColView& col, const Args& a
     if (lane == 0) {
       if (n_null) atomicAdd(&s_null, n_null);
       if (n_nan) atomicAdd(&s_nan, n_nan);
+    }
+#pragma unroll
+    for (int h = 0; h < FREQUENT; h++) {
+      if (uint32_t(h) >= nkeys) break;
+      const uint32_t rows = __reduce_add_sync(0xffffffffu, n_key[h]);
+      if (lane == 0 && rows) atomicAdd(&s_rows[h], rows);
     }
     __syncthreads();
     if (s2 == 0) {
@@ -820,8 +960,12 @@ __device__ __forceinline__ void histogram_body(const ColView& col, const Args& a
       }
     }
     if (threadIdx.x == 0) {
-      a.chunk_cats[2 * c] = s_null;
-      a.chunk_cats[2 * c + 1] = s_nan;
+      a.chunk_cats[CATS * c] = s_null;
+      a.chunk_cats[CATS * c + 1] = s_nan;
+      for (uint32_t h = 0; h < nkeys; h++) {
+        a.chunk_cats[CATS * c + 2 + h] = s_rows[h];
+        s_rows[h] = 0;
+      }
       all_null += s_null;
       all_nan += s_nan;
       s_null = 0;
@@ -834,6 +978,12 @@ __device__ __forceinline__ void histogram_body(const ColView& col, const Args& a
   if (lane == 0) {
     atomicOr(&s_or, (unsigned long long)diff);
     if (values) atomicAdd(&st->n_value, values);
+  }
+#pragma unroll
+  for (int h = 0; h < FREQUENT; h++) {
+    if (uint32_t(h) >= nkeys) break;
+    const uint32_t rows = __reduce_add_sync(0xffffffffu, below[h]);
+    if (lane == 0 && rows) atomicAdd(&st->key_at[h], rows);
   }
   __syncthreads();
   for (uint32_t i = threadIdx.x; i < nb; i += HTHREADS)
@@ -897,19 +1047,27 @@ __device__ __forceinline__ void starts_body(const Args& a) {
   }
   if (rank != 0) return;
   uint32_t all;
-  const uint32_t nulls = t < a.nchunks ? a.chunk_cats[2 * t] : 0u;
-  const uint32_t nans = t < a.nchunks ? a.chunk_cats[2 * t + 1] : 0u;
+  const uint32_t nulls = t < a.nchunks ? a.chunk_cats[CATS * t] : 0u;
+  const uint32_t nans = t < a.nchunks ? a.chunk_cats[CATS * t + 1] : 0u;
   const uint32_t null0 = block_scan<1024>(nulls, s_warp, all);
   const uint32_t nan0 = block_scan<1024>(nans, s_warp, all);
   if (t < a.nchunks) {
-    a.chunk_cats[2 * t] = null0;
-    a.chunk_cats[2 * t + 1] = nan0;
+    a.chunk_cats[CATS * t] = null0;
+    a.chunk_cats[CATS * t + 1] = nan0;
+  }
+  uint32_t apart = 0;                    // rows of the frequent keys
+  for (uint32_t h = 0; h < st->nkeys; h++) {
+    const uint32_t rows = t < a.nchunks ? a.chunk_cats[CATS * t + 2 + h] : 0u;
+    const uint32_t before = block_scan<1024>(rows, s_warp, all);
+    if (t < a.nchunks) a.chunk_cats[CATS * t + 2 + h] = st->key_at[h] + before;
+    if (t == 0) st->key_rows[h] = all;
+    apart += all;
   }
   if (t == 0) {
     a.bpos[nb] = carry;
     st->max_bucket = big;
-    if (carry != st->n_value) atomicOr(a.err, ERR_BOUNDS);
-    if (big > uint32_t(BIG) || carry != st->n_value) {
+    if (carry + apart != st->n_value) atomicOr(a.err, ERR_BOUNDS);
+    if (big > uint32_t(BIG) || carry + apart != st->n_value) {
       st->mode = MODE_FALLBACK;
     } else {
       // The counters of the digit passes' sort: the key's digits that vary. A two-level sort's two
@@ -936,13 +1094,15 @@ struct TileShared {
   uint32_t start[NB], delta[NB], at[NB];
   uint32_t warp[32];
   uint32_t cats[WARPS][2];
+  uint32_t key_cats[WARPS][FREQUENT], key_at[FREQUENT];  // the frequent keys' rows by warp; their next places
+  KeyT apart[FREQUENT];
   uint4 rec[PAY ? TILE : 1];
   KeyT key[TILE];
   // Per staged row: its bin, and without records (which hold the row id) its place in the tile below it.
   std::conditional_t<PAY != 0, uint16_t, uint32_t> word[TILE];
 };
 
-template <typename KeyT, int PAY>
+template <typename KeyT, int PAY, bool FREQ = false>
 __device__ __forceinline__ void level1_body(const ColView& col, const Args& a) {
   extern __shared__ __align__(16) unsigned char tsm[];
   using SM = TileShared<KeyT, PAY>;
@@ -967,10 +1127,15 @@ __device__ __forceinline__ void level1_body(const ColView& col, const Args& a) {
     sm.start[d] = 0;
   }
   const bool cats = col.valid || col.nan_cat;
-  uint32_t null_at = a.chunk_cats[2 * c], nan_at = a.chunk_cats[2 * c + 1];
+  uint32_t null_at = a.chunk_cats[CATS * c], nan_at = a.chunk_cats[CATS * c + 1];
+  const uint32_t nkeys = FREQ ? st->nkeys : 0u;
   const uint32_t nv = st->n_value, nn = st->n_null, nx = st->n_nan;
   null_at += a.nulls_first ? 0u : nv + nx;
   nan_at += a.nulls_first ? nn : nv;
+  if (uint32_t(t) < nkeys) {
+    sm.key_at[t] = a.chunk_cats[CATS * c + 2 + t] + (a.nulls_first ? nn + nx : 0u);
+    sm.apart[t] = KeyT(st->key[t]);
+  }
   KeyT* __restrict__ kout = static_cast<KeyT*>(a.keys[0]);
   uint32_t* __restrict__ iout = a.ids[0];
   uint4* __restrict__ rout = a.rec[0];
@@ -1002,6 +1167,22 @@ __device__ __forceinline__ void level1_body(const ColView& col, const Args& a) {
   for (uint64_t tile = first; tile < end; tile += TILE) {
     uint32_t values, nulls, nans;
     encode_tile(col, tile + (wofs - lane), end, r, values, nulls, nans);
+    uint32_t apart = 0;                 // items of a frequent key
+    auto same_as = [&](KeyT k) {
+      uint32_t same = 0;
+#pragma unroll
+      for (int i = 0; i < ITEMS; i++) same |= uint32_t(r.key[i] == k) << i;
+      return same;
+    };
+    if (nkeys) {
+      for (uint32_t h = 0; h < nkeys; h++) {
+        const uint32_t same = same_as(sm.apart[h]) & values;
+        const uint32_t rows = __reduce_add_sync(0xffffffffu, __popc(same));
+        if (lane == 0) sm.key_cats[warp][h] = rows;
+        apart |= same;
+      }
+      values &= ~apart;
+    }
     uint32_t slot[ITEMS];               // bin << 16 | place among the tile's rows of the bin
 #pragma unroll
     for (int i = 0; i < ITEMS; i++) {
@@ -1086,10 +1267,29 @@ __device__ __forceinline__ void level1_body(const ColView& col, const Args& a) {
       if (tn) stage(nulls, tile_n + wn);
       if (tx) stage(nans, tile_n + tn + wx);
     }
+    // The frequent keys' rows: straight to their places, from here.
+    for (uint32_t h = 0; h < nkeys; h++) {
+      uint32_t p = sm.key_at[h];
+      for (int v = 0; v < warp; v++) p += sm.key_cats[v][h];
+      const uint32_t same = same_as(sm.apart[h]) & apart;
+#pragma unroll
+      for (int i = 0; i < ITEMS; i++) {
+        const bool is = (same >> i) & 1u;
+        const uint32_t m = __ballot_sync(0xffffffffu, is);
+        if (is) {
+          const uint32_t dst = p + __popc(m & lt);
+          if (dst < a.n) store_id(a, dst, uint32_t(tile) + wofs + uint32_t(i) * 32);
+          else atomicOr(a.err, ERR_BOUNDS);
+        }
+        p += __popc(m);
+      }
+    }
     // The next tile's rows arrive while this one leaves.
     if (tile + TILE < end) load_rows(tile + TILE);
     if constexpr (PAY) fence_bulk();
     __syncthreads();
+    if (uint32_t(t) < nkeys)
+      for (int v = 0; v < WARPS; v++) sm.key_at[t] += sm.key_cats[v][t];
     if constexpr (PAY) {
       // Thread d sends bin d's records as one copy; it runs while the next tile is read and ranked.
       static_assert(PER == 1, "one bin a thread");
@@ -1380,7 +1580,7 @@ struct KeyOut {
                   (a.key_desc ? KeyT(~KeyT(0)) : KeyT(0)))) {}
 };
 
-template <typename KeyT, int PAY, int TIES>
+template <typename KeyT, int PAY, int TIES, bool FREQ = false>
 __device__ __forceinline__ void sort_body(const Args& a) {
   extern __shared__ __align__(16) unsigned char lsm[];
   using SM = LocalShared<KeyT, PAY>;
@@ -1393,6 +1593,13 @@ __device__ __forceinline__ void sort_body(const Args& a) {
   const Map<KeyT> map = load_map<KeyT>(st);
   const KeyOut<KeyT> ko(a);
   const int kw = pt_bytes(a.key_pt);
+  const uint32_t nkeys = FREQ ? st->nkeys : 0u;
+  // Rows of the frequent keys before key k: they are not in the buckets.
+  auto apart_before = [&](KeyT k) {
+    uint32_t rows = 0;
+    for (uint32_t h = 0; h < nkeys; h++) rows += k > KeyT(st->key[h]) ? st->key_rows[h] : 0u;
+    return rows;
+  };
   constexpr uint32_t SUB = 32 - BINS_LOG;          // position bits below the bin
   static_assert(CAP <= (1 << BINS_LOG), "a place fits beside the position bits below the bin");
 
@@ -1443,7 +1650,7 @@ __device__ __forceinline__ void sort_body(const Args& a) {
     const uint32_t* __restrict__ iin = a.ids[src] + row0;
     const uint4* __restrict__ rin = a.rec[src] + row0;
     auto id_of = [&](uint32_t p) { return PAY ? rin[p].x : iin[p]; };
-    const uint64_t dst0 = vbase + row0;
+    uint64_t dst0 = vbase + row0;
     if (dst0 + rows > a.n || rows > uint32_t(BIG)) {       // the scan rules both out
       if (t == 0) atomicOr(a.err, ERR_BOUNDS);
       if (PAY && rows <= uint32_t(CAP)) (void)mbar_wait(&sm.full, parity);
@@ -1567,7 +1774,21 @@ __device__ __forceinline__ void sort_body(const Args& a) {
     const uint32_t bn = next_bucket(b + a.sort_grid);
     if (bn < nb) load_rows();
     __syncthreads();
-    if (fast) {
+    // Frequent keys between the bucket's rows: row by row. (Not in a sort of ranks, keys or payload.)
+    bool split = false;
+    if (nkeys && fast) {
+      const uint32_t lo = apart_before(sm.key[0]), hi = apart_before(sm.key[rows - 1]);
+      split = lo != hi;
+      dst0 += split ? 0u : lo;
+      if (dst0 + hi + rows > a.n + (split ? 0u : hi)) {    // the scan rules it out
+        if (t == 0) atomicOr(a.err, ERR_BOUNDS);
+        break;
+      }
+    }
+    if (split) {
+      if constexpr (!PAY)
+        for (uint32_t r = t; r < rows; r += LTHREADS) store_id(a, dst0 + r + apart_before(sm.key[r]), sm.id[r]);
+    } else if (fast) {
       if constexpr (!PAY) {
         if (a.ranks.out) {
           // Equal keys share a bin, so a run of them is at most MAX_BIN rows: the walk to its end is short.
@@ -1665,7 +1886,9 @@ __device__ __forceinline__ void sort_body(const Args& a) {
       for (uint32_t r = t; r < rows; r += LTHREADS) {
         const uint32_t p = sm.slow.place[r];
         const KeyT k = sm.slow.key[r];
-        store_id(a, dst0 + r, id_of(p));
+        const uint64_t dst = dst0 + r + (nkeys ? apart_before(k) : 0u);
+        if (dst < a.n) store_id(a, dst, id_of(p));
+        else atomicOr(a.err, ERR_BOUNDS);
         if constexpr (!PAY) {
           if (a.ranks.out) {
             // The run's end by bisection: the first row not before (or the first after) the key.
@@ -1706,31 +1929,31 @@ __device__ __forceinline__ void sort_body(const Args& a) {
 
 // ---- the launches: of one sort, and of a batch's sorts (one a row of the grid)
 
-template <typename KeyT>
+template <typename KeyT, bool FREQ>
 __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(1024)
 buckets_kernel(const __grid_constant__ ColView col, const __grid_constant__ Args a) {
-  buckets_body<KeyT>(col, a);
+  buckets_body<KeyT, FREQ>(col, a);
 }
-template <typename KeyT>
+template <typename KeyT, bool FREQ>
 __global__ void __launch_bounds__(HTHREADS)
 bucket_histogram_kernel(const __grid_constant__ ColView col, const __grid_constant__ Args a) {
-  histogram_body<KeyT>(col, a);
+  histogram_body<KeyT, FREQ>(col, a);
 }
 template <typename KeyT>
 __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(1024) bucket_starts_kernel(const __grid_constant__ Args a) {
   starts_body<KeyT>(a);
 }
-template <typename KeyT, int PAY>
+template <typename KeyT, int PAY, bool FREQ>
 __global__ void __launch_bounds__(THREADS, 2) level1_kernel(const __grid_constant__ ColView col, const __grid_constant__ Args a) {
-  level1_body<KeyT, PAY>(col, a);
+  level1_body<KeyT, PAY, FREQ>(col, a);
 }
 template <typename KeyT, int PAY>
 __global__ void __launch_bounds__(THREADS, 2) level2_kernel(const __grid_constant__ Args a) {
   level2_body<KeyT, PAY>(a);
 }
-template <typename KeyT, int PAY, int TIES>
+template <typename KeyT, int PAY, int TIES, bool FREQ>
 __global__ void __launch_bounds__(LTHREADS, LBLOCKS) bucket_sort_kernel(const __grid_constant__ Args a) {
-  sort_body<KeyT, PAY, TIES>(a);
+  sort_body<KeyT, PAY, TIES, FREQ>(a);
 }
 
 struct alignas(16) BatchItem {
@@ -1964,7 +2187,7 @@ struct Layout {
     cursor1 = take(size_t(BINS1) * CUR_PAD * 4);
     cursor2 = take(nb * CUR_PAD * 4);
     chunk_bins = take(size_t(chunks_of(n)) * BINS1 * 4);
-    chunk_cats = take(size_t(chunks_of(n)) * 8);
+    chunk_cats = take(size_t(chunks_of(n)) * CATS * 4);
     total = at;
   }
 };
@@ -1974,18 +2197,18 @@ void smem_limit(F fn, size_t bytes) {
   AM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
 }
 
-template <typename KeyT, int PAY, int TIES>
+template <typename KeyT, int PAY, int TIES, bool FREQ = false>
 void launch_moves(const ColView& cv, const Args& a, cudaStream_t s) {
   static std::once_flag once;
   std::call_once(once, [] {
-    smem_limit(level1_kernel<KeyT, PAY>, sizeof(TileShared<KeyT, PAY>));
+    smem_limit(level1_kernel<KeyT, PAY, FREQ>, sizeof(TileShared<KeyT, PAY>));
     smem_limit(level2_kernel<KeyT, PAY>, sizeof(Tile2Shared<KeyT, PAY>));
-    smem_limit(bucket_sort_kernel<KeyT, PAY, TIES>, sizeof(LocalShared<KeyT, PAY>));
+    smem_limit(bucket_sort_kernel<KeyT, PAY, TIES, FREQ>, sizeof(LocalShared<KeyT, PAY>));
   });
   if (!a.one_launch) {
     {
       KernelTimer kt("bucket_level1", s);
-      level1_kernel<KeyT, PAY><<<a.nchunks, THREADS, sizeof(TileShared<KeyT, PAY>), s>>>(cv, a);
+      level1_kernel<KeyT, PAY, FREQ><<<a.nchunks, THREADS, sizeof(TileShared<KeyT, PAY>), s>>>(cv, a);
       AM_CUDA(cudaGetLastError());
     }
     if (a.bucket_cap > a.bins1_cap) {
@@ -1996,32 +2219,44 @@ void launch_moves(const ColView& cv, const Args& a, cudaStream_t s) {
   }
   {
     KernelTimer kt("bucket_sort", s);
-    bucket_sort_kernel<KeyT, PAY, TIES><<<a.sort_grid, LTHREADS, sizeof(LocalShared<KeyT, PAY>), s>>>(a);
+    bucket_sort_kernel<KeyT, PAY, TIES, FREQ><<<a.sort_grid, LTHREADS, sizeof(LocalShared<KeyT, PAY>), s>>>(a);
+    AM_CUDA(cudaGetLastError());
+  }
+}
+
+// The plan and the counts. FREQ: frequent keys are set apart (the other sorts' kernels carry none of it).
+template <typename KeyT, bool FREQ = false>
+void launch_counts(const Sort& b, const Args& a, cudaStream_t s) {
+  {
+    KernelTimer kt("bucket_plan", s);
+    buckets_kernel<KeyT, FREQ><<<CLUSTER, 1024, 0, s>>>(b.col, a);
+    AM_CUDA(cudaGetLastError());
+  }
+  if (a.one_launch) return;
+  static std::once_flag once;
+  std::call_once(once, [] { smem_limit(bucket_histogram_kernel<KeyT, FREQ>, size_t(MAX_BUCKETS) * 4); });
+  {
+    KernelTimer kt("bucket_histogram", s);
+    bucket_histogram_kernel<KeyT, FREQ><<<a.hist_grid, HTHREADS, size_t(a.bucket_cap) * 4, s>>>(b.col, a);
+    AM_CUDA(cudaGetLastError());
+  }
+  {
+    KernelTimer kt("bucket_scan", s);
+    bucket_starts_kernel<KeyT><<<CLUSTER, 1024, 0, s>>>(a);
     AM_CUDA(cudaGetLastError());
   }
 }
 
 template <typename KeyT>
 void launch_all(const Sort& b, const Args& a, int pay, cudaStream_t s) {
-  {
-    KernelTimer kt("bucket_plan", s);
-    buckets_kernel<KeyT><<<CLUSTER, 1024, 0, s>>>(b.col, a);
-    AM_CUDA(cudaGetLastError());
-  }
-  if (!a.one_launch) {
-    static std::once_flag once;
-    std::call_once(once, [] { smem_limit(bucket_histogram_kernel<KeyT>, size_t(MAX_BUCKETS) * 4); });
-    {
-      KernelTimer kt("bucket_histogram", s);
-      bucket_histogram_kernel<KeyT><<<a.hist_grid, HTHREADS, size_t(a.bucket_cap) * 4, s>>>(b.col, a);
-      AM_CUDA(cudaGetLastError());
-    }
-    {
-      KernelTimer kt("bucket_scan", s);
-      bucket_starts_kernel<KeyT><<<CLUSTER, 1024, 0, s>>>(a);
-      AM_CUDA(cudaGetLastError());
+  if constexpr (sizeof(KeyT) == 8) {
+    if (a.frequent) {
+      launch_counts<KeyT, true>(b, a, s);
+      launch_moves<KeyT, 0, TIES_ID, true>(b.col, a, s);
+      return;
     }
   }
+  launch_counts<KeyT>(b, a, s);
   if constexpr (sizeof(KeyT) == 8) {
     if (a.ties.offsets) {
       launch_moves<KeyT, 0, TIES_STRING>(b.col, a, s);
@@ -2107,6 +2342,7 @@ static Args make_args(const Sort& b) {
   a.bins1_cap = b.payload ? BINS1 / 2 : BINS1;
   a.has_payload = b.payload ? 1 : 0;
   a.one_launch = b.n <= SAMPLES ? 1 : 0;
+  a.frequent = b.frequent && !a.one_launch && !b.payload && !b.key_out && !b.ranks.out && !b.ties.offsets && !b.src_ids && b.key_bytes == 8 ? 1 : 0;
   if (a.one_launch) {
     a.bucket_cap = std::min(a.bucket_cap, ONE_CAP);
     a.bins1_cap = ONE_CAP;

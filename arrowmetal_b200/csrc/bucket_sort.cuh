@@ -9,6 +9,7 @@ namespace am {
 namespace bs {
 
 constexpr uint32_t MODE_BUCKETS = 1, MODE_FALLBACK = 2;
+constexpr int FREQUENT = 4;              // keys with too many rows for a bucket that a sort can set apart
 
 // What the sampling, the histogram and the scan decide, read by the kernels after them. All zero when a
 // sort starts.
@@ -20,7 +21,12 @@ struct State {
   uint32_t linear;                       // not 0: the range is cut into this many equal buckets
   uint32_t buckets, s2, bins1;           // buckets; level 1 sorts by bucket >> s2 into bins1 bins
   uint32_t n_value, n_null, n_nan;
-  uint32_t max_bucket, pad;
+  uint32_t max_bucket;
+  // Keys too frequent for a bucket (Sort::frequent), ascending: their rows leave in row order, as null rows
+  // do, to the places from `key_at` on among the values.
+  uint32_t nkeys;
+  unsigned long long key[FREQUENT];
+  uint32_t key_rows[FREQUENT], key_at[FREQUENT];
 };
 
 // Strings behind 8-byte keys of their leading characters (strings.cu): rows of equal keys order by the rest
@@ -70,6 +76,7 @@ struct Sort {
   int key_pt;
   bool key_source;                       // a float order that ties values: null rows, zeros and NaNs keep their own bits
   bool key_desc, nulls_first;
+  bool frequent;                         // set frequent keys apart (an order alone: no payload, key column, ranks or ties)
   uint32_t* err;
   rs::SortSummary* summary;
 };

@@ -216,8 +216,11 @@ __device__ __forceinline__ void histogram_rows(const ColView& col, KeyStats* __r
   }
 }
 
+// `done` (may be NULL): the mode of a bucket sort that makes the key's statistics unnecessary when it ran.
 template <typename KeyT, int THREADS, int ITEMS, bool RANGE = true>
-__global__ void __launch_bounds__(THREADS) key_histogram_kernel(const __grid_constant__ ColView col, KeyStats* __restrict__ st, uint64_t n) {
+__global__ void __launch_bounds__(THREADS) key_histogram_kernel(const __grid_constant__ ColView col, KeyStats* __restrict__ st, uint64_t n,
+                                                                const uint32_t* done = nullptr) {
+  if (done && *done == bs::MODE_BUCKETS) return;
   constexpr uint64_t CHUNK = uint64_t(THREADS) * ITEMS;
   histogram_rows<KeyT, THREADS, ITEMS, RANGE>(col, st, uint64_t(blockIdx.x) * CHUNK, n, uint64_t(gridDim.x) * CHUNK);
 }
@@ -270,6 +273,8 @@ __device__ void plan_body(const PlanArgs& a, KeyStats* __restrict__ st, KeyPlan*
   __shared__ uint8_t s_active[MAX_SLOTS];
   const int t = threadIdx.x;
   const uint32_t n = uint32_t(a.n);
+  // A lexsort whose last key the bucket sort has ordered: that key's slots have nothing to do.
+  const bool last_done = a.last_key_mode && *a.last_key_mode == bs::MODE_BUCKETS;
 
   // 1. Per key: fold a lower key's null / NaN-block rows into its key range when there is room,
   //    else give them key 0 and a category pass; add the folded rows to the histogram.
@@ -315,6 +320,10 @@ __device__ void plan_body(const PlanArgs& a, KeyStats* __restrict__ st, KeyPlan*
   // 2. Which digit passes are not constant.
   for (int sl = 0; sl < a.nslots; sl++) {
     const int k = a.slot_key[sl], d = a.slot_digit[sl];
+    if (last_done && k == a.nkeys - 1) {
+      if (t == 0) s_active[sl] = 0;
+      continue;
+    }
     if (d < 0) {
       if (t == 0) s_active[sl] = (kp[k].fold_mode == 1) ? 1 : 0;
       continue;
@@ -339,7 +348,7 @@ __device__ void plan_body(const PlanArgs& a, KeyStats* __restrict__ st, KeyPlan*
     }
     if ((key0_cats && !any_key0) || !any) s_active[a.slot_key0_first] = 1;
 
-    int ids_src = -1, keys_src = -1;        // -1: identity ids / keys not in a buffer
+    int ids_src = last_done ? 2 : -1, keys_src = -1;        // -1: identity ids / keys not in a buffer
     uint32_t run = 0;
     int last_any = -1;
     for (int sl = 0; sl < a.nslots; sl++) if (s_active[sl]) last_any = sl;
@@ -385,7 +394,7 @@ __device__ void plan_body(const PlanArgs& a, KeyStats* __restrict__ st, KeyPlan*
     sum->value_rows = st[0].n_value;
     sum->null_rows = st[0].n_null;
     sum->nan_rows = st[0].n_nan;
-    sum->passes_run = run;
+    sum->passes_run = run + (last_done ? sum->passes_run : 0u);
     sum->passes_total = uint32_t(a.nslots);
   }
   __syncthreads();
@@ -756,7 +765,7 @@ __device__ __forceinline__ void onesweep_pass(const PassArgs& pa, const ColView&
     si = sm.desc.src_ids;
     di = sm.desc.dst_ids;
     keys_in = sk < 0 ? nullptr : static_cast<const KeyT*>(sk == 0 ? pa.keys[0] : pa.keys[1]) + row_off;
-    ids_in = si < 0 ? nullptr : (si == 0 ? pa.ids[0] : pa.ids[1]) + row_off;
+    ids_in = si < 0 ? nullptr : (si == 0 ? pa.ids[0] : si == 1 ? pa.ids[1] : pa.ids[2]) + row_off;
     keys_out = dk < 0 ? nullptr : static_cast<KeyT*>(dk == 0 ? pa.keys[0] : pa.keys[1]) + row_off;
     ids_out = di < 0 ? nullptr : (di == 0 ? pa.ids[0] : pa.ids[1]) + row_off;
   };
@@ -1839,13 +1848,14 @@ static int pass_blocks_per_sm() {
 
 // `range`: the key range too (a lower key of a multi-key sort).
 template <typename KeyT>
-static void launch_histogram(const ColView& cv, KeyStats* st, uint64_t n, cudaStream_t s, bool range = false) {
+static void launch_histogram(const ColView& cv, KeyStats* st, uint64_t n, cudaStream_t s, bool range = false,
+                             const uint32_t* done = nullptr) {
   constexpr int CHUNK = HIST_THREADS * HIST_ITEMS;
   const uint64_t chunks = (n + CHUNK - 1) / CHUNK;
   const int grid = int(std::min<uint64_t>(chunks, uint64_t(device().sm_count) * 8));
   KernelTimer kt("radix_histogram", s);
-  if (range) key_histogram_kernel<KeyT, HIST_THREADS, HIST_ITEMS, true><<<grid, HIST_THREADS, 0, s>>>(cv, st, n);
-  else key_histogram_kernel<KeyT, HIST_THREADS, HIST_ITEMS, false><<<grid, HIST_THREADS, 0, s>>>(cv, st, n);
+  if (range) key_histogram_kernel<KeyT, HIST_THREADS, HIST_ITEMS, true><<<grid, HIST_THREADS, 0, s>>>(cv, st, n, done);
+  else key_histogram_kernel<KeyT, HIST_THREADS, HIST_ITEMS, false><<<grid, HIST_THREADS, 0, s>>>(cv, st, n, done);
   AM_CUDA(cudaGetLastError());
 }
 
@@ -2334,7 +2344,11 @@ void radix_sort(const std::vector<SortKey>& keys_in, int64_t n64, void* out, int
   const size_t header = (off_sum + sizeof(SortSummary) + 255) & ~size_t(255);
   const size_t kbuf = ((n * max_kb) + 255) & ~size_t(255);
   const size_t ibuf = carry_ids ? ((n * id_bytes) + 255) & ~size_t(255) : 0;
-  ScratchBlock scratch(s, header + 2 * kbuf + 2 * ibuf);
+  // A lexsort's last key by buckets, the digit passes of the other keys from its order on.
+  const bool last_first = K > 1 && pt_key_bytes(keys[K - 1].col->pt) == 8 && n <= bs::MAX_ROWS && !debug_skip_first_tile();
+  const size_t off_order = header + 2 * kbuf + 2 * ibuf;
+  const size_t off_bs = off_order + ibuf;
+  ScratchBlock scratch(s, last_first ? off_bs + bs::scratch_bytes(n) : off_order);
   char* base = scratch.data();
   AM_CUDA(cudaMemsetAsync(base, 0, header, s));
   KeyStats* st = reinterpret_cast<KeyStats*>(base + off_stats);
@@ -2360,10 +2374,32 @@ void radix_sort(const std::vector<SortKey>& keys_in, int64_t n64, void* out, int
   }
 
   std::vector<ColView> views(K);
+  for (int k = 0; k < K; k++) views[k] = make_view(keys[k]);
+  uint32_t* const order = last_first ? reinterpret_cast<uint32_t*>(base + off_order) : nullptr;
+  if (last_first) {
+    AM_CUDA(cudaMemsetAsync(base + off_bs, 0, bs::zeroed_bytes(n), s));
+    const SortKey& key = keys[K - 1];
+    bs::Sort b{};
+    b.col = views[K - 1];
+    b.key_bytes = pt_key_bytes(key.col->pt);
+    b.n = n;
+    b.scratch = base + off_bs;
+    b.keys[0] = kbufA;
+    b.keys[1] = kbufB;
+    b.ids[0] = reinterpret_cast<char*>(ibufA);
+    b.ids[1] = reinterpret_cast<char*>(ibufB);
+    b.out = order;
+    b.key_pt = key.col->pt;
+    b.nulls_first = key.nulls_first;
+    b.frequent = true;
+    b.err = stream_scratch(s, 0).err;
+    b.summary = sum;
+    pa.last_key_mode = &bs::enqueue(b, s)->mode;
+  }
   for (int k = 0; k < K; k++) {
-    views[k] = make_view(keys[k]);
-    if (pt_key_bytes(keys[k].col->pt) == 8) launch_histogram<uint64_t>(views[k], st + k, n, s, k > 0);
-    else launch_histogram<uint32_t>(views[k], st + k, n, s, k > 0);
+    const uint32_t* done = k == K - 1 ? pa.last_key_mode : nullptr;
+    if (pt_key_bytes(keys[k].col->pt) == 8) launch_histogram<uint64_t>(views[k], st + k, n, s, k > 0, done);
+    else launch_histogram<uint32_t>(views[k], st + k, n, s, k > 0, done);
   }
   {
     KernelTimer kt("radix_plan", s);
@@ -2447,7 +2483,12 @@ void radix_sort(const std::vector<SortKey>& keys_in, int64_t n64, void* out, int
     }
   }
   for (int sl = 0; sl < S && !hybrid; sl++) {
-    if (narrow_status) {
+    if (last_first) {
+      const uint64_t n16 = (uint64_t(max_tiles) * NBINS * sizeof(uint32_t) + 15) / 16;
+      const int grid = int(std::min<uint64_t>((n16 + 255) / 256, uint64_t(device().sm_count) * 4));
+      zero_status_kernel<<<std::max(grid, 1), 256, 0, s>>>(pd + sl, reinterpret_cast<uint4*>(sc.status), n16);
+      AM_CUDA(cudaGetLastError());
+    } else if (narrow_status) {
       AM_CUDA(cudaMemsetAsync(sc.status, 0, size_t(max_tiles) * NBINS * sizeof(uint32_t), s));
     } else if (sc.epoch >= (1u << 30) - 1) {
       AM_CUDA(cudaMemsetAsync(sc.status, 0, sc.status_words * sizeof(uint64_t), s));
@@ -2460,6 +2501,7 @@ void radix_sort(const std::vector<SortKey>& keys_in, int64_t n64, void* out, int
     a.keys[1] = kbufB;
     a.ids[0] = ibufA;
     a.ids[1] = ibufB;
+    a.ids[2] = order;
     a.final_out = out;
     a.status = sc.status;
     a.epoch = ++sc.epoch;

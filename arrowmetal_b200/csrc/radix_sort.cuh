@@ -76,6 +76,7 @@ struct SortSummary {
 struct PlanArgs {
   uint64_t n;
   uint64_t hyb_min_rows;                    // value rows from which one 8-byte key takes the two-level sort
+  const uint32_t* last_key_mode;            // not NULL: where this is bs::MODE_BUCKETS, PassArgs::ids[2] holds the last key's order
   int32_t nkeys, nslots, slot_key0_first, index_wide;
   uint8_t key_bytes[MAX_KEYS];
   uint8_t nulls_first[MAX_KEYS];
@@ -120,7 +121,7 @@ struct PassArgs {
   const PassDesc* desc;
   const KeyPlan* kplan;
   void* keys[2];
-  uint32_t* ids[2];
+  uint32_t* ids[3];           // the last: an order that the passes start from
   void* final_out;            // the index output (NULL: none wanted)
   void* status;
   uint32_t* tile_counter;

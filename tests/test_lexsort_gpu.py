@@ -98,3 +98,74 @@ def test_config_shaped_multikey(am, oracle):
     got = ids(am.lexsort_indices([k1, k2], [True, False]))
     want = pc.sort_indices(pa.table({"a": k1, "b": k2}), [("a", "descending"), ("b", "ascending")]).to_numpy()
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("n", [1, 3000, 65_537, 400_003])
+@pytest.mark.parametrize("kinds", [("zipf", "specials"), ("i8", "f32"), ("two", "i64"), ("i64", "i64"), ("i8", "i8"), ("two", "i8", "specials"),
+                                   ("specials", "zipf"), ("ones", "specials"), ("i8", "ones", "mid"), ("f16", "mid")])
+def test_last_key_by_buckets(am, oracle, n, kinds):
+    # The last key ordered by buckets and the others by digit passes from there: every float special in a
+    # leading and in the last key, categories in both, leading keys of one value (one pass has to run), last
+    # keys that no bucket holds (their digit passes run), last keys too narrow for buckets.
+    rng = np.random.default_rng(n + 7 * len(kinds) + len(kinds[0]))
+
+    def make(kind):
+        if kind == "zipf":
+            p = np.arange(1, 201) ** -1.1
+            return rng.integers(-2**31, 2**31, 200).astype(np.int32)[rng.choice(200, n, p=p / p.sum())]
+        if kind in ("specials", "f32", "f16"):
+            v = rng.normal(0, 1e3, n)
+            u = rng.random(n)
+            for value, lo in ((-0.0, 0.0), (0.0, 0.01), (np.inf, 0.02), (-np.inf, 0.03), (np.nan, 0.04), (-np.nan, 0.05)):
+                v[(u >= lo) & (u < lo + 0.01)] = value
+            return v.astype({"specials": np.float64, "f32": np.float32, "f16": np.float16}[kind])
+        if kind == "i8":
+            return rng.integers(-128, 128, n).astype(np.int8)
+        if kind == "two":
+            return rng.integers(0, 2, n).astype(np.int32)
+        if kind == "mid":
+            return rng.integers(0, n // 10 + 1, n)
+        if kind == "ones":
+            return np.full(n, 2**64 - 1, np.uint64)
+        return rng.integers(-2**63, 2**63 - 1, n, dtype=np.int64, endpoint=True)
+
+    for rep in range(3):
+        arrays, opts = [], []
+        for k in kinds:
+            nf = (0.0, 0.05, 0.4)[int(rng.integers(3))]
+            arrays.append(pa.array(make(k), mask=rng.random(n) < nf if nf else None, from_pandas=False))
+            opts.append((bool(rng.integers(2)), ("at_end", "at_start")[int(rng.integers(2))],
+                         ("ieee", "total", "nan_largest")[int(rng.integers(3))]))
+        want = np.arange(n)
+        for a, (d, p, f) in reversed(list(zip(arrays, opts))):
+            want = want[oracle.np_argsort(a.take(pa.array(want)), d, p, f)]
+        got = ids(am.lexsort_indices(arrays, [o[0] for o in opts], [o[1] for o in opts], [o[2] for o in opts]))
+        assert np.array_equal(got, want), opts
+
+
+@pytest.mark.parametrize("n", [65_537, 300_007, 1_500_001])
+@pytest.mark.parametrize("kind", ["specials", "ends", "one", "six", "half"])
+def test_last_key_with_frequent_values(am, oracle, n, kind):
+    # Values of the last key too frequent for a bucket: floats' specials in every order, the smallest and
+    # largest keys, a single value, more values than are set apart, a value of half the rows.
+    rng = np.random.default_rng(n + len(kind))
+    lead = rng.integers(-3, 4, n).astype(np.int32)
+    u = rng.random(n)
+    if kind == "specials":
+        v = rng.normal(0, 1e3, n)
+        for i, x in enumerate((-0.0, 0.0, np.inf, -np.inf, np.nan)):
+            v[(u >= 0.05 * i) & (u < 0.05 * i + 0.05)] = x
+    else:
+        v = rng.integers(-2**62, 2**62, n)
+        picks = {"ends": (-2**63, 2**63 - 1, 0), "one": (12345,), "six": tuple(int(x) for x in rng.integers(-2**62, 2**62, 6)),
+                 "half": (-7,)}[kind]
+        share = 0.5 if kind == "half" else 0.1
+        for i, x in enumerate(picks):
+            v[(u >= share * i) & (u < share * (i + 1))] = x
+    for desc, placement, order in ((False, "at_end", "ieee"), (True, "at_start", "total"), (False, "at_start", "nan_largest")):
+        last = pa.array(v, mask=rng.random(n) < 0.1, from_pandas=False)
+        arrays = [pa.array(lead, mask=rng.random(n) < 0.02), last]
+        want = oracle.np_argsort(last, desc, placement, order)
+        want = want[oracle.np_argsort(arrays[0].take(pa.array(want)), True, "at_end", "ieee")]
+        got = ids(am.lexsort_indices(arrays, [True, desc], ["at_end", placement], ["ieee", order]))
+        assert np.array_equal(got, want), (desc, placement, order)
