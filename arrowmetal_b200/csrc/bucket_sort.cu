@@ -5,13 +5,13 @@
 //      distribution. The sampled key range is cut into 512 equal coarse cells, a coarse cell into up to
 //      2^11 equal fine cells by its share of the sample, a fine cell into equal sub-buckets by its
 //      estimated rows (light neighbours share a bucket): a monotone map key -> bucket of two table reads
-//      and one multiply, whose buckets hold about TARGET rows whatever the distribution.
+//      and one multiply, whose buckets hold about TARGET (CELL_TARGET) rows whatever the distribution.
 //   2. bucket_histogram_kernel reads the column once: exact rows of every bucket, and of every level-1
 //      bin of every chunk (a contiguous range of rows). bucket_starts_kernel turns them into starts, and
 //      decides: when a bucket is larger than BIG rows (heavily repeated keys), nothing has moved yet and
 //      the digit passes sort the column instead.
 //   3. level1_kernel, one CTA a chunk, scatters the chunk's rows to their level-1 bins (the bucket
-//      itself up to BINS1 buckets, else 128 buckets a bin), level2_kernel each bin's rows to their
+//      itself up to BINS1 buckets, else 256 buckets a bin), level2_kernel each bin's rows to their
 //      buckets. A row's place among its tile's rows of a bin comes from one shared-memory atomic, in no
 //      particular order: the row id that moves with it orders equal keys at the end. Rows are staged in
 //      shared memory by bin, so a bin's rows leave as one run. The null and NaN rows go straight to
@@ -52,7 +52,10 @@ constexpr int S2 = 8, BINS2 = 1 << S2;            // buckets a level-1 bin of a 
 static_assert(MAX_BUCKETS / BINS2 <= 256, "level-1 bins of a two-level sort");
 constexpr int CAP = 2048;                         // rows the shared-memory sort of a bucket takes
 constexpr int BIG = 4096;                         // rows its slower form takes
-constexpr uint32_t TARGET = 1300;                 // rows a bucket is meant to hold
+constexpr uint32_t TARGET = 1300;                 // rows a bucket of evenly spread keys is meant to hold
+// With cells, whose densities are estimates: four columns of 5.5M normally distributed float64 keys had
+// their largest bucket at 1,710-2,205 rows with 1,300, and one of more than CAP rows costs 100 us.
+constexpr uint32_t CELL_TARGET = 1100;
 constexpr uint32_t SAMPLES = 65536;               // keys looked at (every key of a shorter column)
 constexpr int CLUSTER = 8;                        // CTAs of the one-cluster kernels
 constexpr uint32_t ONE_CAP = 1024;                // buckets of a column of at most SAMPLES rows
@@ -310,7 +313,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
 // cluster's shared memories. (One CTA alone, its samples read twice from L2, took 60 us for 65,536.)
 struct PlanShared {
   uint32_t coarse_cnt[COARSE];
-  uint32_t half_cnt[2 * FINE];           // the halves of the fine cells
+  union {
+    uint32_t part_cnt[4 * FINE];         // the quarters of the fine cells, up to the plan
+    struct {
+      uint32_t bins[ONE_CAP], start[ONE_CAP];      // then (one launch) the CTA's rows of each bucket, where they go
+    };
+  };
   uint32_t coarse[COARSE];
   uint32_t warp[32];
   uint32_t group[1024];
@@ -318,9 +326,8 @@ struct PlanShared {
   unsigned long long wmax[32], wmin[32];
   uint32_t mode, buckets, linear;        // the plan, from the first CTA
   // One launch for the counts and the moves too (columns of at most SAMPLES rows): the fine cells, the
-  // CTA's rows of each bucket, where they go, its null and NaN rows by item and warp, and their sums.
+  // CTA's null and NaN rows by item and warp, and their sums.
   uint32_t fine[FINE];
-  uint32_t bins[ONE_CAP], start[ONE_CAP];
   uint32_t cats[2][SAMPLES / (1024 * CLUSTER) * 32];
   uint32_t ncats[2];
   unsigned long long diff;
@@ -339,7 +346,7 @@ __device__ __forceinline__ void tell_plan(const Args& a, unsigned long long lo, 
   st->mode = MODE_BUCKETS;
 }
 
-// The first CTA, with the cluster's counts of the half cells: buckets from the fine cells' rows.
+// The first CTA, with the cluster's counts of the quarter cells: buckets from the fine cells' rows.
 template <typename KeyT>
 __device__ void plan_cells(const Args& a, PlanShared& sm, const Map<KeyT>& map, unsigned long long lo, unsigned long long span,
                            uint32_t shc, uint32_t sv, uint32_t nfine, bool full) {
@@ -360,11 +367,17 @@ __device__ void plan_cells(const Args& a, PlanShared& sm, const Map<KeyT>& map, 
     room[q] = 1;
     below[q] = 0;
     if (f >= nfine) continue;
-    const uint32_t h0 = sm.half_cnt[2 * f], h1 = sm.half_cnt[2 * f + 1];
+    const uint4 part = *reinterpret_cast<const uint4*>(&sm.part_cnt[4 * f]);
+    const uint32_t h0 = part.x + part.y, h1 = part.z + part.w, most = max(max(part.x, part.y), max(part.z, part.w));
     const float c = float(h0 + h1), h = float(max(h0, h1));
     rows[q] = full ? h0 + h1 : uint32_t((c + sqrtf(c) + 1.0f) * scale);
-    // Split by the fuller half: keys are not even within a cell that spans a factor of two of a float's range.
-    dense[q] = 2u * (full ? max(h0, h1) : uint32_t((h + sqrtf(h) + 1.0f) * scale));
+    // Split by the fuller half, or by the fullest quarter where the rows of a wide cell crowd there (a
+    // float's cell of eight octaves has half its rows in the last): by the halves alone, two buckets of 6M
+    // normally distributed float64 keys held over CAP rows, and their slow form was the sort's last 100 us
+    // (the buckets' sort 172 us, 66 so).
+    const float e = float(most);
+    dense[q] = full ? max(2u * max(h0, h1), 4u * most)
+                    : uint32_t(max(2.0f * (h + sqrtf(h) + 1.0f), 4.0f * (e + 0.5f * sqrtf(e))) * scale);
     // The fine cell's coarse cell: the last one starting at or before it.
     uint32_t l = 0, r = COARSE;
     while (r - l > 1) {
@@ -380,9 +393,9 @@ __device__ void plan_cells(const Args& a, PlanShared& sm, const Map<KeyT>& map, 
   bad = __syncthreads_or(bad);
   // Buckets: a heavy cell (over half a target) is split into equal parts; light neighbours share one.
   // With more buckets than fit, larger targets.
-  uint32_t target = TARGET, total = 0, base[PER], m[PER];
+  uint32_t target = CELL_TARGET, total = 0, base[PER], m[PER];
   bool start[PER];
-  for (int attempt = 0; attempt < 4 && !bad; attempt++) {
+  for (int attempt = 0; attempt < 8 && !bad; attempt++) {
     const uint32_t half = target / 2;
     uint32_t light = 0;
 #pragma unroll
@@ -415,7 +428,7 @@ __device__ void plan_cells(const Args& a, PlanShared& sm, const Map<KeyT>& map, 
 #pragma unroll
     for (int q = 0; q < PER; q++) base[q] += off;
     if (total + 2 <= a.bucket_cap) break;
-    target += target / 4;
+    target += target / 8;
   }
   if (bad || total + 2 > a.bucket_cap || sv == 0) {
     if (t == 0) {
@@ -465,10 +478,10 @@ template <typename KeyT, int U>
 __device__ uint32_t take_frequent(const Args& a, PlanShared& sm, const KeyT (&key)[U], uint32_t live) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
-  static_assert(COUNTERS <= 2 * FINE && FREQUENT * 64 + FREQUENT + FREQUENT * 2 <= 1024, "they borrow the plan's arrays");
+  static_assert(COUNTERS <= 4 * FINE && FREQUENT * 64 + FREQUENT + FREQUENT * 2 <= 1024, "they borrow the plan's arrays");
   constexpr uint32_t NONE = 0xFFFFFFFFu;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  uint32_t* counter = sm.half_cnt;
+  uint32_t* counter = sm.part_cnt;
   uint32_t* votes = sm.group;                      // by key and bit, then the voters, then the keys' words
   uint32_t* voters = votes + FREQUENT * 64;
   uint32_t* words = voters + FREQUENT;
@@ -485,7 +498,7 @@ __device__ uint32_t take_frequent(const Args& a, PlanShared& sm, const KeyT (&ke
   for (int q = 0; q < COUNTERS / 1024; q++) {
     uint32_t c = 0;
 #pragma unroll
-    for (int r = 0; r < CLUSTER; r++) c += cl.map_shared_rank(&sm, r)->half_cnt[q * 1024 + t];
+    for (int r = 0; r < CLUSTER; r++) c += cl.map_shared_rank(&sm, r)->part_cnt[q * 1024 + t];
     best[q] = (c << COUNTERS_LOG) | uint32_t(q * 1024 + t);
   }
   const uint32_t least = max(4 * SAMPLES / COUNTERS, uint32_t(float(BIG / 2) * float(a.nsamples) / float(a.n)));
@@ -602,7 +615,7 @@ __device__ __forceinline__ void buckets_body(const ColView& col, const Args& a) 
   }
   if constexpr (FREQ) live &= ~take_frequent<KeyT, U>(a, sm, key, live);
   for (int i = t; i < COARSE; i += 1024) sm.coarse_cnt[i] = 0;
-  for (int i = t; i < 2 * FINE; i += 1024) sm.half_cnt[i] = 0;
+  for (int i = t; i < 4 * FINE; i += 1024) sm.part_cnt[i] = 0;
   // The sampled range, over the cluster.
   {
     uint64_t mx = 0, mn = 0;
@@ -713,21 +726,21 @@ __device__ __forceinline__ void buckets_body(const ColView& col, const Args& a) 
       if ((live >> u) & 1u) {
         uint32_t f, frac;
         cell_of(map, sm.coarse, KeyT(key[u] - map.lo), f, frac);
-        atomicAdd(&sm.half_cnt[2 * f + (frac >> 31)], 1u);
+        atomicAdd(&sm.part_cnt[4 * f + (frac >> 30)], 1u);
       }
     cl.sync();
-    if (rank == 0) {
-      for (int i = t; i < 2 * FINE; i += 1024) {
-        uint32_t c = sm.half_cnt[i];
+    // Each CTA sums its share of the counts into the first one's.
+    constexpr int SHARE = 4 * FINE / CLUSTER;
+    static_assert(SHARE <= 1024 && 4 * FINE % CLUSTER == 0, "a count a thread");
+    if (t < SHARE) {
+      const int i = int(rank) * SHARE + t;
+      uint32_t c = 0;
 #pragma unroll
-        for (int r = 1; r < CLUSTER; r++) c += cl.map_shared_rank(&sm, r)->half_cnt[i];
-        sm.half_cnt[i] = c;
-      }
+      for (int r = 0; r < CLUSTER; r++) c += cl.map_shared_rank(&sm, r)->part_cnt[i];
+      cl.map_shared_rank(&sm, 0)->part_cnt[i] = c;
     }
-    if (rank == 0) {
-      __syncthreads();
-      plan_cells<KeyT>(a, sm, map, lo, span, shc, sv, nfine, full);
-    }
+    cl.sync();
+    if (rank == 0) plan_cells<KeyT>(a, sm, map, lo, span, shc, sv, nfine, full);
   }
   cl.sync();                             // no CTA leaves, or goes on, before the plan stands
   if (!a.one_launch) return;
@@ -1344,7 +1357,7 @@ struct Tile2Shared {
   uint8_t bin[TILE];
 };
 
-// Level 2: tiles of one level-1 bin's rows to its 128 buckets. A tile reserves its rows of a bucket with
+// Level 2: tiles of one level-1 bin's rows to its 256 buckets. A tile reserves its rows of a bucket with
 // one atomic.
 template <typename KeyT, int PAY>
 __device__ __forceinline__ void level2_body(const Args& a) {
