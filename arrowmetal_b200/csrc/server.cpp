@@ -167,7 +167,7 @@ bool am_server_t::take_shared(std::vector<ReqPtr>& unit, int64_t* footprint) {
   for (auto& it : cand) {
     const ServeRequest& q = **it;
     if (q.length * 32 < hi - lo) continue;
-    if (in_flight > 0 && in_flight + fp + q.footprint > cap) continue;
+    if (in_flight + fp + q.footprint > cap) continue;      // only a request by itself may exceed the cap
     keep.push_back(it);
     rows += q.length;
     fp += q.footprint;
