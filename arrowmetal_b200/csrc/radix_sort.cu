@@ -19,6 +19,9 @@
 // instead of being written by an iota kernel. A lexsort carries the row ids through every pass, so
 // the reference's "take the next key column, argsort, compose" becomes one gather of the next key
 // inside its first pass.
+//
+// One key of at most bs::MAX_ROWS rows sorts by buckets instead (bucket_sort.cu), and so does the last key of
+// a lexsort; the passes here run behind it when its buckets are too large, all in one cooperative launch.
 #include <algorithm>
 #include <atomic>
 #include <cstddef>
@@ -2344,7 +2347,11 @@ void radix_sort(const std::vector<SortKey>& keys_in, int64_t n64, void* out, int
   const size_t header = (off_sum + sizeof(SortSummary) + 255) & ~size_t(255);
   const size_t kbuf = ((n * max_kb) + 255) & ~size_t(255);
   const size_t ibuf = carry_ids ? ((n * id_bytes) + 255) & ~size_t(255) : 0;
-  // A lexsort's last key by buckets, the digit passes of the other keys from its order on.
+  // A lexsort's last key by buckets, the digit passes of the other keys from its order on: for 8-byte keys,
+  // of which eight digits can vary. After a key of 200 values, by passes and so: float64 1,804 and 1,160 us
+  // at 16M rows, 282 and 242 at 1M, 189 and 164 at 2,000; 40-bit int64 1,343 and 998, 236 and 220, 160 and
+  // 160. A last key that no bucket holds pays for the try: 896 and 977 at 16M, 124 and 190 at 2,000. Four
+  // passes of a 4-byte key cost about what its buckets do (1,105 and 919; 189 and 187; 131 and 133).
   const bool last_first = K > 1 && pt_key_bytes(keys[K - 1].col->pt) == 8 && n <= bs::MAX_ROWS && !debug_skip_first_tile();
   const size_t off_order = header + 2 * kbuf + 2 * ibuf;
   const size_t off_bs = off_order + ibuf;

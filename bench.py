@@ -785,10 +785,10 @@ def algorithmic_bytes(n, m, passes, local_sort=False, records=False):
 
 # DRAM bytes (read + write) per row of the workload, per kernel and step: dram__bytes_read.sum +
 # dram__bytes_write.sum of the kernel's launches in one sort, from one ncu capture of this benchmark at
-# 25,000,000 rows (22.5M value rows: the two-level sort runs as at 50M), divided by the rows. Keyed by
+# 25,000,000 rows (22.5M value rows: a two-level bucket sort as at 50M), divided by the rows. Keyed by
 # whether the payload rode through the sort in records (the table in HBM) or was gathered afterwards.
 TRAFFIC_PER_ROW = {
-    True: {"radix_histogram": 8.26, "radix_onesweep_pass": 83.97, "radix_local_sort": 38.00},
+    True: {"bucket_histogram": 8.27, "bucket_level1": 42.45, "bucket_level2": 41.42, "bucket_sort": 37.57},
     False: {},
 }
 
