@@ -370,14 +370,15 @@ __device__ void plan_cells(const Args& a, PlanShared& sm, const Map<KeyT>& map, 
     const uint4 part = *reinterpret_cast<const uint4*>(&sm.part_cnt[4 * f]);
     const uint32_t h0 = part.x + part.y, h1 = part.z + part.w, most = max(max(part.x, part.y), max(part.z, part.w));
     const float c = float(h0 + h1), h = float(max(h0, h1));
-    rows[q] = full ? h0 + h1 : uint32_t((c + sqrtf(c) + 1.0f) * scale);
+    // (At 50M rows a sampled key stands for 763: a cell of 5,000 rows shows one sample once in a hundred columns.)
+    rows[q] = full ? h0 + h1 : uint32_t((c + 1.5f * sqrtf(c) + 2.5f) * scale);
     // Split by the fuller half, or by the fullest quarter where the rows of a wide cell crowd there (a
     // float's cell of eight octaves has half its rows in the last): by the halves alone, two buckets of 6M
     // normally distributed float64 keys held over CAP rows, and their slow form was the sort's last 100 us
     // (the buckets' sort 172 us, 66 so).
     const float e = float(most);
     dense[q] = full ? max(2u * max(h0, h1), 4u * most)
-                    : uint32_t(max(2.0f * (h + sqrtf(h) + 1.0f), 4.0f * (e + 0.5f * sqrtf(e))) * scale);
+                    : uint32_t(max(2.0f * (h + sqrtf(h) + 2.0f), 4.0f * (e + 0.5f * sqrtf(e))) * scale);
     // The fine cell's coarse cell: the last one starting at or before it.
     uint32_t l = 0, r = COARSE;
     while (r - l > 1) {
