@@ -2723,6 +2723,13 @@ GraphCache& graph_cache() {
   static thread_local GraphCache c;
   return c;
 }
+// Graphs are captured on a stream of the thread's own: on the sort's stream other threads free the arrays of
+// earlier results meanwhile, which a capturing stream refuses.
+cudaStream_t capture_stream() {
+  static thread_local cudaStream_t c = nullptr;
+  if (!c) AM_CUDA(cudaStreamCreateWithFlags(&c, cudaStreamNonBlocking));
+  return c;
+}
 
 bool graphs_enabled() {
   static const bool on = [] {
@@ -2765,16 +2772,17 @@ BatchGraph* find_or_capture(const GroupLayout<KeyT, THREADS, ITEMS>& L, uint32_t
     sl.host = pinned_alloc(L.tables);
     AM_CUDA(cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming));
     cudaGraph_t graph = nullptr;
-    AM_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    const cudaStream_t cs = capture_stream();
+    AM_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
     try {
-      enqueue_group<KeyT, THREADS, ITEMS>(L, g->base, g->status, err, sl.host, false, s);
+      enqueue_group<KeyT, THREADS, ITEMS>(L, g->base, g->status, err, sl.host, false, cs);
     } catch (...) {
       cudaGraph_t discard = nullptr;
-      (void)cudaStreamEndCapture(s, &discard);
+      (void)cudaStreamEndCapture(cs, &discard);
       if (discard) (void)cudaGraphDestroy(discard);
       throw;
     }
-    AM_CUDA(cudaStreamEndCapture(s, &graph));
+    AM_CUDA(cudaStreamEndCapture(cs, &graph));
     const cudaError_t e = cudaGraphInstantiate(&sl.exec, graph, 0);
     (void)cudaGraphDestroy(graph);
     AM_CUDA(e);
@@ -2985,16 +2993,17 @@ void sort_segment_buckets(const std::vector<SortKey>& keys, const std::vector<vo
           sl.host = pinned_alloc(L.tables);
           AM_CUDA(cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming));
           cudaGraph_t graph = nullptr;
-          AM_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+          const cudaStream_t cs = capture_stream();
+          AM_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
           try {
-            enqueue_buckets<KeyT>(L, ng->base, sl.host, host.data(), false, s);
+            enqueue_buckets<KeyT>(L, ng->base, sl.host, host.data(), false, cs);
           } catch (...) {
             cudaGraph_t discard = nullptr;
-            (void)cudaStreamEndCapture(s, &discard);
+            (void)cudaStreamEndCapture(cs, &discard);
             if (discard) (void)cudaGraphDestroy(discard);
             throw;
           }
-          AM_CUDA(cudaStreamEndCapture(s, &graph));
+          AM_CUDA(cudaStreamEndCapture(cs, &graph));
           const cudaError_t e = cudaGraphInstantiate(&sl.exec, graph, 0);
           (void)cudaGraphDestroy(graph);
           AM_CUDA(e);

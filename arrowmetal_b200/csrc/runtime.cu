@@ -176,7 +176,7 @@ void* dmalloc(size_t bytes, cudaStream_t s) {
   return p;
 }
 void dfree(void* p, cudaStream_t s) {
-  if (p) (void)cudaFreeAsync(p, s);
+  if (p && cudaFreeAsync(p, s) != cudaSuccess) (void)cudaGetLastError();    // not the next launch's error
 }
 
 DevBuffer::~DevBuffer() {
