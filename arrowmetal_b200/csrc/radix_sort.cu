@@ -1570,7 +1570,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 8 : THREADS == 256 ?
       const uint32_t r = uint32_t(warp) * (ITEMS * 32) + uint32_t(i) * 32 + lane;
       key[i] = r < size ? keys[start + r] : 0ull;
       if constexpr (REC) id[i] = r;
-      else id[i] = r < size ? ids[start + r] : 0u;
+      else id[i] = ids && r < size ? ids[start + r] : 0u;       // a sorted copy alone has no row ids
     }
     // The tile's empty slots (r >= size) are the last rows in order. They take digit 255 in the ballots
     // but are neither counted nor stored: every row before them keeps its place in [0, size), and their

@@ -82,3 +82,18 @@ def test_order_by_rebuilds_the_key_column(am):
     assert k.null_count == nn
     assert np.array_equal(np.frombuffer(k.buffers()[1], dtype=np.int64)[nn:N], key[order])
     assert np.array_equal(out["p"].to_arrow().to_numpy(), payload[np.concatenate([nulls, order])])
+
+
+@pytest.mark.parametrize("case", ["local_sorts", "fallback_passes", "float_total"])
+def test_sorted_copy_without_row_ids(am, case):
+    # A sorted copy alone carries no row ids through the two-level sort, which serves 8-byte keys above
+    # 62,914,560 rows.
+    n = 62_914_560 + 5001
+    rng = np.random.default_rng(17)
+    v = rng.integers(-2**50, 2**50, n, dtype=np.int64)
+    if case == "fallback_passes":
+        v[rng.random(n) < 0.3] = 123_456_789_012                # one bucket of ~19M rows
+    if case == "float_total":
+        v = v.astype(np.float64)
+    got = am.MetalArray.from_arrow(pa.array(v)).sort(False, "at_end", "total" if case == "float_total" else "ieee")
+    assert np.array_equal(got.to_arrow().to_numpy(), np.sort(v))
