@@ -2958,8 +2958,9 @@ void sort_segment_buckets(const std::vector<SortKey>& keys, const std::vector<vo
   if (!large.empty()) sort_segment_class<KeyT, 512, 8>(keys, outs, large, allow_graph, s);
   if (group.empty()) return;
   BucketLayout<KeyT> L(keys, group);
-  const size_t status_bytes = size_t(L.max_tiles) * NBINS * sizeof(uint32_t);
-  StreamScratch& sc = stream_scratch(s, (status_bytes + 7) / 8);
+  // The passes clear the look-back words 16 bytes at a time: a whole number of those.
+  const size_t status_bytes = (size_t(L.max_tiles) * NBINS * sizeof(uint32_t) + 15) & ~size_t(15);
+  StreamScratch& sc = stream_scratch(s, status_bytes / 8);
   sc.epoch = (1u << 30) - 1;               // its words are used without an epoch: later users start over
   bs::prepare_batch(int(sizeof(KeyT)));
   (void)batch_all_passes_blocks<KeyT>();
@@ -2987,7 +2988,7 @@ void sort_segment_buckets(const std::vector<SortKey>& keys, const std::vector<vo
         ng->lens = L.lens;
         ng->tables = L.tables;
         AM_CUDA(cudaMalloc(reinterpret_cast<void**>(&ng->base), L.total));
-        AM_CUDA(cudaMalloc(&ng->status, std::max<size_t>(status_bytes + 16, 16)));
+        AM_CUDA(cudaMalloc(&ng->status, std::max<size_t>(status_bytes, 16)));
         const std::vector<char> host = L.fill(keys, outs, group, ng->base, ng->status, sc.err);
         for (auto& sl : ng->slot) {
           sl.host = pinned_alloc(L.tables);

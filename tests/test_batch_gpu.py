@@ -193,3 +193,13 @@ def test_batches_by_buckets(am, oracle, kinds):
     for call in range(4):
         opts = [(bool(rng.integers(2)), PLACEMENTS[rng.integers(2)], ORDERS[rng.integers(3)]) for _ in arrays]
         check_batch(am, oracle, arrays, opts)
+
+
+@pytest.mark.parametrize("tiles", [1, 3, 47])
+def test_digit_passes_behind_the_buckets_of_an_odd_number_of_tiles(am, oracle, tiles):
+    # An odd number of 5,120-row tiles is not a whole number of 16-byte pieces of look-back words.
+    rng = np.random.default_rng(tiles)
+    n = 5120 * tiles
+    v = rng.integers(0, 2**40, n, dtype=np.int64)
+    v[rng.random(n) < 0.9] = 77
+    check_batch(am, oracle, [pa.array(v)], [(False, "at_end", "ieee")])
