@@ -8,8 +8,8 @@
 //      and one multiply, whose buckets hold about TARGET (CELL_TARGET) rows whatever the distribution.
 //   2. bucket_histogram_kernel reads the column once: exact rows of every bucket, and of every level-1
 //      bin of every chunk (a contiguous range of rows). bucket_starts_kernel turns them into starts, and
-//      decides: when a bucket is larger than BIG rows (heavily repeated keys), nothing has moved yet and
-//      the digit passes sort the column instead.
+//      decides: when a bucket is larger than one CTA should sort (large_rows; a key repeated very often),
+//      nothing has moved yet and the digit passes sort the column instead.
 //   3. level1_kernel, one CTA a chunk, scatters the chunk's rows to their level-1 bins (the bucket
 //      itself up to BINS1 buckets, else 256 buckets a bin), level2_kernel each bin's rows to their
 //      buckets. A row's place among its tile's rows of a bin comes from one shared-memory atomic, in no
@@ -17,8 +17,14 @@
 //      shared memory by bin, so a bin's rows leave as one run. The null and NaN rows go straight to
 //      their final places, in row order (ballots, and the chunks' counts).
 //   4. bucket_sort_kernel orders each bucket by (key, row id): a counting step over 2,048 bins that
-//      divide the bucket's key range, then comparisons within the bin (a row or two), and writes ids,
-//      rebuilt keys and payload to their final rows.
+//      divide the bucket's key range, then comparisons of (position, row id) within the bin (a row or two), and
+//      writes ids, rebuilt keys and payload to their final rows. Buckets of keys that repeat more often than
+//      a bin may hold, and those of more than CAP rows, are left to bucket_later_kernel: a second counting step, over
+//      row ids, orders the rows of one key, and larger buckets are cut into parts first.
+//
+// Keys that repeat, the order of 16M int64 rows in us (digit passes and two-level sort; buckets with a bitonic sort of
+// crowded ones; this): 10 rows a value 880, 1,454, 676; 50: 1,057, 2,640, 776; 500: 1,608, 1,242, 870; 3,000: 1,193,
+// 1,245, 1,036.
 //
 // The order is the stable sort's: (key, row id) is what a stable sort orders by. What it replaces moved
 // rows stably (nine ballots a row and a look-back over the tiles before it, 8.4 and 5.8 warp
@@ -50,8 +56,9 @@ constexpr uint32_t MAX_BUCKETS = 40960;
 constexpr int BINS1 = 1024;                       // level-1 bins
 constexpr int S2 = 8, BINS2 = 1 << S2;            // buckets a level-1 bin of a two-level sort
 static_assert(MAX_BUCKETS / BINS2 <= 256, "level-1 bins of a two-level sort");
-constexpr int CAP = 2048;                         // rows the shared-memory sort of a bucket takes
-constexpr int BIG = 4096;                         // rows its slower form takes
+constexpr int CAP = 2048;                         // rows the shared-memory sort of a bucket (or a part of one) takes
+constexpr int BIG = 4096;                         // rows a bucket of strings may hold
+constexpr uint32_t LARGE = 16384;                 // rows a bucket of any other keys may hold: it is split by its CTA
 constexpr uint32_t TARGET = 1300;                 // rows a bucket of evenly spread keys is meant to hold
 // With cells, whose densities are estimates: four columns of 5.5M normally distributed float64 keys had
 // their largest bucket at 1,710-2,205 rows with 1,300, and one of more than CAP rows costs 100 us.
@@ -61,19 +68,23 @@ constexpr int CLUSTER = 8;                        // CTAs of the one-cluster ker
 constexpr uint32_t ONE_CAP = 1024;                // buckets of a column of at most SAMPLES rows
 constexpr int BINS = 2048, BINS_LOG = 11;         // bins of the shared-memory sort
 constexpr uint32_t CATS = 2 + FREQUENT;           // a chunk's rows apart from the buckets: null, NaN, each frequent key
-constexpr uint32_t MAX_BIN = 32;                  // rows a bin may hold for the comparisons
+// Rows a bin may hold for the comparisons. 16M int64 keys with 10 rows a value, the order: 676 us where such bins are
+// compared, 843 where later_body takes most of them (24); with 50 rows a value 776 in later_body, 1,113 compared (64).
+constexpr uint32_t MAX_BIN = 40;
 constexpr uint32_t META_SPLIT = 0x80000000u;
 constexpr int CUR_PAD = 8;                        // cursors 32 bytes apart: same-sector atomics queue
 constexpr int THREADS = 512, ITEMS = 7, TILE = THREADS * ITEMS, WARPS = THREADS / 32;
 constexpr int HTHREADS = 1024, HITEMS = 8;
 constexpr int MAX_CHUNKS = 296;                   // two level-1 CTAs on each of 148 SMs
 constexpr int LTHREADS = 256, LITEMS = CAP / LTHREADS, LBLOCKS = 4;
+constexpr int NTHREADS = 256, NITEMS = CAP / NTHREADS, NBLOCKS = 4;      // the buckets that they put off
 
 struct Args {
   State* st;
-  uint32_t *coarse, *fine, *bfirst, *bmeta, *bcount, *bpos, *cursor1, *cursor2, *chunk_bins, *chunk_cats;
+  uint32_t *coarse, *fine, *bfirst, *bmeta, *bcount, *bpos, *later, *cursor1, *cursor2, *chunk_bins, *chunk_cats;
   uint32_t nsamples, nchunks, chunk_rows, bucket_cap, bins1_cap;
-  uint32_t hist_grid, level2_grid, sort_grid;     // CTAs that take part in those steps
+  uint32_t large;                                 // rows a bucket may hold
+  uint32_t hist_grid, level2_grid, sort_grid, later_grid;     // CTAs that take part in those steps
   uint64_t n;
   void* keys[2];
   uint32_t* ids[2];
@@ -389,7 +400,7 @@ __device__ void plan_cells(const Args& a, PlanShared& sm, const Map<KeyT>& map, 
     const uint32_t left = shc - (coarse[l] >> 16);           // key bits below the fine cell
     room[q] = left >= 16 ? 65535u : 1u << left;
     below[q] = uint32_t(sizeof(KeyT)) * 8u - left;
-    if (room[q] == 1u && (c - 4.0f * sqrtf(c)) * scale > float(BIG)) bad = 1;
+    if (room[q] == 1u && (c - 4.0f * sqrtf(c)) * scale > float(a.large)) bad = 1;
   }
   bad = __syncthreads_or(bad);
   // Buckets: a heavy cell (over half a target) is split into equal parts; light neighbours share one.
@@ -810,7 +821,7 @@ __device__ __forceinline__ void buckets_body(const ColView& col, const Args& a) 
   uint32_t values;
   const uint32_t at = block_scan<1024>(rows, sm.warp, values);
   sm.start[t] = at + ahead;
-  const uint32_t over = __syncthreads_or(int(rows > uint32_t(BIG)));
+  const uint32_t over = __syncthreads_or(int(rows > a.large));
   go = go && !over;
   if (rank == 0) {
     if (go && uint32_t(t) < nb) a.bpos[t] = at;
@@ -1081,7 +1092,7 @@ __device__ __forceinline__ void starts_body(const Args& a) {
     a.bpos[nb] = carry;
     st->max_bucket = big;
     if (carry + apart != st->n_value) atomicOr(a.err, ERR_BOUNDS);
-    if (big > uint32_t(BIG) || carry + apart != st->n_value) {
+    if (big > a.large || carry + apart != st->n_value) {
       st->mode = MODE_FALLBACK;
     } else {
       // The counters of the digit passes' sort: the key's digits that vary. A two-level sort's two
@@ -1522,34 +1533,85 @@ __device__ __forceinline__ bool tied_before(const StringTies& s, uint32_t a, uin
   return a < b;
 }
 
-// A CTA's shared memory: the fast form's arrays, or the slower one's keys and places of up to BIG rows.
-template <typename KeyT, int PAY>
-struct LocalShared {
+// What a CTA has at hand: a bucket of the map, or a part of a larger one (split_rows): rows whose positions
+// come from their own keys' range (KIND_KEY), or rows of one key, placed by their ids (KIND_ID).
+constexpr uint32_t KIND_BUCKET = 0, KIND_KEY = 1, KIND_ID = 2;
+// Parts waiting, at most. A split of a large bucket leaves 3 x rows / 1,024 + 2 of them or fewer, one of at most CAP
+// rows 2 x rows / 33 + 4, and one of those waiting is split at a time, at most nine deep (11 bits of the key's or the
+// id's range each).
+constexpr uint32_t PARTS = 256;
+constexpr uint32_t PART_ROWS = CAP / 2;
+static_assert(3 * LARGE / PART_ROWS + 2 * CAP / (MAX_BIN + 1) + 9 * 4 <= PARTS, "the parts of the largest bucket");
+constexpr uint32_t MAX_PAIRED = 8;                 // rows a bin may hold for comparisons, of the buckets put off
+constexpr uint32_t CROWD = MAX_PAIRED + 1;         // their crowded bins start at least so many rows apart
+
+// A CTA's shared memory: the fast form's arrays, or (strings) the slower one's keys and places of up to BIG rows.
+template <typename KeyT>
+struct SlowRows {
+  KeyT key[BIG];
+  uint16_t place[BIG];
+};
+template <typename KeyT, int PAY, int TIES>
+struct FastShared {
   uint64_t full;                        // the bucket's records have arrived
   uint32_t warp[32];
-  uint32_t crowded;
+  uint32_t crowded;                     // some bin holds more than MAX_BIN rows
+  uint32_t some_fast;                   // some bucket of the CTA was ordered by the fast form
   union {
     struct {
       union {
         struct {
-          uint32_t start[BINS + 4];     // rows per bin, then where each bin starts
-          uint32_t word[CAP];           // by bin: the row's position below its bin, then its place in the bucket
+          alignas(16) uint32_t start[BINS / 2 + 4];     // rows per bin, then where each bin starts: 16 bits each
+          uint64_t word[CAP];           // by bin: the row's position, and its id (strings: its place in the bucket) below it
         };
-        KeyT key[CAP];                  // in order
+        struct {                        // in order:
+          KeyT key[CAP];
+          uint32_t id[PAY ? 1 : CAP];
+          uint16_t place[PAY ? CAP : 2];          // the row's place in the bucket
+        };
       };
-      uint32_t id[PAY ? 1 : CAP];       // the rows' ids, as they come; then in order
-      uint16_t place[PAY ? CAP : 2];    // in order: the row's place in the bucket
+      uint32_t in_id[TIES == TIES_STRING ? CAP : 1];      // the rows' ids, as they come
       alignas(16) uint4 rec[PAY ? CAP : 1];     // the rows' records, as they come
     };
-    struct {
-      KeyT key[BIG];
-      uint16_t place[BIG];
-    } slow;
+    std::conditional_t<TIES == TIES_STRING, SlowRows<KeyT>, uint32_t> slow;
   };
 };
+// The same of the buckets put off.
+template <typename KeyT, int PAY>
+struct LaterShared {
+  uint64_t full;
+  uint32_t warp[32];
+  unsigned long long red[3][NTHREADS / 32];
+  uint32_t mixed[CAP / CROWD + 1];      // by crowded bin: its rows are at several positions
+  // The waiting parts: first row; rows, buffers (bit 29) and kind (bits 30 and 31); the rows of their key, where it
+  // is one (ranks).
+  uint32_t part_at[PARTS], part_n[PARTS];
+  uint32_t run_at[PAY ? 1 : PARTS], run_n[PAY ? 1 : PARTS];
+  union {
+    struct {
+      alignas(16) uint32_t start[BINS + 4];       // rows per bin, then where each bin starts
+      uint32_t word[CAP];               // by bin: the row's position below its bin, then its place in the bucket
+    };
+    KeyT key[CAP];                      // in order
+  };
+  uint32_t id[PAY ? 1 : CAP];           // the rows' ids, as they come; then in order
+  uint16_t place[CAP];                  // the words' bins; then, in order, the rows' places in the bucket
+  alignas(16) uint4 rec[PAY ? CAP : 1]; // the rows' records, as they come
+};
 
-// A bucket of more than CAP rows, or with many equal or very close keys: bitonic sort of (key, row id),
-// the ids of equal keys read where the rows are.
+// Read and written as 16-byte vectors, and by bulk copies.
+template <typename SM>
+constexpr bool vectors_aligned() {
+  return offsetof(SM, start) % 16 == 0 && offsetof(SM, rec) % 16 == 0;
+}
+static_assert(vectors_aligned<FastShared<uint32_t, 0, TIES_ID>>() && vectors_aligned<FastShared<uint64_t, 0, TIES_ID>>() &&
+              vectors_aligned<FastShared<uint32_t, 1, TIES_ID>>() && vectors_aligned<FastShared<uint64_t, 1, TIES_ID>>() &&
+              vectors_aligned<FastShared<uint64_t, 0, TIES_STRING>>() && vectors_aligned<LaterShared<uint32_t, 0>>() &&
+              vectors_aligned<LaterShared<uint64_t, 0>>() && vectors_aligned<LaterShared<uint32_t, 1>>() &&
+              vectors_aligned<LaterShared<uint64_t, 1>>(), "shared arrays read as vectors");
+
+// A string bucket of more than CAP rows, or with many equal or very close keys: bitonic sort of (key, the
+// rest of the string, row id), the ids of equal keys read where the rows are.
 template <int TIES, typename KeyT, typename IdOf>
 __device__ __forceinline__ void bitonic_rows(KeyT* key, uint16_t* place, uint32_t size, const KeyT* in, IdOf&& id_of,
                                              const StringTies& ties) {
@@ -1583,6 +1645,359 @@ __device__ __forceinline__ void bitonic_rows(KeyT* key, uint16_t* place, uint32_
   }
 }
 
+// Smallest and largest of every thread's (lo, hi) and (lo2, hi2), to every thread.
+__device__ __forceinline__ uint64_t warp_least(uint64_t v) {
+  const uint32_t h = __reduce_min_sync(0xffffffffu, uint32_t(v >> 32));
+  const uint32_t l = __reduce_min_sync(0xffffffffu, uint32_t(v >> 32) == h ? uint32_t(v) : ~0u);
+  return (uint64_t(h) << 32) | l;
+}
+__device__ __forceinline__ uint32_t warp_least(uint32_t v) { return __reduce_min_sync(0xffffffffu, v); }
+template <typename SM, typename T>
+__device__ __forceinline__ void block_range(SM& sm, T& lo, T& hi, uint32_t& lo2, uint32_t& hi2) {
+  lo = warp_least(lo);
+  hi = T(~warp_least(T(~hi)));
+  lo2 = warp_least(lo2);
+  hi2 = ~warp_least(~hi2);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) {
+    const int w = threadIdx.x >> 5;
+    sm.red[0][w] = lo;
+    sm.red[1][w] = hi;
+    sm.red[2][w] = (uint64_t(hi2) << 32) | lo2;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < NTHREADS / 32; w++) {
+    lo = min(lo, T(sm.red[0][w]));
+    hi = max(hi, T(sm.red[1][w]));
+    lo2 = min(lo2, uint32_t(sm.red[2][w]));
+    hi2 = max(hi2, uint32_t(sm.red[2][w] >> 32));
+  }
+}
+// Shift that brings the top bit of `range` to bit 63 (0 for an empty range).
+__device__ __forceinline__ uint32_t range_shift(uint64_t range) { return range ? uint32_t(__clzll((long long)range)) : 0u; }
+
+// Rows per bin into the bins' starts, over all 2,048; true when some bin holds more than MAX_PAIRED rows.
+template <typename SM>
+__device__ __forceinline__ bool count_scan(SM& sm, uint32_t rows) {
+  constexpr int PER = BINS / NTHREADS;
+  const uint32_t t = threadIdx.x;
+  uint4 c[PER / 4];
+  uint32_t sum = 0, mx = 0, all;
+#pragma unroll
+  for (int q = 0; q < PER / 4; q++) {
+    c[q] = *reinterpret_cast<const uint4*>(&sm.start[t * PER + 4 * q]);
+    sum += c[q].x + c[q].y + c[q].z + c[q].w;
+    mx = max(mx, max(max(c[q].x, c[q].y), max(c[q].z, c[q].w)));
+  }
+  uint32_t s = block_scan<NTHREADS>(sum, sm.warp, all);
+#pragma unroll
+  for (int q = 0; q < PER / 4; q++) {
+    *reinterpret_cast<uint4*>(&sm.start[t * PER + 4 * q]) = make_uint4(s, s + c[q].x, s + c[q].x + c[q].y, s + c[q].x + c[q].y + c[q].z);
+    s += c[q].x + c[q].y + c[q].z + c[q].w;
+  }
+  if (t == NTHREADS - 1) sm.start[BINS] = rows;
+  return __syncthreads_or(int(mx > MAX_PAIRED)) != 0;
+}
+
+// A bucket too large for the fast form, cut into parts that fit it: its rows move to the other buffers
+// (unused by then) by 2,048 bins over the range of their keys, or, all keys being equal, of their row ids;
+// bins of more than `heavy` rows become parts of their own, the others share parts of at most CAP rows. A part that
+// is still too large is split again by its own, 2,048 times smaller range, so every split ends. One CTA does
+// it: the map's buckets are a thousand rows, and only a key repeated thousands of times makes a larger one.
+// Adds the parts to the list; returns their number. Leaves sm.start dirty.
+template <typename KeyT, int PAY, typename SM>
+__device__ __forceinline__ uint32_t split_rows(SM& sm, const Args& a, uint32_t first, uint32_t size, uint32_t side, uint32_t kind,
+                                            uint32_t heavy, uint32_t run_at, uint32_t run_n, uint32_t parts) {
+  const uint32_t t = threadIdx.x;
+  const KeyT* kin = static_cast<const KeyT*>(a.keys[side]) + first;
+  KeyT* kout = static_cast<KeyT*>(a.keys[side ^ 1u]) + first;
+  const uint32_t* iin = a.ids[side] + first;
+  uint32_t* iout = a.ids[side ^ 1u] + first;
+  const uint4* rin = a.rec[side] + first;
+  uint4* rout = a.rec[side ^ 1u] + first;
+  constexpr uint32_t U = 4, STEP = U * NTHREADS;
+  uint64_t lo = ~0ull, hi = 0;
+  uint32_t id0 = ~0u, id1 = 0;
+  for (uint32_t r0 = t; r0 < size; r0 += STEP) {
+#pragma unroll
+    for (uint32_t u = 0; u < U; u++)
+      if (r0 + u * NTHREADS < size) {
+        const uint64_t k = kin[r0 + u * NTHREADS];
+        const uint32_t id = PAY ? rin[r0 + u * NTHREADS].x : iin[r0 + u * NTHREADS];
+        lo = min(lo, k);
+        hi = max(hi, k);
+        id0 = min(id0, id);
+        id1 = max(id1, id);
+      }
+  }
+  block_range(sm, lo, hi, id0, id1);
+  const bool by_id = lo == hi;
+  if (by_id) {
+    if (kind != KIND_ID) {
+      run_at = first;
+      run_n = size;
+    }
+    lo = id0;
+    hi = id1;
+  }
+  const uint32_t sh = range_shift(hi - lo);
+  auto bin_of = [&](uint64_t x) { return uint32_t(((x - lo) << sh) >> (64 - BINS_LOG)); };
+  auto axis = [&](uint32_t r) { return by_id ? uint64_t(PAY ? rin[r].x : iin[r]) : uint64_t(kin[r]); };
+  for (uint32_t x = t; x < BINS; x += NTHREADS) sm.start[x] = 0;
+  __syncthreads();
+  for (uint32_t r0 = t; r0 < size; r0 += STEP) {
+#pragma unroll
+    for (uint32_t u = 0; u < U; u++)
+      if (r0 + u * NTHREADS < size) atomicAdd(&sm.start[bin_of(axis(r0 + u * NTHREADS))], 1u);
+  }
+  __syncthreads();
+  constexpr uint32_t PER = BINS / NTHREADS;
+  {
+    uint32_t c[PER], sum = 0, all;
+#pragma unroll
+    for (uint32_t q = 0; q < PER; q++) {
+      c[q] = sm.start[t * PER + q];
+      sum += c[q];
+    }
+    uint32_t s = block_scan<NTHREADS>(sum, sm.warp, all);
+#pragma unroll
+    for (uint32_t q = 0; q < PER; q++) {
+      sm.start[t * PER + q] = s;
+      sm.word[t * PER + q] = s;                    // the scatter's cursors
+      s += c[q];
+    }
+    if (t == NTHREADS - 1) sm.start[BINS] = size;
+  }
+  __syncthreads();
+  // A part starts at a bin of its own, after one, and where a window of PART_ROWS rows starts.
+  uint32_t flags = 0, total;
+#pragma unroll
+  for (uint32_t q = 0; q < PER; q++) {
+    const uint32_t b = t * PER + q, s = sm.start[b], e = sm.start[b + 1];
+    const uint32_t p = b ? sm.start[b - 1] : 0u;
+    if (b == 0 || e - s > heavy || s - p > heavy || s / PART_ROWS != p / PART_ROWS) flags |= 1u << q;
+  }
+  uint32_t at = parts + block_scan<NTHREADS>(uint32_t(__popc(flags)), sm.warp, total);
+  if (parts + total > PARTS) {                     // ruled out by the bound on the parts
+    if (t == 0) atomicOr(a.err, ERR_BOUNDS);
+    return parts;
+  }
+#pragma unroll
+  for (uint32_t q = 0; q < PER; q++)
+    if ((flags >> q) & 1u) sm.part_at[at++] = first + sm.start[t * PER + q];
+  __syncthreads();
+  for (uint32_t p = t; p < total; p += NTHREADS) {
+    const uint32_t end = p + 1 < total ? sm.part_at[parts + p + 1] : first + size;
+    sm.part_n[parts + p] = (end - sm.part_at[parts + p]) | ((side ^ 1u) << 29) | ((by_id ? KIND_ID : KIND_KEY) << 30);
+    if constexpr (!PAY) {
+      sm.run_at[parts + p] = run_at;
+      sm.run_n[parts + p] = run_n;
+    }
+  }
+  for (uint32_t r0 = t; r0 < size; r0 += STEP) {
+    KeyT k[U];
+    uint32_t id[PAY ? 1 : U];
+    uint4 rec[PAY ? U : 1];
+#pragma unroll
+    for (uint32_t u = 0; u < U; u++)
+      if (r0 + u * NTHREADS < size) {
+        k[u] = kin[r0 + u * NTHREADS];
+        if constexpr (PAY) rec[u] = rin[r0 + u * NTHREADS];
+        else id[u] = iin[r0 + u * NTHREADS];
+      }
+#pragma unroll
+    for (uint32_t u = 0; u < U; u++)
+      if (r0 + u * NTHREADS < size) {
+        uint32_t row;
+        if constexpr (PAY) row = rec[u].x;
+        else row = id[u];
+        const uint32_t p = atomicAdd(&sm.word[bin_of(by_id ? uint64_t(row) : uint64_t(k[u]))], 1u);
+        kout[p] = k[u];
+        if constexpr (PAY) rout[p] = rec[u];
+        else iout[p] = id[u];
+      }
+  }
+  // The parts' records come by bulk copies.
+  if constexpr (PAY) asm volatile("fence.proxy.async;" ::: "memory");
+  __syncthreads();
+  return parts + total;
+}
+
+// The rows of a bucket with many rows at one position, or in one bin: from the words by bin (and sm.place, the
+// words' bins), a bin's rows in neighbouring threads, to the bucket's keys and ids (or places) in order.
+//   Rows at one position are nearly always one key's: they are ranked by row id, and each one's key is compared
+// with that of one of them; only where some differ the ranking is made again by whole keys.
+//   A crowded bin (more than MAX_PAIRED rows) at one position cuts its m places into m cells by row id, which hold a
+// row or two each: a second counting step. At several positions (two repeated keys that share a bin) its rows are
+// compared with one another, up to MAX_MIXED of them; for more the bucket is split by the range of its own keys, every
+// crowded bin a part.
+constexpr uint32_t MAX_MIXED = 256;
+constexpr uint32_t LOW = uint32_t(1 << BINS_LOG) - 1u;       // a word's place
+constexpr uint32_t TIED_DONE = 0, TIED_SPLIT = 1, TIED_TIMEOUT = 2;
+template <typename KeyT, int PAY, typename SM>
+__device__ __forceinline__ uint32_t order_tied(SM& sm, const Args& a, const KeyT* kin, uint32_t rows, bool exact, bool crowded,
+                                               uint32_t parity, uint32_t id0, uint32_t idsh) {
+  const uint32_t t = threadIdx.x;
+  const int ni = int((rows + NTHREADS - 1 - t) / NTHREADS);
+  if constexpr (PAY) {
+    if (!mbar_wait(&sm.full, parity)) {
+      atomicOr(a.err, ERR_LOOKBACK_TIMEOUT);
+      return TIED_TIMEOUT;
+    }
+  }
+  auto id_at = [&](uint32_t p) { return PAY ? sm.rec[PAY ? p : 0].x : sm.id[PAY ? 0 : p]; };
+  // Item i: the row whose word is the (i x NTHREADS + t)-th. Words and places are kept, all else is read again from
+  // shared memory: with ids and bins in registers too they spill (27 local loads a row).
+  uint32_t word[NITEMS], at[NITEMS];
+  uint32_t crowd = 0;                              // items in crowded bins at one position
+  auto bin_of_item = [&](int i, uint32_t& s0, uint32_t& s1) {
+    const uint32_t b = sm.place[t + i * NTHREADS];
+    s0 = sm.start[b];
+    s1 = sm.start[b + 1];
+  };
+#pragma unroll
+  for (int i = 0; i < NITEMS; i++) word[i] = i < ni ? sm.word[t + i * NTHREADS] : 0u;
+  if (crowded) {
+#pragma unroll
+    for (int i = 0; i < NITEMS; i++) {
+      if (i >= ni) break;
+      uint32_t s0, s1;
+      bin_of_item(i, s0, s1);
+      if (s1 - s0 > MAX_PAIRED && (sm.word[s0] ^ word[i]) > LOW) sm.mixed[s0 / CROWD] = 1;
+    }
+    bool split = false;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < NITEMS; i++) {
+      if (i >= ni) break;
+      uint32_t s0, s1;
+      bin_of_item(i, s0, s1);
+      if (s1 - s0 <= MAX_PAIRED) continue;
+      if (!sm.mixed[s0 / CROWD]) crowd |= 1u << i;
+      else split |= s1 - s0 > MAX_MIXED;
+    }
+    if (__syncthreads_or(int(split))) return TIED_SPLIT;
+  }
+  bool differ = false;
+#pragma unroll
+  for (int i = 0; i < NITEMS; i++) {
+    if (i >= ni) break;
+    uint32_t s0, s1;
+    bin_of_item(i, s0, s1);
+    const uint32_t me = word[i], mine = id_at(me & LOW);
+    uint32_t rank = s0, rep = me;
+    if ((crowd >> i) & 1u) {
+      rep = sm.word[s0];
+      rank = s0 + __umulhi((mine - id0) << idsh, s1 - s0);
+    } else if (s1 - s0 > 1) {
+#pragma unroll 1
+      for (uint32_t q = s0; q < s1; q++) {
+        const uint32_t o = sm.word[q];
+        if ((o ^ me) <= LOW) {
+          rep = min(rep, o);
+          rank += id_at(o & LOW) < mine ? 1u : 0u;
+        } else {
+          rank += o < me ? 1u : 0u;
+        }
+      }
+    }
+    at[i] = rank;
+    if (!exact && rep != me) differ |= kin[rep & LOW] != kin[me & LOW];
+  }
+  if (__syncthreads_or(int(differ))) {
+    // Few rows are compared with one another; a larger bin becomes a part, whose own range is 2,048 times smaller.
+    bool split = false;
+#pragma unroll 1
+    for (int i = 0; i < ni; i++) {
+      const uint32_t q = t + i * NTHREADS, me = sm.word[q], mine = id_at(me & LOW), b = sm.place[q];
+      const uint32_t s0 = sm.start[b], s1 = sm.start[b + 1];
+      const KeyT k = kin[me & LOW];
+      if (s1 - s0 > MAX_BIN && !sm.mixed[s0 / CROWD]) {
+        split |= kin[sm.word[s0] & LOW] != k;
+        continue;
+      }
+      uint32_t rank = s0;
+      for (uint32_t x = s0; x < s1; x++) {
+        const uint32_t o = sm.word[x], p = o & LOW;
+        if ((o ^ me) <= LOW) {
+          if (o == me) continue;
+          const KeyT other = kin[p];
+          rank += other < k || (other == k && id_at(p) < mine) ? 1u : 0u;
+        } else {
+          rank += o < me ? 1u : 0u;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < NITEMS; j++)
+        if (j == i) at[j] = rank;
+    }
+    if (__syncthreads_or(int(split))) return TIED_SPLIT;
+  }
+  if (crowded) {
+    for (uint32_t x = t; x < BINS; x += NTHREADS) sm.start[x] = 0;
+    __syncthreads();
+    uint32_t in[NITEMS];
+#pragma unroll
+    for (int i = 0; i < NITEMS; i++) {
+      if (i >= ni) break;
+      in[i] = atomicAdd(&sm.start[at[i]], 1u);
+    }
+    __syncthreads();
+    count_scan(sm, rows);
+#pragma unroll
+    for (int i = 0; i < NITEMS; i++) {
+      if (i >= ni) break;
+      sm.word[sm.start[at[i]] + in[i]] = id_at(word[i] & LOW);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < NITEMS; i++) {
+      if (i >= ni) break;
+      const uint32_t s0 = sm.start[at[i]], s1 = sm.start[at[i] + 1];
+      uint32_t rank = s0;
+      if (s1 - s0 > 1) {
+        const uint32_t mine = id_at(word[i] & LOW);
+#pragma unroll 1
+        for (uint32_t q = s0; q < s1; q++) rank += sm.word[q] < mine ? 1u : 0u;
+      }
+      at[i] = rank;
+    }
+  }
+  // In order: the places, then (the ids of this thread's rows read before others' land there) ids and keys.
+  if constexpr (!PAY) {
+    uint32_t id[NITEMS];
+#pragma unroll
+    for (int i = 0; i < NITEMS; i++) id[i] = i < ni ? sm.id[word[i] & LOW] : 0u;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < NITEMS; i++) {
+      if (i >= ni) break;
+      sm.id[at[i]] = id[i];
+    }
+  } else {
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < NITEMS; i++) {
+      if (i >= ni) break;
+      sm.place[at[i]] = uint16_t(word[i] & LOW);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NITEMS; i++) {
+    if (i >= ni) break;
+    sm.key[at[i]] = kin[word[i] & LOW];
+  }
+  return TIED_DONE;
+}
+
+// Bucket b is left to later_body.
+__device__ __forceinline__ void put_off(const Args& a, uint32_t b) {
+  const uint32_t at = atomicAdd(&a.st->later, 1u);
+  if (at < a.bucket_cap) a.later[at] = b;
+  else atomicOr(a.err, ERR_BOUNDS);
+}
+
 // A row leaves: its id, its key as the column's value, its payload.
 template <typename KeyT>
 struct KeyOut {
@@ -1594,10 +2009,272 @@ struct KeyOut {
                   (a.key_desc ? KeyT(~KeyT(0)) : KeyT(0)))) {}
 };
 
+// A bucket's (or a part's) rows, ordered in shared memory, to their places from `dst0` on. PART: rows [run0, run1)
+// of the values all have this part's key, where that is not empty. False when the records did not come.
+template <typename KeyT, int PAY, bool FREQ, int LTHREADS, bool PART = false, typename SM>
+__device__ __forceinline__ bool write_rows(SM& sm, const Args& a, const KeyOut<KeyT>& ko, uint64_t dst0, uint32_t rows, uint32_t nkeys,
+                                           uint32_t parity, uint64_t run0 = 0, uint64_t run1 = 0) {
+  const uint32_t t = threadIdx.x;
+  constexpr int LITEMS = CAP / LTHREADS;
+  const int ni = int((rows + LTHREADS - 1 - t) / LTHREADS);
+  // Rows of the frequent keys before key k: they are not in the buckets.
+  auto apart_before = [&](KeyT k) {
+    uint32_t n = 0;
+    for (uint32_t h = 0; h < nkeys; h++) n += k > KeyT(a.st->key[h]) ? a.st->key_rows[h] : 0u;
+    return n;
+  };
+  // Frequent keys between the bucket's rows: row by row. (Not in a sort of ranks, keys or payload.)
+  if (FREQ && nkeys) {
+    const uint32_t lo = apart_before(sm.key[0]), hi = apart_before(sm.key[rows - 1]);
+    if (dst0 + hi + rows > a.n) {                          // the scan rules it out
+      if (t == 0) atomicOr(a.err, ERR_BOUNDS);
+      return true;
+    }
+    if constexpr (!PAY)
+      if (lo != hi) {
+        for (uint32_t r = t; r < rows; r += LTHREADS) store_id(a, dst0 + r + apart_before(sm.key[r]), sm.id[r]);
+        return true;
+      }
+    dst0 += lo;
+  }
+  if constexpr (!PAY) {
+    if (a.ranks.out) {
+      // The run of equal keys around a row: by bisection of the ordered keys where a neighbour is equal.
+      for (uint32_t r = t; r < rows; r += LTHREADS) {
+        const KeyT k = sm.key[r];
+        uint32_t p = r;
+        if (a.ranks.mode == RANK_FIRST_OF && r > 0 && sm.key[r - 1] == k) {
+          uint32_t lo = 0;
+          while (lo < p) {
+            const uint32_t mid = (lo + p) >> 1;
+            if (sm.key[mid] < k) lo = mid + 1;
+            else p = mid;
+          }
+        } else if (a.ranks.mode == RANK_LAST_OF && r + 1 < rows && sm.key[r + 1] == k) {
+          uint32_t hi = rows;
+          while (p + 1 < hi) {
+            const uint32_t mid = (p + hi) >> 1;
+            if (sm.key[mid] <= k) p = mid;
+            else hi = mid;
+          }
+        }
+        uint64_t rank = dst0 + p + 1;
+        if (PART && run0 < run1 && a.ranks.mode == RANK_FIRST_OF) rank = run0 + 1;
+        if (PART && run0 < run1 && a.ranks.mode == RANK_LAST_OF) rank = run1;
+        const uint32_t row = sm.id[r];
+        if (row < a.n) a.ranks.out[row] = uint32_t(rank);
+        else atomicOr(a.err, ERR_BOUNDS);
+      }
+    }
+    if (a.out) {
+      if (a.wide) {
+        uint64_t* o = static_cast<uint64_t*>(a.out) + dst0 + t;
+#pragma unroll
+        for (int i = 0; i < LITEMS; i++) {
+          if (i >= ni) break;
+          o[i * LTHREADS] = sm.id[t + i * LTHREADS];
+        }
+      } else {
+        uint32_t* o = static_cast<uint32_t*>(a.out) + dst0 + t;
+#pragma unroll
+        for (int i = 0; i < LITEMS; i++) {
+          if (i >= ni) break;
+          o[i * LTHREADS] = sm.id[t + i * LTHREADS];
+        }
+      }
+    }
+  }
+  if (a.key_out) {
+    if (ko.xored) {
+      KeyT* o = static_cast<KeyT*>(a.key_out) + dst0 + t;
+#pragma unroll
+      for (int i = 0; i < LITEMS; i++) {
+        if (i >= ni) break;
+        o[i * LTHREADS] = sm.key[t + i * LTHREADS] ^ ko.bits;
+      }
+    }
+  }
+  if constexpr (PAY) {
+    if (!mbar_wait(&sm.full, parity)) {
+      atomicOr(a.err, ERR_LOOKBACK_TIMEOUT);
+      return false;
+    }
+  }
+  if (a.key_out && !ko.xored) {
+    for (uint32_t r = t; r < rows; r += LTHREADS) {
+      const KeyT k = sm.key[r];
+      uint64_t v = unkey_bits<KeyT>(k, a.key_pt, a.key_desc);
+      if (a.key_src && (k == KeyT(a.twin0) || k == KeyT(a.twin1))) {
+        uint32_t id;
+        if constexpr (PAY) id = sm.rec[sm.place[r]].x;
+        else id = sm.id[r];
+        v = source_bits(a, id);
+      }
+      store_width(a.key_out, dst0 + r, pt_bytes(a.key_pt), v);
+    }
+  }
+  if constexpr (PAY) {
+    if (a.pay.pair && !a.out) {
+      uint64_t* w = static_cast<uint64_t*>(a.pay.dst[a.pay.wide]) + dst0 + t;
+      uint32_t* h = static_cast<uint32_t*>(a.pay.dst[a.pay.narrow]) + dst0 + t;
+#pragma unroll
+      for (int i = 0; i < LITEMS; i++) {
+        if (i >= ni) break;
+        const uint4 v = sm.rec[sm.place[t + i * LTHREADS]];
+        w[i * LTHREADS] = uint64_t(v.y) | (uint64_t(v.z) << 32);
+        h[i * LTHREADS] = v.w;
+      }
+    } else {
+      for (uint32_t r = t; r < rows; r += LTHREADS) {
+        const uint4 v = sm.rec[sm.place[r]];
+        store_id(a, dst0 + r, v.x);
+        unpack_record(a.pay, v, dst0 + r);
+      }
+    }
+  }
+  return true;
+}
+
+// The buckets that sort_body put off: those with bins of repeated keys, or of more rows than its form takes, which are
+// cut into parts. A launch of its own: within sort_body its registers cost every bucket (16M int64 keys that do not
+// repeat: the buckets' sort 149 us, 193 with this behind its loop, the next bucket's keys waited for to be spilled).
+template <typename KeyT, int PAY, bool FREQ = false>
+__device__ __forceinline__ void later_body(const Args& a) {
+  extern __shared__ __align__(16) unsigned char lsm[];
+  using SM = LaterShared<KeyT, PAY>;
+  SM& sm = *reinterpret_cast<SM*>(lsm);
+  const State* st = a.st;
+  const uint32_t count = st->later;
+  if (blockIdx.x >= count || st->mode != MODE_BUCKETS) return;
+  const uint32_t t = threadIdx.x, src = st->s2 ? 1u : 0u, nkeys = FREQ ? st->nkeys : 0u;
+  const uint64_t vbase = a.nulls_first ? uint64_t(st->n_null) + st->n_nan : 0ull;
+  const KeyOut<KeyT> ko(a);
+  if (PAY && t == 0) mbar_init(&sm.full);
+  uint32_t parts = 0, turn = blockIdx.x, parity = 0;
+  for (;;) {
+    __syncthreads();                               // the last part's memory, and its place in the list, are free
+    uint32_t first, size, side, kind, run_at = 0, run_n = 0;
+    if (parts) {
+      parts--;
+      first = sm.part_at[parts];
+      size = sm.part_n[parts] & 0x1FFFFFFFu;
+      side = (sm.part_n[parts] >> 29) & 1u;
+      kind = sm.part_n[parts] >> 30;
+      if constexpr (!PAY) {
+        run_at = sm.run_at[parts];
+        run_n = sm.run_n[parts];
+      }
+    } else {
+      if (turn >= count) return;
+      const uint32_t b = a.later[turn];
+      turn += gridDim.x;
+      first = a.bpos[b];
+      size = a.bpos[b + 1] - first;
+      side = src;
+      kind = KIND_KEY;
+      if (vbase + first + size > a.n || size > a.large) {         // the scan rules both out
+        if (t == 0) atomicOr(a.err, ERR_BOUNDS);
+        return;
+      }
+    }
+    if (size == 0) continue;
+    __syncthreads();
+    uint32_t heavy = PART_ROWS;                    // split, bins of more rows becoming parts
+    if (size <= uint32_t(CAP)) {
+      if constexpr (PAY) {
+        if (t == 0) bulk_load(sm.rec, a.rec[side] + first, size * 16u, &sm.full);
+      }
+      const KeyT* kin = static_cast<const KeyT*>(a.keys[side]) + first;
+      const int ni = int((size + NTHREADS - 1 - t) / NTHREADS);
+      KeyT key[NITEMS];
+      KeyT klo = KeyT(~KeyT(0)), khi = 0;
+      uint32_t id0 = ~0u, id1 = 0;
+#pragma unroll
+      for (int i = 0; i < NITEMS; i++)
+        if (i < ni) key[i] = kin[t + i * NTHREADS];
+#pragma unroll
+      for (int i = 0; i < NITEMS; i++) {
+        if (i >= ni) break;
+        const uint32_t id = PAY ? a.rec[side][first + t + i * NTHREADS].x : a.ids[side][first + t + i * NTHREADS];
+        if constexpr (!PAY) sm.id[t + i * NTHREADS] = id;
+        id0 = min(id0, id);
+        id1 = max(id1, id);
+      }
+      if (!parts && turn < count) {
+        // The next bucket's rows come from HBM to L2 meanwhile.
+        const uint32_t b = a.later[turn], nf = a.bpos[b], nn = a.bpos[b + 1] - nf;
+        const char* k0 = reinterpret_cast<const char*>(static_cast<const KeyT*>(a.keys[src]) + nf);
+        const char* i0 = PAY ? reinterpret_cast<const char*>(a.rec[src] + nf) : reinterpret_cast<const char*>(a.ids[src] + nf);
+        for (uint32_t x = t * 128u; x < nn * uint32_t(sizeof(KeyT)); x += NTHREADS * 128u) asm volatile("prefetch.global.L2 [%0];" ::"l"(k0 + x));
+        for (uint32_t x = t * 128u; x < nn * (PAY ? 16u : 4u); x += NTHREADS * 128u) asm volatile("prefetch.global.L2 [%0];" ::"l"(i0 + x));
+      }
+      for (uint32_t x = t; x < BINS; x += NTHREADS) sm.start[x] = 0;
+      if (t <= CAP / CROWD) sm.mixed[t] = 0;
+      // Positions: the top bits of the distance from the part's smallest key, or row id; the ids' own range orders crowded bins.
+#pragma unroll
+      for (int i = 0; i < NITEMS; i++) {
+        if (i >= ni) break;
+        klo = min(klo, key[i]);
+        khi = max(khi, key[i]);
+      }
+      block_range(sm, klo, khi, id0, id1);
+      const uint32_t idsh = id1 > id0 ? __clz(id1 - id0) : 0u;
+      const uint64_t lo = kind == KIND_ID ? uint64_t(id0) : uint64_t(klo), hi = kind == KIND_ID ? uint64_t(id1) : uint64_t(khi);
+      const uint32_t sh = range_shift(hi - lo);
+      if (PAY && kind == KIND_ID && !mbar_wait(&sm.full, parity)) {
+        atomicOr(a.err, ERR_LOOKBACK_TIMEOUT);
+        return;
+      }
+      auto pos_of = [&](int i) {
+        uint64_t x = uint64_t(key[i]);
+        if (kind == KIND_ID) x = PAY ? sm.rec[PAY ? t + i * NTHREADS : 0].x : sm.id[PAY ? 0 : t + i * NTHREADS];
+        return uint32_t(((x - lo) << sh) >> 32);
+      };
+      uint32_t at[NITEMS];
+#pragma unroll
+      for (int i = 0; i < NITEMS; i++) {
+        if (i >= ni) break;
+        at[i] = atomicAdd(&sm.start[pos_of(i) >> (32 - BINS_LOG)], 1u);
+      }
+      __syncthreads();
+      const bool crowded = count_scan(sm, size);
+#pragma unroll
+      for (int i = 0; i < NITEMS; i++) {
+        if (i >= ni) break;
+        const uint32_t pos = pos_of(i), bin = pos >> (32 - BINS_LOG), q = sm.start[bin] + at[i];
+        sm.word[q] = (pos << BINS_LOG) | (t + i * NTHREADS);
+        sm.place[q] = uint16_t(bin);
+      }
+      __syncthreads();
+      const uint32_t tied = order_tied<KeyT, PAY>(sm, a, kin, size, sh >= 32u, crowded, parity, id0, idsh);
+      if (tied == TIED_TIMEOUT) return;
+      if (PAY) parity ^= 1u;
+      if (tied != TIED_SPLIT) {
+        __syncthreads();
+        const uint64_t base = kind == KIND_ID ? vbase : 0ull;
+        if (!write_rows<KeyT, PAY, FREQ, NTHREADS, true>(sm, a, ko, vbase + first, size, nkeys, parity ^ (PAY ? 1u : 0u), base + (kind == KIND_ID ? run_at : 0u),
+                                               base + (kind == KIND_ID ? run_at + run_n : 0u)))
+          return;
+        continue;
+      }
+      heavy = MAX_BIN;
+    }
+    parts = split_rows<KeyT, PAY>(sm, a, first, size, side, kind, heavy, run_at, run_n, parts);
+  }
+}
+
+// The 32 bits below the bucket number of (position in the cell, as a fraction of the key's width) x (buckets of the
+// cell). The bucket number comes from the top 32 bits alone, so the bits below can carry past it.
+__device__ __forceinline__ uint32_t position_in(uint32_t z, uint32_t mul) { return z * mul; }
+__device__ __forceinline__ uint32_t position_in(uint64_t z, uint32_t mul) {
+  const uint32_t p = uint32_t(z >> 32) * mul, below = __umulhi(uint32_t(z), mul);
+  return p + below < p ? ~0u : p + below;
+}
+
 template <typename KeyT, int PAY, int TIES, bool FREQ = false>
 __device__ __forceinline__ void sort_body(const Args& a) {
   extern __shared__ __align__(16) unsigned char lsm[];
-  using SM = LocalShared<KeyT, PAY>;
+  using SM = FastShared<KeyT, PAY, TIES>;
   SM& sm = *reinterpret_cast<SM*>(lsm);
   const State* st = a.st;
   if (blockIdx.x >= a.sort_grid || st->mode != MODE_BUCKETS) return;
@@ -1606,16 +2283,12 @@ __device__ __forceinline__ void sort_body(const Args& a) {
   const uint64_t vbase = a.nulls_first ? uint64_t(st->n_null) + st->n_nan : 0ull;
   const Map<KeyT> map = load_map<KeyT>(st);
   const KeyOut<KeyT> ko(a);
-  const int kw = pt_bytes(a.key_pt);
   const uint32_t nkeys = FREQ ? st->nkeys : 0u;
-  // Rows of the frequent keys before key k: they are not in the buckets.
-  auto apart_before = [&](KeyT k) {
-    uint32_t rows = 0;
-    for (uint32_t h = 0; h < nkeys; h++) rows += k > KeyT(st->key[h]) ? st->key_rows[h] : 0u;
-    return rows;
-  };
   constexpr uint32_t SUB = 32 - BINS_LOG;          // position bits below the bin
-  static_assert(CAP <= (1 << BINS_LOG), "a place fits beside the position bits below the bin");
+
+  // Two bins' rows, and then starts, share a word.
+  auto count_in = [&](uint32_t bin) { return (atomicAdd(&sm.start[bin >> 1], 1u << ((bin & 1u) * 16)) >> ((bin & 1u) * 16)) & 0xFFFFu; };
+  auto start_of = [&](uint32_t bin) { return uint32_t(reinterpret_cast<const uint16_t*>(sm.start)[bin]); };
 
   // The bucket at hand: its rows, its part of the map, and this thread's keys of it (item i is the
   // bucket's row i x LTHREADS + t; items below nit).
@@ -1648,9 +2321,10 @@ __device__ __forceinline__ void sort_body(const Args& a) {
   };
   if (t == 0) {
     sm.crowded = 0;
+    sm.some_fast = 0;
     mbar_init(&sm.full);
   }
-  for (int x = t; x < BINS; x += LTHREADS) sm.start[x] = 0;
+  for (int x = t; x < BINS / 2; x += LTHREADS) sm.start[x] = 0;
   __syncthreads();
   uint32_t b = next_bucket(blockIdx.x), parity = 0;
   if (b < nb) {
@@ -1660,18 +2334,14 @@ __device__ __forceinline__ void sort_body(const Args& a) {
   while (b < nb) {
     const uint32_t rows = size, row0 = first;
     const int ni = nit;
-    const KeyT* __restrict__ kin = static_cast<const KeyT*>(a.keys[src]) + row0;
-    const uint32_t* __restrict__ iin = a.ids[src] + row0;
-    const uint4* __restrict__ rin = a.rec[src] + row0;
-    auto id_of = [&](uint32_t p) { return PAY ? rin[p].x : iin[p]; };
-    uint64_t dst0 = vbase + row0;
-    if (dst0 + rows > a.n || rows > uint32_t(BIG)) {       // the scan rules both out
+    const KeyT* kin = static_cast<const KeyT*>(a.keys[src]) + row0;
+    const uint32_t* iin = a.ids[src] + row0;
+    const uint64_t dst0 = vbase + row0;
+    if (dst0 + rows > a.n || rows > a.large) {             // the scan rules both out
       if (t == 0) atomicOr(a.err, ERR_BOUNDS);
       if (PAY && rows <= uint32_t(CAP)) (void)mbar_wait(&sm.full, parity);
       break;
     }
-    // Rows that agree on their positions agree on their keys: no key bits lie below a position's 32.
-    const bool exact = (meta & META_SPLIT) && meta != META_SPLIT && uint32_t(sizeof(KeyT)) * 8u - (f0 >> 16) <= 32u;
     bool fast = rows <= uint32_t(CAP);
     uint32_t at[LITEMS];                           // the row's place among its bin's; by bin; in order
     if (fast) {
@@ -1694,8 +2364,8 @@ __device__ __forceinline__ void sort_body(const Args& a) {
         for (int i = 0; i < LITEMS; i++) {
           if (i >= ni) break;
           const KeyT z = KeyT(KeyT(KeyT(key[i] - map.lo) << sh0) << sh1);      // sh may be the key's width
-          pos[i] = uint32_t(z >> (8 * sizeof(KeyT) - 32)) * mul;
-          at[i] = atomicAdd(&sm.start[pos[i] >> SUB], 1u);
+          pos[i] = position_in(z, mul);
+          at[i] = count_in(pos[i] >> SUB);
         }
       } else {
         const uint32_t cells = meta - f0 + 1u, k = cells > 1u ? 32u - __clz(cells - 1u) : 0u;
@@ -1705,76 +2375,81 @@ __device__ __forceinline__ void sort_body(const Args& a) {
           uint32_t f, frac;
           cell_of(map, a.coarse, KeyT(key[i] - map.lo), f, frac);
           pos[i] = uint32_t(((uint64_t(f - f0) << 32) | frac) >> k);
-          at[i] = atomicAdd(&sm.start[pos[i] >> SUB], 1u);
+          at[i] = count_in(pos[i] >> SUB);
         }
       }
       __syncthreads();
       {
-        constexpr int PER = BINS / LTHREADS;
-        static_assert(PER % 4 == 0, "whole vectors of bins a thread");
-        uint4 c[PER / 4];
+        static_assert(BINS == 8 * LTHREADS, "a vector of bins a thread");
+        const uint4 c = *reinterpret_cast<const uint4*>(&sm.start[t * 4]);
+        const uint32_t w[4] = {c.x, c.y, c.z, c.w};
         uint32_t sum = 0, mx = 0, all;
 #pragma unroll
-        for (int q = 0; q < PER / 4; q++) {
-          c[q] = *reinterpret_cast<const uint4*>(&sm.start[t * PER + 4 * q]);
-          sum += c[q].x + c[q].y + c[q].z + c[q].w;
-          mx = max(mx, max(max(c[q].x, c[q].y), max(c[q].z, c[q].w)));
+        for (int q = 0; q < 4; q++) {
+          sum += (w[q] & 0xFFFFu) + (w[q] >> 16);
+          mx = max(mx, max(w[q] & 0xFFFFu, w[q] >> 16));
         }
         if (mx > MAX_BIN) sm.crowded = 1;
-        uint32_t s = block_scan<LTHREADS>(sum, sm.warp, all);
+        uint32_t s = block_scan<LTHREADS>(sum, sm.warp, all), o[4];
 #pragma unroll
-        for (int q = 0; q < PER / 4; q++) {
-          *reinterpret_cast<uint4*>(&sm.start[t * PER + 4 * q]) =
-              make_uint4(s, s + c[q].x, s + c[q].x + c[q].y, s + c[q].x + c[q].y + c[q].z);
-          s += c[q].x + c[q].y + c[q].z + c[q].w;
+        for (int q = 0; q < 4; q++) {
+          const uint32_t next = s + (w[q] & 0xFFFFu);
+          o[q] = s | (next << 16);
+          s = next + (w[q] >> 16);
         }
-        if (t == LTHREADS - 1) sm.start[BINS] = rows;
+        *reinterpret_cast<uint4*>(&sm.start[t * 4]) = make_uint4(o[0], o[1], o[2], o[3]);
+        if (t == LTHREADS - 1) sm.start[BINS / 2] = rows;
       }
+      if constexpr (PAY)
+        if (!mbar_wait(&sm.full, parity)) atomicOr(a.err, ERR_LOOKBACK_TIMEOUT);
       __syncthreads();
       fast = sm.crowded == 0;
       if (fast) {
 #pragma unroll
         for (int i = 0; i < LITEMS; i++) {
           if (i >= ni) break;
-          const uint32_t s0 = sm.start[pos[i] >> SUB], r = t + i * LTHREADS;
-          sm.word[s0 + at[i]] = (pos[i] << BINS_LOG) | r;
-          if constexpr (!PAY) sm.id[r] = id[i];
-          at[i] = s0;
+          const uint32_t s0 = start_of(pos[i] >> SUB), r = t + i * LTHREADS;
+          uint32_t below;
+          if constexpr (TIES == TIES_STRING) {
+            below = r;
+            sm.in_id[r] = id[i];
+          } else if constexpr (PAY) {
+            below = sm.rec[r].x;
+          } else {
+            below = id[i];
+          }
+          sm.word[s0 + at[i]] = (uint64_t(pos[i]) << 32) | below;
+          at[i] = s0 + at[i];
         }
         __syncthreads();
+        // A row's place: the rows of its bin that come before it, by position and, at one position, by row id. Rows at one
+        // position are nearly always one key's; the keys in order tell whether they are.
+        bool some = false;                         // rows at one position
 #pragma unroll
         for (int i = 0; i < LITEMS; i++) {
           if (i >= ni) break;
-          const uint32_t s0 = at[i], s1 = sm.start[(pos[i] >> SUB) + 1];
+          const uint32_t s0 = start_of(pos[i] >> SUB), s1 = start_of((pos[i] >> SUB) + 1);
           if (s1 - s0 > 1) {
-            // Rows of the bin that come before: by the position bits below the bin; rows that agree on
-            // them too by the whole key, equal keys by row id.
-            const uint32_t me = (pos[i] << BINS_LOG) | (t + i * LTHREADS);
-            uint32_t rank = s0, same = 0;
+            const uint64_t me = sm.word[at[i]];
+            uint32_t rank = s0;
 #pragma unroll 1
             for (uint32_t q = s0; q < s1; q++) {
-              const uint32_t o = sm.word[q];
-              rank += o < me ? 1u : 0u;
-              same += (o ^ me) < uint32_t(1 << BINS_LOG) ? 1u : 0u;
-            }
-            if (same > 1) {
-              rank = s0;
-              const uint32_t mine = PAY ? id_of(me & (BINS - 1)) : sm.id[me & (BINS - 1)];
-#pragma unroll 1
-              for (uint32_t q = s0; q < s1; q++) {
-                const uint32_t o = sm.word[q], p = o & (BINS - 1);
-                if ((o ^ me) >= uint32_t(1 << BINS_LOG)) {
-                  rank += o < me ? 1u : 0u;
-                } else {
-                  const KeyT k = exact ? key[i] : kin[p];
-                  rank += k < key[i] || (k == key[i] && tied_before<TIES>(a.ties, PAY ? id_of(p) : sm.id[p], mine)) ? 1u : 0u;
+              const uint64_t o = sm.word[q];
+              if constexpr (TIES == TIES_STRING) {
+                if (uint32_t(o >> 32) == pos[i] && o != me) {
+                  const KeyT k = kin[uint32_t(o)];
+                  rank += k < key[i] || (k == key[i] && tied_before<TIES>(a.ties, sm.in_id[uint32_t(o)], id[PAY ? 0 : i])) ? 1u : 0u;
+                  continue;
                 }
+              } else {
+                some |= uint32_t(o >> 32) == pos[i] && o != me;
               }
+              rank += o < me ? 1u : 0u;
             }
             at[i] = rank;
           }
         }
-        __syncthreads();
+        some = __syncthreads_or(int(some)) != 0;
 #pragma unroll
         for (int i = 0; i < LITEMS; i++) {
           if (i >= ni) break;
@@ -1782,157 +2457,44 @@ __device__ __forceinline__ void sort_body(const Args& a) {
           if constexpr (PAY) sm.place[at[i]] = uint16_t(t + i * LTHREADS);
           else sm.id[at[i]] = id[i];
         }
+        if (some) {
+          __syncthreads();
+          bool wrong = false;
+          for (uint32_t r = t + 1; r < rows; r += LTHREADS) wrong |= sm.key[r] < sm.key[r - 1];
+          fast = !__syncthreads_or(int(wrong));
+        }
       }
     }
     // The next bucket's keys arrive while this one leaves.
     const uint32_t bn = next_bucket(b + a.sort_grid);
     if (bn < nb) load_rows();
     __syncthreads();
-    // Frequent keys between the bucket's rows: row by row. (Not in a sort of ranks, keys or payload.)
-    bool split = false;
-    if (nkeys && fast) {
-      const uint32_t lo = apart_before(sm.key[0]), hi = apart_before(sm.key[rows - 1]);
-      split = lo != hi;
-      dst0 += split ? 0u : lo;
-      if (dst0 + hi + rows > a.n + (split ? 0u : hi)) {    // the scan rules it out
-        if (t == 0) atomicOr(a.err, ERR_BOUNDS);
-        break;
-      }
-    }
-    if (split) {
-      if constexpr (!PAY)
-        for (uint32_t r = t; r < rows; r += LTHREADS) store_id(a, dst0 + r + apart_before(sm.key[r]), sm.id[r]);
-    } else if (fast) {
-      if constexpr (!PAY) {
-        if (a.ranks.out) {
-          // Equal keys share a bin, so a run of them is at most MAX_BIN rows: the walk to its end is short.
-          for (uint32_t r = t; r < rows; r += LTHREADS) {
-            const KeyT k = sm.key[r];
-            uint32_t p = r + 1;
-            if (a.ranks.mode == RANK_FIRST_OF) {
-              p = r;
-              while (p > 0 && sm.key[p - 1] == k) p--;
-              p++;
-            } else if (a.ranks.mode == RANK_LAST_OF) {
-              while (p < rows && sm.key[p] == k) p++;
-            }
-            const uint32_t row = sm.id[r];
-            if (row < a.n) a.ranks.out[row] = uint32_t(dst0) + p;
-            else atomicOr(a.err, ERR_BOUNDS);
-          }
-        }
-        if (a.out) {
-          if (a.wide) {
-            uint64_t* o = static_cast<uint64_t*>(a.out) + dst0 + t;
-#pragma unroll
-            for (int i = 0; i < LITEMS; i++) {
-              if (i >= ni) break;
-              o[i * LTHREADS] = sm.id[t + i * LTHREADS];
-            }
-          } else {
-            uint32_t* o = static_cast<uint32_t*>(a.out) + dst0 + t;
-#pragma unroll
-            for (int i = 0; i < LITEMS; i++) {
-              if (i >= ni) break;
-              o[i * LTHREADS] = sm.id[t + i * LTHREADS];
-            }
-          }
-        }
-      }
-      if (a.key_out) {
-        if (ko.xored) {
-          KeyT* o = static_cast<KeyT*>(a.key_out) + dst0 + t;
-#pragma unroll
-          for (int i = 0; i < LITEMS; i++) {
-            if (i >= ni) break;
-            o[i * LTHREADS] = sm.key[t + i * LTHREADS] ^ ko.bits;
-          }
-        }
-      }
-      if constexpr (PAY) {
-        if (!mbar_wait(&sm.full, parity)) {
-          atomicOr(a.err, ERR_LOOKBACK_TIMEOUT);
-          return;
-        }
-      }
-      if (a.key_out && !ko.xored) {
-        for (uint32_t r = t; r < rows; r += LTHREADS) {
-          const KeyT k = sm.key[r];
-          uint64_t v = unkey_bits<KeyT>(k, a.key_pt, a.key_desc);
-          if (a.key_src && (k == KeyT(a.twin0) || k == KeyT(a.twin1))) {
-            uint32_t id;
-            if constexpr (PAY) id = sm.rec[sm.place[r]].x;
-            else id = sm.id[r];
-            v = source_bits(a, id);
-          }
-          store_width(a.key_out, dst0 + r, kw, v);
-        }
-      }
-      if constexpr (PAY) {
-        if (a.pay.pair && !a.out) {
-          uint64_t* w = static_cast<uint64_t*>(a.pay.dst[a.pay.wide]) + dst0 + t;
-          uint32_t* h = static_cast<uint32_t*>(a.pay.dst[a.pay.narrow]) + dst0 + t;
-#pragma unroll
-          for (int i = 0; i < LITEMS; i++) {
-            if (i >= ni) break;
-            const uint4 v = sm.rec[sm.place[t + i * LTHREADS]];
-            w[i * LTHREADS] = uint64_t(v.y) | (uint64_t(v.z) << 32);
-            h[i * LTHREADS] = v.w;
-          }
-        } else {
-          for (uint32_t r = t; r < rows; r += LTHREADS) {
-            const uint4 v = sm.rec[sm.place[r]];
-            store_id(a, dst0 + r, v.x);
-            unpack_record(a.pay, v, dst0 + r);
-          }
-        }
-      }
+    if (fast) {
+      if (t == 0) sm.some_fast = 1;
+      if (!write_rows<KeyT, PAY, FREQ, LTHREADS>(sm, a, ko, dst0, rows, nkeys, parity)) return;
+    } else if constexpr (TIES == TIES_STRING) {
+      bitonic_rows<TIES>(sm.slow.key, sm.slow.place, rows, kin, [&](uint32_t p) { return iin[p]; }, a.ties);
+      for (uint32_t r = t; r < rows; r += LTHREADS) store_id(a, dst0 + r, iin[sm.slow.place[r]]);
     } else {
-      // Records of a crowded bucket are on their way into the memory used here.
+      // Left to later_body; in a column of repeated keys, where neither of the CTA's first two buckets was fast,
+      // with all of the CTA's that follow.
+      const bool rest = !sm.some_fast && b >= blockIdx.x + a.sort_grid;
+      if (t == 0) put_off(a, b);
+      if (rest)
+        for (uint32_t x = bn + t * a.sort_grid; x < nb; x += LTHREADS * a.sort_grid)
+          if (a.bpos[x + 1] != a.bpos[x]) put_off(a, x);
       if constexpr (PAY) {
         if (rows <= uint32_t(CAP) && !mbar_wait(&sm.full, parity)) {
           atomicOr(a.err, ERR_LOOKBACK_TIMEOUT);
           return;
         }
-        __syncthreads();
       }
-      bitonic_rows<TIES>(sm.slow.key, sm.slow.place, rows, kin, id_of, a.ties);
-      for (uint32_t r = t; r < rows; r += LTHREADS) {
-        const uint32_t p = sm.slow.place[r];
-        const KeyT k = sm.slow.key[r];
-        const uint64_t dst = dst0 + r + (nkeys ? apart_before(k) : 0u);
-        if (dst < a.n) store_id(a, dst, id_of(p));
-        else atomicOr(a.err, ERR_BOUNDS);
-        if constexpr (!PAY) {
-          if (a.ranks.out) {
-            // The run's end by bisection: the first row not before (or the first after) the key.
-            uint32_t lo = 0, hi = rows;
-            if (a.ranks.mode == RANK_OWN) {
-              lo = r;
-            } else {
-              while (lo < hi) {
-                const uint32_t mid = (lo + hi) >> 1;
-                const KeyT o = sm.slow.key[mid];
-                if (a.ranks.mode == RANK_FIRST_OF ? o < k : o <= k) lo = mid + 1;
-                else hi = mid;
-              }
-            }
-            const uint32_t row = id_of(p);
-            if (row < a.n) a.ranks.out[row] = uint32_t(dst0) + lo + (a.ranks.mode == RANK_LAST_OF ? 0u : 1u);
-            else atomicOr(a.err, ERR_BOUNDS);
-          }
-        }
-        if (a.key_out)
-          store_width(a.key_out, dst0 + r, kw, a.key_src && (k == KeyT(a.twin0) || k == KeyT(a.twin1))
-                                                   ? source_bits(a, id_of(p)) : unkey_bits<KeyT>(k, a.key_pt, a.key_desc));
-        if constexpr (PAY) unpack_record(a.pay, rin[p], dst0 + r);
-      }
-      if constexpr (PAY) fence_bulk();
+      if (rest) return;
     }
     if (PAY && rows <= uint32_t(CAP)) parity ^= 1u;
     b = bn;
     __syncthreads();
-    for (int x = t; x < BINS; x += LTHREADS) sm.start[x] = 0;
+    for (int x = t; x < BINS / 2; x += LTHREADS) sm.start[x] = 0;
     if (t == 0) {
       sm.crowded = 0;
       if (b < nb) load_records();
@@ -1968,6 +2530,10 @@ __global__ void __launch_bounds__(THREADS, 2) level2_kernel(const __grid_constan
 template <typename KeyT, int PAY, int TIES, bool FREQ>
 __global__ void __launch_bounds__(LTHREADS, LBLOCKS) bucket_sort_kernel(const __grid_constant__ Args a) {
   sort_body<KeyT, PAY, TIES, FREQ>(a);
+}
+template <typename KeyT, int PAY, bool FREQ>
+__global__ void __launch_bounds__(NTHREADS, NBLOCKS) bucket_later_kernel(const __grid_constant__ Args a) {
+  later_body<KeyT, PAY, FREQ>(a);
 }
 
 struct alignas(16) BatchItem {
@@ -2007,6 +2573,10 @@ __global__ void __launch_bounds__(THREADS, 2) batch_level2_kernel(const BatchIte
 template <typename KeyT>
 __global__ void __launch_bounds__(LTHREADS, LBLOCKS) batch_sort_kernel(const BatchItem* __restrict__ items) {
   sort_body<KeyT, 0, TIES_ID>(batch_item(items).a);
+}
+template <typename KeyT>
+__global__ void __launch_bounds__(NTHREADS, NBLOCKS) batch_later_kernel(const BatchItem* __restrict__ items) {
+  later_body<KeyT, 0>(batch_item(items).a);
 }
 
 // ---- 5. the first k rows
@@ -2180,8 +2750,11 @@ uint32_t rows_per_chunk(uint64_t n) {
 }
 uint32_t chunks_of(uint64_t n) { return n <= SAMPLES ? 0u : uint32_t((n + rows_per_chunk(n) - 1) / rows_per_chunk(n)); }
 
+// Rows a bucket may hold before the digit passes sort the column instead: one CTA works on it alone.
+uint32_t large_rows(uint64_t n) { return uint32_t(std::min<uint64_t>(LARGE, std::max<uint64_t>(BIG, n / 1024))); }
+
 struct Layout {
-  size_t state, bcount, bmeta, zeroed, coarse, fine, bfirst, bpos, cursor1, cursor2, chunk_bins, chunk_cats, total;
+  size_t state, bcount, bmeta, zeroed, coarse, fine, bfirst, bpos, later, cursor1, cursor2, chunk_bins, chunk_cats, total;
   explicit Layout(uint64_t n) {
     size_t at = 0;
     auto take = [&](size_t bytes) {
@@ -2198,6 +2771,7 @@ struct Layout {
     fine = take(FINE * 4);
     bfirst = take(nb * 4);
     bpos = take((nb + 1) * 4);
+    later = take(nb * 4);
     cursor1 = take(size_t(BINS1) * CUR_PAD * 4);
     cursor2 = take(nb * CUR_PAD * 4);
     chunk_bins = take(size_t(chunks_of(n)) * BINS1 * 4);
@@ -2217,7 +2791,8 @@ void launch_moves(const ColView& cv, const Args& a, cudaStream_t s) {
   std::call_once(once, [] {
     smem_limit(level1_kernel<KeyT, PAY, FREQ>, sizeof(TileShared<KeyT, PAY>));
     smem_limit(level2_kernel<KeyT, PAY>, sizeof(Tile2Shared<KeyT, PAY>));
-    smem_limit(bucket_sort_kernel<KeyT, PAY, TIES, FREQ>, sizeof(LocalShared<KeyT, PAY>));
+    smem_limit(bucket_sort_kernel<KeyT, PAY, TIES, FREQ>, sizeof(FastShared<KeyT, PAY, TIES>));
+    if constexpr (TIES == TIES_ID) smem_limit(bucket_later_kernel<KeyT, PAY, FREQ>, sizeof(LaterShared<KeyT, PAY>));
   });
   if (!a.one_launch) {
     {
@@ -2233,7 +2808,12 @@ void launch_moves(const ColView& cv, const Args& a, cudaStream_t s) {
   }
   {
     KernelTimer kt("bucket_sort", s);
-    bucket_sort_kernel<KeyT, PAY, TIES, FREQ><<<a.sort_grid, LTHREADS, sizeof(LocalShared<KeyT, PAY>), s>>>(a);
+    bucket_sort_kernel<KeyT, PAY, TIES, FREQ><<<a.sort_grid, LTHREADS, sizeof(FastShared<KeyT, PAY, TIES>), s>>>(a);
+    AM_CUDA(cudaGetLastError());
+  }
+  if constexpr (TIES == TIES_ID) {
+    KernelTimer kt("bucket_later", s);
+    bucket_later_kernel<KeyT, PAY, FREQ><<<a.later_grid, NTHREADS, sizeof(LaterShared<KeyT, PAY>), s>>>(a);
     AM_CUDA(cudaGetLastError());
   }
 }
@@ -2318,6 +2898,7 @@ static Args make_args(const Sort& b) {
   a.bmeta = at(L.bmeta);
   a.bcount = at(L.bcount);
   a.bpos = at(L.bpos);
+  a.later = at(L.later);
   a.cursor1 = at(L.cursor1);
   a.cursor2 = at(L.cursor2);
   a.chunk_bins = at(L.chunk_bins);
@@ -2354,6 +2935,7 @@ static Args make_args(const Sort& b) {
   a.sum = b.summary;
   if (b.payload) a.pay = b.rec;
   a.bins1_cap = b.payload ? BINS1 / 2 : BINS1;
+  a.large = b.ties.offsets ? uint32_t(BIG) : large_rows(b.n);
   a.has_payload = b.payload ? 1 : 0;
   a.one_launch = b.n <= SAMPLES ? 1 : 0;
   a.frequent = b.frequent && !a.one_launch && !b.payload && !b.key_out && !b.ranks.out && !b.ties.offsets && !b.src_ids && b.key_bytes == 8 ? 1 : 0;
@@ -2365,6 +2947,7 @@ static Args make_args(const Sort& b) {
   a.hist_grid = std::min(a.nchunks, sms);
   a.level2_grid = uint32_t(std::min<uint64_t>((b.n + TILE - 1) / TILE, sms * 2));
   a.sort_grid = uint32_t(std::min<uint64_t>(b.n / (TARGET / 2) + 3, sms * LBLOCKS));
+  a.later_grid = std::min(a.sort_grid, sms * NBLOCKS);
   return a;
 }
 
@@ -2389,10 +2972,11 @@ namespace {
 template <typename KeyT>
 void launch_batch(const BatchItem* items, const BatchItem* host, uint32_t count, bool timed, cudaStream_t s) {
   prepare_batch(int(sizeof(KeyT)));
-  uint32_t hist = 0, chunks = 0, level2 = 0, sort = 0, cap = 0;
+  uint32_t hist = 0, chunks = 0, level2 = 0, sort = 0, later = 0, cap = 0;
   for (uint32_t i = 0; i < count; i++) {
     const Args& a = host[i].a;
     sort = std::max(sort, a.sort_grid);
+    later = std::max(later, a.later_grid);
     if (a.one_launch) continue;
     hist = std::max(hist, a.hist_grid);
     chunks = std::max(chunks, a.nchunks);
@@ -2421,7 +3005,10 @@ void launch_batch(const BatchItem* items, const BatchItem* host, uint32_t count,
         batch_level2_kernel<KeyT><<<dim3(level2, rows), THREADS, sizeof(Tile2Shared<KeyT, 0>), s>>>(it);
       });
     step("batch_sort", [&] {
-      batch_sort_kernel<KeyT><<<dim3(sort, rows), LTHREADS, sizeof(LocalShared<KeyT, 0>), s>>>(it);
+      batch_sort_kernel<KeyT><<<dim3(sort, rows), LTHREADS, sizeof(FastShared<KeyT, 0, TIES_ID>), s>>>(it);
+    });
+    step("batch_later", [&] {
+      batch_later_kernel<KeyT><<<dim3(later, rows), NTHREADS, sizeof(LaterShared<KeyT, 0>), s>>>(it);
     });
   }
 }
@@ -2432,7 +3019,8 @@ void prepare() {
     smem_limit(batch_histogram_kernel<KeyT>, size_t(MAX_BUCKETS) * 4);
     smem_limit(batch_level1_kernel<KeyT>, sizeof(TileShared<KeyT, 0>));
     smem_limit(batch_level2_kernel<KeyT>, sizeof(Tile2Shared<KeyT, 0>));
-    smem_limit(batch_sort_kernel<KeyT>, sizeof(LocalShared<KeyT, 0>));
+    smem_limit(batch_sort_kernel<KeyT>, sizeof(FastShared<KeyT, 0, TIES_ID>));
+    smem_limit(batch_later_kernel<KeyT>, sizeof(LaterShared<KeyT, 0>));
   });
 }
 }  // namespace

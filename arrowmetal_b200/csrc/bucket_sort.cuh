@@ -22,6 +22,7 @@ struct State {
   uint32_t buckets, s2, bins1;           // buckets; level 1 sorts by bucket >> s2 into bins1 bins
   uint32_t n_value, n_null, n_nan;
   uint32_t max_bucket;
+  uint32_t later;                        // buckets that the fast form put off
   // Keys too frequent for a bucket (Sort::frequent), ascending: their rows leave in row order, as null rows
   // do, to the places from `key_at` on among the values.
   uint32_t nkeys;

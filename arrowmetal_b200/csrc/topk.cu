@@ -671,8 +671,8 @@ static am_array* first_rows(const SortKey& key, int64_t k, cudaStream_t s) {
   const size_t off_rows = off_pairs + cap * 8;
   const size_t off_bs = off_rows + cap * 4;
   const size_t off_keys = up(off_bs + bs::scratch_bytes(cap));
-  const size_t off_ids = off_keys + cap * 8;
-  ScratchBlock scratch(s, off_ids + cap * 4);
+  const size_t off_ids = off_keys + 2 * cap * 8;
+  ScratchBlock scratch(s, off_ids + 2 * cap * 4);
   char* base = scratch.data();
   bs::FirstState* fs = reinterpret_cast<bs::FirstState*>(base);
   uint32_t* rows = reinterpret_cast<uint32_t*>(base + off_rows);
@@ -698,8 +698,10 @@ static am_array* first_rows(const SortKey& key, int64_t k, cudaStream_t s) {
     b.src_keys = base + off_pairs;
     b.src_ids = rows;
     b.scratch = base + off_bs;
-    b.keys[0] = b.keys[1] = base + off_keys;       // one level: only the first is used
-    b.ids[0] = b.ids[1] = base + off_ids;
+    for (int i = 0; i < 2; i++) {
+      b.keys[i] = base + off_keys + size_t(i) * cap * 8;
+      b.ids[i] = base + off_ids + size_t(i) * cap * 4;
+    }
     b.out = out->values->ptr;
     b.err = stream_scratch(s, 0).err;
     b.summary = reinterpret_cast<SortSummary*>(base + off_sum);

@@ -139,3 +139,65 @@ def test_first_rows_are_the_sorts_first(am, n, k, kind):
             want = m.argsort(largest, place, order).to_arrow().to_numpy()[:k]
             got = m.top_k(k, largest, place, order).to_arrow().to_numpy()
             assert np.array_equal(got, want), (nulls, largest, place, order)
+
+
+def repeated(kind, n, rng):
+    """Keys that repeat: `kind` rows a value; two values side by side among distinct keys; sorted runs; a few
+    values far apart on a logarithmic scale; floats with both zeros and NaN."""
+    if isinstance(kind, int):
+        m = max(1, n // kind)
+        return rng.integers(0, 2**40, m)[rng.integers(0, m, n)]
+    if kind == "two_close":
+        v = rng.integers(0, 2**40, n)
+        hit = rng.random(n) < 0.1
+        v[hit] = rng.choice([2**39, 2**39 + 1], int(hit.sum()))
+        return v
+    if kind == "runs":
+        return np.sort(rng.integers(0, max(1, n // 700), n)) * 2**33
+    if kind == "log":
+        v = np.exp2(rng.integers(0, 62, n)).astype(np.int64)
+        return v + rng.integers(0, 3, n)
+    if kind == "int32":
+        m = max(1, n // 40)
+        return rng.integers(-2**31, 2**31, m).astype(np.int32)[rng.integers(0, m, n)]
+    v = rng.standard_normal(max(1, n // 100))[rng.integers(0, max(1, n // 100), n)]
+    for value in (0.0, -0.0, np.nan, np.inf):
+        v[rng.random(n) < 0.003] = value
+    return v
+
+
+@pytest.mark.parametrize("n", [33, 2003, 30_011, 65_537, 1_500_001])
+@pytest.mark.parametrize("kind", [12, 30, 100, 700, 2500, 9000, "two_close", "runs", "log", "int32", "float"])
+def test_keys_that_repeat(am, oracle, n, kind):
+    # Bins of repeated keys, several of them in a bin, and buckets larger than a CTA orders at once: the order,
+    # records, the sorted key column and the ranks.
+    rng = np.random.default_rng(n + len(str(kind)))
+    v = repeated(kind, n, rng)
+    for nulls, desc, place in ((0.0, False, "at_end"), (0.1, True, "at_start")):
+        arr = pa.array(v, mask=rng.random(n) < nulls if nulls else None, from_pandas=False)
+        want = oracle.argsort(arr, desc, place, "ieee", threads=4)
+        m = am.MetalArray.from_arrow(arr)
+        assert np.array_equal(m.argsort(desc, place).to_arrow().to_numpy(), want)
+        p1, p2 = rng.standard_normal(n), rng.integers(-2**31, 2**31, n).astype(np.int32)
+        src = am.PlanSource("t", {"k": m, "a": pa.array(p1), "b": pa.array(p2)})
+        by = [["k", desc, {"nulls": "first" if place == "at_start" else "last"}]]
+        out = am.run_plan({"op": "sort", "by": by, "input": {"op": "scan", "source": "t"}}, [src])
+        assert np.array_equal(out["a"].to_arrow().to_numpy(), p1[want])
+        assert np.array_equal(out["b"].to_arrow().to_numpy(), p2[want])
+        exp = arr.take(pa.array(want))
+        valid = np.asarray(exp.is_valid())
+        width = arr.type.bit_width // 8
+        for got in (m.sort(desc, place).to_arrow(), out["k"].to_arrow()):
+            bits = [np.frombuffer(a.buffers()[1], np.uint8, n * width).reshape(n, width)[valid] for a in (got, exp)]
+            assert np.array_equal(np.asarray(got.is_valid()), valid) and np.array_equal(bits[0], bits[1])
+        # Ranks: runs of equal rows in order (null and NaN rows are equals of one another).
+        key, other = v[want], ~valid | (np.isnan(v[want]) if v.dtype.kind == "f" else False)
+        start = np.ones(n, bool)
+        start[1:] = (other[1:] != other[:-1]) | (~other[1:] & (key[1:] != key[:-1]))
+        run, first = np.cumsum(start) - 1, np.flatnonzero(start)
+        last = np.append(first[1:], n)
+        for tiebreaker, pos in (("min", first[run] + 1), ("max", last[run]), ("first", np.arange(1, n + 1))):
+            ranks = np.empty(n, np.int64)
+            ranks[want] = pos
+            got = m.rank("descending" if desc else "ascending", place, tiebreaker).to_arrow().to_numpy()
+            assert np.array_equal(got, ranks), tiebreaker
