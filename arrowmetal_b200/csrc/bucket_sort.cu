@@ -65,6 +65,7 @@ constexpr uint32_t TARGET = 1300;                 // rows a bucket of evenly spr
 constexpr uint32_t CELL_TARGET = 1100;
 constexpr uint32_t SAMPLES = 65536;               // keys looked at (every key of a shorter column)
 constexpr int CLUSTER = 8;                        // CTAs of the one-cluster kernels
+constexpr uint32_t FUSED_BUCKETS = 8192;          // buckets whose starts the count's last CTA finds
 constexpr uint32_t ONE_CAP = 1024;                // buckets of a column of at most SAMPLES rows
 constexpr int BINS = 2048, BINS_LOG = 11;         // bins of the shared-memory sort
 constexpr uint32_t CATS = 2 + FREQUENT;           // a chunk's rows apart from the buckets: null, NaN, each frequent key
@@ -72,6 +73,15 @@ constexpr uint32_t CATS = 2 + FREQUENT;           // a chunk's rows apart from t
 // compared, 843 where later_body takes most of them (24); with 50 rows a value 776 in later_body, 1,113 compared (64).
 constexpr uint32_t MAX_BIN = 40;
 constexpr uint32_t META_SPLIT = 0x80000000u;
+// From so many rows on, keys that differ in their two low bytes alone take the digit passes, of which they need two:
+// 16M int64 keys of 2,500 values 471 us by passes, 958 by buckets; 4.5M 231 and 304; 1M 115 and 114.
+constexpr uint64_t FEW_DIGITS_ROWS = uint64_t(1) << 20, FEW_DIGITS_SPAN = uint64_t(1) << 16;
+// Four passes of a 4-byte key beat its buckets where keys repeat more than about 16 times (16M int32 rows: 645 us by
+// passes; by buckets 621 with 10 rows a value, 698 with 50, 902 with 3,000; keys that do not repeat 408). Of the
+// sample's 8 x 8,192 keys, about 1.6e8 x (rows a value) / rows meet an equal one.
+constexpr uint64_t PAIRS_ROWS = uint64_t(1) << 22;
+constexpr float PAIRS_LIMIT = 1.6e8f * 16.0f;
+constexpr uint64_t WHOLE_SAMPLE_ROWS = uint64_t(1) << 22;
 constexpr int CUR_PAD = 8;                        // cursors 32 bytes apart: same-sector atomics queue
 constexpr int THREADS = 512, ITEMS = 7, TILE = THREADS * ITEMS, WARPS = THREADS / 32;
 constexpr int HTHREADS = 1024, HITEMS = 8;
@@ -90,6 +100,8 @@ struct Args {
   uint32_t* ids[2];
   uint4* rec[2];                                  // with a payload: row id and payload fields (RecLayout), instead of ids
   void *out, *key_out;
+  uint4* clear;                                   // not NULL: memory that the plan's launch clears, the state among it
+  uint64_t clear16;                               // in 16-byte units
   const void* src_keys;                           // not NULL: the rows are these keys, with these ids, and no column
   const uint32_t* src_ids;
   const void* key_src;                            // not NULL: keys that stand for several values are read here
@@ -335,6 +347,7 @@ struct PlanShared {
   uint32_t group[1024];
   unsigned long long smax[CLUSTER], smin[CLUSTER], scnt[CLUSTER];
   unsigned long long wmax[32], wmin[32];
+  uint32_t pairs[CLUSTER];               // the CTAs' pairs of equal keys, then their most frequent keys
   uint32_t mode, buckets, linear;        // the plan, from the first CTA
   // One launch for the counts and the moves too (columns of at most SAMPLES rows): the fine cells, the
   // CTA's null and NaN rows by item and warp, and their sums.
@@ -592,7 +605,9 @@ __device__ __forceinline__ void buckets_body(const ColView& col, const Args& a) 
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const uint32_t rank = cl.block_rank();
   State* st = a.st;
-  cl.sync();                             // every CTA runs before its shared memory is written
+  if (a.clear)
+    for (uint64_t i = rank * 1024 + t; i < a.clear16; i += 1024 * CLUSTER) a.clear[i] = make_uint4(0, 0, 0, 0);
+  cl.sync();                             // every CTA runs before its shared memory is written; the state is clear
   // The sample: one row of each nsamples-th part of the column, at a mixed offset (no period of the data
   // lines up), or every row. nsamples is SAMPLES or the rows.
   constexpr int U = SAMPLES / (1024 * CLUSTER);
@@ -667,13 +682,49 @@ __device__ __forceinline__ void buckets_body(const ColView& col, const Args& a) 
     sv += uint32_t(sm.scnt[r]);
   }
   const unsigned long long lo = sv ? ~vmin_inv : 0ull, span = sv ? vmax - lo : 0ull;
+  auto give_up = [&] {
+    if (rank == 0 && t == 0) {
+      st->mode = MODE_FALLBACK;
+      sm.mode = MODE_FALLBACK;
+    }
+  };
+  if (!a.one_launch && a.n >= FEW_DIGITS_ROWS && sv && span < FEW_DIGITS_SPAN) {
+    give_up();
+    return;
+  }
   const int bits = max(COARSE_BITS, span ? 64 - __clzll((long long)span) : 0);
   const uint32_t shc = uint32_t(bits - COARSE_BITS);        // key bits below a coarse cell
   const Map<KeyT> map{KeyT(lo), KeyT(span), uint32_t(sizeof(KeyT)) * 8u - uint32_t(bits), 0u, 0u};
 #pragma unroll
   for (int u = 0; u < U; u++)
     if ((live >> u) & 1u) atomicAdd(&sm.coarse_cnt[uint32_t(KeyT(key[u] - map.lo) >> shc)], 1u);
+  const bool count_pairs = sizeof(KeyT) == 4 && a.n >= PAIRS_ROWS;
+  if (count_pairs) {
+    // Sampled keys that meet an equal one of the CTA's, in a table of the last key at each place.
+    uint32_t pairs = 0;
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if ((live >> u) & 1u) {
+        const uint32_t k = uint32_t(key[u]);
+        pairs += atomicExch(&sm.part_cnt[__umulhi(k * 2654435761u, uint32_t(4 * FINE))], k) == k ? 1u : 0u;
+      }
+    pairs = __reduce_add_sync(0xffffffffu, pairs);
+    if (lane == 0) sm.warp[warp] = pairs;
+    __syncthreads();
+    pairs = __reduce_add_sync(0xffffffffu, sm.warp[lane]);
+    if (t < CLUSTER) cl.map_shared_rank(&sm, t)->pairs[rank] = pairs;
+  }
   cl.sync();
+  if (count_pairs) {
+    uint32_t pairs = 0;
+#pragma unroll
+    for (int r = 0; r < CLUSTER; r++) pairs += sm.pairs[r];
+    if (float(pairs) * float(a.n) > PAIRS_LIMIT) {
+      give_up();
+      return;
+    }
+    for (int i = t; i < 4 * FINE; i += 1024) sm.part_cnt[i] = 0;
+  }
   uint32_t in_cell = 0;                  // the sample's keys in coarse cell t
   if (t < COARSE) {
 #pragma unroll
@@ -714,6 +765,49 @@ __device__ __forceinline__ void buckets_body(const ColView& col, const Args& a) 
         planned = true;
       }
     }
+  }
+  if (!planned && !a.one_launch) {
+    // A key with more rows than a bucket may hold ends the attempt here: the sample's keys counted by a hash.
+    constexpr int COUNTERS = 2048;
+    static_assert(COUNTERS <= 4 * FINE && COUNTERS % 1024 == 0, "they borrow the quarters' counters");
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if ((live >> u) & 1u) atomicAdd(&sm.part_cnt[uint32_t((uint64_t(key[u]) * 0x9E3779B97F4A7C15ull) >> 53)], 1u);
+    // Over the cluster where a bucket may hold few of the sample's keys; of a shorter column each CTA's own
+    // keys tell (two cluster barriers and the remote counts less: 5 us of a 1M-row sort).
+    const bool whole = a.n >= WHOLE_SAMPLE_ROWS;
+    if (whole) cl.sync();
+    else __syncthreads();
+    uint32_t most = 0;
+#pragma unroll
+    for (int q = 0; q < COUNTERS / 1024; q++) {
+      uint32_t c = 0;
+      if (whole) {
+#pragma unroll
+        for (int r = 0; r < CLUSTER; r++) c += cl.map_shared_rank(&sm, r)->part_cnt[q * 1024 + t];
+      } else {
+        c = sm.part_cnt[q * 1024 + t];
+      }
+      most = max(most, c);
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 0) sm.warp[warp] = most;
+    __syncthreads();
+    most = __reduce_max_sync(0xffffffffu, sm.warp[lane]);
+    if (t < CLUSTER) cl.map_shared_rank(&sm, t)->pairs[rank] = most;
+    cl.sync();
+    most = 0xFFFFFFFFu;                            // what every CTA saw
+#pragma unroll
+    for (int r = 0; r < CLUSTER; r++) most = min(most, sm.pairs[r]);
+    const float c = float(most), seen = whole ? float(a.nsamples) : float(a.nsamples) / CLUSTER;
+    const float others = (whole ? float(sv) : float(sv) / CLUSTER) / COUNTERS;
+    if ((c - others - 3.0f * sqrtf(c)) * float(a.n) > float(a.large) * seen) {
+      give_up();
+      return;
+    }
+    for (int i = t; i < COUNTERS; i += 1024) sm.part_cnt[i] = 0;
+    __syncthreads();
   }
   if (!planned) {
     // Fine cells of each coarse cell: 2^fb, from its share of the sample (about FINE_GOAL cells over the
@@ -879,7 +973,107 @@ __device__ __forceinline__ void buckets_body(const ColView& col, const Args& a) 
 }
 
 // ---- 2. exact counts
-//
+
+// Bucket starts, cursors, the chunks' null and NaN starts, and the decision: by one cluster, or, up to FUSED_BUCKETS
+// of them, by the count's last CTA (one launch less).
+template <typename KeyT, int CTAS>
+__device__ __forceinline__ void starts_body(const Args& a) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ uint32_t s_warp[32], s_sum[CLUSTER], s_max[CLUSTER];
+  State* st = a.st;
+  if (CTAS > 1) {
+    if (a.one_launch || a.bucket_cap <= FUSED_BUCKETS || st->mode != MODE_BUCKETS) return;
+    cl.sync();                           // every CTA runs before its shared memory is written
+  }
+  constexpr uint32_t PER = 8;
+  static_assert(MAX_BUCKETS <= CLUSTER * 1024 * PER && FUSED_BUCKETS <= 1024 * PER, "one round takes every bucket");
+  const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, rank = CTAS > 1 ? cl.block_rank() : 0u;
+  const uint32_t nb = st->buckets, s2 = st->s2;
+  // CTA r takes the r-th of equal shares (a multiple of PER), a thread PER buckets in a row.
+  const uint32_t share = (nb + CTAS * PER - 1) / (CTAS * PER) * PER;
+  const uint32_t b = rank * share + t * PER;
+  uint32_t c[PER], sum = 0, big = 0;
+#pragma unroll
+  for (uint32_t q = 0; q < PER; q++) {
+    c[q] = t * PER < share && b + q < nb ? __ldcg(a.bcount + b + q) : 0u;
+    sum += c[q];
+    big = max(big, c[q]);
+  }
+  uint32_t tot;
+  uint32_t at = block_scan<1024>(sum, s_warp, tot);
+  big = __reduce_max_sync(0xffffffffu, big);
+  __syncthreads();
+  if (lane == 0) s_warp[warp] = big;
+  __syncthreads();
+  big = __reduce_max_sync(0xffffffffu, s_warp[lane]);
+  if (CTAS > 1) {
+    if (t < uint32_t(CTAS)) {
+      cl.map_shared_rank(s_sum, t)[rank] = tot;
+      cl.map_shared_rank(s_max, t)[rank] = big;
+    }
+    cl.sync();
+  } else {
+    if (t == 0) {
+      s_sum[0] = tot;
+      s_max[0] = big;
+    }
+    __syncthreads();
+  }
+  uint32_t carry = 0;
+  for (uint32_t r = 0; r < uint32_t(CTAS); r++) {
+    if (r < rank) at += s_sum[r];
+    carry += s_sum[r];
+    big = max(big, s_max[r]);
+  }
+#pragma unroll
+  for (uint32_t q = 0; q < PER; q++) {
+    if (t * PER < share && b + q < nb) {
+      a.bpos[b + q] = at;
+      a.cursor2[size_t(b + q) * CUR_PAD] = at;
+      if (((b + q) & ((1u << s2) - 1u)) == 0u) a.cursor1[size_t((b + q) >> s2) * CUR_PAD] = at;
+      at += c[q];
+    }
+  }
+  if (rank != 0) return;
+  uint32_t all;
+  const uint32_t nulls = t < a.nchunks ? __ldcg(a.chunk_cats + CATS * t) : 0u;
+  const uint32_t nans = t < a.nchunks ? __ldcg(a.chunk_cats + CATS * t + 1) : 0u;
+  const uint32_t null0 = block_scan<1024>(nulls, s_warp, all);
+  const uint32_t nan0 = block_scan<1024>(nans, s_warp, all);
+  if (t < a.nchunks) {
+    a.chunk_cats[CATS * t] = null0;
+    a.chunk_cats[CATS * t + 1] = nan0;
+  }
+  uint32_t apart = 0;                    // rows of the frequent keys
+  for (uint32_t h = 0; h < st->nkeys; h++) {
+    const uint32_t rows = t < a.nchunks ? __ldcg(a.chunk_cats + CATS * t + 2 + h) : 0u;
+    const uint32_t before = block_scan<1024>(rows, s_warp, all);
+    if (t < a.nchunks) a.chunk_cats[CATS * t + 2 + h] = __ldcg(&st->key_at[h]) + before;
+    if (t == 0) st->key_rows[h] = all;
+    apart += all;
+  }
+  if (t == 0) {
+    const uint32_t n_value = __ldcg(&st->n_value);
+    a.bpos[nb] = carry;
+    st->max_bucket = big;
+    if (carry + apart != n_value) atomicOr(a.err, ERR_BOUNDS);
+    if (big > a.large || carry + apart != n_value) {
+      st->mode = MODE_FALLBACK;
+    } else {
+      // The counters of the digit passes' sort: the key's digits that vary. A two-level sort's two
+      // passes stand in for them.
+      uint32_t active = 0;
+      for (uint32_t d = 0; d < sizeof(KeyT); d++) active += (__ldcg(&st->diff) >> (8 * d)) & 255u ? 1u : 0u;
+      a.sum->value_rows = n_value;
+      a.sum->null_rows = __ldcg(&st->n_null);
+      a.sum->nan_rows = __ldcg(&st->n_nan);
+      a.sum->passes_run = s2 ? 2u : max(1u, active);
+      a.sum->passes_total = uint32_t(sizeof(KeyT));
+    }
+  }
+}
+
 // One read of the column (63 us for 45M keys and 16,384 bins on a B200: the HBM copy rate). Each CTA
 // takes consecutive chunks; a chunk's level-1 counts are the growth of its bins' sums over the chunk.
 template <typename KeyT, bool FREQ = false>
@@ -1018,93 +1212,15 @@ __device__ __forceinline__ void histogram_body(const ColView& col, const Args& a
     if (all_nan) atomicAdd(&st->n_nan, all_nan);
     atomicOr(&st->diff, s_or);
   }
-}
-
-// One cluster: bucket starts, cursors, the chunks' null and NaN starts, and the decision.
-template <typename KeyT>
-__device__ __forceinline__ void starts_body(const Args& a) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cl = cg::this_cluster();
-  __shared__ uint32_t s_warp[32], s_sum[CLUSTER], s_max[CLUSTER];
-  State* st = a.st;
-  if (a.one_launch || st->mode != MODE_BUCKETS) return;
-  cl.sync();                             // every CTA runs before its shared memory is written
-  constexpr uint32_t PER = 8;
-  static_assert(MAX_BUCKETS <= CLUSTER * 1024 * PER, "one round of the cluster takes every bucket");
-  const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, rank = cl.block_rank();
-  const uint32_t nb = st->buckets, s2 = st->s2;
-  // CTA r takes the r-th of equal shares (a multiple of PER), a thread PER buckets in a row.
-  const uint32_t share = (nb + CLUSTER * PER - 1) / (CLUSTER * PER) * PER;
-  const uint32_t b = rank * share + t * PER;
-  uint32_t c[PER], sum = 0, big = 0;
-#pragma unroll
-  for (uint32_t q = 0; q < PER; q++) {
-    c[q] = t * PER < share && b + q < nb ? a.bcount[b + q] : 0u;
-    sum += c[q];
-    big = max(big, c[q]);
-  }
-  uint32_t tot;
-  uint32_t at = block_scan<1024>(sum, s_warp, tot);
-  big = __reduce_max_sync(0xffffffffu, big);
-  __syncthreads();
-  if (lane == 0) s_warp[warp] = big;
-  __syncthreads();
-  big = __reduce_max_sync(0xffffffffu, s_warp[lane]);
-  if (t < uint32_t(CLUSTER)) {
-    cl.map_shared_rank(s_sum, t)[rank] = tot;
-    cl.map_shared_rank(s_max, t)[rank] = big;
-  }
-  cl.sync();
-  uint32_t carry = 0;
-  for (uint32_t r = 0; r < uint32_t(CLUSTER); r++) {
-    if (r < rank) at += s_sum[r];
-    carry += s_sum[r];
-    big = max(big, s_max[r]);
-  }
-#pragma unroll
-  for (uint32_t q = 0; q < PER; q++) {
-    if (t * PER < share && b + q < nb) {
-      a.bpos[b + q] = at;
-      a.cursor2[size_t(b + q) * CUR_PAD] = at;
-      if (((b + q) & ((1u << s2) - 1u)) == 0u) a.cursor1[size_t((b + q) >> s2) * CUR_PAD] = at;
-      at += c[q];
-    }
-  }
-  if (rank != 0) return;
-  uint32_t all;
-  const uint32_t nulls = t < a.nchunks ? a.chunk_cats[CATS * t] : 0u;
-  const uint32_t nans = t < a.nchunks ? a.chunk_cats[CATS * t + 1] : 0u;
-  const uint32_t null0 = block_scan<1024>(nulls, s_warp, all);
-  const uint32_t nan0 = block_scan<1024>(nans, s_warp, all);
-  if (t < a.nchunks) {
-    a.chunk_cats[CATS * t] = null0;
-    a.chunk_cats[CATS * t + 1] = nan0;
-  }
-  uint32_t apart = 0;                    // rows of the frequent keys
-  for (uint32_t h = 0; h < st->nkeys; h++) {
-    const uint32_t rows = t < a.nchunks ? a.chunk_cats[CATS * t + 2 + h] : 0u;
-    const uint32_t before = block_scan<1024>(rows, s_warp, all);
-    if (t < a.nchunks) a.chunk_cats[CATS * t + 2 + h] = st->key_at[h] + before;
-    if (t == 0) st->key_rows[h] = all;
-    apart += all;
-  }
-  if (t == 0) {
-    a.bpos[nb] = carry;
-    st->max_bucket = big;
-    if (carry + apart != st->n_value) atomicOr(a.err, ERR_BOUNDS);
-    if (big > a.large || carry + apart != st->n_value) {
-      st->mode = MODE_FALLBACK;
-    } else {
-      // The counters of the digit passes' sort: the key's digits that vary. A two-level sort's two
-      // passes stand in for them.
-      uint32_t active = 0;
-      for (uint32_t d = 0; d < sizeof(KeyT); d++) active += (st->diff >> (8 * d)) & 255u ? 1u : 0u;
-      a.sum->value_rows = st->n_value;
-      a.sum->null_rows = st->n_null;
-      a.sum->nan_rows = st->n_nan;
-      a.sum->passes_run = s2 ? 2u : max(1u, active);
-      a.sum->passes_total = uint32_t(sizeof(KeyT));
-    }
+  if (a.bucket_cap <= FUSED_BUCKETS) {
+    __shared__ uint32_t s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&st->counted, 1u) == a.hist_grid - 1 ? 1u : 0u;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    starts_body<KeyT, 1>(a);
   }
 }
 
@@ -2517,7 +2633,7 @@ bucket_histogram_kernel(const __grid_constant__ ColView col, const __grid_consta
 }
 template <typename KeyT>
 __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(1024) bucket_starts_kernel(const __grid_constant__ Args a) {
-  starts_body<KeyT>(a);
+  starts_body<KeyT, CLUSTER>(a);
 }
 template <typename KeyT, int PAY, bool FREQ>
 __global__ void __launch_bounds__(THREADS, 2) level1_kernel(const __grid_constant__ ColView col, const __grid_constant__ Args a) {
@@ -2559,7 +2675,7 @@ __global__ void __launch_bounds__(HTHREADS) batch_histogram_kernel(const BatchIt
 }
 template <typename KeyT>
 __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(1024) batch_starts_kernel(const BatchItem* __restrict__ items) {
-  starts_body<KeyT>(batch_item(items).a);
+  starts_body<KeyT, CLUSTER>(batch_item(items).a);
 }
 template <typename KeyT>
 __global__ void __launch_bounds__(THREADS, 2) batch_level1_kernel(const BatchItem* __restrict__ items) {
@@ -2660,7 +2776,10 @@ first_threshold_kernel(const __grid_constant__ ColView col, uint64_t n, uint64_t
   const float mu = float(k) * float(SAMPLES) / float(n);
   const uint32_t want = uint32_t(mu + 4.0f * sqrtf(mu) + 8.0f);
   if (sv < want) {                       // (the same in every CTA)
-    if (rank == 0 && t == 0) fs->limit = ~0ull;
+    if (rank == 0 && t == 0) {
+      fs->limit = ~0ull;
+      fs->rows = n;
+    }
     cl.sync();
     return;
   }
@@ -2699,16 +2818,26 @@ first_threshold_kernel(const __grid_constant__ ColView col, uint64_t n, uint64_t
   if (rank == 0 && t == 0) {
     const uint64_t x = shift ? (prefix << shift) | ((1ull << shift) - 1ull) : prefix;
     fs->limit = lo + (x < span ? x : span);
+    // Many rows at the limit itself: the first of them, in row order, are enough (evenly spread over the column, with a
+    // margin of four deviations and a quarter).
+    const float equal = shift ? 0.0f : float(sm.pick[2]) * float(n) / float(SAMPLES), wanted = float(k);
+    fs->rows = n;
+    if (equal > 2.0f * wanted + 1024.0f) {
+      const float part = 1.25f * (wanted + 4.0f * sqrtf(wanted) + 64.0f) / equal;
+      if (part < 1.0f) fs->rows = uint64_t(float(n) * part);
+    }
   }
   cl.sync();                             // no CTA leaves while another reads its counts
 }
 
-// Rows whose key is at most the limit, appended as (key, row) pairs; pairs past `cap` are only counted.
+// Rows whose key is below the limit, and those at the limit among the first rows, appended as (key, row) pairs; pairs past `cap` are
+// only counted.
 template <typename KeyT>
 __global__ void __launch_bounds__(256) first_collect_kernel(const __grid_constant__ ColView col, uint64_t n, FirstState* __restrict__ fs,
                                                             uint32_t cap, KeyT* __restrict__ keys, uint32_t* __restrict__ rows) {
   constexpr int NI = 8;
   const KeyT limit = KeyT(fs->limit);
+  const uint64_t equal_rows = fs->rows;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
   const uint64_t step = uint64_t(gridDim.x) * (256 * NI);
   for (uint64_t w0 = uint64_t(blockIdx.x) * (256 * NI) + warp * (NI * 32); w0 < n; w0 += step) {
@@ -2719,7 +2848,7 @@ __global__ void __launch_bounds__(256) first_collect_kernel(const __grid_constan
     uint32_t hit = 0;
 #pragma unroll
     for (int i = 0; i < NI; i++)
-      if (((values >> i) & 1u) && r.key[i] <= limit) hit |= 1u << i;
+      if (((values >> i) & 1u) && (r.key[i] < limit || (r.key[i] == limit && w0 + i * 32 + lane < equal_rows))) hit |= 1u << i;
     if (!__any_sync(0xffffffffu, hit != 0u)) continue;
 #pragma unroll
     for (int i = 0; i < NI; i++) {
@@ -2834,7 +2963,7 @@ void launch_counts(const Sort& b, const Args& a, cudaStream_t s) {
     bucket_histogram_kernel<KeyT, FREQ><<<a.hist_grid, HTHREADS, size_t(a.bucket_cap) * 4, s>>>(b.col, a);
     AM_CUDA(cudaGetLastError());
   }
-  {
+  if (a.bucket_cap > FUSED_BUCKETS) {
     KernelTimer kt("bucket_scan", s);
     bucket_starts_kernel<KeyT><<<CLUSTER, 1024, 0, s>>>(a);
     AM_CUDA(cudaGetLastError());
@@ -2915,6 +3044,8 @@ static Args make_args(const Sort& b) {
   }
   a.ties = b.ties;
   a.ranks = b.ranks;
+  a.clear = static_cast<uint4*>(b.clear);
+  a.clear16 = b.clear ? b.clear_bytes / 16 : 0;
   a.src_keys = b.src_keys;
   a.src_ids = b.src_ids;
   a.out = b.out;
@@ -2935,7 +3066,7 @@ static Args make_args(const Sort& b) {
   a.sum = b.summary;
   if (b.payload) a.pay = b.rec;
   a.bins1_cap = b.payload ? BINS1 / 2 : BINS1;
-  a.large = b.ties.offsets ? uint32_t(BIG) : large_rows(b.n);
+  a.large = b.ties.offsets ? uint32_t(BIG) : b.src_ids ? LARGE : large_rows(b.n);
   a.has_payload = b.payload ? 1 : 0;
   a.one_launch = b.n <= SAMPLES ? 1 : 0;
   a.frequent = b.frequent && !a.one_launch && !b.payload && !b.key_out && !b.ranks.out && !b.ties.offsets && !b.src_ids && b.key_bytes == 8 ? 1 : 0;
@@ -2995,7 +3126,7 @@ void launch_batch(const BatchItem* items, const BatchItem* host, uint32_t count,
     step("batch_plan", [&] { batch_buckets_kernel<KeyT><<<dim3(CLUSTER, rows), 1024, 0, s>>>(it); });
     if (hist) {
       step("batch_histogram", [&] { batch_histogram_kernel<KeyT><<<dim3(hist, rows), HTHREADS, size_t(cap) * 4, s>>>(it); });
-      step("batch_scan", [&] { batch_starts_kernel<KeyT><<<dim3(CLUSTER, rows), 1024, 0, s>>>(it); });
+      if (cap > FUSED_BUCKETS) step("batch_scan", [&] { batch_starts_kernel<KeyT><<<dim3(CLUSTER, rows), 1024, 0, s>>>(it); });
       step("batch_level1", [&] {
         batch_level1_kernel<KeyT><<<dim3(chunks, rows), THREADS, sizeof(TileShared<KeyT, 0>), s>>>(it);
       });

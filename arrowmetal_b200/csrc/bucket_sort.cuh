@@ -12,7 +12,7 @@ constexpr uint32_t MODE_BUCKETS = 1, MODE_FALLBACK = 2;
 constexpr int FREQUENT = 4;              // keys with too many rows for a bucket that a sort can set apart
 
 // What the sampling, the histogram and the scan decide, read by the kernels after them. All zero when a
-// sort starts.
+// sort starts (or cleared by it, Sort::clear).
 struct State {
   unsigned long long lo, span;           // smallest sampled key, and the largest's distance from it
   unsigned long long diff;               // bits in which some value key differs from lo
@@ -23,6 +23,7 @@ struct State {
   uint32_t n_value, n_null, n_nan;
   uint32_t max_bucket;
   uint32_t later;                        // buckets that the fast form put off
+  uint32_t counted;                      // the count's CTAs that are done
   // Keys too frequent for a bucket (Sort::frequent), ascending: their rows leave in row order, as null rows
   // do, to the places from `key_at` on among the values.
   uint32_t nkeys;
@@ -50,9 +51,9 @@ struct RankOut {
   int32_t merge;
 };
 
-// The first rows' selection: keys up to `limit` are kept, `count` of them.
+// The first rows' selection: keys below `limit` are kept, and those at it of the first `rows` rows, `count` of them.
 struct FirstState {
-  unsigned long long limit;
+  unsigned long long limit, rows;
   uint32_t count, pad;
 };
 
@@ -65,6 +66,8 @@ struct Sort {
   const uint32_t* src_ids;
   char* scratch;                         // `scratch_bytes(n)` bytes, the first `zeroed_bytes(n)` zero
   char* zeroed;                          // not NULL: those zero bytes are here instead
+  void* clear;                           // not NULL: `clear_bytes` (a multiple of 16) that the sort itself clears first
+  size_t clear_bytes;
   void* keys[2];                         // n keys each
   char* ids[2];                          // n x 4 bytes, or n x 16 with a payload
   StringTies ties;

@@ -590,7 +590,14 @@ am_array* rank_of(am_array* a, int fn, bool desc, bool nulls_first, bool merge_n
     const SortKey key{a, desc, nulls_first, float_order};
     uint32_t* mode = static_cast<uint32_t*>(perm->ptr) + n;
     const uint32_t* gate = nullptr;
-    if (rank_by_buckets(key, n, fn, merge_nan, static_cast<uint32_t*>(out->values->ptr), static_cast<uint32_t*>(perm->ptr), mode, s))
+    // A key of few distinct values sorts by its dense rank, in one pass; the values are looked for once.
+    if (am_array* few = low_cardinality_ranks(key, s)) {
+      struct Release {
+        am_array* a;
+        ~Release() { release(a); }
+      } owned{few};
+      argsort_any({SortKey{few, false, nulls_first, 0}}, n, perm->ptr, 4, s, nullptr);
+    } else if (rank_by_buckets(key, n, fn, merge_nan, static_cast<uint32_t*>(out->values->ptr), static_cast<uint32_t*>(perm->ptr), mode, s))
       gate = mode;
     else argsort_any({key}, n, perm->ptr, 4, s, nullptr);
     const uint32_t* p = static_cast<const uint32_t*>(perm->ptr);

@@ -268,11 +268,6 @@ __device__ __forceinline__ uint64_t key_max(int bytes) { return bytes == 8 ? ~0u
 
 __device__ void plan_body(const PlanArgs& a, KeyStats* __restrict__ st, KeyPlan* __restrict__ kp,
                           PassDesc* __restrict__ pd, SortSummary* __restrict__ sum) {
-  __shared__ uint32_t s_vals[256];
-  __shared__ uint32_t s_out[256];
-  __shared__ uint32_t s_warp[16];
-  __shared__ uint32_t s_total;
-  __shared__ uint32_t s_max;
   __shared__ uint8_t s_active[MAX_SLOTS];
   const int t = threadIdx.x;
   const uint32_t n = uint32_t(a.n);
@@ -320,27 +315,25 @@ __device__ void plan_body(const PlanArgs& a, KeyStats* __restrict__ st, KeyPlan*
   }
   __syncthreads();
 
-  // 2. Which digit passes are not constant.
-  for (int sl = 0; sl < a.nslots; sl++) {
+  // 2. Which digit passes are not constant: a warp a slot.
+  const int warp = t >> 5, lane = t & 31, warps = int(blockDim.x) >> 5;
+  for (int sl = warp; sl < a.nslots; sl += warps) {
     const int k = a.slot_key[sl], d = a.slot_digit[sl];
+    uint32_t active = 0;
     if (last_done && k == a.nkeys - 1) {
-      if (t == 0) s_active[sl] = 0;
-      continue;
+      active = 0;
+    } else if (d < 0) {
+      active = kp[k].fold_mode == 1 ? 1 : 0;
+    } else {
+      uint32_t c = 0;
+#pragma unroll
+      for (int q = 0; q < 8; q++) c = max(c, st[k].hist[d][q * 32 + lane]);
+      const uint32_t total = (k == 0) ? st[0].n_value : n, most = __reduce_max_sync(0xffffffffu, c);
+      active = (total > 0 && most < total) ? 1 : 0;
     }
-    if (d < 0) {
-      if (t == 0) s_active[sl] = (kp[k].fold_mode == 1) ? 1 : 0;
-      continue;
-    }
-    const uint32_t total = (k == 0) ? st[0].n_value : n;
-    if (t == 0) s_max = 0;
-    __syncthreads();
-    uint32_t c = t < 256 ? st[k].hist[d][t] : 0u;
-    uint32_t m = __reduce_max_sync(0xffffffffu, c);
-    if ((t & 31) == 0) atomicMax(&s_max, m);
-    __syncthreads();
-    if (t == 0) s_active[sl] = (total > 0 && s_max < total) ? 1 : 0;
-    __syncthreads();
+    if (lane == 0) s_active[sl] = uint8_t(active);
   }
+  __syncthreads();
 
   // 3. Buffers: walk the active passes in order, least significant key first.
   if (t == 0) {
@@ -402,28 +395,41 @@ __device__ void plan_body(const PlanArgs& a, KeyStats* __restrict__ st, KeyPlan*
   }
   __syncthreads();
 
-  // 4. Per active pass, every bin's global base.
-  for (int sl = 0; sl < a.nslots; sl++) {
+  // 4. Per active pass, every bin's global base: a warp a pass, eight bins in a row a lane.
+  for (int sl = warp; sl < a.nslots; sl += warps) {
     if (!s_active[sl]) continue;
     const int k = a.slot_key[sl], d = a.slot_digit[sl];
     PassDesc& p = pd[sl];
     if (d < 0) {
       // Category pass: bin 0 / 1 in category order.
-      if (t == 0) {
+      if (lane == 0) {
         const uint32_t nn = st[k].n_null, nv = n - nn;
         const bool first = a.nulls_first[k];
         p.bin_base[0] = 0;
         p.bin_base[1] = first ? nn : nv;
         for (int b = 2; b < NBINS; b++) p.bin_base[b] = 0;
       }
-      __syncthreads();
       continue;
     }
-    if (t < 256) s_vals[t] = st[k].hist[d][t];
-    __syncthreads();
-    block_exclusive_scan_256(s_vals, s_out, &s_total, s_warp);
-    if (t < 256) p.bin_base[t] = s_out[t];
-    if (t == 0) {
+    uint32_t c[8], sum = 0;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      c[q] = st[k].hist[d][lane * 8 + q];
+      sum += c[q];
+    }
+    uint32_t x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    x -= sum;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      p.bin_base[lane * 8 + q] = x;
+      x += c[q];
+    }
+    if (lane == 0) {
       const uint32_t m = st[0].n_value, nn = st[0].n_null, nnan = st[0].n_nan;
       if (k == 0 && a.nulls_first[0]) {
         p.bin_base[NULL_BIN] = 0;
@@ -433,8 +439,8 @@ __device__ void plan_body(const PlanArgs& a, KeyStats* __restrict__ st, KeyPlan*
         p.bin_base[NULL_BIN] = m + nnan;
       }
     }
-    __syncthreads();
   }
+  __syncthreads();
 }
 
 __global__ void __launch_bounds__(256) plan_kernel(PlanArgs a, KeyStats* __restrict__ st, KeyPlan* __restrict__ kp,
@@ -734,7 +740,7 @@ struct PassShared {
 // pass's own (a launch may run several passes one after the other).
 template <typename KeyT, typename StatusT, int THREADS, int ITEMS, bool SEG, bool REC>
 __device__ __forceinline__ void onesweep_pass(const PassArgs& pa, const ColView& col_arg, const PassDesc* pass_desc,
-                                              uint32_t* tickets, uint32_t epoch) {
+                                              uint32_t* tickets, uint32_t epoch, void* look_back) {
   static_assert(THREADS >= NBINS && THREADS % 32 == 0, "one thread per digit bin");
   static_assert(THREADS * ITEMS <= 65536, "tile-local ranks are 16-bit");
   static_assert(!(SEG && REC), "record passes sort one array");
@@ -744,7 +750,7 @@ __device__ __forceinline__ void onesweep_pass(const PassArgs& pa, const ColView&
   constexpr int WARPS = SM::WARPS;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SM& sm = *reinterpret_cast<SM*>(smem_raw);
-  StatusT* __restrict__ status = static_cast<StatusT*>(pa.status);
+  StatusT* __restrict__ status = static_cast<StatusT*>(look_back);
 
   auto copy_words = [](void* dst, const void* src, int words) {
     for (int i = threadIdx.x; i < words; i += THREADS)
@@ -1180,7 +1186,7 @@ __device__ __forceinline__ void onesweep_pass(const PassArgs& pa, const ColView&
 template <typename KeyT, typename StatusT, int THREADS, int ITEMS, bool SEG, bool REC = false>
 __global__ void __launch_bounds__(THREADS, 2)
 onesweep_pass_kernel(const __grid_constant__ PassArgs pa, const __grid_constant__ ColView col) {
-  onesweep_pass<KeyT, StatusT, THREADS, ITEMS, SEG, REC>(pa, col, pa.desc, pa.tile_counter, pa.epoch);
+  onesweep_pass<KeyT, StatusT, THREADS, ITEMS, SEG, REC>(pa, col, pa.desc, pa.tile_counter, pa.epoch, pa.status);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1226,7 +1232,8 @@ struct AllPassesArgs {
   uint32_t* tickets;
   uint32_t* arrived;
   const uint32_t* mode;      // bs::MODE_FALLBACK: run
-  uint64_t status16;         // the look-back words, in 16-byte units
+  uint64_t status16;         // the look-back words of a pass, in 16-byte units (there are twice as many)
+  int32_t counted;           // the key's statistics are there
 };
 
 // False when a barrier ran out.
@@ -1235,21 +1242,28 @@ __device__ __forceinline__ bool run_all_passes(const AllPassesArgs& a, const Col
   uint32_t round = 0;
   constexpr int HI = 4;
   constexpr uint64_t CHUNK = uint64_t(THREADS) * HI;
-  histogram_rows<KeyT, THREADS, HI, false>(col, a.stats, uint64_t(blockIdx.x) * CHUNK, a.plan.n, uint64_t(gridDim.x) * CHUNK);
+  if (!a.counted) histogram_rows<KeyT, THREADS, HI, false>(col, a.stats, uint64_t(blockIdx.x) * CHUNK, a.plan.n, uint64_t(gridDim.x) * CHUNK);
+  // Two sets of look-back words: one pass uses the one while the other is cleared for the next.
+  uint4* words[2] = {static_cast<uint4*>(a.pass.status), static_cast<uint4*>(a.pass.status) + a.status16};
+  auto clear = [&](uint4* w) {
+    for (uint64_t i = uint64_t(blockIdx.x) * THREADS + threadIdx.x; i < a.status16; i += uint64_t(gridDim.x) * THREADS)
+      w[i] = make_uint4(0, 0, 0, 0);
+  };
+  clear(words[0]);
   if (!grid_barrier(a.arrived, round, a.pass.err)) return false;
   if (blockIdx.x == 0) {
     plan_body(a.plan, a.stats, a.kplan, a.desc, a.sum);
-    // The sample and the count read the rows before the passes.
     if (threadIdx.x == 0) a.sum->passes_run += 2;
   }
+  uint32_t turn = 0;
   for (int sl = 0; sl < a.plan.nslots; sl++) {
-    if (!grid_barrier(a.arrived, round, a.pass.err)) return false;
+    // (The first barrier makes the plan visible; the next ones follow a pass.)
+    if (sl == 0 && !grid_barrier(a.arrived, round, a.pass.err)) return false;
     if (!*reinterpret_cast<const volatile uint32_t*>(&a.desc[sl].active)) continue;
-    uint4* words = static_cast<uint4*>(a.pass.status);
-    for (uint64_t i = uint64_t(blockIdx.x) * THREADS + threadIdx.x; i < a.status16; i += uint64_t(gridDim.x) * THREADS)
-      words[i] = make_uint4(0, 0, 0, 0);
-    if (!grid_barrier(a.arrived, round, a.pass.err)) return false;
-    onesweep_pass<KeyT, uint32_t, THREADS, ITEMS, false, REC>(a.pass, col, a.desc + sl, a.tickets + sl, 0u);
+    if (turn && !grid_barrier(a.arrived, round, a.pass.err)) return false;
+    clear(words[(turn + 1) & 1]);
+    onesweep_pass<KeyT, uint32_t, THREADS, ITEMS, false, REC>(a.pass, col, a.desc + sl, a.tickets + sl, 0u, words[turn & 1]);
+    turn++;
   }
   return true;
 }
@@ -1824,6 +1838,7 @@ template <> struct PassConfig<uint32_t> { static constexpr int THREADS = 512, IT
 template <> struct PassConfig<uint64_t> { static constexpr int THREADS = 512, ITEMS = 10; };
 constexpr int HIST_THREADS = 256, HIST_ITEMS = 8;
 constexpr int MAX_ONE_KEY = 8;        // digit passes of one key
+constexpr uint64_t COUNT_APART_ROWS = uint64_t(1) << 23;
 // Ranks leave the bucket sort as random 4-byte stores: while the whole rank column (64 MB here) stays in L2.
 // 8M int64 keys with nulls, min: 867 us by an order, run marks and a scatter, 342 so.
 constexpr uint64_t RANK_BUCKET_ROWS = uint64_t(1) << 24;
@@ -2087,6 +2102,13 @@ static void launch_all_passes(const rs::AllPassesArgs& a, const rs::ColView& cv,
   AM_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(fn), dim3(uint32_t(grid)), dim3(C::THREADS), args, smem, s));
 }
 
+// Keys of one or two bytes need one or two digit passes: 65,537 int16 rows 66 us by passes and 85 by buckets, 1M 85 and 104.
+// Up to bs::MAX_PAIRS rows one launch plans, counts and moves them to buckets.
+static bool few_digits(const SortKey& key, uint64_t n) {
+  const int pt = key.col->pt;
+  return n > bs::MAX_PAIRS && (pt == PT_BOOL || pt == PT_I8 || pt == PT_U8 || pt == PT_I16 || pt == PT_U16);
+}
+
 // One key sorted by buckets (bucket_sort.cu), or, when the device finds a bucket too large, by the digit
 // passes in one launch.
 static void sort_by_buckets(const SortKey& key, const rs::PlanArgs& pa, uint64_t n, int kb, void* out, int index_width,
@@ -2105,17 +2127,19 @@ static void sort_by_buckets(const SortKey& key, const rs::PlanArgs& pa, uint64_t
   const size_t ibuf = up(payload ? n * sizeof(uint4) : n * sizeof(uint32_t));
   ScratchBlock scratch(s, off_keys + 2 * kbuf + 2 * ibuf);
   char* base = scratch.data();
-  AM_CUDA(cudaMemsetAsync(base, 0, off_bs + bs::zeroed_bytes(n), s));
   if (key_dst) alloc_key_column(key_dst, key, n, s);
   const uint64_t tile = min_super();
   const uint64_t tiles = (n + tile - 1) / tile;
-  StreamScratch& sc = stream_scratch(s, size_t(tiles) * NBINS);
+  // Two sets of 32-bit look-back words, each a whole number of 16-byte pieces.
+  StreamScratch& sc = stream_scratch(s, size_t(tiles + 1) * NBINS);
   SortSummary* sum = reinterpret_cast<SortSummary*>(base + off_sum);
 
   bs::Sort b{};
   b.col = make_view(key);
   b.key_bytes = kb;
   b.n = n;
+  b.clear = base;
+  b.clear_bytes = off_bs + bs::zeroed_bytes(n);
   b.scratch = base + off_bs;
   b.payload = payload != nullptr;
   if (payload) b.rec = *payload;
@@ -2168,6 +2192,13 @@ static void sort_by_buckets(const SortKey& key, const rs::PlanArgs& pa, uint64_t
   a.status16 = (tiles * NBINS * sizeof(uint32_t) + 15) / 16;
   // The passes use the stream's look-back words with no epoch: later 64-bit users start over.
   sc.epoch = (1u << 30) - 1;
+  // Many rows are counted by a launch of the shape that reads them fastest (50M int64 rows 140 us; within the
+  // passes' launch, of few threads a row, 330), few within the passes' launch.
+  if (n > COUNT_APART_ROWS) {
+    a.counted = 1;
+    if (kb == 8) launch_histogram<uint64_t>(b.col, a.stats, n, s, false, a.mode);
+    else launch_histogram<uint32_t>(b.col, a.stats, n, s, false, a.mode);
+  }
   if (kb == 8) {
     if (payload) launch_all_passes<uint64_t, true>(a, b.col, n, s);
     else launch_all_passes<uint64_t, false>(a, b.col, n, s);
@@ -2183,13 +2214,8 @@ bool rank_by_buckets(const SortKey& key, int64_t n64, int fn, bool merge_nan, ui
                      cudaStream_t s) {
   using namespace rs;
   const uint64_t n = uint64_t(n64);
-  if (n == 0 || n > RANK_BUCKET_ROWS || pt_var(key.col->pt) || key.col->dictionary || debug_skip_first_tile()) return false;
+  if (n == 0 || n > RANK_BUCKET_ROWS || pt_var(key.col->pt) || key.col->dictionary || few_digits(key, n) || debug_skip_first_tile()) return false;
   if (fn != RANK_MIN && fn != RANK_MAX && fn != RANK_FIRST) return false;
-  // A key of few distinct values sorts by its dense rank in one pass; its order is ranked as before.
-  if (am_array* r = low_cardinality_ranks(key, s)) {
-    am::release(r);
-    return false;
-  }
   PlanArgs pa{};
   const int kb = pt_key_bytes(key.col->pt);
   pa.n = n;
@@ -2219,7 +2245,6 @@ bool string_argsort(const SortKey& key, int64_t n64, void* out, int index_width,
   const size_t kbuf = up(n * 8), ibuf = up(n * 4);
   ScratchBlock scratch(s, off_keys + 2 * kbuf + 2 * ibuf);
   char* base = scratch.data();
-  AM_CUDA(cudaMemsetAsync(base, 0, off_bs + bs::zeroed_bytes(n), s));
   SortSummary* sum = reinterpret_cast<SortSummary*>(base);
   const SortKey first{column.c, key.descending, key.nulls_first, 0};
   bs::Sort b{};
@@ -2231,6 +2256,8 @@ bool string_argsort(const SortKey& key, int64_t n64, void* out, int index_width,
   b.ties.chars = static_cast<const uint32_t*>(chars->ptr) + 8;
   b.ties.wide = a->pt == PT_LSTR ? 1 : 0;
   b.ties.desc = key.descending ? 1 : 0;
+  b.clear = base;
+  b.clear_bytes = off_bs + bs::zeroed_bytes(n);
   b.scratch = base + off_bs;
   for (int i = 0; i < 2; i++) {
     b.keys[i] = base + off_keys + size_t(i) * kbuf;
@@ -2323,7 +2350,7 @@ void radix_sort(const std::vector<SortKey>& keys_in, int64_t n64, void* out, int
   for (auto& k : keys) max_kb = std::max(max_kb, pt_key_bytes(k.col->pt));
 
   // One key of a size that buckets serve: the bucket sort, with the digit passes behind it.
-  if (K == 1 && n <= bs::MAX_ROWS && !debug_skip_first_tile()) {
+  if (K == 1 && n <= bs::MAX_ROWS && !few_digits(keys[0], n) && !debug_skip_first_tile()) {
     sort_by_buckets(keys[0], pa, n, max_kb, out, index_width, key_dst, payload, carry_ids, s, stats);
     return;
   }
@@ -2384,12 +2411,13 @@ void radix_sort(const std::vector<SortKey>& keys_in, int64_t n64, void* out, int
   for (int k = 0; k < K; k++) views[k] = make_view(keys[k]);
   uint32_t* const order = last_first ? reinterpret_cast<uint32_t*>(base + off_order) : nullptr;
   if (last_first) {
-    AM_CUDA(cudaMemsetAsync(base + off_bs, 0, bs::zeroed_bytes(n), s));
     const SortKey& key = keys[K - 1];
     bs::Sort b{};
     b.col = views[K - 1];
     b.key_bytes = pt_key_bytes(key.col->pt);
     b.n = n;
+    b.clear = base + off_bs;
+    b.clear_bytes = bs::zeroed_bytes(n);
     b.scratch = base + off_bs;
     b.keys[0] = kbufA;
     b.keys[1] = kbufB;
@@ -2958,8 +2986,8 @@ void sort_segment_buckets(const std::vector<SortKey>& keys, const std::vector<vo
   if (!large.empty()) sort_segment_class<KeyT, 512, 8>(keys, outs, large, allow_graph, s);
   if (group.empty()) return;
   BucketLayout<KeyT> L(keys, group);
-  // The passes clear the look-back words 16 bytes at a time: a whole number of those.
-  const size_t status_bytes = (size_t(L.max_tiles) * NBINS * sizeof(uint32_t) + 15) & ~size_t(15);
+  // The passes clear the look-back words 16 bytes at a time: a whole number of those, twice.
+  const size_t status_bytes = 2 * ((size_t(L.max_tiles) * NBINS * sizeof(uint32_t) + 15) & ~size_t(15));
   StreamScratch& sc = stream_scratch(s, status_bytes / 8);
   sc.epoch = (1u << 30) - 1;               // its words are used without an epoch: later users start over
   bs::prepare_batch(int(sizeof(KeyT)));

@@ -690,13 +690,14 @@ static am_array* first_rows(const SortKey& key, int64_t k, cudaStream_t s) {
     out->null_count = 0;
     out->perm_of = int64_t(n);
     out->last_stream = s;
-    AM_CUDA(cudaMemsetAsync(base + off_bs, 0, bs::zeroed_bytes(count), s));
     bs::Sort b{};
     b.col = col;
     b.key_bytes = kb;
     b.n = count;
     b.src_keys = base + off_pairs;
     b.src_ids = rows;
+    b.clear = base + off_bs;
+    b.clear_bytes = bs::zeroed_bytes(count);
     b.scratch = base + off_bs;
     for (int i = 0; i < 2; i++) {
       b.keys[i] = base + off_keys + size_t(i) * cap * 8;

@@ -291,3 +291,24 @@ def test_ranks_out_of_the_buckets(am, oracle, n, kind):
     rows = np.empty(n, np.uint32)
     rows[order] = np.arange(1, n + 1)
     assert np.array_equal(np_of(m.row_number()), rows)
+
+
+def test_rank_of_few_values_looks_for_them_once(am):
+    # The ranks of a large column of few values come from its dense rank: one search for the values a call.
+    rng = np.random.default_rng(77)
+    n = (1 << 22) + 5
+    v = rng.integers(0, 100, n) * 7919
+    for _ in range(2):
+        m = am.MetalArray.from_arrow(pa.array(v))
+        m.rank()
+        am.synchronize()
+        am.profile_reset()
+        am.profile(True)
+        got = m.rank().to_arrow().to_numpy()
+        am.synchronize()
+        launches = {k: c for k, (c, _) in am.profile_entries().items()}
+        am.profile(False)
+        assert launches["low_cardinality_probe"] == 1 and launches["low_cardinality_rank"] == 1
+        values, counts = np.unique(v, return_counts=True)
+        first = np.concatenate([[0], np.cumsum(counts)[:-1]]) + 1
+        assert np.array_equal(got, first[np.searchsorted(values, v)])

@@ -83,3 +83,18 @@ def test_top_k_at_the_order_by_scale(am):
     order = vi[np.argsort(key[vi], kind="stable")]
     for k in (10, 1000, 1_000_000):
         assert np.array_equal(ids(col.top_k(k, False)), order[:k])
+
+
+@pytest.mark.parametrize("rows_a_value", [300, 5000, 60_000])
+@pytest.mark.parametrize("k", [1, 1000, 20_000])
+def test_repeated_keys_at_the_limit(am, oracle, rows_a_value, k):
+    # More rows share the k-th key than the selection wants: the first of them in row order are taken, wherever they are.
+    n = 1_200_007
+    rng = np.random.default_rng(rows_a_value + k)
+    m = n // rows_a_value
+    v = rng.integers(0, 2**40, m)[rng.integers(0, m, n)]
+    for keys in (v, np.sort(v), v.astype(np.float64)):
+        arr = pa.array(keys, mask=rng.random(n) < 0.05)
+        for largest in (True, False):
+            want = oracle.argsort(arr, largest, "at_end", threads=4)[:k]
+            assert np.array_equal(am.MetalArray.from_arrow(arr).top_k(k, largest).to_arrow().to_numpy(), want)
