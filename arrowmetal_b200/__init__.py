@@ -83,7 +83,7 @@ class BatchShape(ctypes.Structure):
 class SortStats(ctypes.Structure):
     _fields_ = [("rows", _I64), ("value_rows", _I64), ("passes_run", ctypes.c_int32),
                 ("passes_skipped", ctypes.c_int32), ("kernel_us", ctypes.c_double),
-                ("payload_in_records", ctypes.c_int32), ("reserved", ctypes.c_int32)]
+                ("payload_in_records", ctypes.c_int32), ("method", ctypes.c_int32)]
 
 
 def _sig(name, res, args):
@@ -772,7 +772,8 @@ def last_sort_stats():
     s = SortStats()
     _ok(_lib.am_last_sort_stats(ctypes.byref(s)))
     return {"rows": s.rows, "value_rows": s.value_rows, "passes_run": s.passes_run,
-            "passes_skipped": s.passes_skipped, "payload_in_records": bool(s.payload_in_records)}
+            "passes_skipped": s.passes_skipped, "payload_in_records": bool(s.payload_in_records),
+            "method": ("digit_passes", "two_level", "buckets")[s.method]}
 
 
 def batch_tuning():

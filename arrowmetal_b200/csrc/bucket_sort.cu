@@ -930,7 +930,8 @@ __device__ __forceinline__ void buckets_body(const ColView& col, const Args& a) 
         a.sum->value_rows = values;
         a.sum->null_rows = nn;
         a.sum->nan_rows = nx;
-        a.sum->passes_run = max(1u, active);
+        a.sum->passes_run = active;
+        a.sum->method = 2;
         a.sum->passes_total = uint32_t(sizeof(KeyT));
       } else {
         st->mode = MODE_FALLBACK;
@@ -1061,14 +1062,14 @@ __device__ __forceinline__ void starts_body(const Args& a) {
     if (big > a.large || carry + apart != n_value) {
       st->mode = MODE_FALLBACK;
     } else {
-      // The counters of the digit passes' sort: the key's digits that vary. A two-level sort's two
-      // passes stand in for them.
+      // The counters: no digit pass runs; the key's digits that vary stand in for them.
       uint32_t active = 0;
       for (uint32_t d = 0; d < sizeof(KeyT); d++) active += (__ldcg(&st->diff) >> (8 * d)) & 255u ? 1u : 0u;
       a.sum->value_rows = n_value;
       a.sum->null_rows = __ldcg(&st->n_null);
       a.sum->nan_rows = __ldcg(&st->n_nan);
-      a.sum->passes_run = s2 ? 2u : max(1u, active);
+      a.sum->passes_run = active;
+      a.sum->method = 2;
       a.sum->passes_total = uint32_t(sizeof(KeyT));
     }
   }

@@ -390,8 +390,9 @@ __device__ void plan_body(const PlanArgs& a, KeyStats* __restrict__ st, KeyPlan*
     sum->value_rows = st[0].n_value;
     sum->null_rows = st[0].n_null;
     sum->nan_rows = st[0].n_nan;
-    sum->passes_run = run + (last_done ? sum->passes_run : 0u);
+    sum->passes_run = run;
     sum->passes_total = uint32_t(a.nslots);
+    sum->method = 0;
   }
   __syncthreads();
 
@@ -1251,10 +1252,7 @@ __device__ __forceinline__ bool run_all_passes(const AllPassesArgs& a, const Col
   };
   clear(words[0]);
   if (!grid_barrier(a.arrived, round, a.pass.err)) return false;
-  if (blockIdx.x == 0) {
-    plan_body(a.plan, a.stats, a.kplan, a.desc, a.sum);
-    if (threadIdx.x == 0) a.sum->passes_run += 2;
-  }
+  if (blockIdx.x == 0) plan_body(a.plan, a.stats, a.kplan, a.desc, a.sum);
   uint32_t turn = 0;
   for (int sl = 0; sl < a.plan.nslots; sl++) {
     // (The first barrier makes the plan visible; the next ones follow a pass.)
@@ -1523,6 +1521,7 @@ __global__ void __launch_bounds__(256) bucket_scan_kernel(HybridState* __restric
   if (v >= 0) {
     hs->variant = uint32_t(v);
     sum->passes_run = 2;                 // the local sorts stand in for the others
+    sum->method = 1;
   } else {
     hs->fallback = 1;
     for (uint32_t i = 0; i < hs->nfall; i++) steps[2 + i].active = 1;
@@ -1982,6 +1981,7 @@ void fill_last_sort_stats(am_sort_stats* out) {
   out->value_rows = h->value_rows;
   out->passes_run = int32_t(h->passes_run);
   out->passes_skipped = int32_t(h->passes_total - h->passes_run);
+  out->method = int32_t(h->method);
 }
 
 void key_statistics(const SortKey& k, rs::KeyStats* st, cudaStream_t s) {

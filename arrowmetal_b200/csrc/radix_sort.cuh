@@ -70,7 +70,7 @@ struct PassDesc {
 };
 
 struct SortSummary {
-  uint32_t value_rows, null_rows, nan_rows, passes_run, passes_total, pad[3];
+  uint32_t value_rows, null_rows, nan_rows, passes_run, passes_total, method, pad[2];      // method: am_sort_stats'
 };
 
 struct PlanArgs {

@@ -258,9 +258,11 @@ typedef struct am_batch_shape {
 } am_batch_shape;
 int  am_cuda_batch_tuning(am_batch_shape* out, int64_t capacity, int64_t* count);
 
-/* Per-call counters of the calling thread's last sort: rows, radix passes run and skipped, the device
- * time of the sort's kernels in microseconds (0 unless am_cuda_profile(1) is on), and whether the
- * payload columns rode through the sort in row records (1) instead of a gather afterwards (0). */
+/* Per-call counters of the calling thread's last sort: rows, radix passes run and skipped (the digits that do not
+ * vary), the device time of the sort's kernels in microseconds (0 unless am_cuda_profile(1) is on), whether the
+ * payload columns rode through the sort in row records (1) instead of a gather afterwards (0), and the method:
+ * digit passes (0), two of them and then sorts of their buckets in shared memory (1), or buckets alone (2: no
+ * pass ran; the two counts are the key's digits that vary and that do not). */
 typedef struct am_sort_stats {
   int64_t rows;
   int64_t value_rows;
@@ -268,7 +270,7 @@ typedef struct am_sort_stats {
   int32_t passes_skipped;
   double  kernel_us;
   int32_t payload_in_records;
-  int32_t reserved;
+  int32_t method;
 } am_sort_stats;
 int  am_last_sort_stats(am_sort_stats* out);
 /* Kernel timing with CUDA events around every launch of this library (1 on, 0 off), and the

@@ -3,7 +3,7 @@ frame whose other columns are fixed-width, complete on the device, without nulls
 bytes a row moves each row's record (its id and payload) through the passes and unpacks it where the
 row reaches its final place, so no gather follows. The result must equal pyarrow's sort_indices + take
 (or the oracle's order at the large sizes), on every path the device can pick: one pass, several
-passes, the two-level sort's local sorts and its fallback passes; for 8- and 4-byte keys, floats in
+passes, the bucket sort, and (above 62,914,560 rows) the two-level sort's local sorts and its fallback passes; for 8- and 4-byte keys, floats in
 totalOrder, both directions and null placements, every payload layout, sliced columns. Frames that do
 not qualify take the gather and must give the same answer."""
 import numpy as np
@@ -135,7 +135,7 @@ def test_frames_that_take_the_gather(am, why):
     check(out, table, pc.sort_indices(table, [("k", "ascending")]).to_numpy())
 
 
-N_LARGE = 36_000_000        # 5% nulls leave more than 2^25 value rows: the two-level sort
+N_LARGE = 62_914_560 + 1000        # one key of more rows than the bucket sort takes: the two-level sort
 
 
 @pytest.mark.parametrize("case", ["local_sorts", "fallback_passes"])
@@ -149,6 +149,7 @@ def test_two_level_sort_with_records(am, oracle, case):
     for desc, nf in ((False, False), (True, True)):
         out, st = run(am, cols, "k", desc, nf)
         assert st["payload_in_records"] and st["passes_run"] == (2 if case == "local_sorts" else 2 + 5)
+        assert st["method"] == ("two_level" if case == "local_sorts" else "digit_passes")
         order = oracle.argsort(k, desc, "at_start" if nf else "at_end", threads=8)
         for name in ("p0", "p1"):
             want = cols[name].to_numpy()[order]

@@ -155,7 +155,13 @@ def test_stats_report_skipped_passes(am):
     st = am.last_sort_stats()
     assert st["rows"] == 1_000_000
     assert st["passes_run"] == 5 and st["passes_skipped"] == 3
+    assert st["method"] == "buckets"          # (of which the counts are the digits that vary and that do not)
     assert 880_000 < st["value_rows"] < 920_000
+    # A value that no bucket holds: the five passes run.
+    v = np.where(rng.random(1_000_000) < 0.2, 2**39, rng.integers(0, 2**40, 1_000_000))
+    am.MetalArray.from_arrow(pa.array(v)).argsort()
+    st = am.last_sort_stats()
+    assert st["passes_run"] == 5 and st["passes_skipped"] == 3 and st["method"] == "digit_passes"
 
 
 def test_chunked_import(am, oracle):
