@@ -57,8 +57,8 @@ constexpr int BINS1 = 1024;                       // level-1 bins
 constexpr int S2 = 8, BINS2 = 1 << S2;            // buckets a level-1 bin of a two-level sort
 static_assert(MAX_BUCKETS / BINS2 <= 256, "level-1 bins of a two-level sort");
 constexpr int CAP = 2048;                         // rows the shared-memory sort of a bucket (or a part of one) takes
-constexpr int BIG = 4096;                         // rows a bucket of strings may hold
-constexpr uint32_t LARGE = 16384;                 // rows a bucket of any other keys may hold: it is split by its CTA
+constexpr int BIG = 4096;                         // rows of one key whose strings differ that a bucket may hold
+constexpr uint32_t LARGE = 16384;                 // rows a bucket may hold at most: it is split by its CTA
 constexpr uint32_t TARGET = 1300;                 // rows a bucket of evenly spread keys is meant to hold
 // With cells, whose densities are estimates: four columns of 5.5M normally distributed float64 keys had
 // their largest bucket at 1,710-2,205 rows with 1,300, and one of more than CAP rows costs 100 us.
@@ -1622,9 +1622,20 @@ __device__ __forceinline__ void level2_body(const Args& a) {
 
 constexpr int TIES_ID = 0, TIES_STRING = 1;
 
-// Row a before row b, their keys being equal: by row id, or first by the strings behind them.
+// Row a before row b, their keys being equal: by row id, or first by the strings behind them, eight bytes at a time.
+// Of each string the first TIE_BYTES are looked at: where those of both agree and more follow, `far` says that the
+// derived keys must order the column (one CTA would compare them for as long as they are: 4,000 rows of a shared
+// 100 KB took 6e7 dependent reads a thread).
+constexpr uint64_t TIE_BYTES = 512;
+__device__ __forceinline__ uint64_t eight_bytes(const uint8_t* p) {          // big-endian, from any address; two aligned words
+  const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+  const uint64_t* w = reinterpret_cast<const uint64_t*>(at & ~uintptr_t(7));
+  const uint32_t sh = uint32_t(at & 7u) * 8u;
+  const uint64_t v = sh ? (w[0] >> sh) | (w[1] << (64 - sh)) : w[0];
+  return (uint64_t(__byte_perm(uint32_t(v), 0, 0x0123)) << 32) | __byte_perm(uint32_t(v >> 32), 0, 0x0123);
+}
 template <int TIES>
-__device__ __forceinline__ bool tied_before(const StringTies& s, uint32_t a, uint32_t b) {
+__device__ __forceinline__ bool tied_before(const StringTies& s, uint32_t a, uint32_t b, bool& far, bool strings_alone = false) {
   if constexpr (TIES == TIES_STRING) {
     uint64_t oa, ob, la, lb;
     if (s.wide) {
@@ -1640,14 +1651,27 @@ __device__ __forceinline__ bool tied_before(const StringTies& s, uint32_t a, uin
       la = uint64_t(uint32_t(o[a + 1ull])) - oa;
       lb = uint64_t(uint32_t(o[b + 1ull])) - ob;
     }
-    const uint64_t n = la < lb ? la : lb;
-    for (uint64_t i = *s.chars; i < n; i++) {
+    const uint64_t n = la < lb ? la : lb, end = n < TIE_BYTES ? n : TIE_BYTES;
+    uint64_t i = *s.chars;
+    // Whole eight bytes of both strings, then single ones (a string's last word could end past the column's bytes).
+    for (; i + 16 <= end; i += 8) {
+      const uint64_t x = eight_bytes(s.bytes + oa + i), y = eight_bytes(s.bytes + ob + i);
+      if (x != y) return (x < y) != (s.desc != 0);
+    }
+    for (; i < end; i++) {
       const uint8_t x = s.bytes[oa + i], y = s.bytes[ob + i];
       if (x != y) return (x < y) != (s.desc != 0);
     }
+    if (n > end) far = true;
     if (la != lb) return (la < lb) != (s.desc != 0);
+    if (strings_alone) return false;
   }
   return a < b;
+}
+
+// Two strings whose keys are equal are equal.
+__device__ __forceinline__ bool same_string(const StringTies& s, uint32_t a, uint32_t b, bool& far) {
+  return !tied_before<TIES_STRING>(s, a, b, far, true) && !tied_before<TIES_STRING>(s, b, a, far, true);
 }
 
 // What a CTA has at hand: a bucket of the map, or a part of a larger one (split_rows): rows whose positions
@@ -1662,12 +1686,7 @@ static_assert(3 * LARGE / PART_ROWS + 2 * CAP / (MAX_BIN + 1) + 9 * 4 <= PARTS, 
 constexpr uint32_t MAX_PAIRED = 8;                 // rows a bin may hold for comparisons, of the buckets put off
 constexpr uint32_t CROWD = MAX_PAIRED + 1;         // their crowded bins start at least so many rows apart
 
-// A CTA's shared memory: the fast form's arrays, or (strings) the slower one's keys and places of up to BIG rows.
-template <typename KeyT>
-struct SlowRows {
-  KeyT key[BIG];
-  uint16_t place[BIG];
-};
+// A CTA's shared memory.
 template <typename KeyT, int PAY, int TIES>
 struct FastShared {
   uint64_t full;                        // the bucket's records have arrived
@@ -1676,25 +1695,25 @@ struct FastShared {
   uint32_t some_fast;                   // some bucket of the CTA was ordered by the fast form
   union {
     struct {
-      union {
-        struct {
-          alignas(16) uint32_t start[BINS / 2 + 4];     // rows per bin, then where each bin starts: 16 bits each
-          uint64_t word[CAP];           // by bin: the row's position, and its id (strings: its place in the bucket) below it
-        };
-        struct {                        // in order:
-          KeyT key[CAP];
-          uint32_t id[PAY ? 1 : CAP];
-          uint16_t place[PAY ? CAP : 2];          // the row's place in the bucket
-        };
-      };
-      uint32_t in_id[TIES == TIES_STRING ? CAP : 1];      // the rows' ids, as they come
-      alignas(16) uint4 rec[PAY ? CAP : 1];     // the rows' records, as they come
+      alignas(16) uint32_t start[BINS / 2 + 4];     // rows per bin, then where each bin starts: 16 bits each
+      uint64_t word[CAP];               // by bin: the row's position, and its id (strings: its place in the bucket) below it
     };
-    std::conditional_t<TIES == TIES_STRING, SlowRows<KeyT>, uint32_t> slow;
+    struct {                            // in order:
+      KeyT key[CAP];
+      uint32_t id[PAY ? 1 : CAP];
+      uint16_t place[PAY ? CAP : 2];    // the row's place in the bucket
+    };
   };
+  uint32_t in_id[TIES == TIES_STRING ? CAP : 1];      // the rows' ids, as they come
+  alignas(16) uint4 rec[PAY ? CAP : 1]; // the rows' records, as they come
 };
-// The same of the buckets put off.
-template <typename KeyT, int PAY>
+// The same of the buckets put off; and the keys and places of up to BIG strings' rows, in a bitonic sort.
+template <typename KeyT>
+struct SlowRows {
+  KeyT key[BIG];
+  uint16_t place[BIG];
+};
+template <typename KeyT, int PAY, int TIES = TIES_ID>
 struct LaterShared {
   uint64_t full;
   uint32_t warp[32];
@@ -1706,14 +1725,19 @@ struct LaterShared {
   uint32_t run_at[PAY ? 1 : PARTS], run_n[PAY ? 1 : PARTS];
   union {
     struct {
-      alignas(16) uint32_t start[BINS + 4];       // rows per bin, then where each bin starts
-      uint32_t word[CAP];               // by bin: the row's position below its bin, then its place in the bucket
+      union {
+        struct {
+          alignas(16) uint32_t start[BINS + 4];   // rows per bin, then where each bin starts
+          uint32_t word[CAP];           // by bin: the row's position below its bin, then its place in the bucket
+        };
+        KeyT key[CAP];                  // in order
+      };
+      uint32_t id[PAY ? 1 : CAP];       // the rows' ids, as they come; then in order
+      uint16_t place[CAP];              // the words' bins; then, in order, the rows' places in the bucket
+      alignas(16) uint4 rec[PAY ? CAP : 1];       // the rows' records, as they come
     };
-    KeyT key[CAP];                      // in order
+    std::conditional_t<TIES == TIES_STRING, SlowRows<KeyT>, uint32_t> slow;
   };
-  uint32_t id[PAY ? 1 : CAP];           // the rows' ids, as they come; then in order
-  uint16_t place[CAP];                  // the words' bins; then, in order, the rows' places in the bucket
-  alignas(16) uint4 rec[PAY ? CAP : 1]; // the rows' records, as they come
 };
 
 // Read and written as 16-byte vectors, and by bulk copies.
@@ -1725,29 +1749,30 @@ static_assert(vectors_aligned<FastShared<uint32_t, 0, TIES_ID>>() && vectors_ali
               vectors_aligned<FastShared<uint32_t, 1, TIES_ID>>() && vectors_aligned<FastShared<uint64_t, 1, TIES_ID>>() &&
               vectors_aligned<FastShared<uint64_t, 0, TIES_STRING>>() && vectors_aligned<LaterShared<uint32_t, 0>>() &&
               vectors_aligned<LaterShared<uint64_t, 0>>() && vectors_aligned<LaterShared<uint32_t, 1>>() &&
-              vectors_aligned<LaterShared<uint64_t, 1>>(), "shared arrays read as vectors");
+              vectors_aligned<LaterShared<uint64_t, 1>>() && vectors_aligned<LaterShared<uint64_t, 0, TIES_STRING>>(), "shared arrays read as vectors");
 
-// A string bucket of more than CAP rows, or with many equal or very close keys: bitonic sort of (key, the
-// rest of the string, row id), the ids of equal keys read where the rows are.
+// Strings that differ behind many equal keys: bitonic sort of (key, the rest of the string, row id), the ids of
+// equal keys read where the rows are.
 template <int TIES, typename KeyT, typename IdOf>
 __device__ __forceinline__ void bitonic_rows(KeyT* key, uint16_t* place, uint32_t size, const KeyT* in, IdOf&& id_of,
-                                             const StringTies& ties) {
+                                             const StringTies& ties, bool& far) {
   uint32_t p = 2;
   while (p < size) p <<= 1;
-  for (uint32_t i = threadIdx.x; i < p; i += LTHREADS) {
+  for (uint32_t i = threadIdx.x; i < p; i += NTHREADS) {
     key[i] = i < size ? in[i] : KeyT(~KeyT(0));
     place[i] = uint16_t(i);             // places from `size` on come after every row
   }
   __syncthreads();
   for (uint32_t k = 2; k <= p; k <<= 1) {
+    if (__syncthreads_or(int(far))) return;          // the order is not used
     for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-      for (uint32_t q = threadIdx.x; q < p / 2; q += LTHREADS) {
+      for (uint32_t q = threadIdx.x; q < p / 2; q += NTHREADS) {
         const uint32_t i = 2 * q - (q & (j - 1)), l = i + j;
         const KeyT ki = key[i], kl = key[l];
         bool less = kl < ki;
         if (kl == ki) {
           const uint32_t pi = place[i], pl = place[l];
-          less = pl >= size ? false : pi >= size ? true : tied_before<TIES>(ties, id_of(pl), id_of(pi));
+          less = pl >= size ? false : pi >= size ? true : tied_before<TIES>(ties, id_of(pl), id_of(pi), far);
         }
         if (less == ((i & k) == 0)) {
           key[i] = kl;
@@ -1823,7 +1848,8 @@ __device__ __forceinline__ bool count_scan(SM& sm, uint32_t rows) {
 // is still too large is split again by its own, 2,048 times smaller range, so every split ends. One CTA does
 // it: the map's buckets are a thousand rows, and only a key repeated thousands of times makes a larger one.
 // Adds the parts to the list; returns their number. Leaves sm.start dirty.
-template <typename KeyT, int PAY, typename SM>
+constexpr uint32_t NOT_SPLIT = ~0u;                // strings of one key that differ
+template <typename KeyT, int PAY, int TIES, typename SM>
 __device__ __forceinline__ uint32_t split_rows(SM& sm, const Args& a, uint32_t first, uint32_t size, uint32_t side, uint32_t kind,
                                             uint32_t heavy, uint32_t run_at, uint32_t run_n, uint32_t parts) {
   const uint32_t t = threadIdx.x;
@@ -1852,6 +1878,12 @@ __device__ __forceinline__ uint32_t split_rows(SM& sm, const Args& a, uint32_t f
   const bool by_id = lo == hi;
   if (by_id) {
     if (kind != KIND_ID) {
+      if constexpr (TIES == TIES_STRING) {
+        bool differ = false, far = false;
+        for (uint32_t r = t; r < size && !far; r += NTHREADS) differ |= !same_string(a.ties, iin[r], iin[0], far);
+        if (far) a.st->mode = MODE_FALLBACK;
+        if (__syncthreads_or(int(differ || far))) return NOT_SPLIT;
+      }
       run_at = first;
       run_n = size;
     }
@@ -2255,10 +2287,10 @@ __device__ __forceinline__ bool write_rows(SM& sm, const Args& a, const KeyOut<K
 // The buckets that sort_body put off: those with bins of repeated keys, or of more rows than its form takes, which are
 // cut into parts. A launch of its own: within sort_body its registers cost every bucket (16M int64 keys that do not
 // repeat: the buckets' sort 149 us, 193 with this behind its loop, the next bucket's keys waited for to be spilled).
-template <typename KeyT, int PAY, bool FREQ = false>
+template <typename KeyT, int PAY, bool FREQ = false, int TIES = TIES_ID>
 __device__ __forceinline__ void later_body(const Args& a) {
   extern __shared__ __align__(16) unsigned char lsm[];
-  using SM = LaterShared<KeyT, PAY>;
+  using SM = LaterShared<KeyT, PAY, TIES>;
   SM& sm = *reinterpret_cast<SM*>(lsm);
   const State* st = a.st;
   const uint32_t count = st->later;
@@ -2268,6 +2300,21 @@ __device__ __forceinline__ void later_body(const Args& a) {
   const KeyOut<KeyT> ko(a);
   if (PAY && t == 0) mbar_init(&sm.full);
   uint32_t parts = 0, turn = blockIdx.x, parity = 0;
+  // Rows whose strings differ behind equal keys.
+  auto by_strings = [&](uint32_t first, uint32_t size, uint32_t side) {
+    if constexpr (TIES == TIES_STRING) {
+      const uint32_t* iin = a.ids[side] + first;
+      bool far = size > uint32_t(BIG);
+      if (!far) {
+        __syncthreads();
+        bitonic_rows<TIES>(sm.slow.key, sm.slow.place, size, static_cast<const KeyT*>(a.keys[side]) + first,
+                           [&](uint32_t p) { return iin[p]; }, a.ties, far);
+        far = __syncthreads_or(int(far)) != 0;     // (the sort then ended early: its places are in no order)
+        for (uint32_t r = t; r < size && !far; r += NTHREADS) store_id(a, vbase + first + r, iin[sm.slow.place[r]]);
+      }
+      if (far) a.st->mode = MODE_FALLBACK;
+    }
+  };
   for (;;) {
     __syncthreads();                               // the last part's memory, and its place in the list, are free
     uint32_t first, size, side, kind, run_at = 0, run_n = 0;
@@ -2368,6 +2415,17 @@ __device__ __forceinline__ void later_body(const Args& a) {
       if (PAY) parity ^= 1u;
       if (tied != TIED_SPLIT) {
         __syncthreads();
+        if constexpr (TIES == TIES_STRING) {
+          // Equal keys are in row order: right where their strings are equal (a part of one key's rows was looked at whole).
+          bool differ = false, far = false;
+          for (uint32_t r = t + 1; r < size && kind != KIND_ID && !far; r += NTHREADS)
+            if (sm.key[r] == sm.key[r - 1]) differ |= !same_string(a.ties, sm.id[r], sm.id[r - 1], far);
+          if (far) a.st->mode = MODE_FALLBACK;
+          if (__syncthreads_or(int(differ || far))) {
+            by_strings(first, size, side);
+            continue;
+          }
+        }
         const uint64_t base = kind == KIND_ID ? vbase : 0ull;
         if (!write_rows<KeyT, PAY, FREQ, NTHREADS, true>(sm, a, ko, vbase + first, size, nkeys, parity ^ (PAY ? 1u : 0u), base + (kind == KIND_ID ? run_at : 0u),
                                                base + (kind == KIND_ID ? run_at + run_n : 0u)))
@@ -2376,7 +2434,9 @@ __device__ __forceinline__ void later_body(const Args& a) {
       }
       heavy = MAX_BIN;
     }
-    parts = split_rows<KeyT, PAY>(sm, a, first, size, side, kind, heavy, run_at, run_n, parts);
+    const uint32_t split = split_rows<KeyT, PAY, TIES>(sm, a, first, size, side, kind, heavy, run_at, run_n, parts);
+    if (TIES == TIES_STRING && split == NOT_SPLIT) by_strings(first, size, side);
+    else parts = split;
   }
 }
 
@@ -2444,6 +2504,7 @@ __device__ __forceinline__ void sort_body(const Args& a) {
   for (int x = t; x < BINS / 2; x += LTHREADS) sm.start[x] = 0;
   __syncthreads();
   uint32_t b = next_bucket(blockIdx.x), parity = 0;
+  bool far = false;                                // strings that agree for longer than a tie looks
   if (b < nb) {
     load_rows();
     if (t == 0) load_records();
@@ -2555,7 +2616,7 @@ __device__ __forceinline__ void sort_body(const Args& a) {
               if constexpr (TIES == TIES_STRING) {
                 if (uint32_t(o >> 32) == pos[i] && o != me) {
                   const KeyT k = kin[uint32_t(o)];
-                  rank += k < key[i] || (k == key[i] && tied_before<TIES>(a.ties, sm.in_id[uint32_t(o)], id[PAY ? 0 : i])) ? 1u : 0u;
+                  rank += k < key[i] || (k == key[i] && tied_before<TIES>(a.ties, sm.in_id[uint32_t(o)], id[PAY ? 0 : i], far)) ? 1u : 0u;
                   continue;
                 }
               } else {
@@ -2589,9 +2650,6 @@ __device__ __forceinline__ void sort_body(const Args& a) {
     if (fast) {
       if (t == 0) sm.some_fast = 1;
       if (!write_rows<KeyT, PAY, FREQ, LTHREADS>(sm, a, ko, dst0, rows, nkeys, parity)) return;
-    } else if constexpr (TIES == TIES_STRING) {
-      bitonic_rows<TIES>(sm.slow.key, sm.slow.place, rows, kin, [&](uint32_t p) { return iin[p]; }, a.ties);
-      for (uint32_t r = t; r < rows; r += LTHREADS) store_id(a, dst0 + r, iin[sm.slow.place[r]]);
     } else {
       // Left to later_body; in a column of repeated keys, where neither of the CTA's first two buckets was fast,
       // with all of the CTA's that follow.
@@ -2618,6 +2676,7 @@ __device__ __forceinline__ void sort_body(const Args& a) {
     }
     __syncthreads();
   }
+  if (TIES == TIES_STRING && far) a.st->mode = MODE_FALLBACK;
 }
 
 // ---- the launches: of one sort, and of a batch's sorts (one a row of the grid)
@@ -2648,9 +2707,9 @@ template <typename KeyT, int PAY, int TIES, bool FREQ>
 __global__ void __launch_bounds__(LTHREADS, LBLOCKS) bucket_sort_kernel(const __grid_constant__ Args a) {
   sort_body<KeyT, PAY, TIES, FREQ>(a);
 }
-template <typename KeyT, int PAY, bool FREQ>
+template <typename KeyT, int PAY, bool FREQ, int TIES>
 __global__ void __launch_bounds__(NTHREADS, NBLOCKS) bucket_later_kernel(const __grid_constant__ Args a) {
-  later_body<KeyT, PAY, FREQ>(a);
+  later_body<KeyT, PAY, FREQ, TIES>(a);
 }
 
 struct alignas(16) BatchItem {
@@ -2922,7 +2981,7 @@ void launch_moves(const ColView& cv, const Args& a, cudaStream_t s) {
     smem_limit(level1_kernel<KeyT, PAY, FREQ>, sizeof(TileShared<KeyT, PAY>));
     smem_limit(level2_kernel<KeyT, PAY>, sizeof(Tile2Shared<KeyT, PAY>));
     smem_limit(bucket_sort_kernel<KeyT, PAY, TIES, FREQ>, sizeof(FastShared<KeyT, PAY, TIES>));
-    if constexpr (TIES == TIES_ID) smem_limit(bucket_later_kernel<KeyT, PAY, FREQ>, sizeof(LaterShared<KeyT, PAY>));
+    smem_limit(bucket_later_kernel<KeyT, PAY, FREQ, TIES>, sizeof(LaterShared<KeyT, PAY, TIES>));
   });
   if (!a.one_launch) {
     {
@@ -2941,9 +3000,9 @@ void launch_moves(const ColView& cv, const Args& a, cudaStream_t s) {
     bucket_sort_kernel<KeyT, PAY, TIES, FREQ><<<a.sort_grid, LTHREADS, sizeof(FastShared<KeyT, PAY, TIES>), s>>>(a);
     AM_CUDA(cudaGetLastError());
   }
-  if constexpr (TIES == TIES_ID) {
+  {
     KernelTimer kt("bucket_later", s);
-    bucket_later_kernel<KeyT, PAY, FREQ><<<a.later_grid, NTHREADS, sizeof(LaterShared<KeyT, PAY>), s>>>(a);
+    bucket_later_kernel<KeyT, PAY, FREQ, TIES><<<a.later_grid, NTHREADS, sizeof(LaterShared<KeyT, PAY, TIES>), s>>>(a);
     AM_CUDA(cudaGetLastError());
   }
 }
@@ -3067,7 +3126,7 @@ static Args make_args(const Sort& b) {
   a.sum = b.summary;
   if (b.payload) a.pay = b.rec;
   a.bins1_cap = b.payload ? BINS1 / 2 : BINS1;
-  a.large = b.ties.offsets ? uint32_t(BIG) : b.src_ids ? LARGE : large_rows(b.n);
+  a.large = b.src_ids ? LARGE : large_rows(b.n);
   a.has_payload = b.payload ? 1 : 0;
   a.one_launch = b.n <= SAMPLES ? 1 : 0;
   a.frequent = b.frequent && !a.one_launch && !b.payload && !b.key_out && !b.ranks.out && !b.ties.offsets && !b.src_ids && b.key_bytes == 8 ? 1 : 0;

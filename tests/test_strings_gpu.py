@@ -229,3 +229,21 @@ def test_string_order_by_buckets(am, n, kind):
             for desc, place in ((False, "at_end"), (True, "at_start")):
                 want = pc.sort_indices(pa.table({"s": part}), [("s", "descending" if desc else "ascending")], null_placement=place)
                 assert np.array_equal(m.argsort(desc, place).to_arrow().to_numpy(), want.to_numpy()), (typ, desc)
+
+
+@pytest.mark.parametrize("shared", [13, 90, 511, 512, 513, 4000])
+def test_strings_that_agree_far_past_their_key(am, shared):
+    # Rows of one 8-byte key: their ties compare eight bytes at a time, and past 512 bytes the derived keys order
+    # the column. Tails of every length (and none), equal strings, other strings around them, both directions.
+    rng = np.random.default_rng(shared)
+    head = "".join(rng.choice(list("abcdefgh"), shared))
+    rows = []
+    for i in range(3500):
+        tail = "".join(rng.choice(list("abc"), int(rng.integers(0, 12))))
+        rows.append(head + tail if i % 4 else "".join(rng.choice(list("abcdefgh"), int(rng.integers(0, 30)))))
+    for kind in (pa.utf8(), pa.large_utf8()):
+        arr = pa.array(rows, kind)
+        for desc in (False, True):
+            want = pc.array_sort_indices(arr, order="descending" if desc else "ascending").to_numpy()
+            got = am.MetalArray.from_arrow(arr.slice(0)).argsort(desc).to_arrow().to_numpy()
+            assert np.array_equal(got, want), (kind, desc)
