@@ -97,7 +97,7 @@ struct Args {
   uint32_t hist_grid, level2_grid, sort_grid, later_grid;     // CTAs that take part in those steps
   uint64_t n;
   void* keys[2];
-  uint32_t* ids[2];
+  uint32_t* ids[2];                               // NULL: no row ids (a sorted copy of an invertible key alone)
   uint4* rec[2];                                  // with a payload: row id and payload fields (RecLayout), instead of ids
   void *out, *key_out;
   uint4* clear;                                   // not NULL: memory that the plan's launch clears, the state among it
@@ -952,7 +952,7 @@ __device__ __forceinline__ void buckets_body(const ColView& col, const Args& a) 
         if (dst < values) {
           static_cast<KeyT*>(a.keys[0])[dst] = key[u];
           if (a.has_payload) a.rec[0][dst] = build_record(a.pay, row);
-          else a.ids[0][dst] = a.src_ids ? a.src_ids[row] : row;
+          else if (a.ids[0]) a.ids[0][dst] = a.src_ids ? a.src_ids[row] : row;
         } else {
           atomicOr(a.err, ERR_BOUNDS);
         }
@@ -1453,7 +1453,8 @@ __device__ __forceinline__ void level1_body(const ColView& col, const Args& a) {
         continue;
       }
       kout[dst] = sm.key[j];
-      if constexpr (!PAY) iout[dst] = uint32_t(tile) + (word & 0xFFFFu);
+      if constexpr (!PAY)
+        if (iout) iout[dst] = uint32_t(tile) + (word & 0xFFFFu);
     }
     for (uint32_t j = tile_n + t; j < tile_n + tn + tx; j += THREADS) {
       const uint32_t q = j - tile_n, row = uint32_t(tile) + sm.word[j];
@@ -1557,7 +1558,7 @@ __device__ __forceinline__ void level2_body(const Args& a) {
     const RecT* rp = rin + row0 + t;
 #pragma unroll
     for (int i = 0; i < ITEMS; i++) {
-      if (i >= ni) break;
+      if (i >= ni || !rin) break;
       rec[i] = rp[i * THREADS];
     }
     __syncthreads();
@@ -1587,7 +1588,7 @@ __device__ __forceinline__ void level2_body(const Args& a) {
       if (i >= ni) break;
       const uint32_t b = slot[i] >> 16, pos = sm.start[b] + (slot[i] & 0xFFFFu);
       sm.key[pos] = key[i];
-      sm.rec[pos] = rec[i];
+      if (rin) sm.rec[pos] = rec[i];
       sm.bin[pos] = uint8_t(b);
     }
     if (q + 1 < t1) load(q + 1);
@@ -1611,7 +1612,8 @@ __device__ __forceinline__ void level2_body(const Args& a) {
         continue;
       }
       kout[dst] = sm.key[j];
-      if constexpr (!PAY) rout[dst] = sm.rec[j];
+      if constexpr (!PAY)
+        if (rin) rout[dst] = sm.rec[j];
     }
     __syncthreads();
   }
@@ -1855,8 +1857,9 @@ __device__ __forceinline__ uint32_t split_rows(SM& sm, const Args& a, uint32_t f
   const uint32_t t = threadIdx.x;
   const KeyT* kin = static_cast<const KeyT*>(a.keys[side]) + first;
   KeyT* kout = static_cast<KeyT*>(a.keys[side ^ 1u]) + first;
-  const uint32_t* iin = a.ids[side] + first;
-  uint32_t* iout = a.ids[side ^ 1u] + first;
+  const bool ids = PAY || a.ids[0];              // else the rows' places stand in for them
+  const uint32_t* iin = ids ? a.ids[side] + first : nullptr;
+  uint32_t* iout = ids ? a.ids[side ^ 1u] + first : nullptr;
   const uint4* rin = a.rec[side] + first;
   uint4* rout = a.rec[side ^ 1u] + first;
   constexpr uint32_t U = 4, STEP = U * NTHREADS;
@@ -1867,7 +1870,7 @@ __device__ __forceinline__ uint32_t split_rows(SM& sm, const Args& a, uint32_t f
     for (uint32_t u = 0; u < U; u++)
       if (r0 + u * NTHREADS < size) {
         const uint64_t k = kin[r0 + u * NTHREADS];
-        const uint32_t id = PAY ? rin[r0 + u * NTHREADS].x : iin[r0 + u * NTHREADS];
+        const uint32_t id = PAY ? rin[r0 + u * NTHREADS].x : ids ? iin[r0 + u * NTHREADS] : r0 + u * NTHREADS;
         lo = min(lo, k);
         hi = max(hi, k);
         id0 = min(id0, id);
@@ -1892,7 +1895,7 @@ __device__ __forceinline__ uint32_t split_rows(SM& sm, const Args& a, uint32_t f
   }
   const uint32_t sh = range_shift(hi - lo);
   auto bin_of = [&](uint64_t x) { return uint32_t(((x - lo) << sh) >> (64 - BINS_LOG)); };
-  auto axis = [&](uint32_t r) { return by_id ? uint64_t(PAY ? rin[r].x : iin[r]) : uint64_t(kin[r]); };
+  auto axis = [&](uint32_t r) { return by_id ? uint64_t(PAY ? rin[r].x : ids ? iin[r] : r) : uint64_t(kin[r]); };
   for (uint32_t x = t; x < BINS; x += NTHREADS) sm.start[x] = 0;
   __syncthreads();
   for (uint32_t r0 = t; r0 < size; r0 += STEP) {
@@ -1953,7 +1956,7 @@ __device__ __forceinline__ uint32_t split_rows(SM& sm, const Args& a, uint32_t f
       if (r0 + u * NTHREADS < size) {
         k[u] = kin[r0 + u * NTHREADS];
         if constexpr (PAY) rec[u] = rin[r0 + u * NTHREADS];
-        else id[u] = iin[r0 + u * NTHREADS];
+        else id[u] = ids ? iin[r0 + u * NTHREADS] : r0 + u * NTHREADS;
       }
 #pragma unroll
     for (uint32_t u = 0; u < U; u++)
@@ -1964,7 +1967,7 @@ __device__ __forceinline__ uint32_t split_rows(SM& sm, const Args& a, uint32_t f
         const uint32_t p = atomicAdd(&sm.word[bin_of(by_id ? uint64_t(row) : uint64_t(k[u]))], 1u);
         kout[p] = k[u];
         if constexpr (PAY) rout[p] = rec[u];
-        else iout[p] = id[u];
+        else if (ids) iout[p] = id[u];
       }
   }
   // The parts' records come by bulk copies.
@@ -2359,7 +2362,8 @@ __device__ __forceinline__ void later_body(const Args& a) {
 #pragma unroll
       for (int i = 0; i < NITEMS; i++) {
         if (i >= ni) break;
-        const uint32_t id = PAY ? a.rec[side][first + t + i * NTHREADS].x : a.ids[side][first + t + i * NTHREADS];
+        const uint32_t id = PAY ? a.rec[side][first + t + i * NTHREADS].x
+                                : a.ids[0] ? a.ids[side][first + t + i * NTHREADS] : t + i * NTHREADS;
         if constexpr (!PAY) sm.id[t + i * NTHREADS] = id;
         id0 = min(id0, id);
         id1 = max(id1, id);
@@ -2369,8 +2373,9 @@ __device__ __forceinline__ void later_body(const Args& a) {
         const uint32_t b = a.later[turn], nf = a.bpos[b], nn = a.bpos[b + 1] - nf;
         const char* k0 = reinterpret_cast<const char*>(static_cast<const KeyT*>(a.keys[src]) + nf);
         const char* i0 = PAY ? reinterpret_cast<const char*>(a.rec[src] + nf) : reinterpret_cast<const char*>(a.ids[src] + nf);
+        const uint32_t ib = PAY ? 16u : a.ids[0] ? 4u : 0u;
         for (uint32_t x = t * 128u; x < nn * uint32_t(sizeof(KeyT)); x += NTHREADS * 128u) asm volatile("prefetch.global.L2 [%0];" ::"l"(k0 + x));
-        for (uint32_t x = t * 128u; x < nn * (PAY ? 16u : 4u); x += NTHREADS * 128u) asm volatile("prefetch.global.L2 [%0];" ::"l"(i0 + x));
+        for (uint32_t x = t * 128u; x < nn * ib; x += NTHREADS * 128u) asm volatile("prefetch.global.L2 [%0];" ::"l"(i0 + x));
       }
       for (uint32_t x = t; x < BINS; x += NTHREADS) sm.start[x] = 0;
       if (t <= CAP / CROWD) sm.mixed[t] = 0;
@@ -2513,7 +2518,7 @@ __device__ __forceinline__ void sort_body(const Args& a) {
     const uint32_t rows = size, row0 = first;
     const int ni = nit;
     const KeyT* kin = static_cast<const KeyT*>(a.keys[src]) + row0;
-    const uint32_t* iin = a.ids[src] + row0;
+    const uint32_t* iin = a.ids[src] ? a.ids[src] + row0 : nullptr;        // NULL: places stand in for the ids
     const uint64_t dst0 = vbase + row0;
     if (dst0 + rows > a.n || rows > a.large) {             // the scan rules both out
       if (t == 0) atomicOr(a.err, ERR_BOUNDS);
@@ -2529,7 +2534,7 @@ __device__ __forceinline__ void sort_body(const Args& a) {
 #pragma unroll
         for (int i = 0; i < LITEMS; i++) {
           if (i >= ni) break;
-          id[i] = iin[t + i * LTHREADS];
+          id[i] = iin ? iin[t + i * LTHREADS] : t + i * LTHREADS;
         }
       }
       // A row's position in the bucket's key range, as 32 bits: in a split cell the part of

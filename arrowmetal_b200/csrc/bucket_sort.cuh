@@ -69,7 +69,7 @@ struct Sort {
   void* clear;                           // not NULL: `clear_bytes` (a multiple of 16) that the sort itself clears first
   size_t clear_bytes;
   void* keys[2];                         // n keys each
-  char* ids[2];                          // n x 4 bytes, or n x 16 with a payload
+  char* ids[2];                          // n x 4 bytes, or n x 16 with a payload; NULL: the sorted key column alone is wanted
   StringTies ties;
   RankOut ranks;
   bool payload;

@@ -2124,7 +2124,9 @@ static void sort_by_buckets(const SortKey& key, const rs::PlanArgs& pa, uint64_t
   const size_t off_bs = up(off_sum + sizeof(SortSummary));
   const size_t off_keys = up(off_bs + bs::scratch_bytes(n));
   const size_t kbuf = up(n * size_t(kb));
-  const size_t ibuf = up(payload ? n * sizeof(uint4) : n * sizeof(uint32_t));
+  // A sorted copy of an invertible key alone moves keys alone.
+  const bool with_ids = carry_ids || !key_invertible(key);
+  const size_t ibuf = with_ids ? up(payload ? n * sizeof(uint4) : n * sizeof(uint32_t)) : 0;
   ScratchBlock scratch(s, off_keys + 2 * kbuf + 2 * ibuf);
   char* base = scratch.data();
   if (key_dst) alloc_key_column(key_dst, key, n, s);
@@ -2148,7 +2150,7 @@ static void sort_by_buckets(const SortKey& key, const rs::PlanArgs& pa, uint64_t
   b.wide = index_width == 8;
   for (int i = 0; i < 2; i++) {
     b.keys[i] = base + off_keys + size_t(i) * kbuf;
-    b.ids[i] = base + off_keys + 2 * kbuf + size_t(i) * ibuf;
+    b.ids[i] = with_ids ? base + off_keys + 2 * kbuf + size_t(i) * ibuf : nullptr;
   }
   if (key_dst) b.key_out = key_dst->values->ptr;
   b.key_pt = key.col->pt;

@@ -180,3 +180,23 @@ def test_empty_and_all_null(am):
     z = am.MetalArray.from_arrow(pa.array([None] * 5000, type=pa.float64()))
     assert ids(z.argsort()).tolist() == list(range(5000))
     assert ids(z.argsort(True, "at_start")).tolist() == list(range(5000))
+
+
+def test_a_sorted_copy_moves_keys_alone():
+    # Its scratch is two buffers of keys beside the copy, and no row ids: 8 + 2 x 8 bytes a row, not 8 more.
+    import subprocess
+    import sys
+    code = """
+import numpy as np, pyarrow as pa, torch
+import arrowmetal_b200 as am
+n = 30_000_000
+m = am.MetalArray.from_arrow(pa.array(np.random.default_rng(1).integers(0, 2**40, n)))
+am.synchronize()
+before = torch.cuda.mem_get_info()[0]
+s = m.sort()
+am.synchronize()
+used = before - torch.cuda.mem_get_info()[0]
+assert np.array_equal(s.to_arrow().to_numpy(), np.sort(m.to_arrow().to_numpy()))
+assert used < 28 * n, used / n
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=300)
