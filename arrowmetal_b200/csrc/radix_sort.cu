@@ -3204,9 +3204,11 @@ void sort_segment_group(const std::vector<SortKey>& keys, const std::vector<void
       cudaEvent_t e0, e1;
       AM_CUDA(cudaEventCreate(&e0));
       AM_CUDA(cudaEventCreate(&e1));
+      // The first large scratch grows the pool: not in the first candidate's time.
+      dfree(dmalloc(size_t(cls_rows[c]) * 2 * (sizeof(KeyT) + 4), s), s);
       for (size_t k = 0; k < cand.size(); k++) {
-        // Once before: the first run of a shape loads its kernels and grows the scratch.
-        run_segment_shape<KeyT>(cand[k], keys, outs, cls[c], false, s);
+        // One array before: the first run of a shape loads its kernels.
+        run_segment_shape<KeyT>(cand[k], keys, outs, {cls[c].front()}, false, s);
         AM_CUDA(cudaEventRecord(e0, s));
         run_segment_shape<KeyT>(cand[k], keys, outs, cls[c], false, s);
         AM_CUDA(cudaEventRecord(e1, s));
