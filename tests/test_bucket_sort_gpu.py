@@ -77,11 +77,13 @@ def test_sliced_columns(am, oracle, offset):
     assert np.array_equal(m.argsort().to_arrow().to_numpy(), oracle.argsort(part))
 
 
-def test_concurrent_threads(am, oracle):
-    # Each thread sorts on its own stream, with its own scratch.
+@pytest.mark.parametrize("kind", ["normal", "one_value", "repeats"])
+def test_concurrent_threads(am, oracle, kind):
+    # Each thread sorts on its own stream, with its own scratch: by buckets, by the digit passes of one launch behind
+    # them (with barriers over the grid), and by buckets of repeated keys.
     import threading
     rng = np.random.default_rng(3)
-    arrays = [pa.array(rng.standard_normal(300_000 + 1000 * i)) for i in range(4)]
+    arrays = [pa.array(keys(kind, 300_000 + 1000 * i, rng), from_pandas=False) for i in range(4)]
     want = [oracle.argsort(a) for a in arrays]
     bad = []
 
@@ -97,6 +99,62 @@ def test_concurrent_threads(am, oracle):
     for t in threads:
         t.join()
     assert not bad
+
+
+def sampled_rows(n):
+    """The rows that a sort of more than 65,536 looks at first: one of each 65,536th part, at a mixed offset."""
+    j = np.arange(65_536, dtype=np.uint64)
+    lo, hi = j * n // 65_536, (j + 1) * n // 65_536
+    mask = np.uint64(0xFFFFFFFF)
+    h = (j * 2654435761) & mask
+    h ^= h >> np.uint64(15)
+    h = (h * 2246822519) & mask
+    h ^= h >> np.uint64(13)
+    return (lo + ((h * (hi - lo)) >> np.uint64(32))).astype(np.int64)
+
+
+@pytest.mark.parametrize("n", [70_001, 1_000_003, 5_000_011])
+@pytest.mark.parametrize("kind", ["sorted", "reversed", "pipe", "stride", "sample_apart", "sample_below"])
+def test_orders_that_mislead_the_sample(am, oracle, n, kind):
+    # Columns already in order, periods of the sample's stride, and rows that lie outside the sampled keys' range
+    # (all of them beside one key, or all above it).
+    rng = np.random.default_rng(n)
+    v = rng.integers(0, 2**40, n)
+    if kind == "sorted":
+        v = np.sort(v)
+    elif kind == "reversed":
+        v = np.sort(v)[::-1].copy()
+    elif kind == "pipe":
+        v = np.abs(np.arange(n) - n // 2) * 2**18
+    elif kind == "stride":
+        v = (np.arange(n) % max(2, n // 65_536)) * 2**30 + rng.integers(0, 2**20, n)
+    elif kind == "sample_apart":
+        v[sampled_rows(n)] = 2**39 + rng.integers(0, 50, 65_536)
+    else:
+        v += 2**41
+        v[sampled_rows(n)] = rng.integers(0, 2**30, 65_536)
+    arr = pa.array(v)
+    m = am.MetalArray.from_arrow(arr)
+    for desc in (False, True):
+        want = oracle.argsort(arr, desc, threads=4)
+        assert np.array_equal(m.argsort(desc).to_arrow().to_numpy(), want)
+        assert np.array_equal(m.sort(desc).to_arrow().to_numpy(), v[want])
+
+
+@pytest.mark.parametrize("n", [10_000_019, 1 << 24, (1 << 24) + 1])
+def test_ranks_of_large_columns(am, oracle, n):
+    # Both sides of the rows up to which ranks leave the buckets.
+    rng = np.random.default_rng(n)
+    v = rng.integers(0, 2**40, n) if n % 2 else rng.integers(0, n // 50, n) * 7919
+    arr = pa.array(v)
+    order = oracle.argsort(arr, threads=8)
+    key = v[order]
+    start = np.ones(n, bool)
+    start[1:] = key[1:] != key[:-1]
+    first = np.flatnonzero(start)[np.cumsum(start) - 1]
+    ranks = np.empty(n, np.int64)
+    ranks[order] = first + 1
+    assert np.array_equal(am.MetalArray.from_arrow(arr).rank().to_arrow().to_numpy(), ranks)
 
 
 @pytest.mark.parametrize("kind,order", [("normal", "ieee"), ("normal32", "nan_largest"), ("normal32", "ieee"), ("one_value", "ieee")])
