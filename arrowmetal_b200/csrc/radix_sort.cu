@@ -2756,9 +2756,15 @@ GraphCache& graph_cache() {
 // Graphs are captured on a stream of the thread's own: on the sort's stream other threads free the arrays of
 // earlier results meanwhile, which a capturing stream refuses.
 cudaStream_t capture_stream() {
-  static thread_local cudaStream_t c = nullptr;
-  if (!c) AM_CUDA(cudaStreamCreateWithFlags(&c, cudaStreamNonBlocking));
-  return c;
+  struct Own {
+    cudaStream_t s = nullptr;
+    ~Own() {
+      if (s) (void)cudaStreamDestroy(s);
+    }
+  };
+  static thread_local Own own;
+  if (!own.s) AM_CUDA(cudaStreamCreateWithFlags(&own.s, cudaStreamNonBlocking));
+  return own.s;
 }
 
 bool graphs_enabled() {
