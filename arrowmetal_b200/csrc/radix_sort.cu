@@ -1838,6 +1838,7 @@ template <> struct PassConfig<uint64_t> { static constexpr int THREADS = 512, IT
 constexpr int HIST_THREADS = 256, HIST_ITEMS = 8;
 constexpr int MAX_ONE_KEY = 8;        // digit passes of one key
 constexpr uint64_t COUNT_APART_ROWS = uint64_t(1) << 23;
+constexpr uint64_t LAST_KEY_ROWS = uint64_t(1) << 21;      // of a lexsort, see radix_sort
 // Ranks leave the bucket sort as random 4-byte stores: while the whole rank column (64 MB here) stays in L2.
 // 8M int64 keys with nulls, min: 867 us by an order, run marks and a scatter, 342 so.
 constexpr uint64_t RANK_BUCKET_ROWS = uint64_t(1) << 24;
@@ -2376,12 +2377,12 @@ void radix_sort(const std::vector<SortKey>& keys_in, int64_t n64, void* out, int
   const size_t header = (off_sum + sizeof(SortSummary) + 255) & ~size_t(255);
   const size_t kbuf = ((n * max_kb) + 255) & ~size_t(255);
   const size_t ibuf = carry_ids ? ((n * id_bytes) + 255) & ~size_t(255) : 0;
-  // A lexsort's last key by buckets, the digit passes of the other keys from its order on: for 8-byte keys,
-  // of which eight digits can vary. After a key of 200 values, by passes and so: float64 1,804 and 1,160 us
-  // at 16M rows, 282 and 242 at 1M, 189 and 164 at 2,000; 40-bit int64 1,343 and 998, 236 and 220, 160 and
-  // 160. A last key that no bucket holds pays for the try: 896 and 977 at 16M, 124 and 190 at 2,000. Four
-  // passes of a 4-byte key cost about what its buckets do (1,105 and 919; 189 and 187; 131 and 133).
-  const bool last_first = K > 1 && pt_key_bytes(keys[K - 1].col->pt) == 8 && n <= bs::MAX_ROWS && !debug_skip_first_tile();
+  // A lexsort's last key by buckets, the digit passes of the other keys from its order on: for 8-byte keys of many
+  // rows, of which eight digits can vary. After a key of 200 values, by passes and so: float64 1,803 and 1,136 us at 16M
+  // rows; 40-bit int64 1,336 and 991. At 1M rows 271 and 248, 228 and 219, and where the last key repeats
+  // the passes are faster (30,000 rows a value 264 and 343, 222 and 297; at 2,003 rows 99 and 160): few rows are left to them. At 16M a last
+  // key of 500 rows a value costs 1,784 and 1,485, 1,327 and 1,412. Four passes of a 4-byte key cost about what its buckets do.
+  const bool last_first = K > 1 && pt_key_bytes(keys[K - 1].col->pt) == 8 && n >= LAST_KEY_ROWS && n <= bs::MAX_ROWS && !debug_skip_first_tile();
   const size_t off_order = header + 2 * kbuf + 2 * ibuf;
   const size_t off_bs = off_order + ibuf;
   ScratchBlock scratch(s, last_first ? off_bs + bs::scratch_bytes(n) : off_order);
