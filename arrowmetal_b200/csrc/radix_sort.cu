@@ -1839,9 +1839,6 @@ constexpr int HIST_THREADS = 256, HIST_ITEMS = 8;
 constexpr int MAX_ONE_KEY = 8;        // digit passes of one key
 constexpr uint64_t COUNT_APART_ROWS = uint64_t(1) << 23;
 constexpr uint64_t LAST_KEY_ROWS = uint64_t(1) << 21;      // of a lexsort, see radix_sort
-// Ranks leave the bucket sort as random 4-byte stores: while the whole rank column (64 MB here) stays in L2.
-// 8M int64 keys with nulls, min: 867 us by an order, run marks and a scatter, 342 so.
-constexpr uint64_t RANK_BUCKET_ROWS = uint64_t(1) << 24;
 
 template <typename KeyT, int ITEMS = PassConfig<KeyT>::ITEMS, int THREADS = PassConfig<KeyT>::THREADS, bool REC = false>
 static size_t pass_smem() {
@@ -2213,11 +2210,13 @@ static void sort_by_buckets(const SortKey& key, const rs::PlanArgs& pa, uint64_t
   finish_sort(key, n, key_dst, sum, payload != nullptr, stats, s);
 }
 
+// Ranks leave the bucket sort as random 4-byte stores, and still take less than an order, run marks and a scatter
+// where the rank column is larger than L2: int64 min, 8M rows 867 and 342 us, 20M 1,399 and 693, 50M 4,322 and 2,662.
 bool rank_by_buckets(const SortKey& key, int64_t n64, int fn, bool merge_nan, uint32_t* ranks, uint32_t* perm, uint32_t* mode,
                      cudaStream_t s) {
   using namespace rs;
   const uint64_t n = uint64_t(n64);
-  if (n == 0 || n > RANK_BUCKET_ROWS || pt_var(key.col->pt) || key.col->dictionary || few_digits(key, n) || debug_skip_first_tile()) return false;
+  if (n == 0 || n > bs::MAX_ROWS || pt_var(key.col->pt) || key.col->dictionary || few_digits(key, n) || debug_skip_first_tile()) return false;
   if (fn != RANK_MIN && fn != RANK_MAX && fn != RANK_FIRST) return false;
   PlanArgs pa{};
   const int kb = pt_key_bytes(key.col->pt);
