@@ -1328,7 +1328,7 @@ __global__ void __launch_bounds__(256) key_validity_kernel(const SortSummary* __
 // ------------------------------------------------------------------------------------------------
 // The large single-key sort: two passes on the top digits, then local sorts in shared memory.
 //
-// One 8-byte key over at least 2^25 value rows with three or more active digits. Two onesweep passes
+// One 8-byte key of more rows than the bucket sort takes, with three or more active digits. Two onesweep passes
 // on the two highest active digits (the lower of them first: LSD order) leave the value rows grouped
 // by those digits -- at most 65,536 buckets, a few hundred rows each at the benchmark's size -- with
 // every bucket in row order. Each bucket is then sorted by the remaining active digits inside one
@@ -2359,7 +2359,7 @@ void radix_sort(const std::vector<SortKey>& keys_in, int64_t n64, void* out, int
 
   // Per-call scratch: stats, plans, pass descriptors, tickets, summary (one memset), then the
   // ping-pong key and id buffers.
-  // A single 8-byte key over at least 2^21 rows may take the two-level sort (the device decides).
+  // A single 8-byte key (of more rows than buckets take) may take the two-level sort: the device decides.
   pa.hyb_min_rows = hybrid_min_rows();
   const bool hybrid = K == 1 && pt_key_bytes(keys[0].col->pt) == 8 && n < (uint64_t(1) << 32) &&
                       n >= (pa.hyb_min_rows ? pa.hyb_min_rows : HYB_MIN_ANY);
@@ -3210,11 +3210,13 @@ void sort_segment_group(const std::vector<SortKey>& keys, const std::vector<void
       cudaEvent_t e0, e1;
       AM_CUDA(cudaEventCreate(&e0));
       AM_CUDA(cudaEventCreate(&e1));
-      // The first large scratch grows the pool: not in the first candidate's time.
-      dfree(dmalloc(size_t(cls_rows[c]) * 2 * (sizeof(KeyT) + 4), s), s);
+      const size_t largest = *std::max_element(cls[c].begin(), cls[c].end(),
+                                               [&](size_t x, size_t y) { return keys[x].col->length < keys[y].col->length; });
       for (size_t k = 0; k < cand.size(); k++) {
-        // One array before: the first run of a shape loads its kernels.
-        run_segment_shape<KeyT>(cand[k], keys, outs, {cls[c].front()}, false, s);
+        // Once before: the first candidate's run grows the pool (its scratch is the largest), and a shape's first run
+        // loads its kernels, for which the largest array is enough.
+        if (k == 0) run_segment_shape<KeyT>(cand[k], keys, outs, cls[c], false, s);
+        else run_segment_shape<KeyT>(cand[k], keys, outs, {largest}, false, s);
         AM_CUDA(cudaEventRecord(e0, s));
         run_segment_shape<KeyT>(cand[k], keys, outs, cls[c], false, s);
         AM_CUDA(cudaEventRecord(e1, s));
