@@ -23,8 +23,8 @@
 //      row ids, orders the rows of one key, and larger buckets are cut into parts first.
 //
 // Keys that repeat, the order of 16M int64 rows in us (digit passes and two-level sort; buckets with a bitonic sort of
-// crowded ones; this): 10 rows a value 880, 1,454, 676; 50: 1,057, 2,640, 776; 500: 1,608, 1,242, 870; 3,000: 1,193,
-// 1,245, 1,036.
+// crowded ones; this): 10 rows a value 880, 1,454, 689; 50: 1,057, 2,640, 777; 500: 1,608, 1,242, 880; 3,000: 1,193,
+// 1,245, 1,047.
 //
 // The order is the stable sort's: (key, row id) is what a stable sort orders by. What it replaces moved
 // rows stably (nine ballots a row and a look-back over the tiles before it, 8.4 and 5.8 warp
@@ -85,7 +85,6 @@ constexpr uint64_t WHOLE_SAMPLE_ROWS = uint64_t(1) << 22;
 constexpr int CUR_PAD = 8;                        // cursors 32 bytes apart: same-sector atomics queue
 constexpr int THREADS = 512, ITEMS = 7, TILE = THREADS * ITEMS, WARPS = THREADS / 32;
 constexpr int HTHREADS = 1024, HITEMS = 8;
-constexpr int MAX_CHUNKS = 296;                   // two level-1 CTAs on each of 148 SMs
 constexpr int LTHREADS = 256, LITEMS = CAP / LTHREADS, LBLOCKS = 4;
 constexpr int NTHREADS = 256, NITEMS = CAP / NTHREADS, NBLOCKS = 4;      // the buckets that they put off
 
@@ -2938,8 +2937,10 @@ static uint32_t bucket_cap(uint64_t n) {
   return uint32_t(std::min<uint64_t>(MAX_BUCKETS, (want + 1023) & ~uint64_t(1023)));
 }
 namespace {
+// A chunk a level-1 CTA, two of them an SM; at most as many as the starts have threads.
 uint32_t rows_per_chunk(uint64_t n) {
-  const uint64_t per = (n + MAX_CHUNKS - 1) / MAX_CHUNKS;
+  const uint64_t chunks = std::min<uint64_t>(1024, uint64_t(device().sm_count) * 2);
+  const uint64_t per = (n + chunks - 1) / chunks;
   return uint32_t((per + TILE - 1) / TILE * TILE);
 }
 uint32_t chunks_of(uint64_t n) { return n <= SAMPLES ? 0u : uint32_t((n + rows_per_chunk(n) - 1) / rows_per_chunk(n)); }
@@ -3203,8 +3204,11 @@ void launch_batch(const BatchItem* items, const BatchItem* host, uint32_t count,
     step("batch_sort", [&] {
       batch_sort_kernel<KeyT><<<dim3(sort, rows), LTHREADS, sizeof(FastShared<KeyT, 0, TIES_ID>), s>>>(it);
     });
+    // A share of the chip an array (its CTAs take as many buckets as there are): 592 CTAs each of 1,024 arrays,
+    // nearly all idle, took 4 ms.
+    const uint32_t each = std::max<uint32_t>(1, std::min<uint32_t>(later, 2 * NBLOCKS * uint32_t(device().sm_count) / rows));
     step("batch_later", [&] {
-      batch_later_kernel<KeyT><<<dim3(later, rows), NTHREADS, sizeof(LaterShared<KeyT, 0>), s>>>(it);
+      batch_later_kernel<KeyT><<<dim3(each, rows), NTHREADS, sizeof(LaterShared<KeyT, 0>), s>>>(it);
     });
   }
 }
