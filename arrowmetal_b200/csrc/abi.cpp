@@ -927,7 +927,8 @@ int am_sort_ex2(am_array* a, int descending, int null_placement, int float_order
   return guard([&] {
     std::vector<SortKey> k(1);
     k[0] = SortKey{a, descending != 0, null_placement == 1, float_order};
-    // A key map that is a bijection: the sorted column is rebuilt from the sorted keys, no gather
+    // A key map that is a bijection, or a float order (which ties zeros and NaNs; those few values are read
+    // back from the column): the sorted column is rebuilt from the sorted keys, no gather
     // (the reference's sortedByInvertingKeys, Sources/ArrowMetal/Kernels/Sort.swift:509-619).
     if (a->length > 0 && float_order_ok(float_order) >= 0 && key_rebuildable(k[0])) {
       check_index_rows(a->length, "sort");

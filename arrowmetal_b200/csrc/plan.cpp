@@ -205,9 +205,9 @@ Frame sort_frame(Frame f, const std::vector<KeySpec>& keys) {
     if (i < 0) throw invalid("plan: unknown sort column \"" + k.col + "\"");
     which.push_back(i);
   }
-  // One integer (or totalOrder float) key over an unpermuted frame: the last pass rebuilds the sorted
-  // key column from the sorted keys while it writes the permutation, and the other columns come
-  // through one fused gather. The key column is never gathered.
+  // One integer or float key over an unpermuted frame: the sort rebuilds the sorted key column from the
+  // sorted keys (the few values that a float order ties are read back from the column), and the other
+  // columns ride along in records or come through one fused gather. The key column is never gathered.
   if (keys.size() == 1 && !f.perm && f.rows > 0) {
     SortKey key{f.cols[size_t(which[0])], keys[0].desc, keys[0].nulls_first, keys[0].float_order};
     if (key.float_order < 0 || key.float_order > 2) throw invalid("unknown float_order " + std::to_string(key.float_order));
