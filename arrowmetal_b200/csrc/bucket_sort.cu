@@ -1750,7 +1750,8 @@ static_assert(vectors_aligned<FastShared<uint32_t, 0, TIES_ID>>() && vectors_ali
               vectors_aligned<FastShared<uint32_t, 1, TIES_ID>>() && vectors_aligned<FastShared<uint64_t, 1, TIES_ID>>() &&
               vectors_aligned<FastShared<uint64_t, 0, TIES_STRING>>() && vectors_aligned<LaterShared<uint32_t, 0>>() &&
               vectors_aligned<LaterShared<uint64_t, 0>>() && vectors_aligned<LaterShared<uint32_t, 1>>() &&
-              vectors_aligned<LaterShared<uint64_t, 1>>() && vectors_aligned<LaterShared<uint64_t, 0, TIES_STRING>>(), "shared arrays read as vectors");
+              vectors_aligned<LaterShared<uint64_t, 1>>() && vectors_aligned<LaterShared<uint64_t, 0, TIES_STRING>>(),
+              "shared arrays read as vectors");
 
 // Strings that differ behind many equal keys: bitonic sort of (key, the rest of the string, row id), the ids of
 // equal keys read where the rows are.
@@ -2373,8 +2374,10 @@ __device__ __forceinline__ void later_body(const Args& a) {
         const char* k0 = reinterpret_cast<const char*>(static_cast<const KeyT*>(a.keys[src]) + nf);
         const char* i0 = PAY ? reinterpret_cast<const char*>(a.rec[src] + nf) : reinterpret_cast<const char*>(a.ids[src] + nf);
         const uint32_t ib = PAY ? 16u : a.ids[0] ? 4u : 0u;
-        for (uint32_t x = t * 128u; x < nn * uint32_t(sizeof(KeyT)); x += NTHREADS * 128u) asm volatile("prefetch.global.L2 [%0];" ::"l"(k0 + x));
-        for (uint32_t x = t * 128u; x < nn * ib; x += NTHREADS * 128u) asm volatile("prefetch.global.L2 [%0];" ::"l"(i0 + x));
+        for (uint32_t x = t * 128u; x < nn * uint32_t(sizeof(KeyT)); x += NTHREADS * 128u)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(k0 + x));
+        for (uint32_t x = t * 128u; x < nn * ib; x += NTHREADS * 128u)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(i0 + x));
       }
       for (uint32_t x = t; x < BINS; x += NTHREADS) sm.start[x] = 0;
       if (t <= CAP / CROWD) sm.mixed[t] = 0;
@@ -2430,9 +2433,9 @@ __device__ __forceinline__ void later_body(const Args& a) {
             continue;
           }
         }
-        const uint64_t base = kind == KIND_ID ? vbase : 0ull;
-        if (!write_rows<KeyT, PAY, FREQ, NTHREADS, true>(sm, a, ko, vbase + first, size, nkeys, parity ^ (PAY ? 1u : 0u), base + (kind == KIND_ID ? run_at : 0u),
-                                               base + (kind == KIND_ID ? run_at + run_n : 0u)))
+        // A part of one key's rows: where they all are.
+        const uint64_t run0 = kind == KIND_ID ? vbase + run_at : 0ull, run1 = kind == KIND_ID ? run0 + run_n : 0ull;
+        if (!write_rows<KeyT, PAY, FREQ, NTHREADS, true>(sm, a, ko, vbase + first, size, nkeys, parity ^ (PAY ? 1u : 0u), run0, run1))
           return;
         continue;
       }

@@ -1243,7 +1243,8 @@ __device__ __forceinline__ bool run_all_passes(const AllPassesArgs& a, const Col
   uint32_t round = 0;
   constexpr int HI = 4;
   constexpr uint64_t CHUNK = uint64_t(THREADS) * HI;
-  if (!a.counted) histogram_rows<KeyT, THREADS, HI, false>(col, a.stats, uint64_t(blockIdx.x) * CHUNK, a.plan.n, uint64_t(gridDim.x) * CHUNK);
+  if (!a.counted)
+    histogram_rows<KeyT, THREADS, HI, false>(col, a.stats, uint64_t(blockIdx.x) * CHUNK, a.plan.n, uint64_t(gridDim.x) * CHUNK);
   // Two sets of look-back words: one pass uses the one while the other is cleared for the next.
   uint4* words[2] = {static_cast<uint4*>(a.pass.status), static_cast<uint4*>(a.pass.status) + a.status16};
   auto clear = [&](uint4* w) {
